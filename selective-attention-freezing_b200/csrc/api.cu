@@ -67,8 +67,10 @@ TensorMapEncodeFn tensor_map_encoder() {
   return fn;
 }
 
-int make_tensor_map_bf16(CUtensorMap* out, const void* base, int rank, const uint64_t* dims,
-                         const uint64_t* strides_bytes, const uint32_t* box, bool l2_256) {
+namespace {
+
+int make_tensor_map(CUtensorMap* out, CUtensorMapDataType type, const void* base, int rank, const uint64_t* dims,
+                    const uint64_t* strides_bytes, const uint32_t* box, bool l2_256) {
   TensorMapEncodeFn enc = tensor_map_encoder();
   if (!enc) return fail(SAF_ERR_CUDA, "cuTensorMapEncodeTiled is not available from this driver");
   cuuint64_t d[5], s[4];
@@ -79,12 +81,24 @@ int make_tensor_map_bf16(CUtensorMap* out, const void* base, int rank, const uin
     es[i] = 1;
     if (i > 0) s[i - 1] = strides_bytes[i];
   }
-  CUresult r = enc(out, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, (cuuint32_t)rank, const_cast<void*>(base), d, s, b, es,
+  CUresult r = enc(out, type, (cuuint32_t)rank, const_cast<void*>(base), d, s, b, es,
                    CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
                    l2_256 ? CU_TENSOR_MAP_L2_PROMOTION_L2_256B : CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
                    CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS) return fail(SAF_ERR_CUDA, "cuTensorMapEncodeTiled failed with CUresult %d", (int)r);
   return SAF_OK;
+}
+
+}  // namespace
+
+int make_tensor_map_bf16(CUtensorMap* out, const void* base, int rank, const uint64_t* dims,
+                         const uint64_t* strides_bytes, const uint32_t* box, bool l2_256) {
+  return make_tensor_map(out, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, base, rank, dims, strides_bytes, box, l2_256);
+}
+
+int make_tensor_map_f32(CUtensorMap* out, const void* base, int rank, const uint64_t* dims,
+                        const uint64_t* strides_bytes, const uint32_t* box) {
+  return make_tensor_map(out, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, base, rank, dims, strides_bytes, box, false);
 }
 
 bool tma_rows_ok(const SafTensor& t) {
@@ -333,7 +347,9 @@ static int frozen_pv_common(const SafFrozenPvArgs* p, void* stream, bool bwd) {
 int saf_frozen_pv_fwd(const SafFrozenPvArgs* args, void* stream) { return frozen_pv_common(args, stream, false); }
 int saf_frozen_pv_bwd(const SafFrozenPvArgs* args, void* stream) { return frozen_pv_common(args, stream, true); }
 
-static int validate_linear(const SafIndexedLinearArgs* a) {
+}  // extern "C"
+
+int saf::validate_linear_args(const SafIndexedLinearArgs* a) {
   if (!a) return fail(SAF_ERR_INVALID, "null argument struct");
   if (a->struct_size != (int32_t)sizeof(SafIndexedLinearArgs))
     return fail(SAF_ERR_INVALID, "SafIndexedLinearArgs size mismatch: caller %d, library %d", a->struct_size,
@@ -364,8 +380,10 @@ static int validate_linear(const SafIndexedLinearArgs* a) {
   return SAF_OK;
 }
 
+extern "C" {
+
 int saf_indexed_linear_fwd(const SafIndexedLinearArgs* args, void* stream) {
-  int rc = validate_linear(args);
+  int rc = validate_linear_args(args);
   if (rc) return rc;
   if (args->M == 0 || args->n_slabs == 0) return SAF_OK;
   if (!args->out) return fail(SAF_ERR_INVALID, "out must be non-null");
@@ -379,17 +397,17 @@ int saf_indexed_linear_fwd(const SafIndexedLinearArgs* args, void* stream) {
 
 int saf_indexed_linear_bwd_dx(const SafIndexedLinearArgs* args, const void* dout, int64_t lddo, void* dx,
                               int64_t lddx, const void* bias, void* stream) {
-  int rc = validate_linear(args);
+  int rc = validate_linear_args(args);
   if (rc) return rc;
   if (args->M == 0) return SAF_OK;
   if (!dout || !dx) return fail(SAF_ERR_INVALID, "dout and dx must be non-null");
-  rc = launch_gemm_bwd_dx_sm100(*args, dout, lddo, dx, lddx, bias, (cudaStream_t)stream);
+  rc = launch_gemm_bwd_dx_sm100(*args, dout, lddo, dx, lddx, bias, false, (cudaStream_t)stream);
   if (rc != SAF_ERR_UNSUPPORTED) return rc;
   return launch_gemm_bwd_dx(*args, dout, lddo, dx, lddx, bias, (cudaStream_t)stream);
 }
 
 int saf_indexed_linear_bwd_dw(const SafIndexedLinearArgs* args, const void* dout, int64_t lddo, void* stream) {
-  int rc = validate_linear(args);
+  int rc = validate_linear_args(args);
   if (rc) return rc;
   if (args->n_slabs == 0) return SAF_OK;
   if (!dout) return fail(SAF_ERR_INVALID, "dout must be non-null");

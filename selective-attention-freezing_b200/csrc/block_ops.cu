@@ -114,9 +114,63 @@ __global__ void __launch_bounds__(LN_WARPS * 32) layernorm_generic_kernel(const 
   }
 }
 
+// fp32 -> bf16 of several arrays in one launch: the residual stream and the master weights of a training layer enter
+// the tensor-core products this way once per pass.  Memory-bound: 32 bytes in and 16 out per thread and step.
+constexpr int CAST_THREADS = 256, CAST_STEPS = 4;
+constexpr int64_t CAST_BLOCK = (int64_t)CAST_THREADS * CAST_STEPS * 8;    // elements of one block
+struct CastParams {
+  CastSegment seg[MAX_CAST_SEGMENTS];
+  unsigned block0[MAX_CAST_SEGMENTS + 1];
+  int n;
+};
+
+__global__ void __launch_bounds__(CAST_THREADS) cast_bf16_kernel(const __grid_constant__ CastParams p) {
+  int s = 0;
+  while (s + 1 < p.n && blockIdx.x >= p.block0[s + 1]) ++s;
+  const float4* src = reinterpret_cast<const float4*>(p.seg[s].src);
+  uint4* dst = reinterpret_cast<uint4*>(p.seg[s].dst);
+  const int64_t n8 = p.seg[s].n >> 3;
+  const int64_t i0 = (int64_t)(blockIdx.x - p.block0[s]) * (CAST_BLOCK / 8) + threadIdx.x;
+  float4 a[CAST_STEPS], b[CAST_STEPS];
+#pragma unroll
+  for (int k = 0; k < CAST_STEPS; ++k) {
+    const int64_t i = i0 + k * CAST_THREADS;
+    if (i < n8) {
+      a[k] = __ldcs(src + 2 * i);
+      b[k] = __ldcs(src + 2 * i + 1);
+    }
+  }
+#pragma unroll
+  for (int k = 0; k < CAST_STEPS; ++k) {
+    const int64_t i = i0 + k * CAST_THREADS;
+    if (i < n8) {
+      const __nv_bfloat162 w[4] = {__floats2bfloat162_rn(a[k].x, a[k].y), __floats2bfloat162_rn(a[k].z, a[k].w),
+                                   __floats2bfloat162_rn(b[k].x, b[k].y), __floats2bfloat162_rn(b[k].z, b[k].w)};
+      dst[i] = *reinterpret_cast<const uint4*>(w);
+    }
+  }
+}
+
 bool ln_al16(const void* p) { return ((uintptr_t)p & 15) == 0; }
 
 }  // namespace
+
+int launch_cast_bf16(const CastSegment* seg, int n, cudaStream_t st) {
+  CastParams p;
+  memset(&p, 0, sizeof(p));
+  p.n = n;
+  unsigned blocks = 0;
+  for (int i = 0; i < n; ++i) {
+    p.seg[i] = seg[i];
+    p.block0[i] = blocks;
+    blocks += (unsigned)((seg[i].n + CAST_BLOCK - 1) / CAST_BLOCK);
+  }
+  p.block0[n] = blocks;
+  if (!blocks) return SAF_OK;
+  cast_bf16_kernel<<<blocks, CAST_THREADS, 0, st>>>(p);
+  count_launch();
+  return check_launch("cast_bf16_kernel");
+}
 
 int launch_layernorm(const void* x, int64_t ldx, const void* w, const void* b, void* out, int64_t ldo, int M, int C,
                      float eps, int dtype, int rms, cudaStream_t st) {

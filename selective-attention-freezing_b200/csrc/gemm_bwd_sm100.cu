@@ -11,6 +11,17 @@
 //       rows the two blocks own (the reference zero-fills and index_copy_'s a dense product instead).
 // Same persistent, warp-specialised CTA as the forward GEMM: warp 0 TMA, warp 1 MMA issuer, warps 2-5
 // epilogue; 128x256 tiles, K step 64, 4 stages, two TMEM accumulators.  All waits are bounded.
+//
+// A training layer keeps fp32 master weights and an fp32 residual stream, so both products also exist with an fp32
+// result (F32OUT: the accumulator leaves the kernel unrounded, 32 columns per 16 KB staging block), and DW can be
+// split over the tokens: work unit (tile, split) writes its partial tile to an fp32 workspace and a finishing kernel
+// adds the splits in a fixed order, writes the gradient of whole weight matrices in their own dtype and puts the
+// exact zeros of rows no slab owns -- one pass instead of a zero fill, a bf16 product and a conversion.  A narrow layer
+// needs the split: at 12 x 64 the products have 18 to 45 tiles for 148 SMs, and their K range is the token count.
+// All weight gradients of one layer, 12 x 64, 8192 tokens: 260 us (three products on at most 36 CTAs, without fills
+// and conversions) -> 44 + 9 us; 16 x 128, 16384 tokens: 510 -> 495 + 31 us, the zero fills and conversions (0.1 ms) gone.
+#include <algorithm>
+
 #include "saf_internal.h"
 #include "sm100_prims.cuh"
 
@@ -45,6 +56,7 @@ struct BwdGemmParams {
   const void* bias;          // DX only: bf16 over the J output columns, or null
   int* status;
   int halves;                // see BlockTable
+  int splits, split_rows;    // DW into a workspace: parts of the K range, workspace rows of one part
 };
 
 struct BSmem {
@@ -52,7 +64,8 @@ struct BSmem {
   uint32_t tmem_base;
 };
 
-template <int MODE>
+// F32OUT: DX writes fp32, DW writes its part of the product to the workspace (mapO: splits * split_rows rows)
+template <int MODE, bool F32OUT>
 __global__ void __launch_bounds__(BGEMM_THREADS, 1)
 indexed_gemm_bwd_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUtensorMap mapB,
                         const __grid_constant__ CUtensorMap mapW0, const __grid_constant__ CUtensorMap mapW1,
@@ -65,7 +78,17 @@ indexed_gemm_bwd_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_c
   uint8_t* out_stage = smem + NSTG * BSTAGE;
   BSmem* sl = reinterpret_cast<BSmem*>(out_stage + BOUT_BYTES);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int total_tiles = p.tiles_m * p.tiles_n;
+  const int splits = (MODE == MODE_DW && F32OUT) ? p.splits : 1;
+  const int total_tiles = p.tiles_m * p.tiles_n * splits;    // work units: (tile, part of the K range)
+  // unit -> row tile, column tile and its K steps; the parts of a tile are neighbours, the first ones a step longer
+  auto unit = [&](int u, int& tm, int& tn, int& sp, int& kb0, int& kb1) {
+    const int tile = u / splits;
+    sp = u - tile * splits;
+    tm = tile / p.tiles_n;
+    tn = tile - tm * p.tiles_n;
+    kb0 = (int)((int64_t)p.KB * sp / splits);
+    kb1 = (int)((int64_t)p.KB * (sp + 1) / splits);
+  };
   const CUtensorMap* wm[4] = {&mapW0, &mapW1, &mapW2, &mapW3};
 
   if (tid == 0) {
@@ -94,10 +117,11 @@ indexed_gemm_bwd_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_c
       uint32_t it = 0;
       bool ok = true;
       for (int tile = blockIdx.x; tile < total_tiles && ok; tile += gridDim.x) {
-        const int tm = tile / p.tiles_n, tn = tile - tm * p.tiles_n;
+        int tm, tn, sp, kb0, kb1;
+        unit(tile, tm, tn, sp, kb0, kb1);
         const int nsub = min(4, (p.J - tn * BN + 63) / 64);                      // 64-column blocks of B
         const int nrow = (MODE == MODE_DW) ? min(2, p.n_blocks - tm * 2) : 2;    // 64-feature blocks of A
-        for (int kb = 0; kb < p.KB; ++kb, ++it) {
+        for (int kb = kb0; kb < kb1; ++kb, ++it) {
           const int s = it % NSTG;
           if (!mbar_wait(&sl->empty[s], ((it / NSTG) & 1) ^ 1)) {
             dev_set_error(p.status, SAF_DEV_TIMEOUT_TMA, 60);
@@ -138,7 +162,9 @@ indexed_gemm_bwd_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_c
       }
       tc_fence_after();
       const uint32_t d = tmem + buf * BN;
-      for (int kb = 0; kb < p.KB; ++kb, ++it) {
+      int tm, tn, sp, kb0, kb1;
+      unit(tile, tm, tn, sp, kb0, kb1);
+      for (int kb = kb0; kb < kb1; ++kb, ++it) {
         const int s = it % NSTG;
         if (!mbar_wait(&sl->full[s], (it / NSTG) & 1)) {
           dev_set_error(p.status, SAF_DEV_TIMEOUT_MMA, 62);
@@ -153,7 +179,7 @@ indexed_gemm_bwd_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_c
           for (int k4 = 0; k4 < BK / 16; ++k4) {
             const uint64_t ad = (MODE == MODE_DW) ? umma_smem_desc_sw128(a + k4 * 2048, ATOM, 1024)
                                                   : umma_smem_desc_sw128(a + k4 * 32, 16, 1024);
-            umma_ss(d, ad, umma_smem_desc_sw128(b + k4 * 2048, ATOM, 1024), idesc, (kb | k4) != 0);
+            umma_ss(d, ad, umma_smem_desc_sw128(b + k4 * 2048, ATOM, 1024), idesc, kb > kb0 || k4 > 0);
           }
           umma_commit(&sl->empty[s]);
         }
@@ -169,7 +195,8 @@ indexed_gemm_bwd_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_c
     uint32_t lt = 0;
     uint32_t n_out = 0;                         // output blocks stored so far (staging block = parity)
     for (int tile = blockIdx.x; tile < total_tiles; tile += gridDim.x, ++lt) {
-      const int tm = tile / p.tiles_n, tn = tile - tm * p.tiles_n;
+      int tm, tn, sp, kb0, kb1;
+      unit(tile, tm, tn, sp, kb0, kb1);
       const int nsub = min(4, (p.J - tn * BN + 63) / 64);
       const int nrow = (MODE == MODE_DW) ? min(2, p.n_blocks - tm * 2) : 2;
       const int buf = lt & 1;
@@ -179,6 +206,28 @@ indexed_gemm_bwd_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_c
       }
       tc_fence_after();
       const uint32_t tsrc = tmem + ((uint32_t)(quad * 32) << 16) + buf * BN;
+      if constexpr (F32OUT) {
+        const int orow = (MODE == MODE_DW) ? sp * p.split_rows + tm * BM : tm * BM;
+        const int n32 = min(2 * nsub, (p.J - tn * BN + 31) / 32);
+        for (int u = 0; u < n32; ++u) {             // 32 fp32 columns: 128-byte rows, 16 KB
+          const int ob = (n_out++) & 1;
+          if (etid == 0) tma_store_wait_read1();
+          named_bar_sync(1, 128);
+          uint32_t r0[32];
+          tmem_ld32(tsrc + u * 32, r0);
+          tmem_ld_wait();
+          uint8_t* dst = out_stage + ob * (BOUT_BYTES / 2) + row * 128;
+#pragma unroll
+          for (int c = 0; c < 8; ++c)
+            *reinterpret_cast<uint4*>(dst + ((c ^ (row & 7)) << 4)) = make_uint4(r0[c * 4], r0[c * 4 + 1], r0[c * 4 + 2], r0[c * 4 + 3]);
+          fence_proxy_async_smem();
+          named_bar_sync(1, 128);
+          if (etid == 0) {
+            tma_store_2d(&mapO, out_stage + ob * (BOUT_BYTES / 2), tn * BN + u * 32, orow);
+            tma_store_commit();
+          }
+        }
+      } else
       for (int u = 0; u < nsub; ++u) {
         // the two staging blocks take turns over all stores of the CTA (nsub may be odd)
         const int ob = (n_out++) & 1;
@@ -246,6 +295,14 @@ int map2(CUtensorMap* m, const void* base, uint64_t cols, uint64_t rows, int64_t
   return make_tensor_map_bf16(m, base, 2, dims, strides, box, true);
 }
 
+// fp32 output: 32 columns x 128 rows per store, row stride ld elements
+int map2_f32(CUtensorMap* m, const void* base, uint64_t cols, uint64_t rows, int64_t ld) {
+  uint64_t dims[2] = {cols, rows};
+  uint64_t strides[2] = {0, (uint64_t)ld * 4};
+  uint32_t box[2] = {32, 128};
+  return make_tensor_map_f32(m, base, 2, dims, strides, box);
+}
+
 bool common_ok(const SafIndexedLinearArgs& a, const void* dout, int64_t lddo) {
   if (a.dtype != SAF_BF16 || a.slab % 32 || (a.n_slabs * a.slab) % 64 || a.n_slabs <= 0 || a.M <= 0) return false;
   if (a.n_slabs * a.slab / 64 > BMAX_SUB) return false;
@@ -282,15 +339,15 @@ void fill_blocks(const SafIndexedLinearArgs& a, BlockTable* tb) {
     }
 }
 
-template <int MODE>
+template <int MODE, bool F32OUT = false>
 int launch_mode(const CUtensorMap& ma, const CUtensorMap& mb, const CUtensorMap* mw, const CUtensorMap& mo,
                 const BwdGemmParams& p, const BlockTable& tb, cudaStream_t st) {
   const int sm_count = device_sm_count();
   const size_t smem = 1024 + NSTG * BSTAGE + BOUT_BYTES + sizeof(BSmem);
   static PerDeviceOnce smem_once;
-  if (int rc = ensure_dyn_smem(indexed_gemm_bwd_kernel<MODE>, (int)smem, smem_once)) return rc;
-  const int grid = std::min(sm_count, p.tiles_m * p.tiles_n);
-  indexed_gemm_bwd_kernel<MODE><<<grid, BGEMM_THREADS, smem, st>>>(ma, mb, mw[0], mw[1], mw[2], mw[3], mo, p, tb);
+  if (int rc = ensure_dyn_smem(indexed_gemm_bwd_kernel<MODE, F32OUT>, (int)smem, smem_once)) return rc;
+  const int grid = std::min(sm_count, p.tiles_m * p.tiles_n * std::max(1, p.splits));
+  indexed_gemm_bwd_kernel<MODE, F32OUT><<<grid, BGEMM_THREADS, smem, st>>>(ma, mb, mw[0], mw[1], mw[2], mw[3], mo, p, tb);
   count_launch();
   return check_launch(MODE == MODE_DX ? "indexed_gemm_bwd_kernel<dx>" : "indexed_gemm_bwd_kernel<dw>");
 }
@@ -298,9 +355,9 @@ int launch_mode(const CUtensorMap& ma, const CUtensorMap& mb, const CUtensorMap*
 }  // namespace
 
 int launch_gemm_bwd_dx_sm100(const SafIndexedLinearArgs& a, const void* dout, int64_t lddo, void* dx, int64_t lddx,
-                             const void* bias, cudaStream_t st) {
+                             const void* bias, bool f32_out, cudaStream_t st) {
   if (!common_ok(a, dout, lddo)) return SAF_ERR_UNSUPPORTED;
-  if (lddx % 8 || !al16(dx)) return SAF_ERR_UNSUPPORTED;
+  if (lddx % (f32_out ? 4 : 8) || !al16(dx) || (f32_out && bias)) return SAF_ERR_UNSUPPORTED;
   const int N = a.n_slabs * a.slab;
   CUtensorMap ma, mw[4], mo;
   int rc;
@@ -309,7 +366,9 @@ int launch_gemm_bwd_dx_sm100(const SafIndexedLinearArgs& a, const void* dout, in
     const int ww = w < a.n_weights ? w : 0;
     if ((rc = map2(&mw[w], a.weights[ww], (uint64_t)a.C, (uint64_t)a.rows_w[ww], a.ldw[ww], is_halves(a) ? 32 : 64))) return rc;
   }
-  if ((rc = map2(&mo, dx, (uint64_t)a.C, (uint64_t)a.M, lddx, 128))) return rc;
+  if (f32_out) rc = map2_f32(&mo, dx, (uint64_t)a.C, (uint64_t)a.M, lddx);
+  else rc = map2(&mo, dx, (uint64_t)a.C, (uint64_t)a.M, lddx, 128);
+  if (rc) return rc;
   BlockTable tb;
   fill_blocks(a, &tb);
   BwdGemmParams p;
@@ -320,6 +379,7 @@ int launch_gemm_bwd_dx_sm100(const SafIndexedLinearArgs& a, const void* dout, in
   p.tiles_n = (a.C + BN - 1) / BN;
   p.bias = bias;
   p.status = a.status;
+  if (f32_out) return launch_mode<MODE_DX, true>(ma, ma, mw, mo, p, tb, st);
   return launch_mode<MODE_DX>(ma, ma, mw, mo, p, tb, st);
 }
 
@@ -347,6 +407,137 @@ int launch_gemm_bwd_dw_sm100(const SafIndexedLinearArgs& a, const void* dout, in
   p.tiles_n = (a.C + BN - 1) / BN;
   p.status = a.status;
   return launch_mode<MODE_DW>(ma, mb, mw, ma, p, tb, st);
+}
+
+// ---- DW through a workspace: splits over the tokens, whole gradient matrices out ----------------------------------
+namespace {
+
+constexpr int FIN_RUNS = 1024;                  // 32-row runs of the gradient matrices of one call
+constexpr int FIN_THREADS = 256;
+struct FinishTable {
+  int16_t src[FIN_RUNS];                        // position of the run in the stacked product (in runs), -1: zeros
+};
+struct FinishParams {
+  const float* ws;
+  void* out[SAF_MAX_WEIGHTS];
+  int run0[SAF_MAX_WEIGHTS + 1];                // first run of each matrix
+  int n, C4, splits;                            // matrices; 16-byte columns; parts
+  int64_t part;                                 // floats of one part (split_rows * C)
+  int f32;
+};
+
+// gradient[row] = sum over the parts of the workspace row its run came from, or zero.  Memory-bound: one float4
+// column per thread and row, consecutive threads along the row.
+__global__ void __launch_bounds__(FIN_THREADS) dw_finish_kernel(const __grid_constant__ FinishParams p,
+                                                                const __grid_constant__ FinishTable tb) {
+  const int run = blockIdx.y;
+  int w = 0;
+  while (w + 1 < p.n && run >= p.run0[w + 1]) ++w;
+  const int src = tb.src[run];
+  const int64_t row0 = (int64_t)(run - p.run0[w]) * 32;
+  for (int idx = blockIdx.x * FIN_THREADS + threadIdx.x; idx < 32 * p.C4; idx += gridDim.x * FIN_THREADS) {
+    const int r = idx / p.C4, c = idx - r * p.C4;
+    float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (src >= 0) {
+      const float4* q = reinterpret_cast<const float4*>(p.ws) + ((int64_t)src * 32 + r) * p.C4 + c;
+      const int64_t step = p.part >> 2;
+      s = *q;
+      for (int k = 1; k < p.splits; ++k) {
+        const float4 t = q[k * step];
+        s.x += t.x; s.y += t.y; s.z += t.z; s.w += t.w;
+      }
+    }
+    const int64_t o = (row0 + r) * p.C4 + c;
+    if (p.f32) reinterpret_cast<float4*>(p.out[w])[o] = s;
+    else reinterpret_cast<uint2*>(p.out[w])[o] = make_uint2(pack_bf16(s.x, s.y), pack_bf16(s.z, s.w));
+  }
+}
+
+struct DwPlan {
+  int splits, split_rows;
+};
+
+// Parts of the token range.  A row of tiles that does not fill the SMs, or leaves a nearly empty last wave, is split
+// until (waves x K steps per unit), plus about 6 K steps of accumulator drain per unit and the workspace traffic of the
+// extra part (written and read once, in K steps of 0.28 us over all SMs), is smallest.
+DwPlan dw_plan(int n_blocks, int C, int M) {
+  const int sms = device_sm_count();
+  const int tiles_m = (n_blocks + 1) / 2, tiles = tiles_m * ((C + BN - 1) / BN), KB = (M + BK - 1) / BK;
+  int best = 1;
+  double best_cost = 1e30;
+  for (int s = 1; s <= std::min(16, KB); ++s) {
+    const int waves = (tiles * s + sms - 1) / sms;
+    const double traffic = 2.0 * s * tiles_m * BM * (double)C * 4.0 / 5e12 / 0.28e-6;
+    const double cost = waves * ((KB + s - 1) / s + 6.0) + traffic;
+    if (cost < best_cost) {
+      best_cost = cost;
+      best = s;
+    }
+  }
+  return {best, tiles_m * BM};
+}
+
+}  // namespace
+
+int64_t gemm_dw_workspace_bytes(int n_rows, int C, int M) {
+  const DwPlan d = dw_plan((n_rows + 63) / 64, C, M);
+  return (int64_t)d.splits * d.split_rows * C * 4;
+}
+
+// a.weights: the gradient matrices, contiguous (rows_w, C) in fp32 (f32_out) or bf16, every row of them written
+int launch_gemm_bwd_dw_full_sm100(const SafIndexedLinearArgs& a, const void* dout, int64_t lddo, float* ws,
+                                  int64_t ws_bytes, bool f32_out, cudaStream_t st) {
+  if (!common_ok(a, dout, lddo)) return SAF_ERR_UNSUPPORTED;
+  if (a.ldx % 8 || !al16(a.x) || !al16(ws)) return SAF_ERR_UNSUPPORTED;
+  const int N = a.n_slabs * a.slab;
+  FinishTable ft;
+  FinishParams fp;
+  memset(&fp, 0, sizeof(fp));
+  int runs = 0;
+  for (int w = 0; w < a.n_weights; ++w) {
+    if (a.rows_w[w] % 32 || a.ldw[w] != a.C) return SAF_ERR_UNSUPPORTED;
+    fp.run0[w] = runs;
+    runs += a.rows_w[w] / 32;
+    fp.out[w] = const_cast<void*>(a.weights[w]);
+  }
+  if (runs > FIN_RUNS) return SAF_ERR_UNSUPPORTED;
+  fp.run0[a.n_weights] = runs;
+  for (int i = 0; i < runs; ++i) ft.src[i] = -1;
+  const int per = a.slab / 32;
+  for (int g = 0; g < a.n_slabs; ++g) {
+    if (a.slab_row0[g] % 32) return SAF_ERR_UNSUPPORTED;
+    for (int u = 0; u < per; ++u) ft.src[fp.run0[a.slab_weight[g]] + a.slab_row0[g] / 32 + u] = (int16_t)(g * per + u);
+  }
+  const DwPlan d = dw_plan(N / 64, a.C, a.M);
+  if (ws_bytes < (int64_t)d.splits * d.split_rows * a.C * 4) return fail(SAF_ERR_INVALID, "dW workspace is too small");
+  CUtensorMap ma, mb, mo;
+  int rc;
+  if ((rc = map2(&ma, dout, (uint64_t)N, (uint64_t)a.M, lddo, 64))) return rc;
+  if ((rc = map2(&mb, a.x, (uint64_t)a.C, (uint64_t)a.M, a.ldx, 64))) return rc;
+  if ((rc = map2_f32(&mo, ws, (uint64_t)a.C, (uint64_t)d.splits * d.split_rows, a.C))) return rc;
+  BlockTable tb;
+  memset(&tb, 0, sizeof(tb));
+  BwdGemmParams p;
+  memset(&p, 0, sizeof(p));
+  p.I = N; p.J = a.C; p.KB = (a.M + BK - 1) / BK; p.n_blocks = N / 64;
+  p.tiles_m = (p.n_blocks + 1) / 2;
+  p.tiles_n = (a.C + BN - 1) / BN;
+  p.splits = d.splits;
+  p.split_rows = d.split_rows;
+  p.status = a.status;
+  const CUtensorMap mw[4] = {ma, ma, ma, ma};
+  if ((rc = launch_mode<MODE_DW, true>(ma, mb, mw, mo, p, tb, st))) return rc;
+  fp.ws = ws;
+  fp.n = a.n_weights;
+  fp.C4 = a.C / 4;
+  fp.splits = d.splits;
+  fp.part = (int64_t)d.split_rows * a.C;
+  fp.f32 = f32_out ? 1 : 0;
+  const int per_run = (32 * fp.C4 + FIN_THREADS - 1) / FIN_THREADS;
+  const dim3 grid((unsigned)std::min(per_run, std::max(1, 8 * device_sm_count() / runs)), (unsigned)runs);
+  dw_finish_kernel<<<grid, FIN_THREADS, 0, st>>>(fp, ft);
+  count_launch();
+  return check_launch("dw_finish_kernel");
 }
 
 }  // namespace saf

@@ -67,6 +67,7 @@ struct GemmParams {
   const __nv_bfloat16* residual; // added to the output, or null
   int64_t ldr;
   int halves;                    // weight blocks arrive as two 32-row TMA boxes (see SubTable)
+  int32_t* zero2;                // two ints this launch clears for the next one on the stream (a tile queue), or null
 };
 
 // exact-form GELU, 0.5 x (1 + erf(x / sqrt 2)), with erf from Abramowitz-Stegun 7.1.26 (|error| < 1.5e-7):
@@ -122,6 +123,10 @@ indexed_gemm_kernel(const __grid_constant__ CUtensorMap mapX, const __grid_const
   const int tile_hi = (int)((int64_t)(unit + 1) * total_tiles / n_units);
 
   if (tid == 0) {
+    if (p.zero2 && blockIdx.x == 0) {
+      p.zero2[0] = 0;
+      p.zero2[1] = 0;
+    }
     for (int s = 0; s < STAGES; ++s) {
       mbar_init(&sl->full[s], 1);
       mbar_init(&sl->empty[s], 1);
@@ -433,7 +438,7 @@ bool aligned16(const void* p) { return ((uintptr_t)p & 15) == 0; }
 
 }  // namespace
 
-int launch_gemm_sm100(const SafIndexedLinearArgs& a, cudaStream_t st) {
+int launch_gemm_sm100(const SafIndexedLinearArgs& a, cudaStream_t st, int32_t* zero2) {
   if (a.dtype != SAF_BF16) return SAF_ERR_UNSUPPORTED;
   // slabs of 64 or 128 rows are whole 64-row weight blocks; other multiples of 32 (head_dim 96) are served as runs
   // of 32 rows, two per block, when the total width still fills whole 64-column blocks.  The rotation is fused in
@@ -517,6 +522,7 @@ int launch_gemm_sm100(const SafIndexedLinearArgs& a, cudaStream_t st) {
   p.residual = reinterpret_cast<const __nv_bfloat16*>(a.residual);
   p.ldr = a.ldr;
   p.halves = halves ? 1 : 0;
+  p.zero2 = zero2;
 
   const int sm_count = device_sm_count();
   // CTA pairs on 256-row tiles when the product is large enough to fill the machine with them

@@ -89,19 +89,32 @@ int launch_flash_fwd_sm100(const SafMixedAttnArgs& a, uint32_t want, uint32_t* h
 // dense-stored frozen heads as a TMA-staged lower-triangular GEMM (bf16 patterns)
 int launch_dense_pv_sm100(const SafMixedAttnArgs& a, uint32_t* handled_states, cudaStream_t st);
 int launch_flash_bwd_sm100(const SafMixedAttnBwdArgs& a, uint32_t* handled_states, cudaStream_t st);
-int launch_gemm_sm100(const SafIndexedLinearArgs& a, cudaStream_t st);
+// `zero2`: two device ints the launch clears for the next launch on the stream (not touched when it returns UNSUPPORTED)
+int launch_gemm_sm100(const SafIndexedLinearArgs& a, cudaStream_t st, int32_t* zero2 = nullptr);
 int launch_gemm_generic(const SafIndexedLinearArgs& a, cudaStream_t st);
 int launch_gemm_bwd_dx(const SafIndexedLinearArgs& a, const void* dout, int64_t lddo, void* dx, int64_t lddx,
                        const void* bias, cudaStream_t st);
 int launch_gemm_bwd_dw(const SafIndexedLinearArgs& a, const void* dout, int64_t lddo, cudaStream_t st);
 // tcgen05 versions of the two backward products; SAF_ERR_UNSUPPORTED when the call does not qualify
 int launch_gemm_bwd_dx_sm100(const SafIndexedLinearArgs& a, const void* dout, int64_t lddo, void* dx, int64_t lddx,
-                             const void* bias, cudaStream_t st);
+                             const void* bias, bool f32_out, cudaStream_t st);
 int launch_gemm_bwd_dw_sm100(const SafIndexedLinearArgs& a, const void* dout, int64_t lddo, cudaStream_t st);
+// dW of whole matrices through an fp32 workspace (splits over the tokens, zero rows included); see the kernel file
+int64_t gemm_dw_workspace_bytes(int n_rows, int C, int M);
+int launch_gemm_bwd_dw_full_sm100(const SafIndexedLinearArgs& a, const void* dout, int64_t lddo, float* ws,
+                                  int64_t ws_bytes, bool f32_out, cudaStream_t st);
 int launch_rope_slabs(void* x, int64_t ld, int M, int n_slabs, int slab, int T, const int32_t* slab_rope,
                       const float* cosT, const float* sinT, int dtype, int inverse, cudaStream_t st);
 int launch_layernorm(const void* x, int64_t ldx, const void* w, const void* b, void* out, int64_t ldo, int M, int C,
                      float eps, int dtype, int rms, cudaStream_t st);
+struct CastSegment {
+  const float* src;
+  void* dst;               // bf16
+  int64_t n;               // elements, a multiple of 8; both pointers 16-byte aligned
+};
+constexpr int MAX_CAST_SEGMENTS = 6;
+int launch_cast_bf16(const CastSegment* seg, int n, cudaStream_t st);   // fp32 -> bf16, all segments in one launch
+int validate_linear_args(const SafIndexedLinearArgs* a);
 int launch_logz(const float* alpha, const float* rho, float* z, int H, int S, int rows, cudaStream_t st);   // rows >= `rows` get 0
 int launch_pattern_grad(const SafPatternGradArgs& a, cudaStream_t st);
 int launch_attn_stats_sm100(const SafAttnStatsArgs& a, cudaStream_t st);
@@ -115,6 +128,8 @@ TensorMapEncodeFn tensor_map_encoder();
 // rank-`rank` bf16 map, 128B swizzle; dims/strides innermost first, strides in BYTES for dims 1..rank-1
 int make_tensor_map_bf16(CUtensorMap* out, const void* base, int rank, const uint64_t* dims,
                          const uint64_t* strides_bytes, const uint32_t* box, bool l2_256);
+int make_tensor_map_f32(CUtensorMap* out, const void* base, int rank, const uint64_t* dims,
+                        const uint64_t* strides_bytes, const uint32_t* box);
 
 // a (B, Hn, T, HD) bf16 tensor that TMA can tile: 16-byte aligned base, unit last stride, other strides multiples of 8
 bool tma_rows_ok(const SafTensor& t);

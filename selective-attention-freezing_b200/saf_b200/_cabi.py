@@ -90,6 +90,29 @@ class SafAttnStatsArgs(C.Structure):
     ]
 
 
+class SafAttnLayerArgs(C.Structure):
+    _fields_ = [
+        ("struct_size", C.c_int32), ("C", C.c_int32), ("x_dtype", C.c_int32), ("w_dtype", C.c_int32), ("train", C.c_int32),
+        ("attn", SafMixedAttnArgs), ("live", C.POINTER(C.c_int32)),
+        ("x", C.c_void_p), ("ldx", C.c_int64),
+        ("wq", C.c_void_p), ("wk", C.c_void_p), ("wv", C.c_void_p), ("wo", C.c_void_p),
+        ("bq", C.c_void_p), ("bk", C.c_void_p), ("bv", C.c_void_p), ("bo", C.c_void_p),
+        ("rope_cos", C.c_void_p), ("rope_sin", C.c_void_p),
+        ("residual", C.c_void_p), ("ldr", C.c_int64), ("out", C.c_void_p), ("ldo", C.c_int64),
+        ("work", C.c_void_p), ("work_bytes", C.c_int64),
+        ("event_before", C.c_void_p), ("event_after", C.c_void_p),
+    ]
+
+
+class SafAttnLayerBwdArgs(C.Structure):
+    _fields_ = [
+        ("struct_size", C.c_int32), ("need_dy", C.c_int32), ("fwd", SafAttnLayerArgs),
+        ("dout", C.c_void_p), ("lddo", C.c_int64), ("dx", C.c_void_p),
+        ("dwq", C.c_void_p), ("dwk", C.c_void_p), ("dwv", C.c_void_p), ("dwo", C.c_void_p),
+        ("work", C.c_void_p), ("work_bytes", C.c_int64),
+    ]
+
+
 STATS_PROBS, STATS_LOGITS = 0, 1
 ACT_NONE, ACT_GELU, ACT_SWIGLU = 0, 1, 2
 
@@ -99,6 +122,7 @@ EXPORTS = (
     "saf_indexed_linear_fwd", "saf_indexed_linear_bwd_dx", "saf_indexed_linear_bwd_dw",
     "saf_decomposed_logz", "saf_rope_slabs", "saf_layernorm_fwd", "saf_rmsnorm_fwd",
     "saf_pattern_normalisers", "saf_pattern_param_grad", "saf_attention_moments",
+    "saf_attn_layer_workspace", "saf_attn_layer_fwd", "saf_attn_layer_bwd",
     "saf_selftest_wait_timeout", "saf_selftest_per_device_once", "saf_selftest_mma_rate",
 )
 
@@ -125,10 +149,13 @@ def _load():
                      ("saf_frozen_pv_fwd", SafFrozenPvArgs), ("saf_frozen_pv_bwd", SafFrozenPvArgs),
                      ("saf_indexed_linear_fwd", SafIndexedLinearArgs),
                      ("saf_pattern_param_grad", SafPatternGradArgs),
-                     ("saf_attention_moments", SafAttnStatsArgs)):
+                     ("saf_attention_moments", SafAttnStatsArgs),
+                     ("saf_attn_layer_fwd", SafAttnLayerArgs), ("saf_attn_layer_bwd", SafAttnLayerBwdArgs)):
         f = getattr(lib, name)
         f.argtypes = [C.POINTER(at), C.c_void_p]
         f.restype = C.c_int
+    lib.saf_attn_layer_workspace.argtypes = [C.POINTER(SafAttnLayerArgs), C.POINTER(C.c_int64)]
+    lib.saf_attn_layer_workspace.restype = C.c_int
     lib.saf_indexed_linear_bwd_dx.argtypes = [C.POINTER(SafIndexedLinearArgs), C.c_void_p, C.c_int64, C.c_void_p,
                                               C.c_int64, C.c_void_p, C.c_void_p]
     lib.saf_indexed_linear_bwd_dx.restype = C.c_int

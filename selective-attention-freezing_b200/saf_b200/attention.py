@@ -26,6 +26,7 @@ import torch
 import torch.nn as nn
 import torch.nn.functional as F
 
+from . import layer as _layer
 from . import ops
 
 BAND_ROWS = ops.BAND_ROWS
@@ -291,6 +292,7 @@ class SafCausalSelfAttention(nn.Module):
         sd = self.sd_params()
         self._sd = (sd[:, 0].contiguous(), sd[:, 1].contiguous()) if self._sd_any else None
         self._patt_cast = None      # compact copy of the dense heads' patterns in the activation dtype, built on demand
+        self._plan = _layer.LayerPlan(states, self._live, hd, self.n_embd, self._fz_mask_i32, self._hidx_i32, self._sd)
         self._mask_frozen_only = None   # head states with live heads masked out (training with attention dropout)
         self._fz_dirty = False
 
@@ -364,6 +366,26 @@ class SafCausalSelfAttention(nn.Module):
                 self._patt_cast = (patt[dense].to(act_dt), torch.tensor(slot, dtype=torch.int32, device=patt.device))
             patt, pidx = self._patt_cast
         nuf = len(self._live)
+        if act_dt == torch.bfloat16 and nuf and (self.dropout == 0.0 or not self.training):
+            grad = torch.is_grad_enabled()
+            w = [self.q_proj.weight, self.k_proj.weight, self.v_proj.weight, self.c_proj.weight]
+            bias = self.q_proj.bias is not None
+            # without autocast, training wants x and the weights in one dtype (the separate operators say so)
+            mixed = grad and not torch.is_autocast_enabled("cuda") and w[0].dtype != x.dtype
+            if not (grad and bias) and not mixed and _layer.usable(self._plan, x, w, grad):
+                learn = None
+                if grad and dec[0] is not None and (dec[0].requires_grad or dec[1].requires_grad):
+                    from . import trainable_patterns as tp
+                    learn = dec[:2]
+                    dec = (dec[0].detach(), dec[1].detach(), tp.current_normalisers(dec[0], dec[1], T))
+                bs = None
+                if bias:
+                    bs = [m.bias.to(act_dt) for m in (self.q_proj, self.k_proj, self.v_proj, self.c_proj)]
+                measure = self._measure if self._stats is not None or self._logit_stats is not None else None
+                out = _layer.attention_layer(self._plan, x, w, rp, patt=patt if 1 in self._states else None, pidx=pidx,
+                                             decomposed=dec, learn=learn, biases=bs, residual=None if grad else residual,
+                                             measure=measure)
+                return residual + out if grad and residual is not None else out
         if not torch.is_grad_enabled() and act_dt == torch.bfloat16 and (self.dropout == 0.0 or not self.training):
             # inference: one GEMM, canonical weights read in place, RoPE in the epilogue
             w = [m.weight if m.weight.dtype == act_dt else m.weight.to(act_dt) for m in (self.q_proj, self.k_proj, self.v_proj)]

@@ -1,0 +1,243 @@
+"""The attention layer through `saf_attn_layer_fwd` / `saf_attn_layer_bwd`: one library call per direction over one
+workspace, instead of an operator, an allocation and an autograd node for every product of the layer.
+
+The forward's workspace holds the bf16 copies of fp32 inputs (autocast), the fused projection, the attention output and
+the row statistics; a training call saves it for the backward, which works on the projection's own layout and returns
+gradients in the dtypes of x and the weights.  Same mathematics as `linear_rows2` + `linear_rows` + `fused_mixed_attn` +
+`linear_rows` with rotation fused (nanogpt/model.py:946-1077)."""
+import ctypes as C
+
+import torch
+
+from . import ops
+from ._cabi import SafAttnLayerArgs, SafAttnLayerBwdArgs, SafMixedAttnArgs, lib, check, SAF_BF16, SAF_F32
+
+_DT = {torch.float32: SAF_F32, torch.bfloat16: SAF_BF16}
+HEAD_DIMS = (64, 96, 128)
+MAX_BLOCKS = 160          # 64-row blocks of one backward product
+
+
+class LayerPlan:
+    """What a freeze set fixes: head states and slots.  Device tensors are kept, pointers are taken per call."""
+
+    def __init__(self, states, live, head_dim, width, frozen, hidx, sink_decay=None, kvidx=None, n_kv=0):
+        H, U = len(states), len(live)
+        self.H, self.U, self.hd, self.C, self.n_kv = H, U, head_dim, width, n_kv
+        self.frozen, self.hidx, self.sink_decay, self.kvidx = frozen, hidx, sink_decay, kvidx
+        self._states = (C.c_int32 * H)(*states)
+        self._live = (C.c_int32 * max(U, 1))(*live)
+        a = SafAttnLayerArgs()
+        a.struct_size = C.sizeof(SafAttnLayerArgs)
+        a.C = width
+        a.live = self._live
+        t = a.attn
+        t.struct_size = C.sizeof(SafMixedAttnArgs)
+        t.dtype, t.H, t.U, t.HD, t.HKV, t.force_state = SAF_BF16, H, U, head_dim, n_kv, -1
+        t.sm_scale = head_dim ** -0.5
+        t.frozen_host = self._states
+        self._template = bytes(a)
+        self._sizes = {}
+
+    def width(self):
+        return (self.U + 2 * self.n_kv if self.n_kv else 2 * self.U + self.H) * self.hd
+
+    def shapes_ok(self, training):
+        """Sizes the tensor-core products of both directions take."""
+        blocks = max(self.width(), self.C) // 64
+        return (self.hd in HEAD_DIMS and self.U > 0 and self.width() % 64 == 0 and self.C % 64 == 0
+                and (not training or (blocks <= MAX_BLOCKS and self.H * self.hd % 64 == 0 and self.C + 3 * self.H * self.hd <= 32 * 1024)))
+
+    def args(self, c):
+        """The C struct of one call `c` (a _Call), every pointer taken from the tensors it holds now."""
+        a = SafAttnLayerArgs.from_buffer_copy(self._template)
+        t = a.attn
+        x = c.x
+        t.B, t.T = c.B, c.T
+        t.status = ops._status_ptr(x.device)
+        t.frozen, t.hidx = self.frozen.data_ptr(), self.hidx.data_ptr()
+        if self.kvidx is not None:
+            t.kvidx = self.kvidx.data_ptr()
+        if self.sink_decay is not None:
+            t.sd_alpha, t.sd_rho = self.sink_decay[0].data_ptr(), self.sink_decay[1].data_ptr()
+        if c.patt is not None:
+            t.patt = ops._st(c.patt)
+            t.S = c.patt.shape[1]
+            t.patt_dtype = ops._dt(c.patt)
+            if c.pidx is not None:
+                t.pidx = c.pidx.data_ptr()
+        if c.alpha is not None:
+            t.alpha, t.rho, t.z = ops._st(c.alpha), ops._st(c.rho), ops._st(c.z)
+            t.SD = c.alpha.shape[1]
+            t.dec_dtype = ops._dt(c.alpha)
+        a.x_dtype, a.w_dtype, a.train = _DT[x.dtype], _DT[c.w[0].dtype], c.train
+        a.x, a.ldx = x.data_ptr(), x.stride(0)
+        a.wq, a.wk, a.wv, a.wo = [w.data_ptr() for w in c.w]
+        if c.rope is not None:
+            a.rope_cos, a.rope_sin = c.rope[0].data_ptr(), c.rope[1].data_ptr()
+        return a
+
+    def sizes(self, a):
+        """(forward bytes, backward bytes, offset of the projection, offset of the attention output)."""
+        t = a.attn
+        key = (t.B, t.T, a.x_dtype, a.w_dtype, a.train)
+        got = self._sizes.get(key)
+        if got is None:
+            out = (C.c_int64 * 4)()
+            check(lib.saf_attn_layer_workspace(C.byref(a), out))
+            if len(self._sizes) >= 64:
+                self._sizes.clear()
+            got = self._sizes[key] = tuple(out)
+        return got
+
+
+class _Call:
+    """Tensors of one layer call, in the form the library reads them."""
+    __slots__ = ("B", "T", "x", "w", "train", "rope", "patt", "pidx", "alpha", "rho", "z")
+
+
+def usable(plan, x, weights, training):
+    """True when the whole layer can run through the library's layer entry."""
+    dt = weights[0].dtype
+    return (x.dtype in _DT and dt in _DT and x.numel() > 0 and plan.shapes_ok(training) and x.data_ptr() % 16 == 0
+            and all(w.dtype == dt and w.is_contiguous() and w.data_ptr() % 16 == 0 for w in weights))
+
+
+def _rows(x):
+    x2 = ops._as_2d(x)
+    if x.dtype == torch.float32:
+        return x2.contiguous()
+    return x2 if x2.stride(0) % 8 == 0 else x2.contiguous()
+
+
+def _blob(n, device):
+    return torch.empty(n, dtype=torch.uint8, device=device)
+
+
+def _forward(plan, c, biases=None, residual=None):
+    """Enqueues the layer; returns (out (tokens, C) bf16, workspace, sizes)."""
+    a = plan.args(c)
+    sz = plan.sizes(a)
+    dev = c.x.device
+    work = _blob(sz[0], dev)
+    out = torch.empty((c.B * c.T, plan.C), dtype=torch.bfloat16, device=dev)
+    a.out, a.ldo = out.data_ptr(), plan.C
+    a.work, a.work_bytes = work.data_ptr(), sz[0]
+    if biases is not None:
+        a.bq, a.bk, a.bv, a.bo = [None if b is None else b.data_ptr() for b in biases]
+    if residual is not None:
+        a.residual, a.ldr = residual.data_ptr(), residual.stride(0)
+    events = ops.attention_event_pair()
+    if events is not None:
+        a.event_before, a.event_after = events
+    ops._call(c.x, lib.saf_attn_layer_fwd, C.byref(a))
+    return out, work, sz
+
+
+def projection_views(plan, work, sz, B, T):
+    """q, k, v (B, heads, T, hd) and the attention output y inside a forward workspace."""
+    W, hd = plan.width(), plan.hd
+    n = B * T * W
+    qkv = work[sz[2]:sz[2] + 2 * n].view(torch.bfloat16).view(B, T, W // hd, hd)
+    nk = plan.n_kv or plan.U
+    y = work[sz[3]:sz[3] + 2 * B * T * plan.H * hd].view(torch.bfloat16).view(B, T, plan.H, hd)
+    q, k, v = qkv[:, :, :plan.U], qkv[:, :, plan.U:plan.U + nk], qkv[:, :, plan.U + nk:]
+    return q.transpose(1, 2), k.transpose(1, 2), v.transpose(1, 2), y.transpose(1, 2)
+
+
+class _LayerFunction(torch.autograd.Function):
+    """(x, wq, wk, wv, wo, alpha, rho) -> layer output; alpha / rho are passed when they learn."""
+
+    @staticmethod
+    def forward(ctx, x, wq, wk, wv, wo, alpha_p, rho_p, plan, c, measure):
+        out, work, sz = _forward(plan, c)
+        if measure is not None:
+            q, k, _, _ = projection_views(plan, work, sz, c.B, c.T)
+            measure(q, k)
+        ctx.plan, ctx.sz, ctx.bt = plan, sz, (c.B, c.T)
+        ctx.x_like, ctx.w_cast = (x.shape, x.dtype), wq.dtype != torch.bfloat16
+        # (converted tensors live in the workspace: the originals are not needed again)
+        kept = [work, c.x if x.dtype == torch.bfloat16 else None]
+        kept += [None] * 4 if ctx.w_cast else [wq, wk, wv, wo]
+        kept += [c.patt, c.pidx, c.alpha, c.rho, c.z, *(c.rope or (None, None))]
+        ctx.save_for_backward(*kept, plan.frozen, plan.hidx, *(plan.sink_decay or ()))
+        ctx.w_like = [(w.shape, w.dtype) for w in (wq, wk, wv, wo)]
+        ctx.learns = alpha_p is not None
+        return out.view(*x.shape[:-1], plan.C)
+
+    @staticmethod
+    @torch.autograd.function.once_differentiable
+    def backward(ctx, dout):
+        work, x2, wq, wk, wv, wo, patt, pidx, alpha, rho, z, cos, sin = ctx.saved_tensors[:13]
+        plan, sz = ctx.plan, ctx.sz
+        B, T = ctx.bt
+        dev = dout.device
+        need = ctx.needs_input_grad
+        d2 = ops._as_2d(dout)
+        if d2.dtype != torch.bfloat16:
+            d2 = d2.to(torch.bfloat16)
+        if d2.stride(0) % 8 or d2.data_ptr() % 16:
+            d2 = d2.contiguous()
+        x_shape, x_dtype = ctx.x_like
+        c = _Call()
+        c.B, c.T, c.train = B, T, 1
+        # a converted tensor is read from the workspace; its argument only tells the dtype and layout
+        c.x = x2 if x2 is not None else work.view(torch.float32)[:plan.C].view(1, plan.C)
+        c.w = [wq, wk, wv, wo] if wq is not None else [work.view(torch.float32)] * 4
+        c.rope = (cos, sin) if cos is not None else None
+        c.patt, c.pidx, c.alpha, c.rho, c.z = patt, pidx, alpha, rho, z
+        g = SafAttnLayerBwdArgs()
+        g.struct_size = C.sizeof(SafAttnLayerBwdArgs)
+        g.fwd = plan.args(c)
+        g.fwd.work, g.fwd.work_bytes = work.data_ptr(), sz[0]
+        g.dout, g.lddo = d2.data_ptr(), d2.stride(0)
+        scratch = _blob(sz[1], dev)
+        g.work, g.work_bytes = scratch.data_ptr(), sz[1]
+        dx, dw = None, [None] * 4
+        if need[0]:
+            dx = torch.empty(x_shape, dtype=x_dtype, device=dev)
+            g.dx = dx.data_ptr()
+        if need[1] or need[2] or need[3]:
+            for i in range(3):
+                dw[i] = torch.empty(ctx.w_like[i][0], dtype=ctx.w_like[i][1], device=dev)
+            g.dwq, g.dwk, g.dwv = [t.data_ptr() for t in dw[:3]]
+        if need[4]:
+            dw[3] = torch.empty(ctx.w_like[3][0], dtype=ctx.w_like[3][1], device=dev)
+            g.dwo = dw[3].data_ptr()
+        g.need_dy = int(ctx.learns)
+        ops._call(d2, lib.saf_attn_layer_bwd, C.byref(g))
+        da = dr = None
+        if ctx.learns:
+            from .trainable_patterns import pattern_param_grad
+            _, _, v, y = projection_views(plan, work, sz, B, T)
+            dy = scratch[:2 * B * T * plan.H * plan.hd].view(torch.bfloat16).view(B, T, plan.H, plan.hd).transpose(1, 2)
+            da, dr = pattern_param_grad(dy, y, v, alpha, rho, z, plan.frozen)
+        return (dx, *[t if need[1 + i] else None for i, t in enumerate(dw)], da, dr, None, None, None)
+
+
+def attention_layer(plan, x, weights, rope, *, patt=None, pidx=None, decomposed=(None, None, None), learn=None,
+                    biases=None, residual=None, measure=None):
+    """x (B, T, C) -> bf16 (B, T, C).  weights: q, k, v, o; decomposed: (alpha, rho, z) buffers; learn: (alpha, rho)
+    parameters that receive gradients (decomposed then holds their detached values and current normalisers);
+    measure: called with the rotated q, k of the live heads.  Biases and residual go with inference."""
+    c = _Call()
+    c.B, c.T = x.shape[0], x.shape[1]
+    c.x, c.w, c.rope = _rows(x.detach()), weights, rope
+    c.patt, c.pidx = patt, pidx
+    c.alpha, c.rho, c.z = decomposed
+    if torch.is_grad_enabled() and (x.requires_grad or learn is not None or any(w.requires_grad for w in weights)):
+        c.train = 1
+        ap, rp = learn if learn is not None else (None, None)
+        return _LayerFunction.apply(x, *weights, ap, rp, plan, c, measure)
+    c.train = 0
+    r2 = None
+    if residual is not None:
+        r2 = ops._as_2d(residual)
+        if r2.dtype != torch.bfloat16:
+            r2 = r2.to(torch.bfloat16)
+        if r2.stride(0) % 8 or r2.data_ptr() % 16:
+            r2 = r2.contiguous()
+    out, work, sz = _forward(plan, c, biases, r2)
+    if measure is not None:
+        q, k, _, _ = projection_views(plan, work, sz, c.B, c.T)
+        measure(q, k)
+    return out.view(c.B, c.T, plan.C)

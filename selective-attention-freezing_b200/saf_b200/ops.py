@@ -46,7 +46,9 @@ def _ptr(t):
 
 
 def _stream(t):
-    return C.c_void_p(torch.cuda.current_stream(t.device).cuda_stream)
+    """Raw handle of the current stream of t's device."""
+    d = t.device.index
+    return C.c_void_p(torch._C._cuda_getCurrentRawStream(torch.cuda.current_device() if d is None else d))
 
 
 def _call(t, fn, *args):
@@ -296,6 +298,17 @@ def attention_timing(enable):
     got = _ATTN_EVENTS
     _ATTN_EVENTS = [] if enable else None
     return got
+
+
+def attention_event_pair():
+    """Raw handles of a new event pair of the running probe, for a library call that records them itself; else None."""
+    if _ATTN_EVENTS is None:
+        return None
+    e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+    e0.record()          # (an event gets its handle at its first record)
+    e1.record()
+    _ATTN_EVENTS.append((e0, e1))
+    return e0.cuda_event, e1.cuda_event
 
 
 class _FusedMixedAttn(torch.autograd.Function):
