@@ -383,6 +383,26 @@ typedef struct SafAttnLayerBwdArgs {
   int64_t work_bytes;
 } SafAttnLayerBwdArgs;
 
+/* A whole pre-norm transformer block at inference: x1 = x + attention(norm(x)), out = x1 + mlp(norm(x1)).  LayerNorm and
+ * GELU (Block.forward, nanogpt/model.py:1237-1240) or, with rms / gated, RMSNorm and the gated SiLU MLP of the
+ * Qwen-shaped blocks.  bf16 throughout. */
+typedef struct SafBlockArgs {
+  int32_t struct_size;
+  int32_t rms, gated;
+  int32_t hidden;           /* width of the MLP, a multiple of 64 (gated: 128)        */
+  float eps;
+  SafAttnLayerArgs layer;   /* its x and out are the block's; residual and train are not used; work is the block's
+                               workspace, saf_block_workspace() bytes                  */
+  const void *n1_w, *n1_b;  /* (C,); biases may be null                               */
+  const void *n2_w, *n2_b;
+  const void *w_in, *w_up;  /* (hidden, C): c_fc, or gate and up                      */
+  const void *b_in;         /* (hidden,) or null                                      */
+  const void* w_out;        /* (C, hidden)                                            */
+  const void* b_out;        /* (C,) or null                                           */
+} SafBlockArgs;
+int saf_block_workspace(const SafBlockArgs* args, int64_t* bytes);
+int saf_block_fwd(const SafBlockArgs* args, void* stream);
+
 /* sizes[4]: bytes of the forward's and of the backward's workspace (0 without `train`), byte offsets of the
  * projection (B*T, width) and of the attention output (B*T, H*HD) in the forward's.  Host-only. */
 int saf_attn_layer_workspace(const SafAttnLayerArgs* args, int64_t* sizes);

@@ -11,6 +11,8 @@ namespace {
 
 constexpr int LN_WARPS = 8;
 constexpr int LN_MAX_CHUNKS = 8;   // 16-byte chunks per lane held in registers: C <= 2048 on the vector path
+// (the kernel is compiled per chunk count: with room for 8 chunks a 768-wide row held a third of its registers and
+// the SM a third of the loads in flight)
 
 __device__ __forceinline__ void unpack8(const uint4& u, float (&f)[8]) {
   const uint32_t w[4] = {u.x, u.y, u.z, u.w};
@@ -21,6 +23,7 @@ __device__ __forceinline__ void unpack8(const uint4& u, float (&f)[8]) {
   }
 }
 
+template <int NC>
 __global__ void __launch_bounds__(LN_WARPS * 32) layernorm_bf16_kernel(const __nv_bfloat16* __restrict__ x, int64_t ldx,
                                                                        const __nv_bfloat16* __restrict__ w,
                                                                        const __nv_bfloat16* __restrict__ b,
@@ -30,10 +33,10 @@ __global__ void __launch_bounds__(LN_WARPS * 32) layernorm_bf16_kernel(const __n
   if (row >= M) return;
   const int n_chunks = C >> 3;                     // 8 elements each
   const uint4* xr = reinterpret_cast<const uint4*>(x + (int64_t)row * ldx);
-  float v[LN_MAX_CHUNKS][8];
+  float v[NC][8];
   float s = 0.f;
 #pragma unroll
-  for (int k = 0; k < LN_MAX_CHUNKS; ++k) {
+  for (int k = 0; k < NC; ++k) {
     const int c = lane + 32 * k;
     if (c < n_chunks) {
       unpack8(xr[c], v[k]);
@@ -46,7 +49,7 @@ __global__ void __launch_bounds__(LN_WARPS * 32) layernorm_bf16_kernel(const __n
   const float mean = rms ? 0.f : s / (float)C;
   float q = 0.f;
 #pragma unroll
-  for (int k = 0; k < LN_MAX_CHUNKS; ++k) {
+  for (int k = 0; k < NC; ++k) {
     if (lane + 32 * k < n_chunks) {
 #pragma unroll
       for (int e = 0; e < 8; ++e) {
@@ -62,7 +65,7 @@ __global__ void __launch_bounds__(LN_WARPS * 32) layernorm_bf16_kernel(const __n
   const uint4* br = reinterpret_cast<const uint4*>(b);
   uint4* orow = reinterpret_cast<uint4*>(out + (int64_t)row * ldo);
 #pragma unroll
-  for (int k = 0; k < LN_MAX_CHUNKS; ++k) {
+  for (int k = 0; k < NC; ++k) {
     const int c = lane + 32 * k;
     if (c < n_chunks) {
       float wv[8], bv[8];
@@ -178,10 +181,19 @@ int launch_layernorm(const void* x, int64_t ldx, const void* w, const void* b, v
   if (dtype == SAF_BF16) {
     const bool vec = C % 8 == 0 && C <= 256 * LN_MAX_CHUNKS && ldx % 8 == 0 && ldo % 8 == 0 && ln_al16(x) && ln_al16(w) &&
                      ln_al16(out) && (!b || ln_al16(b));
-    if (vec)
-      layernorm_bf16_kernel<<<grid, LN_WARPS * 32, 0, st>>>(
-          reinterpret_cast<const __nv_bfloat16*>(x), ldx, reinterpret_cast<const __nv_bfloat16*>(w),
-          reinterpret_cast<const __nv_bfloat16*>(b), reinterpret_cast<__nv_bfloat16*>(out), ldo, M, C, eps, rms);
+    if (vec) {
+      const auto xb = reinterpret_cast<const __nv_bfloat16*>(x), wb = reinterpret_cast<const __nv_bfloat16*>(w),
+                 bb = reinterpret_cast<const __nv_bfloat16*>(b);
+      const auto ob = reinterpret_cast<__nv_bfloat16*>(out);
+      switch ((C + 255) / 256) {
+        case 1: layernorm_bf16_kernel<1><<<grid, LN_WARPS * 32, 0, st>>>(xb, ldx, wb, bb, ob, ldo, M, C, eps, rms); break;
+        case 2: layernorm_bf16_kernel<2><<<grid, LN_WARPS * 32, 0, st>>>(xb, ldx, wb, bb, ob, ldo, M, C, eps, rms); break;
+        case 3: layernorm_bf16_kernel<3><<<grid, LN_WARPS * 32, 0, st>>>(xb, ldx, wb, bb, ob, ldo, M, C, eps, rms); break;
+        case 4: layernorm_bf16_kernel<4><<<grid, LN_WARPS * 32, 0, st>>>(xb, ldx, wb, bb, ob, ldo, M, C, eps, rms); break;
+        case 5: case 6: layernorm_bf16_kernel<6><<<grid, LN_WARPS * 32, 0, st>>>(xb, ldx, wb, bb, ob, ldo, M, C, eps, rms); break;
+        default: layernorm_bf16_kernel<LN_MAX_CHUNKS><<<grid, LN_WARPS * 32, 0, st>>>(xb, ldx, wb, bb, ob, ldo, M, C, eps, rms);
+      }
+    }
     else
       layernorm_generic_kernel<__nv_bfloat16><<<grid, LN_WARPS * 32, 0, st>>>(
           reinterpret_cast<const __nv_bfloat16*>(x), ldx, reinterpret_cast<const __nv_bfloat16*>(w),

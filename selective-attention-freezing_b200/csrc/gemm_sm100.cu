@@ -27,20 +27,23 @@
 namespace saf {
 namespace {
 
-constexpr int GM = 128, GN = 256, GK = 64;   // 128x256 tiles: 96 B/clk/SM of operand traffic at full MMA rate
-constexpr int SUBS = GN / 64;                // 64-column blocks per tile
+constexpr int GM = 128, GK = 64;             // rows of one CTA's accumulator, K step
 constexpr int A_BYTES = GM * GK * 2;            // 16 KB
 constexpr int SUB_BYTES = 64 * GK * 2;          // 8 KB: one 64-row block of weights
-constexpr int MAX_STAGES = 6;
+constexpr int MAX_STAGES = 8;
 // PAIR: two CTAs of a cluster share one 256 x 256 tile through tcgen05 cta_group::2.  Each CTA loads its 128 rows of x
 // and HALF of the weight tile (two 64-row blocks), so the operand traffic per SM drops from 96 to 64 bytes per clock at
 // the full MMA rate -- what one SM can pull from L2 -- and a stage shrinks to 32 KB (6 stages instead of 4).
-template <bool PAIR>
+// SUBS: 64-column blocks of a tile.  4 (128x256 tiles, 96 B/clk of operand traffic per SM at the full MMA rate) is the form
+// for products with tiles to spare; 2 and 1 cut a small product into enough tiles to occupy the SMs (pick_subs).
+template <bool PAIR, int SUBS>
 struct GCfg {
-  static constexpr int STAGES = PAIR ? 6 : 4;
-  static constexpr int B_SUBS = PAIR ? 2 : SUBS;                       // weight blocks a CTA loads per stage
-  static constexpr int STAGE_BYTES = A_BYTES + B_SUBS * SUB_BYTES;     // 32 KB / 48 KB
+  static constexpr int GN = SUBS * 64;                                 // columns of a tile
+  static constexpr int B_SUBS = PAIR ? SUBS / 2 : SUBS;                // weight blocks a CTA loads per stage
+  static constexpr int STAGE_BYTES = A_BYTES + B_SUBS * SUB_BYTES;     // 48 / 32 / 24 KB
+  static constexpr int STAGES = STAGE_BYTES > 32768 ? 4 : (STAGE_BYTES > 24576 ? 6 : 8);
   static constexpr int ROWS = PAIR ? 2 * GM : GM;                      // rows of a tile
+  static constexpr int TMEM_COLS = 2 * GN;                             // two accumulators
 };
 constexpr int OUT_BYTES = 2 * GM * 64 * 2;      // two 16 KB staging blocks for the TMA stores
 constexpr int MAX_SUB = 288;                    // 64-row blocks of output features (N <= 18432)
@@ -69,6 +72,27 @@ struct GemmParams {
   int halves;                    // weight blocks arrive as two 32-row TMA boxes (see SubTable)
   int32_t* zero2;                // two ints this launch clears for the next one on the stream (a tile queue), or null
 };
+
+// Width of a single-CTA tile, in 64-column blocks.  With few rows the 256-column tiles leave most SMs idle (777 rows of
+// a 12 x 64 layer: 21 to 84 tiles on 148 SMs, 18 us a product), so the narrower form that finishes first is taken: waves
+// of tiles, each KB K steps at the pace of its MMA (256 columns 128 cycles, 128: 64, 64: 48, bound by the A operand's
+// shared-memory reads; four per step) plus its blocks' way out.  `least`: blocks that belong together (a 128-row
+// rotated slab, a gate/up pair).
+int pick_subs(int tiles_m, int N, int KB, int least) {
+  const int sms = device_sm_count();
+  int best = 4;
+  double best_t = 1e30;
+  for (int subs = 4; subs >= least; subs >>= 1) {
+    const int tiles = tiles_m * ((N / 64 + subs - 1) / subs);
+    const double step = subs == 4 ? 512.0 : (subs == 2 ? 256.0 : 192.0);
+    const double t = (double)((tiles + sms - 1) / sms) * KB * step + 1200.0 * subs;
+    if (t < best_t) {
+      best_t = t;
+      best = subs;
+    }
+  }
+  return best;
+}
 
 // exact-form GELU, 0.5 x (1 + erf(x / sqrt 2)), with erf from Abramowitz-Stegun 7.1.26 (|error| < 1.5e-7):
 // one reciprocal and one exponential on the special-function unit, the rest FMAs
@@ -99,7 +123,7 @@ struct SmemLayout {
   uint32_t tmem_base;
 };
 
-template <bool PAIR>
+template <bool PAIR, int SUBS>
 __global__ void __launch_bounds__(GEMM_THREADS, 1)
 indexed_gemm_kernel(const __grid_constant__ CUtensorMap mapX, const __grid_constant__ CUtensorMap mapW0,
                     const __grid_constant__ CUtensorMap mapW1, const __grid_constant__ CUtensorMap mapW2,
@@ -107,8 +131,8 @@ indexed_gemm_kernel(const __grid_constant__ CUtensorMap mapX, const __grid_const
                     const __grid_constant__ GemmParams p, const __grid_constant__ SubTable tb) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
-  using C = GCfg<PAIR>;
-  constexpr int STAGES = C::STAGES, STAGE_BYTES = C::STAGE_BYTES;
+  using C = GCfg<PAIR, SUBS>;
+  constexpr int STAGES = C::STAGES, STAGE_BYTES = C::STAGE_BYTES, GN = C::GN;
   uint8_t* stage_base = smem;
   uint8_t* out_stage = smem + STAGES * STAGE_BYTES;
   SmemLayout* sl = reinterpret_cast<SmemLayout*>(out_stage + OUT_BYTES);
@@ -139,10 +163,10 @@ indexed_gemm_kernel(const __grid_constant__ CUtensorMap mapX, const __grid_const
   }
   if (warp == 1) {
     if constexpr (PAIR) {
-      tmem_alloc_pair(&sl->tmem_base, 512);
+      tmem_alloc_pair(&sl->tmem_base, C::TMEM_COLS);
       tmem_relinquish_pair();
     } else {
-      tmem_alloc(&sl->tmem_base, 512);
+      tmem_alloc(&sl->tmem_base, C::TMEM_COLS);
       tmem_relinquish();
     }
   }
@@ -328,7 +352,7 @@ indexed_gemm_kernel(const __grid_constant__ CUtensorMap mapX, const __grid_const
 #pragma unroll
           for (int j = 0; j < 64; ++j) v[j] = gelu_erf(v[j]);
         }
-        if (swiglu) {   // v holds the gate block; the up block is the next 64 accumulator columns
+        if (SUBS > 1 && swiglu) {   // v holds the gate block; the up block is the next 64 accumulator columns
           uint32_t q0[32], q1[32];
           tmem_ld32(tsrc + (u + 1) * 64, q0);
           tmem_ld32(tsrc + (u + 1) * 64 + 32, q1);
@@ -374,7 +398,7 @@ indexed_gemm_kernel(const __grid_constant__ CUtensorMap mapX, const __grid_const
             }
           } else {
             // slab 128: partner block is the other 64-column block of the same tile
-            const int pu = u ^ 1;
+            const int pu = (u ^ 1) & (SUBS - 1);   // (a rotated 128-row slab never meets one-block tiles)
             uint32_t q0[32], q1[32];
             tmem_ld32(tsrc + pu * 64, q0);
             tmem_ld32(tsrc + pu * 64 + 32, q1);
@@ -428,13 +452,28 @@ indexed_gemm_kernel(const __grid_constant__ CUtensorMap mapX, const __grid_const
   __syncthreads();
   if constexpr (PAIR) {
     cluster_sync_all();               // nothing of the peer's is touched after this point
-    if (warp == 1) tmem_dealloc_pair(tmem, 512);
+    if (warp == 1) tmem_dealloc_pair(tmem, C::TMEM_COLS);
   } else {
-    if (warp == 1) tmem_dealloc(tmem, 512);
+    if (warp == 1) tmem_dealloc(tmem, C::TMEM_COLS);
   }
 }
 
 bool aligned16(const void* p) { return ((uintptr_t)p & 15) == 0; }
+
+template <int SUBS>
+int launch_single(const CUtensorMap& mx, const CUtensorMap* mw, const CUtensorMap& mo, GemmParams p, const SubTable& tb,
+                  cudaStream_t st) {
+  using C = GCfg<false, SUBS>;
+  constexpr size_t smem = 1024 + C::STAGES * C::STAGE_BYTES + OUT_BYTES + sizeof(SmemLayout);
+  static_assert(smem <= 227 * 1024, "single-CTA kernel shared memory");
+  static PerDeviceOnce smem_once;
+  if (int rc = ensure_dyn_smem(indexed_gemm_kernel<false, SUBS>, (int)smem, smem_once)) return rc;
+  p.tiles_n = (p.N + C::GN - 1) / C::GN;
+  const int grid = std::min(device_sm_count(), p.tiles_m * p.tiles_n);
+  indexed_gemm_kernel<false, SUBS><<<grid, GEMM_THREADS, smem, st>>>(mx, mw[0], mw[1], mw[2], mw[3], mo, p, tb);
+  count_launch();
+  return check_launch("indexed_gemm_kernel");
+}
 
 }  // namespace
 
@@ -512,8 +551,6 @@ int launch_gemm_sm100(const SafIndexedLinearArgs& a, cudaStream_t st, int32_t* z
   GemmParams p;
   memset(&p, 0, sizeof(p));
   p.M = a.M; p.N = N; p.K = a.C; p.T = a.T; p.slab = a.slab;
-  p.tiles_m = (a.M + GM - 1) / GM;
-  p.tiles_n = (N + GN - 1) / GN;
   for (int w = 0; w < a.n_weights; ++w) p.bias[w] = a.biases[w];
   p.cosT = a.rope_cos;
   p.sinT = a.rope_sin;
@@ -528,12 +565,15 @@ int launch_gemm_sm100(const SafIndexedLinearArgs& a, cudaStream_t st, int32_t* z
   // CTA pairs on 256-row tiles when the product is large enough to fill the machine with them
   const char* pair_env = getenv("SAF_B200_GEMM_PAIR");
   const bool pair_off = pair_env && pair_env[0] == '0' && pair_env[1] == 0;
-  if (!pair_off && a.M >= 2 * GM * 32 && N >= GN) {
-    constexpr size_t smem_p = 1024 + GCfg<true>::STAGES * GCfg<true>::STAGE_BYTES + OUT_BYTES + sizeof(SmemLayout);
+  if (!pair_off && a.M >= 2 * GM * 32 && N >= 256) {
+    using C = GCfg<true, 4>;
+    constexpr size_t smem_p = 1024 + C::STAGES * C::STAGE_BYTES + OUT_BYTES + sizeof(SmemLayout);
     static_assert(smem_p <= 227 * 1024, "pair kernel shared memory");
+    auto kernel = indexed_gemm_kernel<true, 4>;
     static PerDeviceOnce smem_once_p;
-    if ((rc = ensure_dyn_smem(indexed_gemm_kernel<true>, (int)smem_p, smem_once_p))) return rc;
-    p.tiles_m = (a.M + 2 * GM - 1) / (2 * GM);
+    if ((rc = ensure_dyn_smem(kernel, (int)smem_p, smem_once_p))) return rc;
+    p.tiles_m = (a.M + C::ROWS - 1) / C::ROWS;
+    p.tiles_n = (N + C::GN - 1) / C::GN;
     cudaLaunchConfig_t cfg;
     memset(&cfg, 0, sizeof(cfg));
     cudaLaunchAttribute attr[1];
@@ -553,7 +593,7 @@ int launch_gemm_sm100(const SafIndexedLinearArgs& a, cudaStream_t st, int32_t* z
     if (pairs <= 0) {
       cfg.gridDim = dim3(sm_count & ~1);
       int n = 0;
-      if (cudaOccupancyMaxActiveClusters(&n, indexed_gemm_kernel<true>, &cfg) != cudaSuccess || n <= 0) {
+      if (cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) != cudaSuccess || n <= 0) {
         cudaGetLastError();
         n = sm_count / 2;
       }
@@ -562,7 +602,7 @@ int launch_gemm_sm100(const SafIndexedLinearArgs& a, cudaStream_t st, int32_t* z
     }
     pairs = std::min(pairs, p.tiles_m * p.tiles_n);
     cfg.gridDim = dim3(2 * pairs);
-    cudaError_t e = cudaLaunchKernelEx(&cfg, indexed_gemm_kernel<true>, mx, mw[0], mw[1], mw[2], mw[3], mo, p, tb);
+    cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, mx, mw[0], mw[1], mw[2], mw[3], mo, p, tb);
     if (e != cudaSuccess) {
       cudaGetLastError();
       return fail(SAF_ERR_CUDA, "indexed_gemm_kernel<pair> launch: %s", cudaGetErrorString(e));
@@ -570,13 +610,14 @@ int launch_gemm_sm100(const SafIndexedLinearArgs& a, cudaStream_t st, int32_t* z
     count_launch();
     if ((rc = check_launch("indexed_gemm_kernel<pair>"))) return rc;
   } else {
-    constexpr size_t smem = 1024 + GCfg<false>::STAGES * GCfg<false>::STAGE_BYTES + OUT_BYTES + sizeof(SmemLayout);
-    static PerDeviceOnce smem_once;
-    if ((rc = ensure_dyn_smem(indexed_gemm_kernel<false>, (int)smem, smem_once))) return rc;
-    const int grid = std::min(sm_count, p.tiles_m * p.tiles_n);
-    indexed_gemm_kernel<false><<<grid, GEMM_THREADS, smem, st>>>(mx, mw[0], mw[1], mw[2], mw[3], mo, p, tb);
-    count_launch();
-    if ((rc = check_launch("indexed_gemm_kernel"))) return rc;
+    const bool together = a.act == SAF_ACT_SWIGLU || (!halves && a.slab == 128 && a.slab_rope);
+    p.tiles_m = (a.M + GM - 1) / GM;
+    switch (pick_subs(p.tiles_m, N, (a.C + GK - 1) / GK, together ? 2 : 1)) {
+      case 1: rc = launch_single<1>(mx, mw, mo, p, tb, st); break;
+      case 2: rc = launch_single<2>(mx, mw, mo, p, tb, st); break;
+      default: rc = launch_single<4>(mx, mw, mo, p, tb, st); break;
+    }
+    if (rc) return rc;
   }
   if (rope_after)
     return launch_rope_slabs(a.out, a.ldo, a.M, a.n_slabs, a.slab, a.T, a.slab_rope, a.rope_cos, a.rope_sin, a.dtype, 0, st);

@@ -364,3 +364,112 @@ int saf_attn_layer_bwd(const SafAttnLayerBwdArgs* args, void* stream) {
 }
 
 }  // extern "C"
+
+// ---- the transformer block around the layer (inference) ----------------------------------------------------------------
+namespace {
+
+struct BlockLayout {
+  int64_t layer, normed, x1, hidden, total;
+};
+BlockLayout block_layout(const SafBlockArgs& b) {
+  const Dims d = dims_of(b.layer);
+  BlockLayout l;
+  l.layer = 0;
+  int64_t at = up(fwd_layout(b.layer, d).total);
+  l.normed = at;
+  at += up(d.tok * d.C * 2);
+  l.x1 = at;
+  at += up(d.tok * d.C * 2);
+  l.hidden = at;
+  at += up(d.tok * b.hidden * 2);
+  l.total = at;
+  return l;
+}
+
+int validate_block(const SafBlockArgs* b) {
+  if (!b) return fail(SAF_ERR_INVALID, "null argument struct");
+  if (b->struct_size != (int32_t)sizeof(SafBlockArgs))
+    return fail(SAF_ERR_INVALID, "SafBlockArgs size mismatch: caller %d, library %d", b->struct_size, (int)sizeof(SafBlockArgs));
+  if (int rc = validate_layer(&b->layer)) return rc;
+  if (b->layer.x_dtype != SAF_BF16 || b->layer.w_dtype != SAF_BF16 || b->layer.train)
+    return fail(SAF_ERR_UNSUPPORTED, "the block entry is bf16 inference");
+  if (b->hidden <= 0 || b->hidden % (b->gated ? 128 : 64) || b->layer.C % 64) return fail(SAF_ERR_UNSUPPORTED, "width %d, hidden %d", b->layer.C, b->hidden);
+  return SAF_OK;
+}
+
+// out = [residual +] act(x W^T + b) over whole matrices in 64-row blocks; gated: blocks of the two weights alternate
+int mlp_linear(const void* x, int M, int K, const void* w0, const void* w1, const void* bias, int N, int act, const void* residual,
+               int64_t ldr, void* out, int64_t ldo, int32_t* status, void* stream) {
+  constexpr int MAX = 1024;
+  int32_t weight[MAX], row0[MAX];
+  const int per = w1 ? 2 : 1, n = N / 64 * per;
+  if (n > MAX) return fail(SAF_ERR_LIMIT, "MLP width %d", N);
+  for (int i = 0; i < n; ++i) {
+    weight[i] = w1 ? i & 1 : 0;
+    row0[i] = i / per * 64;
+  }
+  SafIndexedLinearArgs g;
+  memset(&g, 0, sizeof(g));
+  g.struct_size = (int32_t)sizeof(g);
+  g.dtype = SAF_BF16;
+  g.M = M; g.C = K;
+  g.n_weights = per;
+  g.slab = 64;
+  g.n_slabs = n;
+  g.x = x; g.ldx = K;
+  g.weights[0] = w0; g.weights[1] = w1;
+  g.biases[0] = bias;
+  g.ldw[0] = g.ldw[1] = K;
+  g.rows_w[0] = g.rows_w[1] = N;
+  g.slab_weight = weight; g.slab_row0 = row0;
+  g.out = out; g.ldo = ldo;
+  g.status = status;
+  g.act = act;
+  g.residual = residual; g.ldr = ldr;
+  return saf_indexed_linear_fwd(&g, stream);
+}
+
+}  // namespace
+
+extern "C" {
+
+int saf_block_workspace(const SafBlockArgs* args, int64_t* bytes) {
+  if (int rc = validate_block(args)) return rc;
+  if (!bytes) return fail(SAF_ERR_INVALID, "null pointer");
+  *bytes = block_layout(*args).total;
+  return SAF_OK;
+}
+
+int saf_block_fwd(const SafBlockArgs* args, void* stream) {
+  int rc = validate_block(args);
+  if (rc) return rc;
+  const SafBlockArgs& b = *args;
+  const Dims d = dims_of(b.layer);
+  const BlockLayout l = block_layout(b);
+  if (!b.layer.x || !b.layer.out || !b.n1_w || !b.n2_w || !b.w_in || !b.w_out || (b.gated && !b.w_up)) return fail(SAF_ERR_INVALID, "null pointer");
+  if (!b.layer.work || ((uintptr_t)b.layer.work & 255) || b.layer.work_bytes < l.total)
+    return fail(SAF_ERR_INVALID, "workspace too small or not aligned to 256 bytes");
+  if (b.rms && (b.n1_b || b.n2_b)) return fail(SAF_ERR_INVALID, "RMSNorm has no bias");
+  cudaStream_t st = (cudaStream_t)stream;
+  uint8_t* work = reinterpret_cast<uint8_t*>(b.layer.work);
+  void *normed = work + l.normed, *x1 = work + l.x1, *hidden = work + l.hidden;
+  const int M = (int)d.tok;
+  if ((rc = launch_layernorm(b.layer.x, b.layer.ldx, b.n1_w, b.n1_b, normed, d.C, M, d.C, b.eps, SAF_BF16, b.rms, st))) return rc;
+  SafAttnLayerArgs a = b.layer;
+  a.x = normed;
+  a.ldx = d.C;
+  a.residual = b.layer.x;
+  a.ldr = b.layer.ldx;
+  a.out = x1;
+  a.ldo = d.C;
+  a.work_bytes = l.normed;
+  if ((rc = saf_attn_layer_fwd(&a, stream))) return rc;
+  if ((rc = launch_layernorm(x1, d.C, b.n2_w, b.n2_b, normed, d.C, M, d.C, b.eps, SAF_BF16, b.rms, st))) return rc;
+  int32_t* status = b.layer.attn.status;
+  if ((rc = mlp_linear(normed, M, d.C, b.w_in, b.gated ? b.w_up : nullptr, b.b_in, b.hidden, b.gated ? SAF_ACT_SWIGLU : SAF_ACT_GELU,
+                       nullptr, 0, hidden, b.hidden, status, stream)))
+    return rc;
+  return mlp_linear(hidden, M, b.hidden, b.w_out, nullptr, b.b_out, d.C, SAF_ACT_NONE, x1, d.C, b.layer.out, b.layer.ldo, status, stream);
+}
+
+}  // extern "C"

@@ -113,6 +113,15 @@ class SafAttnLayerBwdArgs(C.Structure):
     ]
 
 
+class SafBlockArgs(C.Structure):
+    _fields_ = [
+        ("struct_size", C.c_int32), ("rms", C.c_int32), ("gated", C.c_int32), ("hidden", C.c_int32), ("eps", C.c_float),
+        ("layer", SafAttnLayerArgs),
+        ("n1_w", C.c_void_p), ("n1_b", C.c_void_p), ("n2_w", C.c_void_p), ("n2_b", C.c_void_p),
+        ("w_in", C.c_void_p), ("w_up", C.c_void_p), ("b_in", C.c_void_p), ("w_out", C.c_void_p), ("b_out", C.c_void_p),
+    ]
+
+
 STATS_PROBS, STATS_LOGITS = 0, 1
 ACT_NONE, ACT_GELU, ACT_SWIGLU = 0, 1, 2
 
@@ -123,6 +132,7 @@ EXPORTS = (
     "saf_decomposed_logz", "saf_rope_slabs", "saf_layernorm_fwd", "saf_rmsnorm_fwd",
     "saf_pattern_normalisers", "saf_pattern_param_grad", "saf_attention_moments",
     "saf_attn_layer_workspace", "saf_attn_layer_fwd", "saf_attn_layer_bwd",
+    "saf_block_workspace", "saf_block_fwd",
     "saf_selftest_wait_timeout", "saf_selftest_per_device_once", "saf_selftest_mma_rate",
 )
 
@@ -150,12 +160,15 @@ def _load():
                      ("saf_indexed_linear_fwd", SafIndexedLinearArgs),
                      ("saf_pattern_param_grad", SafPatternGradArgs),
                      ("saf_attention_moments", SafAttnStatsArgs),
-                     ("saf_attn_layer_fwd", SafAttnLayerArgs), ("saf_attn_layer_bwd", SafAttnLayerBwdArgs)):
+                     ("saf_attn_layer_fwd", SafAttnLayerArgs), ("saf_attn_layer_bwd", SafAttnLayerBwdArgs),
+                     ("saf_block_fwd", SafBlockArgs)):
         f = getattr(lib, name)
         f.argtypes = [C.POINTER(at), C.c_void_p]
         f.restype = C.c_int
     lib.saf_attn_layer_workspace.argtypes = [C.POINTER(SafAttnLayerArgs), C.POINTER(C.c_int64)]
     lib.saf_attn_layer_workspace.restype = C.c_int
+    lib.saf_block_workspace.argtypes = [C.POINTER(SafBlockArgs), C.POINTER(C.c_int64)]
+    lib.saf_block_workspace.restype = C.c_int
     lib.saf_indexed_linear_bwd_dx.argtypes = [C.POINTER(SafIndexedLinearArgs), C.c_void_p, C.c_int64, C.c_void_p,
                                               C.c_int64, C.c_void_p, C.c_void_p]
     lib.saf_indexed_linear_bwd_dx.restype = C.c_int

@@ -292,7 +292,7 @@ class SafCausalSelfAttention(nn.Module):
         sd = self.sd_params()
         self._sd = (sd[:, 0].contiguous(), sd[:, 1].contiguous()) if self._sd_any else None
         self._patt_cast = None      # compact copy of the dense heads' patterns in the activation dtype, built on demand
-        self._plan = _layer.LayerPlan(states, self._live, hd, self.n_embd, self._fz_mask_i32, self._hidx_i32, self._sd)
+        self._plan = _layer.LayerPlan(states, self._live, hd, self.n_embd)
         self._mask_frozen_only = None   # head states with live heads masked out (training with attention dropout)
         self._fz_dirty = False
 
@@ -347,45 +347,66 @@ class SafCausalSelfAttention(nn.Module):
             self._last_attn = att.detach()
         return att @ v
 
-    def _attend_cheap(self, x, rope=None, residual=None):
-        B, T, C = x.shape
-        nh, hd = self.n_head, self.head_dim
-        rp = self._rope_f32(rope, T, x.device)
-        patt, pidx = self.dyn_pattern, None
-        dec = (self.dyn_alpha, self.dyn_rho, self.dyn_z) if self._dec_any else (None, None, None)
-        act_dt = torch.get_autocast_dtype("cuda") if torch.is_autocast_enabled("cuda") else x.dtype
+    def _patterns(self, act_dt):
+        """(patt, pidx) of the dense heads as the kernels take them."""
+        patt = self.dyn_pattern
         if act_dt == torch.bfloat16 and patt is not None and patt.dtype != act_dt and 1 in self._states:
             # The kernels multiply the pattern in the activation dtype (the reference casts P to v's dtype in
             # registers, kernel/frozen_attn.py:81).  A compact bf16 copy of the dense heads' planes, made once per
             # freeze set, gives the same products and lets them run on the TMA-fed tensor-core path.
             if self._patt_cast is None:
-                dense = [h for h in range(nh) if self._states[h] == 1]
-                slot = [0] * nh
+                dense = [h for h in range(self.n_head) if self._states[h] == 1]
+                slot = [0] * self.n_head
                 for i, h in enumerate(dense):
                     slot[h] = i
                 self._patt_cast = (patt[dense].to(act_dt), torch.tensor(slot, dtype=torch.int32, device=patt.device))
-            patt, pidx = self._patt_cast
+            return self._patt_cast
+        return patt, None
+
+    def _layer_call(self, x, rope):
+        """Arguments of `layer.attention_layer` for this call, or None when the layer runs operator by operator: fp32,
+        head widths the tensor-core kernels do not take, attention dropout, bias gradients."""
+        act_dt = torch.get_autocast_dtype("cuda") if torch.is_autocast_enabled("cuda") else x.dtype
+        if act_dt != torch.bfloat16 or not self._live or (self.dropout > 0.0 and self.training):
+            return None
+        grad = torch.is_grad_enabled()
+        w = (self.q_proj.weight, self.k_proj.weight, self.v_proj.weight, self.c_proj.weight)
+        bias = self.q_proj.bias is not None
+        # without autocast, training wants x and the weights in one dtype (the separate operators say so)
+        mixed = grad and w[0].dtype != x.dtype and not torch.is_autocast_enabled("cuda")
+        if (grad and bias) or mixed or not _layer.usable(self._plan, x, w, grad):
+            return None
+        T = x.shape[1]
+        call = dict(weights=w, rope=self._rope_f32(rope, T, x.device), frozen=self._fz_mask_i32, hidx=self._hidx_i32,
+                    sink_decay=self._sd)
+        if 1 in self._states:
+            call["patt"], call["pidx"] = self._patterns(act_dt)
+        if self._dec_any:
+            dec = (self.dyn_alpha, self.dyn_rho, self.dyn_z)
+            if grad and (dec[0].requires_grad or dec[1].requires_grad):
+                from . import trainable_patterns as tp
+                call["learn"] = dec[:2]
+                dec = (dec[0].detach(), dec[1].detach(), tp.current_normalisers(dec[0], dec[1], T))
+            call["decomposed"] = dec
+        if bias:
+            call["biases"] = [m.bias.to(act_dt) for m in (self.q_proj, self.k_proj, self.v_proj, self.c_proj)]
+        if self._stats is not None or self._logit_stats is not None:
+            call["measure"] = self._measure
+        return call
+
+    def _attend_cheap(self, x, rope=None, residual=None):
+        B, T, C = x.shape
+        nh, hd = self.n_head, self.head_dim
+        call = self._layer_call(x, rope)
+        if call is not None:
+            if torch.is_grad_enabled() and residual is not None:
+                return residual + _layer.attention_layer(self._plan, x, **call)
+            return _layer.attention_layer(self._plan, x, residual=residual, **call)
+        rp = self._rope_f32(rope, T, x.device)
+        dec = (self.dyn_alpha, self.dyn_rho, self.dyn_z) if self._dec_any else (None, None, None)
+        act_dt = torch.get_autocast_dtype("cuda") if torch.is_autocast_enabled("cuda") else x.dtype
+        patt, pidx = self._patterns(act_dt)
         nuf = len(self._live)
-        if act_dt == torch.bfloat16 and nuf and (self.dropout == 0.0 or not self.training):
-            grad = torch.is_grad_enabled()
-            w = [self.q_proj.weight, self.k_proj.weight, self.v_proj.weight, self.c_proj.weight]
-            bias = self.q_proj.bias is not None
-            # without autocast, training wants x and the weights in one dtype (the separate operators say so)
-            mixed = grad and not torch.is_autocast_enabled("cuda") and w[0].dtype != x.dtype
-            if not (grad and bias) and not mixed and _layer.usable(self._plan, x, w, grad):
-                learn = None
-                if grad and dec[0] is not None and (dec[0].requires_grad or dec[1].requires_grad):
-                    from . import trainable_patterns as tp
-                    learn = dec[:2]
-                    dec = (dec[0].detach(), dec[1].detach(), tp.current_normalisers(dec[0], dec[1], T))
-                bs = None
-                if bias:
-                    bs = [m.bias.to(act_dt) for m in (self.q_proj, self.k_proj, self.v_proj, self.c_proj)]
-                measure = self._measure if self._stats is not None or self._logit_stats is not None else None
-                out = _layer.attention_layer(self._plan, x, w, rp, patt=patt if 1 in self._states else None, pidx=pidx,
-                                             decomposed=dec, learn=learn, biases=bs, residual=None if grad else residual,
-                                             measure=measure)
-                return residual + out if grad and residual is not None else out
         if not torch.is_grad_enabled() and act_dt == torch.bfloat16 and (self.dropout == 0.0 or not self.training):
             # inference: one GEMM, canonical weights read in place, RoPE in the epilogue
             w = [m.weight if m.weight.dtype == act_dt else m.weight.to(act_dt) for m in (self.q_proj, self.k_proj, self.v_proj)]

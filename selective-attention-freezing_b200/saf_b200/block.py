@@ -9,6 +9,7 @@ import torch
 import torch.nn as nn
 import torch.nn.functional as F
 
+from . import layer as _layer
 from . import ops
 from .attention import SafCausalSelfAttention
 
@@ -60,5 +61,26 @@ class SafBlock(nn.Module):
         self.mlp = MLP(config)
 
     def forward(self, x, rope=None):
+        y = self._fused(x, rope)
+        if y is not None:
+            return y
         x = self.main_block(self.ln_1(x), rope=rope, residual=x)     # residual added in c_proj's epilogue
         return self.mlp(self.ln_2(x), residual=x)
+
+    def _fused(self, x, rope):
+        """The whole block as one library call (bf16 inference), or None when a piece has to run on its own."""
+        if torch.is_grad_enabled() or not x.is_cuda or x.dtype != torch.bfloat16 or torch.is_autocast_enabled("cuda"):
+            return None
+        m, mlp = self.main_block, self.mlp
+        if m._capture or (self.training and mlp.dropout.p > 0.0):
+            return None
+        if m._fz_dirty:
+            m._refresh_freeze_cache()
+        call = m._layer_call(x, rope)
+        if call is None:
+            return None
+        n1, n2 = (self.ln_1.weight, self.ln_1.bias), (self.ln_2.weight, self.ln_2.bias)
+        w = (mlp.c_fc.weight, None, mlp.c_fc.bias, mlp.c_proj.weight, mlp.c_proj.bias)
+        if not _layer.block_usable(m._plan, x, (*call["weights"], *n1, *n2, *w), w[0].shape[0], False):
+            return None
+        return _layer.block(m._plan, x, call, n1, n2, w, 1e-5)

@@ -25,6 +25,7 @@ import torch
 import torch.nn as nn
 import torch.nn.functional as F
 
+from . import layer as _layer
 from . import ops
 from .attention import rope_tables
 from .workloads import WORKLOADS
@@ -80,6 +81,8 @@ class SafGqaAttention(nn.Module):
         self.register_buffer("dec_rho", None)
         self.register_buffer("dec_z", None)
         self._live = list(range(H))
+        self._states = [0] * H
+        self._plan = None
         self._rope_key = None
 
     # ---- freeze state -----------------------------------------------------------------------
@@ -98,6 +101,7 @@ class SafGqaAttention(nn.Module):
         for h in sink_decay:
             states[h] = 3
         self._live = [h for h in range(H) if states[h] == 0]
+        self._states, self._plan = states, None
         hidx, pidx = [0] * H, [0] * H
         for slot, h in enumerate(self._live):
             hidx[h] = slot
@@ -134,12 +138,37 @@ class SafGqaAttention(nn.Module):
             self._rope_key = key
         return self._rope_tabs
 
+    def _layer_call(self, x, position_embeddings):
+        """Arguments of `layer.attention_layer`, or None when the layer runs operator by operator (fp32, q/k norm
+        between projection and rotation, no live head)."""
+        if x.dtype != torch.bfloat16 or self.q_norm is not None or not self._live or torch.is_grad_enabled():
+            return None
+        w = (self.q_proj.weight, self.k_proj.weight, self.v_proj.weight, self.o_proj.weight)
+        if self._plan is None:
+            self._plan = _layer.LayerPlan(self._states, self._live, self.head_dim, self.hidden, n_kv=self.n_kv)
+        if w[0].dtype != x.dtype or not _layer.usable(self._plan, x, w, False):
+            return None
+        call = dict(weights=w, rope=self._rope(*position_embeddings, x.shape[1]), frozen=self.frozen_mask_i32, hidx=self.hidx_i32,
+                    kvidx=self.kvidx_i32)
+        if getattr(self, "_has_sd", False):
+            call["sink_decay"] = (self.sd_alpha, self.sd_rho)
+        if self.prior_pattern is not None:
+            call["patt"], call["pidx"] = self.prior_pattern, self.pidx_i32
+        if self.dec_alpha is not None:
+            call["decomposed"] = (self.dec_alpha, self.dec_rho, self.dec_z)
+        if self.q_proj.bias is not None:
+            call["biases"] = [self.q_proj.bias, self.k_proj.bias, self.v_proj.bias, None]
+        return call
+
     def forward(self, hidden_states, position_embeddings, residual=None):
         """(B, T, hidden) -> (B, T, hidden), o_proj included (and `residual` added when given)."""
         if torch.is_grad_enabled() and any(p.requires_grad for p in self.parameters()):
             raise NotImplementedError("grouped-query mixed attention is forward-only (as in the reference)")
         x = hidden_states
         B, T, _ = x.shape
+        call = self._layer_call(x, position_embeddings) if x.is_cuda else None
+        if call is not None:
+            return _layer.attention_layer(self._plan, x, residual=residual, **call)
         hd, H, HKV = self.head_dim, self.n_head, self.n_kv
         U = len(self._live)
         cos, sin = self._rope(*position_embeddings, T)
@@ -199,6 +228,16 @@ class SafQwenBlock(nn.Module):
         self.mlp = GatedMLP(config)
 
     def forward(self, x, position_embeddings):
+        if x.is_cuda and x.dtype == torch.bfloat16 and not torch.is_grad_enabled():
+            m, mlp = self.self_attn, self.mlp
+            call = m._layer_call(x, position_embeddings)
+            if call is not None:
+                n1, n2 = self.input_layernorm, self.post_attention_layernorm
+                w = (mlp.gate_proj.weight, mlp.up_proj.weight, None, mlp.down_proj.weight, None)
+                used = (*call["weights"], *call.get("biases", ()), n1.weight, n2.weight, *w)
+                if n1.variance_epsilon == n2.variance_epsilon and _layer.block_usable(m._plan, x, used, w[0].shape[0], True):
+                    return _layer.block(m._plan, x, call, (n1.weight, None), (n2.weight, None), w, n1.variance_epsilon,
+                                        rms=True, gated=True)
         x = self.self_attn(self.input_layernorm(x), position_embeddings, residual=x)
         return self.mlp(self.post_attention_layernorm(x), residual=x)
 

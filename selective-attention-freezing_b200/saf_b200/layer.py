@@ -10,7 +10,7 @@ import ctypes as C
 import torch
 
 from . import ops
-from ._cabi import SafAttnLayerArgs, SafAttnLayerBwdArgs, SafMixedAttnArgs, lib, check, SAF_BF16, SAF_F32
+from ._cabi import SafAttnLayerArgs, SafAttnLayerBwdArgs, SafBlockArgs, SafMixedAttnArgs, lib, check, SAF_BF16, SAF_F32
 
 _DT = {torch.float32: SAF_F32, torch.bfloat16: SAF_BF16}
 HEAD_DIMS = (64, 96, 128)
@@ -18,12 +18,11 @@ MAX_BLOCKS = 160          # 64-row blocks of one backward product
 
 
 class LayerPlan:
-    """What a freeze set fixes: head states and slots.  Device tensors are kept, pointers are taken per call."""
+    """What a freeze set fixes on the host: head states and slots, and the argument struct with them filled in."""
 
-    def __init__(self, states, live, head_dim, width, frozen, hidx, sink_decay=None, kvidx=None, n_kv=0):
+    def __init__(self, states, live, head_dim, width, n_kv=0):
         H, U = len(states), len(live)
         self.H, self.U, self.hd, self.C, self.n_kv = H, U, head_dim, width, n_kv
-        self.frozen, self.hidx, self.sink_decay, self.kvidx = frozen, hidx, sink_decay, kvidx
         self._states = (C.c_int32 * H)(*states)
         self._live = (C.c_int32 * max(U, 1))(*live)
         a = SafAttnLayerArgs()
@@ -54,11 +53,11 @@ class LayerPlan:
         x = c.x
         t.B, t.T = c.B, c.T
         t.status = ops._status_ptr(x.device)
-        t.frozen, t.hidx = self.frozen.data_ptr(), self.hidx.data_ptr()
-        if self.kvidx is not None:
-            t.kvidx = self.kvidx.data_ptr()
-        if self.sink_decay is not None:
-            t.sd_alpha, t.sd_rho = self.sink_decay[0].data_ptr(), self.sink_decay[1].data_ptr()
+        t.frozen, t.hidx = c.frozen.data_ptr(), c.hidx.data_ptr()
+        if c.kvidx is not None:
+            t.kvidx = c.kvidx.data_ptr()
+        if c.sink_decay is not None:
+            t.sd_alpha, t.sd_rho = c.sink_decay[0].data_ptr(), c.sink_decay[1].data_ptr()
         if c.patt is not None:
             t.patt = ops._st(c.patt)
             t.S = c.patt.shape[1]
@@ -92,7 +91,14 @@ class LayerPlan:
 
 class _Call:
     """Tensors of one layer call, in the form the library reads them."""
-    __slots__ = ("B", "T", "x", "w", "train", "rope", "patt", "pidx", "alpha", "rho", "z")
+    __slots__ = ("B", "T", "x", "w", "train", "rope", "frozen", "hidx", "kvidx", "sink_decay", "patt", "pidx", "alpha", "rho", "z")
+
+    def __init__(self, B, T, x, w, train, rope, frozen, hidx, kvidx=None, sink_decay=None, patt=None, pidx=None,
+                 decomposed=(None, None, None)):
+        self.B, self.T, self.x, self.w, self.train, self.rope = B, T, x, w, train, rope
+        self.frozen, self.hidx, self.kvidx, self.sink_decay = frozen, hidx, kvidx, sink_decay
+        self.patt, self.pidx = patt, pidx
+        self.alpha, self.rho, self.z = decomposed
 
 
 def usable(plan, x, weights, training):
@@ -159,7 +165,7 @@ class _LayerFunction(torch.autograd.Function):
         kept = [work, c.x if x.dtype == torch.bfloat16 else None]
         kept += [None] * 4 if ctx.w_cast else [wq, wk, wv, wo]
         kept += [c.patt, c.pidx, c.alpha, c.rho, c.z, *(c.rope or (None, None))]
-        ctx.save_for_backward(*kept, plan.frozen, plan.hidx, *(plan.sink_decay or ()))
+        ctx.save_for_backward(*kept, c.frozen, c.hidx, *(c.sink_decay or ()))
         ctx.w_like = [(w.shape, w.dtype) for w in (wq, wk, wv, wo)]
         ctx.learns = alpha_p is not None
         return out.view(*x.shape[:-1], plan.C)
@@ -167,7 +173,8 @@ class _LayerFunction(torch.autograd.Function):
     @staticmethod
     @torch.autograd.function.once_differentiable
     def backward(ctx, dout):
-        work, x2, wq, wk, wv, wo, patt, pidx, alpha, rho, z, cos, sin = ctx.saved_tensors[:13]
+        work, x2, wq, wk, wv, wo, patt, pidx, alpha, rho, z, cos, sin, frozen, hidx = ctx.saved_tensors[:15]
+        sink_decay = ctx.saved_tensors[15:] or None
         plan, sz = ctx.plan, ctx.sz
         B, T = ctx.bt
         dev = dout.device
@@ -178,13 +185,11 @@ class _LayerFunction(torch.autograd.Function):
         if d2.stride(0) % 8 or d2.data_ptr() % 16:
             d2 = d2.contiguous()
         x_shape, x_dtype = ctx.x_like
-        c = _Call()
-        c.B, c.T, c.train = B, T, 1
         # a converted tensor is read from the workspace; its argument only tells the dtype and layout
-        c.x = x2 if x2 is not None else work.view(torch.float32)[:plan.C].view(1, plan.C)
-        c.w = [wq, wk, wv, wo] if wq is not None else [work.view(torch.float32)] * 4
-        c.rope = (cos, sin) if cos is not None else None
-        c.patt, c.pidx, c.alpha, c.rho, c.z = patt, pidx, alpha, rho, z
+        x_arg = x2 if x2 is not None else work.view(torch.float32)[:plan.C].view(1, plan.C)
+        w_arg = [wq, wk, wv, wo] if wq is not None else [work.view(torch.float32)] * 4
+        c = _Call(B, T, x_arg, w_arg, 1, (cos, sin) if cos is not None else None, frozen, hidx, None, sink_decay, patt, pidx,
+                  (alpha, rho, z))
         g = SafAttnLayerBwdArgs()
         g.struct_size = C.sizeof(SafAttnLayerBwdArgs)
         g.fwd = plan.args(c)
@@ -210,34 +215,77 @@ class _LayerFunction(torch.autograd.Function):
             from .trainable_patterns import pattern_param_grad
             _, _, v, y = projection_views(plan, work, sz, B, T)
             dy = scratch[:2 * B * T * plan.H * plan.hd].view(torch.bfloat16).view(B, T, plan.H, plan.hd).transpose(1, 2)
-            da, dr = pattern_param_grad(dy, y, v, alpha, rho, z, plan.frozen)
+            da, dr = pattern_param_grad(dy, y, v, alpha, rho, z, frozen)
         return (dx, *[t if need[1 + i] else None for i, t in enumerate(dw)], da, dr, None, None, None)
 
 
-def attention_layer(plan, x, weights, rope, *, patt=None, pidx=None, decomposed=(None, None, None), learn=None,
-                    biases=None, residual=None, measure=None):
+def _bf16_rows(x):
+    x2 = ops._as_2d(x)
+    if x2.dtype != torch.bfloat16:
+        x2 = x2.to(torch.bfloat16)
+    return x2.contiguous() if x2.stride(0) % 8 or x2.data_ptr() % 16 else x2
+
+
+def attention_layer(plan, x, weights, rope, frozen, hidx, *, kvidx=None, sink_decay=None, patt=None, pidx=None,
+                    decomposed=(None, None, None), learn=None, biases=None, residual=None, measure=None):
     """x (B, T, C) -> bf16 (B, T, C).  weights: q, k, v, o; decomposed: (alpha, rho, z) buffers; learn: (alpha, rho)
     parameters that receive gradients (decomposed then holds their detached values and current normalisers);
     measure: called with the rotated q, k of the live heads.  Biases and residual go with inference."""
-    c = _Call()
-    c.B, c.T = x.shape[0], x.shape[1]
-    c.x, c.w, c.rope = _rows(x.detach()), weights, rope
-    c.patt, c.pidx = patt, pidx
-    c.alpha, c.rho, c.z = decomposed
-    if torch.is_grad_enabled() and (x.requires_grad or learn is not None or any(w.requires_grad for w in weights)):
-        c.train = 1
+    grad = torch.is_grad_enabled() and (x.requires_grad or learn is not None or any(w.requires_grad for w in weights))
+    c = _Call(x.shape[0], x.shape[1], _rows(x.detach()), weights, int(grad), rope, frozen, hidx, kvidx, sink_decay, patt, pidx,
+              decomposed)
+    if grad:
         ap, rp = learn if learn is not None else (None, None)
         return _LayerFunction.apply(x, *weights, ap, rp, plan, c, measure)
-    c.train = 0
-    r2 = None
-    if residual is not None:
-        r2 = ops._as_2d(residual)
-        if r2.dtype != torch.bfloat16:
-            r2 = r2.to(torch.bfloat16)
-        if r2.stride(0) % 8 or r2.data_ptr() % 16:
-            r2 = r2.contiguous()
-    out, work, sz = _forward(plan, c, biases, r2)
+    out, work, sz = _forward(plan, c, biases, None if residual is None else _bf16_rows(residual))
     if measure is not None:
         q, k, _, _ = projection_views(plan, work, sz, c.B, c.T)
         measure(q, k)
     return out.view(c.B, c.T, plan.C)
+
+
+def block_usable(plan, x, tensors, hidden, gated):
+    """bf16 inference of the whole block: every weight and norm in bf16, widths in whole 64-row blocks."""
+    return (x.dtype == torch.bfloat16 and hidden % (128 if gated else 64) == 0 and hidden // 64 * (2 if gated else 1) <= 288
+            and all(t is None or (t.dtype == torch.bfloat16 and t.is_contiguous() and t.data_ptr() % 16 == 0) for t in tensors))
+
+
+def block(plan, x, call, norm1, norm2, mlp, eps, *, rms=False, gated=False):
+    """One pre-norm block, x (B, T, C) bf16 -> (B, T, C), in one library call.  call: the keyword arguments of
+    `attention_layer`; norm: (weight, bias); mlp: (w_in, w_up, b_in, w_out, b_out)."""
+    kw = dict(call)
+    weights, rope, frozen, hidx = kw.pop("weights"), kw.pop("rope"), kw.pop("frozen"), kw.pop("hidx")
+    biases, measure = kw.pop("biases", None), kw.pop("measure", None)
+    kw.pop("learn", None)
+    c = _Call(x.shape[0], x.shape[1], _bf16_rows(x), weights, 0, rope, frozen, hidx, **kw)
+    g = SafBlockArgs()
+    g.struct_size = C.sizeof(SafBlockArgs)
+    g.rms, g.gated, g.hidden, g.eps = int(rms), int(gated), mlp[0].shape[0], eps
+    a = plan.args(c)
+    if biases is not None:
+        a.bq, a.bk, a.bv, a.bo = [None if b is None else b.data_ptr() for b in biases]
+    sz = plan.sizes(a)
+    tok, Cw = c.B * c.T, plan.C
+    dev = x.device
+    key = ("block", c.B, c.T, g.hidden)
+    n = plan._sizes.get(key)
+    if n is None:
+        g.layer = a
+        out = C.c_int64()
+        check(lib.saf_block_workspace(C.byref(g), C.byref(out)))
+        n = plan._sizes[key] = out.value
+    work = _blob(n, dev)
+    out = torch.empty((tok, Cw), dtype=torch.bfloat16, device=dev)
+    a.out, a.ldo = out.data_ptr(), Cw
+    a.work, a.work_bytes = work.data_ptr(), n
+    events = ops.attention_event_pair()
+    if events is not None:
+        a.event_before, a.event_after = events
+    g.layer = a
+    g.n1_w, g.n1_b, g.n2_w, g.n2_b = [None if t is None else t.data_ptr() for t in (*norm1, *norm2)]
+    g.w_in, g.w_up, g.b_in, g.w_out, g.b_out = [None if t is None else t.data_ptr() for t in mlp]
+    ops._call(c.x, lib.saf_block_fwd, C.byref(g))
+    if measure is not None:
+        q, k, _, _ = projection_views(plan, work, sz, c.B, c.T)
+        measure(q, k)
+    return out.view(c.B, c.T, Cw)
