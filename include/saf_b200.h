@@ -367,6 +367,7 @@ typedef struct SafAttnLayerArgs {
   void* work;               /* 256-byte aligned, saf_attn_layer_workspace() bytes     */
   int64_t work_bytes;
   void *event_before, *event_after; /* cudaEvent_t recorded around the attention launch, or null */
+  int32_t after_library_launch; /* 1: the last launch on the stream is this library's and wrote no weights (0 is always right) */
 } SafAttnLayerArgs;
 
 typedef struct SafAttnLayerBwdArgs {

@@ -5,6 +5,7 @@
 // y = x / sqrt(mean(x^2) + eps) * weight.
 // HBM-bound: one warp per row, 16-byte loads, the row stays in registers between the two passes.
 #include "saf_internal.h"
+#include "sm100_prims.cuh"
 
 namespace saf {
 namespace {
@@ -30,6 +31,8 @@ __global__ void __launch_bounds__(LN_WARPS * 32) layernorm_bf16_kernel(const __n
                                                                        __nv_bfloat16* __restrict__ out, int64_t ldo, int M,
                                                                        int C, float eps, int rms) {
   const int row = blockIdx.x * LN_WARPS + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  pdl_wait();
+  pdl_trigger();
   if (row >= M) return;
   const int n_chunks = C >> 3;                     // 8 elements each
   const uint4* xr = reinterpret_cast<const uint4*>(x + (int64_t)row * ldx);
@@ -94,6 +97,8 @@ __global__ void __launch_bounds__(LN_WARPS * 32) layernorm_generic_kernel(const 
                                                                           T* __restrict__ out, int64_t ldo, int M, int C,
                                                                           float eps, int rms) {
   const int row = blockIdx.x * LN_WARPS + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  pdl_wait();
+  pdl_trigger();
   if (row >= M) return;
   const T* xr = x + (int64_t)row * ldx;
   float s = 0.f;
@@ -128,6 +133,8 @@ struct CastParams {
 };
 
 __global__ void __launch_bounds__(CAST_THREADS) cast_bf16_kernel(const __grid_constant__ CastParams p) {
+  pdl_wait();
+  pdl_trigger();
   int s = 0;
   while (s + 1 < p.n && blockIdx.x >= p.block0[s + 1]) ++s;
   const float4* src = reinterpret_cast<const float4*>(p.seg[s].src);
@@ -170,9 +177,7 @@ int launch_cast_bf16(const CastSegment* seg, int n, cudaStream_t st) {
   }
   p.block0[n] = blocks;
   if (!blocks) return SAF_OK;
-  cast_bf16_kernel<<<blocks, CAST_THREADS, 0, st>>>(p);
-  count_launch();
-  return check_launch("cast_bf16_kernel");
+  return launch_pdl("cast_bf16_kernel", cast_bf16_kernel, dim3(blocks), CAST_THREADS, 0, st, 1, p);
 }
 
 int launch_layernorm(const void* x, int64_t ldx, const void* w, const void* b, void* out, int64_t ldo, int M, int C,
@@ -185,26 +190,25 @@ int launch_layernorm(const void* x, int64_t ldx, const void* w, const void* b, v
       const auto xb = reinterpret_cast<const __nv_bfloat16*>(x), wb = reinterpret_cast<const __nv_bfloat16*>(w),
                  bb = reinterpret_cast<const __nv_bfloat16*>(b);
       const auto ob = reinterpret_cast<__nv_bfloat16*>(out);
+      auto go = [&](auto kernel) {
+        return launch_pdl("layernorm_kernel", kernel, dim3(grid), LN_WARPS * 32, 0, st, 1, xb, ldx, wb, bb, ob, ldo, M, C, eps, rms);
+      };
       switch ((C + 255) / 256) {
-        case 1: layernorm_bf16_kernel<1><<<grid, LN_WARPS * 32, 0, st>>>(xb, ldx, wb, bb, ob, ldo, M, C, eps, rms); break;
-        case 2: layernorm_bf16_kernel<2><<<grid, LN_WARPS * 32, 0, st>>>(xb, ldx, wb, bb, ob, ldo, M, C, eps, rms); break;
-        case 3: layernorm_bf16_kernel<3><<<grid, LN_WARPS * 32, 0, st>>>(xb, ldx, wb, bb, ob, ldo, M, C, eps, rms); break;
-        case 4: layernorm_bf16_kernel<4><<<grid, LN_WARPS * 32, 0, st>>>(xb, ldx, wb, bb, ob, ldo, M, C, eps, rms); break;
-        case 5: case 6: layernorm_bf16_kernel<6><<<grid, LN_WARPS * 32, 0, st>>>(xb, ldx, wb, bb, ob, ldo, M, C, eps, rms); break;
-        default: layernorm_bf16_kernel<LN_MAX_CHUNKS><<<grid, LN_WARPS * 32, 0, st>>>(xb, ldx, wb, bb, ob, ldo, M, C, eps, rms);
+        case 1: return go(layernorm_bf16_kernel<1>);
+        case 2: return go(layernorm_bf16_kernel<2>);
+        case 3: return go(layernorm_bf16_kernel<3>);
+        case 4: return go(layernorm_bf16_kernel<4>);
+        case 5: case 6: return go(layernorm_bf16_kernel<6>);
+        default: return go(layernorm_bf16_kernel<LN_MAX_CHUNKS>);
       }
     }
-    else
-      layernorm_generic_kernel<__nv_bfloat16><<<grid, LN_WARPS * 32, 0, st>>>(
-          reinterpret_cast<const __nv_bfloat16*>(x), ldx, reinterpret_cast<const __nv_bfloat16*>(w),
-          reinterpret_cast<const __nv_bfloat16*>(b), reinterpret_cast<__nv_bfloat16*>(out), ldo, M, C, eps, rms);
-  } else {
-    layernorm_generic_kernel<float><<<grid, LN_WARPS * 32, 0, st>>>(
-        reinterpret_cast<const float*>(x), ldx, reinterpret_cast<const float*>(w), reinterpret_cast<const float*>(b),
-        reinterpret_cast<float*>(out), ldo, M, C, eps, rms);
+    return launch_pdl("layernorm_kernel", layernorm_generic_kernel<__nv_bfloat16>, dim3(grid), LN_WARPS * 32, 0, st, 1,
+                      reinterpret_cast<const __nv_bfloat16*>(x), ldx, reinterpret_cast<const __nv_bfloat16*>(w),
+                      reinterpret_cast<const __nv_bfloat16*>(b), reinterpret_cast<__nv_bfloat16*>(out), ldo, M, C, eps, rms);
   }
-  count_launch();
-  return check_launch("layernorm_kernel");
+  return launch_pdl("layernorm_kernel", layernorm_generic_kernel<float>, dim3(grid), LN_WARPS * 32, 0, st, 1,
+                    reinterpret_cast<const float*>(x), ldx, reinterpret_cast<const float*>(w), reinterpret_cast<const float*>(b),
+                    reinterpret_cast<float*>(out), ldo, M, C, eps, rms);
 }
 
 }  // namespace saf

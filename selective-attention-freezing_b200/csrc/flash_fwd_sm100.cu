@@ -740,6 +740,8 @@ flash_fwd_persistent_kernel(const __grid_constant__ CUtensorMap mapQ, const __gr
   using C = Cfg<HD>;
   const int bh_count = p.B * p.H;
   if ((int)blockIdx.x < bh_count) {          // scan slots, as in flash_fwd_kernel
+    pdl_wait();
+    pdl_trigger();
     const int b = blockIdx.x / p.H, h = blockIdx.x % p.H;
     const int state = p.force_state >= 0 ? p.force_state : p.frozen[h];
     if (state == SAF_SINK_DECAY && p.has_scan) {
@@ -763,6 +765,8 @@ flash_fwd_persistent_kernel(const __grid_constant__ CUtensorMap mapQ, const __gr
     return;
   }
   if ((int)blockIdx.x < bh_count + p.dense_slots) {   // dense-pattern role
+    pdl_wait();
+    pdl_trigger();
     extern __shared__ uint8_t dense_smem_raw[];
     uint8_t* dsm = (uint8_t*)(((uintptr_t)dense_smem_raw + 1023) & ~(uintptr_t)1023);
     dense_pv_cta<HD>(mapP, mapV64, mapO, p.dense, (int)blockIdx.x - bh_count, dsm);
@@ -804,7 +808,9 @@ flash_fwd_persistent_kernel(const __grid_constant__ CUtensorMap mapQ, const __gr
     tmem_relinquish();
   }
   tc_fence_before();
+  pdl_wait();            // every thread: all roles read or write global memory below
   __syncthreads();
+  if (tid == 0) pdl_trigger();
   tc_fence_after();
   const uint32_t tmem = bars->tmem_base;
 
@@ -1318,9 +1324,8 @@ int launch_typed(const SafMixedAttnArgs& a, uint32_t want, cudaStream_t st) {
     if ((rc = ensure_dyn_smem(flash_fwd_persistent_kernel<HD>, Cfg<HD>::SMEM_PERSIST, smem_once_p))) return rc;
     const int workers = std::min(device_sm_count(), p.n_items);
     const unsigned grid = (unsigned)(p.lead + workers);
-    flash_fwd_persistent_kernel<HD><<<grid, FLASH_THREADS, Cfg<HD>::SMEM_PERSIST, st>>>(mq, mk, mv, mo, mpat, mv64, p);
-    count_launch();
-    return check_launch("flash_fwd_persistent_kernel");
+    return launch_pdl("flash_fwd_persistent_kernel", flash_fwd_persistent_kernel<HD>, dim3(grid), FLASH_THREADS, Cfg<HD>::SMEM_PERSIST, st,
+                      1, mq, mk, mv, mo, mpat, mv64, p);
   }
   static PerDeviceOnce smem_once;
   if ((rc = ensure_dyn_smem(flash_fwd_kernel<HD>, Cfg<HD>::SMEM_BYTES, smem_once))) return rc;

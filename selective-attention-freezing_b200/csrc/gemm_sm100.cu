@@ -70,6 +70,7 @@ struct GemmParams {
   const __nv_bfloat16* residual; // added to the output, or null
   int64_t ldr;
   int halves;                    // weight blocks arrive as two 32-row TMA boxes (see SubTable)
+  int weights_early;             // the first weight tiles may be loaded before the previous kernel is complete
   int32_t* zero2;                // two ints this launch clears for the next one on the stream (a tile queue), or null
 };
 
@@ -147,10 +148,6 @@ indexed_gemm_kernel(const __grid_constant__ CUtensorMap mapX, const __grid_const
   const int tile_hi = (int)((int64_t)(unit + 1) * total_tiles / n_units);
 
   if (tid == 0) {
-    if (p.zero2 && blockIdx.x == 0) {
-      p.zero2[0] = 0;
-      p.zero2[1] = 0;
-    }
     for (int s = 0; s < STAGES; ++s) {
       mbar_init(&sl->full[s], 1);
       mbar_init(&sl->empty[s], 1);
@@ -182,45 +179,57 @@ indexed_gemm_kernel(const __grid_constant__ CUtensorMap mapX, const __grid_const
       tma_prefetch_desc(&mapX);
       uint32_t it = 0;
       bool ok = true;
+      // announce a stage's bytes and load its weight tile / its rows of x.
+      // PAIR: this CTA's 128 rows of x and its two of the tile's four weight blocks.  Every byte of both CTAs is
+      // counted on the even CTA's barrier, which its MMA warp waits on: the even CTA's producer announces the
+      // pair's bytes there (a local arrive), the odd CTA's producer only issues its loads -- they cannot land
+      // before the barrier's previous phase is over, because its own empty barrier opens after that.
+      // (a last column tile of two blocks is computed as a 256 x 128 product: one block per CTA)
+      auto load_w = [&](int tn, int kb, int s) {
+        const int nsub = min(SUBS, (p.N - tn * GN) / 64);
+        uint8_t* b = stage_base + s * STAGE_BYTES + A_BYTES;
+        const int per = PAIR ? (nsub == 2 ? 1 : C::B_SUBS) : SUBS;
+        const int mine = PAIR ? max(0, min(per, nsub - rank * per)) : nsub;
+        if (!PAIR) mbar_expect_tx(&sl->full[s], A_BYTES + nsub * SUB_BYTES);
+        else if (rank == 0) mbar_expect_tx(&sl->full[s], 2 * A_BYTES + nsub * SUB_BYTES);
+        const uint32_t bar = PAIR ? cluster_addr_of(&sl->full[s], 0) : 0;
+        for (int u = 0; u < mine; ++u) {
+          const int sb = tn * SUBS + rank * per + u;
+          if constexpr (PAIR) tma_load_2d_pair(b + u * SUB_BYTES, wm[tb.weight[sb]], bar, kb * GK, tb.row0[sb]);
+          else tma_load_2d(b + u * SUB_BYTES, wm[tb.weight[sb]], &sl->full[s], kb * GK, tb.row0[sb]);
+          if (p.halves) {   // the maps' boxes are 32 rows: the second run lands behind the first (4 swizzle atoms on)
+            if constexpr (PAIR) tma_load_2d_pair(b + u * SUB_BYTES + SUB_BYTES / 2, wm[tb.weightb[sb]], bar, kb * GK, tb.row0b[sb]);
+            else tma_load_2d(b + u * SUB_BYTES + SUB_BYTES / 2, wm[tb.weightb[sb]], &sl->full[s], kb * GK, tb.row0b[sb]);
+          }
+        }
+      };
+      auto load_x = [&](int tm, int kb, int s) {
+        uint8_t* a = stage_base + s * STAGE_BYTES;
+        if constexpr (PAIR) tma_load_2d_pair(a, &mapX, cluster_addr_of(&sl->full[s], 0), kb * GK, tm * C::ROWS + rank * GM);
+        else tma_load_2d(a, &mapX, &sl->full[s], kb * GK, tm * GM);
+      };
+      // the first ring of weight tiles depends on no earlier kernel (the caller says so)
+      const int early = p.weights_early && tile_lo < tile_hi ? min(KB, STAGES) : 0;
+      for (int kb = 0; kb < early; ++kb) load_w(tile_lo % p.tiles_n, kb, kb);
+      pdl_wait();
+      if (p.zero2 && blockIdx.x == 0) {
+        p.zero2[0] = 0;
+        p.zero2[1] = 0;
+      }
+      pdl_trigger();
       for (int tile = tile_lo; tile < tile_hi && ok; ++tile) {
         const int tm = tile / p.tiles_n, tn = tile - tm * p.tiles_n;
-        const int nsub = min(SUBS, (p.N - tn * GN) / 64);
         for (int kb = 0; kb < KB; ++kb, ++it) {
           const int s = it % STAGES;
-          if (!mbar_wait(&sl->empty[s], ((it / STAGES) & 1) ^ 1)) {
-            dev_set_error(p.status, SAF_DEV_TIMEOUT_TMA, 10);
-            ok = false;
-            break;
-          }
-          uint8_t* a = stage_base + s * STAGE_BYTES;
-          uint8_t* b = a + A_BYTES;
-          if constexpr (PAIR) {
-            // this CTA's 128 rows of x and its two of the tile's four weight blocks.  Every byte of both CTAs is
-            // counted on the even CTA's barrier, which its MMA warp waits on: the even CTA's producer announces the
-            // pair's bytes there (a local arrive), the odd CTA's producer only issues its loads -- they cannot land
-            // before the barrier's previous phase is over, because its own empty barrier opens after that.
-            // (a last column tile of two blocks is computed as a 256 x 128 product: one block per CTA)
-            const int per = nsub == 2 ? 1 : C::B_SUBS;
-            const int mine = max(0, min(per, nsub - rank * per));
-            const uint32_t bar = cluster_addr_of(&sl->full[s], 0);
-            if (rank == 0) mbar_expect_tx(&sl->full[s], 2 * A_BYTES + nsub * SUB_BYTES);
-            tma_load_2d_pair(a, &mapX, bar, kb * GK, tm * C::ROWS + rank * GM);
-            for (int u = 0; u < mine; ++u) {
-              const int sb = tn * SUBS + rank * per + u;
-              tma_load_2d_pair(b + u * SUB_BYTES, wm[tb.weight[sb]], bar, kb * GK, tb.row0[sb]);
-              if (p.halves)
-                tma_load_2d_pair(b + u * SUB_BYTES + SUB_BYTES / 2, wm[tb.weightb[sb]], bar, kb * GK, tb.row0b[sb]);
+          if (it >= (uint32_t)early) {
+            if (!mbar_wait(&sl->empty[s], ((it / STAGES) & 1) ^ 1)) {
+              dev_set_error(p.status, SAF_DEV_TIMEOUT_TMA, 10);
+              ok = false;
+              break;
             }
-          } else {
-            mbar_expect_tx(&sl->full[s], A_BYTES + nsub * SUB_BYTES);
-            tma_load_2d(a, &mapX, &sl->full[s], kb * GK, tm * GM);
-            for (int u = 0; u < nsub; ++u) {
-              const int sb = tn * SUBS + u;
-              tma_load_2d(b + u * SUB_BYTES, wm[tb.weight[sb]], &sl->full[s], kb * GK, tb.row0[sb]);
-              if (p.halves)   // the maps' boxes are 32 rows: the second run lands behind the first (4 swizzle atoms on)
-                tma_load_2d(b + u * SUB_BYTES + SUB_BYTES / 2, wm[tb.weightb[sb]], &sl->full[s], kb * GK, tb.row0b[sb]);
-            }
+            load_w(tn, kb, s);
           }
+          load_x(tm, kb, s);
         }
       }
     }
@@ -274,6 +283,7 @@ indexed_gemm_kernel(const __grid_constant__ CUtensorMap mapX, const __grid_const
     }
   } else if (warp >= 2) {
     // epilogue warps 2..5 -> TMEM lane quadrant (warp % 4)
+    pdl_wait();
     const int quad = warp & 3;
     const int row = quad * 32 + lane;           // row inside the tile
     const int etid = tid - 64;                  // 0..127
@@ -470,14 +480,13 @@ int launch_single(const CUtensorMap& mx, const CUtensorMap* mw, const CUtensorMa
   if (int rc = ensure_dyn_smem(indexed_gemm_kernel<false, SUBS>, (int)smem, smem_once)) return rc;
   p.tiles_n = (p.N + C::GN - 1) / C::GN;
   const int grid = std::min(device_sm_count(), p.tiles_m * p.tiles_n);
-  indexed_gemm_kernel<false, SUBS><<<grid, GEMM_THREADS, smem, st>>>(mx, mw[0], mw[1], mw[2], mw[3], mo, p, tb);
-  count_launch();
-  return check_launch("indexed_gemm_kernel");
+  return launch_pdl("indexed_gemm_kernel", indexed_gemm_kernel<false, SUBS>, dim3(grid), GEMM_THREADS, smem, st, 1, mx, mw[0], mw[1],
+                    mw[2], mw[3], mo, p, tb);
 }
 
 }  // namespace
 
-int launch_gemm_sm100(const SafIndexedLinearArgs& a, cudaStream_t st, int32_t* zero2) {
+int launch_gemm_sm100(const SafIndexedLinearArgs& a, cudaStream_t st, int32_t* zero2, bool weights_early) {
   if (a.dtype != SAF_BF16) return SAF_ERR_UNSUPPORTED;
   // slabs of 64 or 128 rows are whole 64-row weight blocks; other multiples of 32 (head_dim 96) are served as runs
   // of 32 rows, two per block, when the total width still fills whole 64-column blocks.  The rotation is fused in
@@ -560,6 +569,7 @@ int launch_gemm_sm100(const SafIndexedLinearArgs& a, cudaStream_t st, int32_t* z
   p.ldr = a.ldr;
   p.halves = halves ? 1 : 0;
   p.zero2 = zero2;
+  p.weights_early = weights_early ? 1 : 0;
 
   const int sm_count = device_sm_count();
   // CTA pairs on 256-row tiles when the product is large enough to fill the machine with them
@@ -574,23 +584,23 @@ int launch_gemm_sm100(const SafIndexedLinearArgs& a, cudaStream_t st, int32_t* z
     if ((rc = ensure_dyn_smem(kernel, (int)smem_p, smem_once_p))) return rc;
     p.tiles_m = (a.M + C::ROWS - 1) / C::ROWS;
     p.tiles_n = (N + C::GN - 1) / C::GN;
-    cudaLaunchConfig_t cfg;
-    memset(&cfg, 0, sizeof(cfg));
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = 2;
-    attr[0].val.clusterDim.y = 1;
-    attr[0].val.clusterDim.z = 1;
-    cfg.blockDim = dim3(GEMM_THREADS);
-    cfg.dynamicSmemBytes = smem_p;
-    cfg.stream = st;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
     // pairs that can be resident at once (an SM without a free neighbour in its GPC stays out)
     static std::atomic<int> pairs_cache[SAF_MAX_DEVICES];
     const int dev = current_device();
     int pairs = (dev >= 0 && dev < SAF_MAX_DEVICES) ? pairs_cache[dev].load(std::memory_order_acquire) : 0;
     if (pairs <= 0) {
+      cudaLaunchConfig_t cfg;
+      memset(&cfg, 0, sizeof(cfg));
+      cudaLaunchAttribute attr[1];
+      attr[0].id = cudaLaunchAttributeClusterDimension;
+      attr[0].val.clusterDim.x = 2;
+      attr[0].val.clusterDim.y = 1;
+      attr[0].val.clusterDim.z = 1;
+      cfg.blockDim = dim3(GEMM_THREADS);
+      cfg.dynamicSmemBytes = smem_p;
+      cfg.stream = st;
+      cfg.attrs = attr;
+      cfg.numAttrs = 1;
       cfg.gridDim = dim3(sm_count & ~1);
       int n = 0;
       if (cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) != cudaSuccess || n <= 0) {
@@ -601,14 +611,9 @@ int launch_gemm_sm100(const SafIndexedLinearArgs& a, cudaStream_t st, int32_t* z
       if (dev >= 0 && dev < SAF_MAX_DEVICES) pairs_cache[dev].store(pairs, std::memory_order_release);
     }
     pairs = std::min(pairs, p.tiles_m * p.tiles_n);
-    cfg.gridDim = dim3(2 * pairs);
-    cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, mx, mw[0], mw[1], mw[2], mw[3], mo, p, tb);
-    if (e != cudaSuccess) {
-      cudaGetLastError();
-      return fail(SAF_ERR_CUDA, "indexed_gemm_kernel<pair> launch: %s", cudaGetErrorString(e));
-    }
-    count_launch();
-    if ((rc = check_launch("indexed_gemm_kernel<pair>"))) return rc;
+    if ((rc = launch_pdl("indexed_gemm_kernel<pair>", kernel, dim3(2 * pairs), GEMM_THREADS, smem_p, st, 2, mx, mw[0], mw[1], mw[2], mw[3],
+                         mo, p, tb)))
+      return rc;
   } else {
     const bool together = a.act == SAF_ACT_SWIGLU || (!halves && a.slab == 128 && a.slab_rope);
     p.tiles_m = (a.M + GM - 1) / GM;

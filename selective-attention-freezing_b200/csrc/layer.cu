@@ -280,7 +280,7 @@ int saf_attn_layer_fwd(const SafAttnLayerArgs* args, void* stream) {
   g.out = work + l.qkv;
   g.ldo = d.width();
   // the projection also clears the attention launch's tile queue
-  rc = launch_gemm_sm100(g, st, t.sched);
+  rc = launch_gemm_sm100(g, st, t.sched, a.w_dtype == SAF_BF16 && a.after_library_launch);
   if (rc == SAF_ERR_UNSUPPORTED) {
     t.sched = nullptr;
     rc = saf_indexed_linear_fwd(&g, stream);
@@ -293,7 +293,9 @@ int saf_attn_layer_fwd(const SafAttnLayerArgs* args, void* stream) {
   go.ldo = a.ldo;
   go.residual = a.residual;
   go.ldr = a.ldr;
-  return saf_indexed_linear_fwd(&go, stream);
+  // (behind the attention launch, which writes no weights)
+  rc = launch_gemm_sm100(go, st, nullptr, true);
+  return rc == SAF_ERR_UNSUPPORTED ? saf_indexed_linear_fwd(&go, stream) : rc;
 }
 
 int saf_attn_layer_bwd(const SafAttnLayerBwdArgs* args, void* stream) {
@@ -426,7 +428,9 @@ int mlp_linear(const void* x, int M, int K, const void* w0, const void* w1, cons
   g.status = status;
   g.act = act;
   g.residual = residual; g.ldr = ldr;
-  return saf_indexed_linear_fwd(&g, stream);
+  if (int rc = validate_linear_args(&g)) return rc;
+  const int rc = launch_gemm_sm100(g, (cudaStream_t)stream, nullptr, true);     // behind a norm or another product
+  return rc == SAF_ERR_UNSUPPORTED ? saf_indexed_linear_fwd(&g, stream) : rc;
 }
 
 }  // namespace
@@ -463,6 +467,7 @@ int saf_block_fwd(const SafBlockArgs* args, void* stream) {
   a.out = x1;
   a.ldo = d.C;
   a.work_bytes = l.normed;
+  a.after_library_launch = 1;       // the norm, which writes no weights
   if ((rc = saf_attn_layer_fwd(&a, stream))) return rc;
   if ((rc = launch_layernorm(x1, d.C, b.n2_w, b.n2_b, normed, d.C, M, d.C, b.eps, SAF_BF16, b.rms, st))) return rc;
   int32_t* status = b.layer.attn.status;

@@ -8,6 +8,7 @@
 #include <stdio.h>
 
 #include <atomic>
+#include <utility>
 
 #include "../../include/saf_b200.h"
 
@@ -52,6 +53,38 @@ int ensure_dyn_smem(K kernel, int bytes, PerDeviceOnce& once) {
   return SAF_OK;
 }
 
+// Launch with programmatic dependent launch allowed (see pdl_wait in sm100_prims.cuh): on a chain of short kernels the
+// launch latency, the barrier / TMEM / descriptor set-up and the loads that depend on no predecessor run under the
+// kernel before.  cluster = 2: CTA pairs.
+template <typename... P, typename... A>
+int launch_pdl(const char* what, void (*kernel)(P...), dim3 grid, unsigned threads, size_t smem, cudaStream_t st, int cluster,
+               A&&... args) {
+  cudaLaunchConfig_t cfg{};
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.numAttrs = 1;
+  if (cluster > 1) {
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim.x = cluster;
+    attr[1].val.clusterDim.y = 1;
+    attr[1].val.clusterDim.z = 1;
+    cfg.numAttrs = 2;
+  }
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cfg.attrs = attr;
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, std::forward<A>(args)...);
+  if (e != cudaSuccess) {
+    cudaGetLastError();
+    return fail(SAF_ERR_CUDA, "%s: %s", what, cudaGetErrorString(e));
+  }
+  count_launch();
+  return SAF_OK;
+}
+
 // ---- element conversion -----------------------------------------------------
 template <typename T> __device__ __forceinline__ float to_f(T x);
 template <> __device__ __forceinline__ float to_f<float>(float x) { return x; }
@@ -89,8 +122,10 @@ int launch_flash_fwd_sm100(const SafMixedAttnArgs& a, uint32_t want, uint32_t* h
 // dense-stored frozen heads as a TMA-staged lower-triangular GEMM (bf16 patterns)
 int launch_dense_pv_sm100(const SafMixedAttnArgs& a, uint32_t* handled_states, cudaStream_t st);
 int launch_flash_bwd_sm100(const SafMixedAttnBwdArgs& a, uint32_t* handled_states, cudaStream_t st);
-// `zero2`: two device ints the launch clears for the next launch on the stream (not touched when it returns UNSUPPORTED)
-int launch_gemm_sm100(const SafIndexedLinearArgs& a, cudaStream_t st, int32_t* zero2 = nullptr);
+// `zero2`: two device ints the launch clears for the next launch on the stream (not touched when it returns UNSUPPORTED).
+// `weights_early`: the launch before this one on the stream does not write the weights, so the first weight tiles may be
+// loaded while it still runs
+int launch_gemm_sm100(const SafIndexedLinearArgs& a, cudaStream_t st, int32_t* zero2 = nullptr, bool weights_early = false);
 int launch_gemm_generic(const SafIndexedLinearArgs& a, cudaStream_t st);
 int launch_gemm_bwd_dx(const SafIndexedLinearArgs& a, const void* dout, int64_t lddo, void* dx, int64_t lddx,
                        const void* bias, cudaStream_t st);

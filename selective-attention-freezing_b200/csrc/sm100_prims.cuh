@@ -92,6 +92,18 @@ __device__ __forceinline__ void dev_set_error(int* err, int code, int where) {
 }
 
 // ---------------------------------------------------------------------------
+// programmatic dependent launch
+// ---------------------------------------------------------------------------
+// Kernels launched through launch_pdl() may start while the kernel before them on the stream still runs.  Everything
+// they read or write in global memory that an earlier kernel may touch comes after pdl_wait(), which returns when all
+// earlier kernels are complete and their writes visible; each thread that accesses global memory calls it (or is ordered
+// behind one that did by a barrier).  pdl_trigger() lets the next kernel start; it always follows the CTA's own
+// pdl_wait(), so a kernel that has started can rely on everything BEFORE its predecessor being complete, and only its
+// predecessor's own writes are still in flight until its pdl_wait() returns.
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
+// ---------------------------------------------------------------------------
 // proxy fences
 // ---------------------------------------------------------------------------
 __device__ __forceinline__ void fence_proxy_async_smem() {

@@ -100,7 +100,7 @@ class SafAttnLayerArgs(C.Structure):
         ("rope_cos", C.c_void_p), ("rope_sin", C.c_void_p),
         ("residual", C.c_void_p), ("ldr", C.c_int64), ("out", C.c_void_p), ("ldo", C.c_int64),
         ("work", C.c_void_p), ("work_bytes", C.c_int64),
-        ("event_before", C.c_void_p), ("event_after", C.c_void_p),
+        ("event_before", C.c_void_p), ("event_after", C.c_void_p), ("after_library_launch", C.c_int32),
     ]
 
 
