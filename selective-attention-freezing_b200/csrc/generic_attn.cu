@@ -1,11 +1,13 @@
 // CUDA-core (fp32 FMA) mixed attention: forward and backward for every head state,
 // element type, stride pattern and head_dim <= 128.  This is the path for fp32
 // inputs (true fp32 accumulation, the 2e-5 contract of kernel/fused_attn.py:36-37),
-// for shapes the tensor-core kernels do not take, and for the backward pass.
+// for shapes the tensor-core kernels do not take, and for the backward pass.  Live fp32 heads of 64
+// columns in 16-byte rows go to attn_f32.cu.
 //
 // Work decomposition follows the reference's Triton kernels
 // (kernel/fused_attn.py:228-289 forward, 291-540 backward): one CTA per 64-row
 // tile per (batch, head), causal tile skipping, head state read per CTA.
+#include "head_index.cuh"
 #include "saf_internal.h"
 
 namespace saf {
@@ -17,26 +19,6 @@ constexpr int BN = 64;      // keys per step
 constexpr int PADW = 65;    // padded row length of transposed tiles
 constexpr int NT = 256;
 constexpr float LOG2E = 1.4426950408889634f;
-
-struct HeadIdx {
-  int b, h, state, hq, hk, hv, hp;
-};
-
-__device__ __forceinline__ HeadIdx head_index(const SafMixedAttnArgs& a, int bh) {
-  HeadIdx x;
-  x.b = bh / a.H;
-  x.h = bh % a.H;
-  x.state = a.force_state >= 0 ? a.force_state : a.frozen[x.h];
-  x.hq = a.hidx ? a.hidx[x.h] : x.h;
-  if (a.HKV > 0) {
-    x.hk = x.hv = a.kvidx ? a.kvidx[x.h] : 0;
-  } else {
-    x.hk = x.hq;
-    x.hv = x.h;
-  }
-  x.hp = a.pidx ? a.pidx[x.h] : x.h;
-  return x;
-}
 
 // load one (rows x hd) tile of a (.., T, hd) head into smem, transposed: dst[d*PADW + r]
 template <typename T, bool ROPE>
@@ -568,14 +550,21 @@ int bwd_typed(const SafMixedAttnBwdArgs& g, uint32_t mask, cudaStream_t st) {
   const SafMixedAttnArgs& a = g.fwd;
   const int hd = a.HD;
   int rc;
-  const bool any_live = (mask & 1u) != 0;
+  bool any_live = (mask & 1u) != 0;
   if (any_live) {
     dim3 gd((a.T + (NT / 32) - 1) / (NT / 32), a.B * a.H);
     generic_delta_kernel<T><<<gd, NT, 0, st>>>(g);
     count_launch();
     if ((rc = check_launch("generic_delta_kernel"))) return rc;
+    rc = launch_attn_f32_bwd(g, st);
+    if (rc == SAF_OK) {
+      any_live = false;
+      mask &= ~1u;
+    } else if (rc != SAF_ERR_UNSUPPORTED) {
+      return rc;
+    }
   }
-  {
+  if (mask) {
     const size_t smem = sizeof(float) * ((size_t)4 * hd * PADW + (size_t)2 * BN * PADW);
     if ((rc = set_smem(generic_dkdv_kernel<T>, smem))) return rc;
     dim3 grid((a.T + BN - 1) / BN, a.B * a.H);
@@ -599,6 +588,12 @@ int bwd_typed(const SafMixedAttnBwdArgs& g, uint32_t mask, cudaStream_t st) {
 int launch_generic_fwd(const SafMixedAttnArgs& a, uint32_t states_mask, cudaStream_t st) {
   if (a.HD > 128) return fail(SAF_ERR_UNSUPPORTED, "head_dim %d > 128", a.HD);
   if (a.T == 0 || a.B == 0 || a.H == 0) return SAF_OK;
+  if (states_mask & 1u) {
+    const int rc = launch_attn_f32_fwd(a, st);
+    if (rc == SAF_OK) states_mask &= ~1u;
+    else if (rc != SAF_ERR_UNSUPPORTED) return rc;
+    if (!states_mask) return SAF_OK;
+  }
   switch (a.dtype) {
     case SAF_F32: return fwd_typed<float>(a, states_mask, st);
     case SAF_BF16: return fwd_typed<__nv_bfloat16>(a, states_mask, st);
