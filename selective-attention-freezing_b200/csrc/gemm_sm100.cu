@@ -12,9 +12,14 @@
 // Persistent, warp-specialised CTA (1 per SM):
 //   warp 0      TMA producer: x tile 128x64 and four 64x64 weight blocks per stage (128B swizzle)
 //   warp 1      MMA issuer: tcgen05.mma 128x256x16, bf16 -> fp32 in TMEM, 2 accumulator buffers (512 columns)
-//   warps 2..5  epilogue, 64 columns at a time: TMEM -> registers (bias, RoPE) -> bf16 -> swizzled smem
-//               -> TMA store (two staging blocks in flight).  The row's cos/sin values are fetched once
-//               per row of tiles, before the accumulator is waited for, so their latency hides behind the MMAs.
+//   warps 4..11 epilogue, two groups of four warps, 64 columns each at a time: TMEM -> registers (bias, RoPE) -> bf16
+//               -> swizzled smem -> TMA store (one staging block per group).  The row's cos/sin values are fetched
+//               once per row of tiles, before the accumulator is waited for, so their latency hides behind the MMAs.
+//               With K = 768 a tile's products take 6144 cycles; one group of four warps needed longer than that for
+//               a GELU or (by far) a rotation of 128-row slabs, whose 64 cos and 64 sin values it had to read anew for
+//               every tile: 65536 x 1536 -> 1664, 128-row slabs, 692 -> 453 us; 65536 x 768 -> 1920, 64-row, 209 -> 180.
+//               A residual comes by TMA into the block's own staging place, fetched into L2 while the products run:
+//               65536 x 768 -> 768 with residual 125 -> 90 us (row by row from global memory before).
 // Large products run the same kernel as CTA PAIRS (template parameter PAIR, a cluster of two): one 256x256 tile per
 // pair through tcgen05.mma.cta_group::2, each CTA loading its 128 rows of x and half of the weight tile (see GCfg).
 // All waits are bounded; a wait that runs out sets *status and the CTA drains.
@@ -47,7 +52,9 @@ struct GCfg {
 };
 constexpr int OUT_BYTES = 2 * GM * 64 * 2;      // two 16 KB staging blocks for the TMA stores
 constexpr int MAX_SUB = 288;                    // 64-row blocks of output features (N <= 18432)
-constexpr int GEMM_THREADS = 192;   // TMA warp, MMA warp, one epilogue warpgroup
+constexpr int GEMM_THREADS = 384;   // TMA warp, MMA warp, two idle ones; two epilogue groups of four warps
+// registers: 384 x 168 at launch; the first four warps keep 72, the epilogue takes 208 (128 * 72 + 256 * 208 <= 384 * 168)
+constexpr int REGS_ISSUE = 72, REGS_EPI = 208;
 
 struct SubTable {
   int32_t row0[MAX_SUB];
@@ -62,6 +69,7 @@ struct SubTable {
 struct GemmParams {
   int M, N, K, T, slab;
   int tiles_m, tiles_n;
+  int group_n, runs;             // column tiles walked together; units walk runs of tiles (see the tile order)
   const void* bias[SAF_MAX_WEIGHTS];
   const float* cosT;
   const float* sinT;
@@ -69,6 +77,7 @@ struct GemmParams {
   int act;                       // SAF_ACT_*
   const __nv_bfloat16* residual; // added to the output, or null
   int64_t ldr;
+  int residual_tma;              // the residual's blocks come through mapR (no rotation, no gate: columns as the output's)
   int halves;                    // weight blocks arrive as two 32-row TMA boxes (see SubTable)
   int weights_early;             // the first weight tiles may be loaded before the previous kernel is complete
   int32_t* zero2;                // two ints this launch clears for the next one on the stream (a tile queue), or null
@@ -120,7 +129,7 @@ __device__ __forceinline__ float silu_mul(float g, float u) {
 }
 
 struct SmemLayout {
-  uint64_t full[MAX_STAGES], empty[MAX_STAGES], acc_full[2], acc_empty[2];
+  uint64_t full[MAX_STAGES], empty[MAX_STAGES], acc_full[2], acc_empty[2], res[2];
   uint32_t tmem_base;
 };
 
@@ -129,6 +138,7 @@ __global__ void __launch_bounds__(GEMM_THREADS, 1)
 indexed_gemm_kernel(const __grid_constant__ CUtensorMap mapX, const __grid_constant__ CUtensorMap mapW0,
                     const __grid_constant__ CUtensorMap mapW1, const __grid_constant__ CUtensorMap mapW2,
                     const __grid_constant__ CUtensorMap mapW3, const __grid_constant__ CUtensorMap mapO,
+                    const __grid_constant__ CUtensorMap mapR,
                     const __grid_constant__ GemmParams p, const __grid_constant__ SubTable tb) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
@@ -140,12 +150,25 @@ indexed_gemm_kernel(const __grid_constant__ CUtensorMap mapX, const __grid_const
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int KB = (p.K + GK - 1) / GK;
   const int total_tiles = p.tiles_m * p.tiles_n;
-  // each CTA walks a contiguous run of tiles (column tile fastest): consecutive tiles share their rows, so the
-  // row's cos / sin values stay in registers and the x tile stays hot in L2
   const int rank = PAIR ? (int)cluster_ctarank() : 0;                 // which 128 rows of the tile are this CTA's
   const int unit = PAIR ? blockIdx.x >> 1 : blockIdx.x, n_units = PAIR ? gridDim.x >> 1 : gridDim.x;
-  const int tile_lo = (int)((int64_t)unit * total_tiles / n_units);
-  const int tile_hi = (int)((int64_t)(unit + 1) * total_tiles / n_units);
+  // Tile order: column tiles in groups whose weights stay in L2, inside a group all columns of one row tile first; the
+  // units take neighbouring tiles at the same time, so a row of x is fetched from memory once per group, by the units that
+  // need it together.  (Each unit walking the columns of rows of its own has 74 x 256 rows of x in use at once: at
+  // K = 8960 that is 340 MB, and x comes from memory once per column tile.  65536 x 8960 -> 1536 with that order and its
+  // sibling 1536 -> 2 x 8960 2372 us on average, now 1882.)  A rotated product keeps the runs: its epilogue holds the
+  // row's cos / sin values over the run, and reading them anew for every tile cost more than x from memory
+  // (65536 x 768 -> 1920: 180 us with runs, 260 without; at 128-row slabs no difference).
+  const int tile_lo = p.runs ? (int)((int64_t)unit * total_tiles / n_units) : unit;
+  const int tile_hi = p.runs ? (int)((int64_t)(unit + 1) * total_tiles / n_units) : total_tiles;
+  const int tile_step = p.runs ? 1 : n_units;
+  auto decode = [&](int tile, int& tm, int& tn) {
+    const int per_group = p.tiles_m * p.group_n;
+    const int g = tile / per_group, rem = tile - g * per_group;
+    const int width = min(p.group_n, p.tiles_n - g * p.group_n);
+    tm = rem / width;
+    tn = g * p.group_n + rem - tm * width;
+  };
 
   if (tid == 0) {
     for (int s = 0; s < STAGES; ++s) {
@@ -154,8 +177,10 @@ indexed_gemm_kernel(const __grid_constant__ CUtensorMap mapX, const __grid_const
     }
     for (int b = 0; b < 2; ++b) {
       mbar_init(&sl->acc_full[b], 1);
-      mbar_init(&sl->acc_empty[b], PAIR ? 8 : 4);       // one arrival per epilogue warp (of both CTAs)
+      mbar_init(&sl->acc_empty[b], PAIR ? 16 : 8);      // one arrival per epilogue warp (of both CTAs)
     }
+    mbar_init(&sl->res[0], 1);
+    mbar_init(&sl->res[1], 1);
     fence_mbar_init();
   }
   if (warp == 1) {
@@ -173,265 +198,276 @@ indexed_gemm_kernel(const __grid_constant__ CUtensorMap mapX, const __grid_const
   tc_fence_after();
   const uint32_t tmem = sl->tmem_base;
 
-  if (warp == 0) {
-    if (lane == 0) {
-      const CUtensorMap* wm[4] = {&mapW0, &mapW1, &mapW2, &mapW3};
-      tma_prefetch_desc(&mapX);
-      uint32_t it = 0;
-      bool ok = true;
-      // announce a stage's bytes and load its weight tile / its rows of x.
-      // PAIR: this CTA's 128 rows of x and its two of the tile's four weight blocks.  Every byte of both CTAs is
-      // counted on the even CTA's barrier, which its MMA warp waits on: the even CTA's producer announces the
-      // pair's bytes there (a local arrive), the odd CTA's producer only issues its loads -- they cannot land
-      // before the barrier's previous phase is over, because its own empty barrier opens after that.
-      // (a last column tile of two blocks is computed as a 256 x 128 product: one block per CTA)
-      auto load_w = [&](int tn, int kb, int s) {
-        const int nsub = min(SUBS, (p.N - tn * GN) / 64);
-        uint8_t* b = stage_base + s * STAGE_BYTES + A_BYTES;
-        const int per = PAIR ? (nsub == 2 ? 1 : C::B_SUBS) : SUBS;
-        const int mine = PAIR ? max(0, min(per, nsub - rank * per)) : nsub;
-        if (!PAIR) mbar_expect_tx(&sl->full[s], A_BYTES + nsub * SUB_BYTES);
-        else if (rank == 0) mbar_expect_tx(&sl->full[s], 2 * A_BYTES + nsub * SUB_BYTES);
-        const uint32_t bar = PAIR ? cluster_addr_of(&sl->full[s], 0) : 0;
-        for (int u = 0; u < mine; ++u) {
-          const int sb = tn * SUBS + rank * per + u;
-          if constexpr (PAIR) tma_load_2d_pair(b + u * SUB_BYTES, wm[tb.weight[sb]], bar, kb * GK, tb.row0[sb]);
-          else tma_load_2d(b + u * SUB_BYTES, wm[tb.weight[sb]], &sl->full[s], kb * GK, tb.row0[sb]);
-          if (p.halves) {   // the maps' boxes are 32 rows: the second run lands behind the first (4 swizzle atoms on)
-            if constexpr (PAIR) tma_load_2d_pair(b + u * SUB_BYTES + SUB_BYTES / 2, wm[tb.weightb[sb]], bar, kb * GK, tb.row0b[sb]);
-            else tma_load_2d(b + u * SUB_BYTES + SUB_BYTES / 2, wm[tb.weightb[sb]], &sl->full[s], kb * GK, tb.row0b[sb]);
-          }
-        }
-      };
-      auto load_x = [&](int tm, int kb, int s) {
-        uint8_t* a = stage_base + s * STAGE_BYTES;
-        if constexpr (PAIR) tma_load_2d_pair(a, &mapX, cluster_addr_of(&sl->full[s], 0), kb * GK, tm * C::ROWS + rank * GM);
-        else tma_load_2d(a, &mapX, &sl->full[s], kb * GK, tm * GM);
-      };
-      // the first ring of weight tiles depends on no earlier kernel (the caller says so)
-      const int early = p.weights_early && tile_lo < tile_hi ? min(KB, STAGES) : 0;
-      for (int kb = 0; kb < early; ++kb) load_w(tile_lo % p.tiles_n, kb, kb);
-      pdl_wait();
-      if (p.zero2 && blockIdx.x == 0) {
-        p.zero2[0] = 0;
-        p.zero2[1] = 0;
-      }
-      pdl_trigger();
-      for (int tile = tile_lo; tile < tile_hi && ok; ++tile) {
-        const int tm = tile / p.tiles_n, tn = tile - tm * p.tiles_n;
-        for (int kb = 0; kb < KB; ++kb, ++it) {
-          const int s = it % STAGES;
-          if (it >= (uint32_t)early) {
-            if (!mbar_wait(&sl->empty[s], ((it / STAGES) & 1) ^ 1)) {
-              dev_set_error(p.status, SAF_DEV_TIMEOUT_TMA, 10);
-              ok = false;
-              break;
+  if (warp < 4) {
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(REGS_ISSUE));
+    if (warp == 0) {
+      if (lane == 0) {
+        const CUtensorMap* wm[4] = {&mapW0, &mapW1, &mapW2, &mapW3};
+        tma_prefetch_desc(&mapX);
+        uint32_t it = 0;
+        bool ok = true;
+        // announce a stage's bytes and load its weight tile / its rows of x.
+        // PAIR: this CTA's 128 rows of x and its two of the tile's four weight blocks.  Every byte of both CTAs is
+        // counted on the even CTA's barrier, which its MMA warp waits on: the even CTA's producer announces the
+        // pair's bytes there (a local arrive), the odd CTA's producer only issues its loads -- they cannot land
+        // before the barrier's previous phase is over, because its own empty barrier opens after that.
+        // (a last column tile of two blocks is computed as a 256 x 128 product: one block per CTA)
+        auto load_w = [&](int tn, int kb, int s) {
+          const int nsub = min(SUBS, (p.N - tn * GN) / 64);
+          uint8_t* b = stage_base + s * STAGE_BYTES + A_BYTES;
+          const int per = PAIR ? (nsub == 2 ? 1 : C::B_SUBS) : SUBS;
+          const int mine = PAIR ? max(0, min(per, nsub - rank * per)) : nsub;
+          if (!PAIR) mbar_expect_tx(&sl->full[s], A_BYTES + nsub * SUB_BYTES);
+          else if (rank == 0) mbar_expect_tx(&sl->full[s], 2 * A_BYTES + nsub * SUB_BYTES);
+          const uint32_t bar = PAIR ? cluster_addr_of(&sl->full[s], 0) : 0;
+          for (int u = 0; u < mine; ++u) {
+            const int sb = tn * SUBS + rank * per + u;
+            if constexpr (PAIR) tma_load_2d_pair(b + u * SUB_BYTES, wm[tb.weight[sb]], bar, kb * GK, tb.row0[sb]);
+            else tma_load_2d(b + u * SUB_BYTES, wm[tb.weight[sb]], &sl->full[s], kb * GK, tb.row0[sb]);
+            if (p.halves) {   // the maps' boxes are 32 rows: the second run lands behind the first (4 swizzle atoms on)
+              if constexpr (PAIR) tma_load_2d_pair(b + u * SUB_BYTES + SUB_BYTES / 2, wm[tb.weightb[sb]], bar, kb * GK, tb.row0b[sb]);
+              else tma_load_2d(b + u * SUB_BYTES + SUB_BYTES / 2, wm[tb.weightb[sb]], &sl->full[s], kb * GK, tb.row0b[sb]);
             }
-            load_w(tn, kb, s);
           }
-          load_x(tm, kb, s);
+        };
+        auto load_x = [&](int tm, int kb, int s) {
+          uint8_t* a = stage_base + s * STAGE_BYTES;
+          if constexpr (PAIR) tma_load_2d_pair(a, &mapX, cluster_addr_of(&sl->full[s], 0), kb * GK, tm * C::ROWS + rank * GM);
+          else tma_load_2d(a, &mapX, &sl->full[s], kb * GK, tm * GM);
+        };
+        // the first ring of weight tiles depends on no earlier kernel (the caller says so)
+        const int early = p.weights_early && tile_lo < tile_hi ? min(KB, STAGES) : 0;
+        int tm, tn;
+        decode(tile_lo, tm, tn);
+        for (int kb = 0; kb < early; ++kb) load_w(tn, kb, kb);
+        pdl_wait();
+        if (p.zero2 && blockIdx.x == 0) {
+          p.zero2[0] = 0;
+          p.zero2[1] = 0;
+        }
+        pdl_trigger();
+        for (int tile = tile_lo; tile < tile_hi && ok; tile += tile_step) {
+          decode(tile, tm, tn);
+          if (p.residual_tma)     // the epilogue's residual blocks are in L2 by the time the products are done
+            for (int u = 0; u < min(SUBS, (p.N - tn * GN) / 64); ++u) tma_prefetch_2d(&mapR, tn * GN + u * 64, tm * C::ROWS + rank * GM);
+          for (int kb = 0; kb < KB; ++kb, ++it) {
+            const int s = it % STAGES;
+            if (it >= (uint32_t)early) {
+              if (!mbar_wait(&sl->empty[s], ((it / STAGES) & 1) ^ 1)) {
+                dev_set_error(p.status, SAF_DEV_TIMEOUT_TMA, 10);
+                ok = false;
+                break;
+              }
+              load_w(tn, kb, s);
+            }
+            load_x(tm, kb, s);
+          }
         }
       }
-    }
-  } else if (warp == 1 && rank == 0) {
-    // the whole warp walks the schedule (uniform addresses); one elected lane issues.  In a pair only the even
-    // CTA issues: its instructions read both CTAs' stages and write both CTAs' accumulators.
-    const bool leader = elect_one();
-    const uint32_t idesc_full = umma_idesc_bf16(C::ROWS, GN, 0, 0);
-    const uint32_t idesc_half = umma_idesc_bf16(C::ROWS, GN / 2, 0, 0);   // pair: a last column tile of two blocks
-    const uint32_t sbase = smem_u32(stage_base);
-    uint32_t it = 0, lt = 0;
-    bool ok = true;
-    for (int tile = tile_lo; tile < tile_hi && ok; ++tile, ++lt) {
-      const int buf = lt & 1;
-      if (!mbar_wait(&sl->acc_empty[buf], ((lt >> 1) & 1) ^ 1)) {
-        dev_set_error(p.status, SAF_DEV_TIMEOUT_MMA, 11);
-        break;
-      }
-      tc_fence_after();
-      const uint32_t d = tmem + buf * GN;
-      const int tn_ = tile % p.tiles_n;
-      const uint32_t idesc = (PAIR && (p.N - tn_ * GN) / 64 == 2) ? idesc_half : idesc_full;
-      for (int kb = 0; kb < KB; ++kb, ++it) {
-        const int s = it % STAGES;
-        if (!mbar_wait(&sl->full[s], (it / STAGES) & 1)) {
-          dev_set_error(p.status, SAF_DEV_TIMEOUT_MMA, 12);
-          ok = false;
+    } else if (warp == 1 && rank == 0) {
+      // the whole warp walks the schedule (uniform addresses); one elected lane issues.  In a pair only the even
+      // CTA issues: its instructions read both CTAs' stages and write both CTAs' accumulators.
+      const bool leader = elect_one();
+      const uint32_t idesc_full = umma_idesc_bf16(C::ROWS, GN, 0, 0);
+      const uint32_t idesc_half = umma_idesc_bf16(C::ROWS, GN / 2, 0, 0);   // pair: a last column tile of two blocks
+      const uint32_t sbase = smem_u32(stage_base);
+      uint32_t it = 0, lt = 0;
+      bool ok = true;
+      for (int tile = tile_lo; tile < tile_hi && ok; tile += tile_step, ++lt) {
+        const int buf = lt & 1;
+        if (!mbar_wait(&sl->acc_empty[buf], ((lt >> 1) & 1) ^ 1)) {
+          dev_set_error(p.status, SAF_DEV_TIMEOUT_MMA, 11);
           break;
         }
         tc_fence_after();
-        const uint32_t a = sbase + s * STAGE_BYTES;
-        const uint32_t b = a + A_BYTES;
-        if (leader) {
-          const uint64_t ad0 = umma_smem_desc_sw128(a, 16, 1024), bd0 = umma_smem_desc_sw128(b, 16, 1024);
-#pragma unroll
-          for (int k4 = 0; k4 < GK / 16; ++k4) {
-            const uint64_t ad = umma_desc_advance(ad0, k4 * 32), bd = umma_desc_advance(bd0, k4 * 32);
-            if constexpr (PAIR) umma_ss_pair(d, ad, bd, idesc, (kb | k4) != 0);
-            else umma_ss(d, ad, bd, idesc, (kb | k4) != 0);
+        const uint32_t d = tmem + buf * GN;
+        int tm_, tn_;
+        decode(tile, tm_, tn_);
+        const uint32_t idesc = (PAIR && (p.N - tn_ * GN) / 64 == 2) ? idesc_half : idesc_full;
+        for (int kb = 0; kb < KB; ++kb, ++it) {
+          const int s = it % STAGES;
+          if (!mbar_wait(&sl->full[s], (it / STAGES) & 1)) {
+            dev_set_error(p.status, SAF_DEV_TIMEOUT_MMA, 12);
+            ok = false;
+            break;
           }
-          if constexpr (PAIR) umma_commit_pair(&sl->empty[s]);      // frees the stage in both CTAs
-          else umma_commit(&sl->empty[s]);
+          tc_fence_after();
+          const uint32_t a = sbase + s * STAGE_BYTES;
+          const uint32_t b = a + A_BYTES;
+          if (leader) {
+            const uint64_t ad0 = umma_smem_desc_sw128(a, 16, 1024), bd0 = umma_smem_desc_sw128(b, 16, 1024);
+#pragma unroll
+            for (int k4 = 0; k4 < GK / 16; ++k4) {
+              const uint64_t ad = umma_desc_advance(ad0, k4 * 32), bd = umma_desc_advance(bd0, k4 * 32);
+              if constexpr (PAIR) umma_ss_pair(d, ad, bd, idesc, (kb | k4) != 0);
+              else umma_ss(d, ad, bd, idesc, (kb | k4) != 0);
+            }
+            if constexpr (PAIR) umma_commit_pair(&sl->empty[s]);      // frees the stage in both CTAs
+            else umma_commit(&sl->empty[s]);
+          }
+          __syncwarp();
+        }
+        if (ok && leader) {
+          if constexpr (PAIR) umma_commit_pair(&sl->acc_full[buf]);
+          else umma_commit(&sl->acc_full[buf]);
         }
         __syncwarp();
       }
-      if (ok && leader) {
-        if constexpr (PAIR) umma_commit_pair(&sl->acc_full[buf]);
-        else umma_commit(&sl->acc_full[buf]);
-      }
-      __syncwarp();
     }
-  } else if (warp >= 2) {
-    // epilogue warps 2..5 -> TMEM lane quadrant (warp % 4)
+  } else {
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(REGS_EPI));
+    // epilogue warps 4..11 -> TMEM lane quadrant (warp % 4); two groups of four warps take turns over the 64-column blocks
     pdl_wait();
-    const int quad = warp & 3;
+    const int quad = warp & 3, grp = (warp - 4) >> 2;
     const int row = quad * 32 + lane;           // row inside the tile
-    const int etid = tid - 64;                  // 0..127
+    const bool chief = (tid & 127) == 0;        // loads and stores its group's blocks
+    const bool swiglu = p.act == SAF_ACT_SWIGLU;
+    // a rotated 128-row slab is two blocks: group g rotates columns 32g .. 32g+31 of the first with those of the second,
+    // so that a thread needs 32 cos and 32 sin values of its row (held over the row's tiles), and both fill both blocks
+    const bool wide = p.slab == 128 && p.cosT;
+    const int bar_id = wide ? 3 : 1 + grp, bar_n = wide ? 256 : 128;
+    uint8_t* stg = out_stage + grp * (OUT_BYTES / 2);
     uint32_t lt = 0;
-    uint32_t n_out = 0;                         // output blocks stored so far (staging block = parity)
     int tm_held = -1;                           // row tile whose cos / sin values the registers hold
     float4 cs4[8], sn4[8];
-    for (int tile = tile_lo; tile < tile_hi; ++tile, ++lt) {
-      const int tm = tile / p.tiles_n, tn = tile - tm * p.tiles_n;
+    // the residual block of this group's first output block at or behind (tile, step), into its free staging block
+    uint32_t n_res = 0;
+    auto ask_residual = [&](int tile, int st) {
+      for (; tile < tile_hi; tile += tile_step, st = 0) {
+        int tm, tn;
+        decode(tile, tm, tn);
+        const int nsub = min(SUBS, (p.N - tn * GN) / 64), u = 2 * st + grp;
+        if (u >= nsub) continue;
+        mbar_expect_tx(&sl->res[grp], GM * 64 * 2);
+        tma_load_2d(stg, &mapR, &sl->res[grp], tn * GN + u * 64, tm * C::ROWS + rank * GM);
+        return;
+      }
+    };
+    if (p.residual_tma && chief) ask_residual(tile_lo, 0);
+    for (int tile = tile_lo; tile < tile_hi; tile += tile_step, ++lt) {
+      int tm, tn;
+      decode(tile, tm, tn);
       const int nsub = min(SUBS, (p.N - tn * GN) / 64);
       const int buf = lt & 1;
       const int m = tm * C::ROWS + rank * GM + row;
-      const int t = (p.T > 0) ? (m % p.T) : 0;
-      // head_dim 64: this row's 32 cos and 32 sin values, shared by every rotated block of the tile
-      if (p.slab == 64 && p.cosT && tm != tm_held) {
+      if (p.cosT && !p.halves && tm != tm_held) {
         tm_held = tm;
-        const float4* cr4 = reinterpret_cast<const float4*>(p.cosT + (int64_t)t * 64);
-        const float4* sr4 = reinterpret_cast<const float4*>(p.sinT + (int64_t)t * 64);
+        const int64_t at = (int64_t)(p.T > 0 ? m % p.T : 0) * p.slab + (wide ? grp * 32 : 0);   // (the tables repeat per half)
+        const float4* cr4 = reinterpret_cast<const float4*>(p.cosT + at);
+        const float4* sr4 = reinterpret_cast<const float4*>(p.sinT + at);
 #pragma unroll
         for (int j4 = 0; j4 < 8; ++j4) {
           cs4[j4] = cr4[j4];
           sn4[j4] = sr4[j4];
         }
       }
-      if (!mbar_wait(&sl->acc_full[buf], (lt >> 1) & 1)) {
-        dev_set_error(p.status, SAF_DEV_TIMEOUT_EPI, 13);
-        break;
-      }
-      tc_fence_after();
       const uint32_t tsrc = tmem + ((uint32_t)(quad * 32) << 16) + buf * GN;
-      const bool swiglu = p.act == SAF_ACT_SWIGLU;
-      for (int u = 0; u < nsub; ++u) {
-        // gated MLP: blocks come in (gate, up) pairs; the even block of a pair produces the 64 output columns
-        if (swiglu && (u & 1)) continue;
-        // the two staging blocks take turns over ALL stores of the CTA (a column tile may hold an odd number of
-        // output blocks: alternating by u alone would reuse the block whose store was issued last);
-        // the one whose turn it is is free once the store issued two output blocks ago has read it
-        const int ob = (n_out++) & 1;
-        if (etid == 0) tma_store_wait_read1();
-        named_bar_sync(1, 128);
+      // gated MLP: blocks come in (gate, up) pairs, a group takes a pair and produces 64 output columns
+      const int n_steps = swiglu ? (nsub + 3) / 4 : (nsub + 1) / 2;
+      for (int st = 0; st < n_steps; ++st) {
+        const int u = swiglu ? (2 * st + grp) * 2 : 2 * st + grp;
+        const bool mine = u < nsub;
+        const int out_col = swiglu ? (tn * GN + u * 64) / 2 : tn * GN + u * 64;
+        if (st == 0) {
+          if (!mbar_wait(&sl->acc_full[buf], (lt >> 1) & 1)) {
+            dev_set_error(p.status, SAF_DEV_TIMEOUT_EPI, 13);
+            if (p.residual_tma && mine) mbar_wait(&sl->res[grp], n_res & 1);   // its copy is on its way: let it land
+            tile = tile_hi;
+            break;
+          }
+          tc_fence_after();
+        }
         const int sb = tn * SUBS + u;
-        const int w = tb.weight[sb];
-        const int rp = tb.rope[sb];
-        // column offset of this 64-block inside its slab (slab = 64: 0; slab = 128: 0 or 64)
-        const int in_slab = (sb * 64) % p.slab;
+        const bool both = wide && tb.rope[sb];   // (a rotated 128-row slab never meets one-block tiles)
         float v[64];
-        {
+        if (mine) {
           uint32_t r0[32], r1[32];
-          tmem_ld32(tsrc + u * 64, r0);
-          tmem_ld32(tsrc + u * 64 + 32, r1);
+          tmem_ld32(tsrc + (both ? 2 * st * 64 + grp * 32 : u * 64), r0);
+          tmem_ld32(tsrc + (both ? (2 * st + 1) * 64 + grp * 32 : u * 64 + 32), r1);
           tmem_ld_wait();
 #pragma unroll
           for (int j = 0; j < 32; ++j) {
             v[j] = __uint_as_float(r0[j]);
             v[32 + j] = __uint_as_float(r1[j]);
           }
+          if (SUBS > 1 && swiglu) {   // v holds the gate block; the up block is the next 64 accumulator columns
+#pragma unroll
+            for (int c = 0; c < 64; c += 16) {
+              uint32_t q[16];
+              tmem_ld16(tsrc + (u + 1) * 64 + c, q);
+              tmem_ld_wait();
+#pragma unroll
+              for (int j = 0; j < 16; ++j) v[c + j] = silu_mul(v[c + j], __uint_as_float(q[j]));
+            }
+          }
         }
-        if (p.halves) {
-          const int wb = tb.weightb[sb];
-          if (p.bias[w]) {
-            const __nv_bfloat16* bp = reinterpret_cast<const __nv_bfloat16*>(p.bias[w]) + tb.row0[sb];
+        if (st == n_steps - 1) {   // the accumulator has been read: the MMA warp may overwrite it
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) {
+            if constexpr (PAIR) mbar_arrive_cluster(cluster_addr_of(&sl->acc_empty[buf], 0));   // the even CTA's MMA warp waits
+            else mbar_arrive(&sl->acc_empty[buf]);
+          }
+        }
+        if (!mine) continue;
+        {
+          // bias of the columns in v[0..31] and v[32..63]
+          const int sa = both ? tn * SUBS + 2 * st : sb;
+          const int wa = tb.weight[sa], wb = p.halves ? tb.weightb[sb] : wa;
+          const int ra = tb.row0[sa] + (both ? grp * 32 : 0);
+          const int rb = both ? tb.row0[sa + 1] + grp * 32 : (p.halves ? tb.row0b[sb] : ra + 32);
+          if (p.bias[wa]) {
+            const __nv_bfloat16* bp = reinterpret_cast<const __nv_bfloat16*>(p.bias[wa]) + ra;
 #pragma unroll
             for (int j = 0; j < 32; ++j) v[j] += __bfloat162float(bp[j]);
           }
           if (p.bias[wb]) {
-            const __nv_bfloat16* bp = reinterpret_cast<const __nv_bfloat16*>(p.bias[wb]) + tb.row0b[sb];
+            const __nv_bfloat16* bp = reinterpret_cast<const __nv_bfloat16*>(p.bias[wb]) + rb;
 #pragma unroll
             for (int j = 0; j < 32; ++j) v[32 + j] += __bfloat162float(bp[j]);
           }
-        } else if (p.bias[w]) {
-          const __nv_bfloat16* bp = reinterpret_cast<const __nv_bfloat16*>(p.bias[w]) + tb.row0[sb];
-#pragma unroll
-          for (int j = 0; j < 64; ++j) v[j] += __bfloat162float(bp[j]);
         }
         if (p.act == SAF_ACT_GELU) {
 #pragma unroll
           for (int j = 0; j < 64; ++j) v[j] = gelu_erf(v[j]);
         }
-        if (SUBS > 1 && swiglu) {   // v holds the gate block; the up block is the next 64 accumulator columns
-          uint32_t q0[32], q1[32];
-          tmem_ld32(tsrc + (u + 1) * 64, q0);
-          tmem_ld32(tsrc + (u + 1) * 64 + 32, q1);
-          tmem_ld_wait();
-#pragma unroll
-          for (int j = 0; j < 32; ++j) {
-            v[j] = silu_mul(v[j], __uint_as_float(q0[j]));
-            v[32 + j] = silu_mul(v[32 + j], __uint_as_float(q1[j]));
+        if (p.residual) {
+          if (p.residual_tma) {     // the block is in staging; this thread's row takes its sums back to the same place
+            if (!mbar_wait(&sl->res[grp], (n_res++) & 1)) dev_set_error(p.status, SAF_DEV_TIMEOUT_EPI, 14);
           }
-        }
-        const int out_col = swiglu ? (tn * GN + u * 64) / 2 : tn * GN + u * 64;
-        if (p.residual && m < p.M) {   // this row's 64 residual values: one 128-byte line
-          const uint4* rr = reinterpret_cast<const uint4*>(p.residual + (int64_t)m * p.ldr + out_col);
+          const __nv_bfloat16* rr = p.residual + (int64_t)m * p.ldr + tn * GN;
 #pragma unroll
-          for (int c8 = 0; c8 < 8; ++c8) {
-            const uint4 q = rr[c8];
+          for (int c = 0; c < 8; ++c) {
+            uint4 q = make_uint4(0, 0, 0, 0);
+            if (p.residual_tma) q = *reinterpret_cast<const uint4*>(stg + row * 128 + ((c ^ (row & 7)) << 4));
+            else if (m < p.M) q = *reinterpret_cast<const uint4*>(rr + (both ? (2 * st + (c >> 2)) * 64 + grp * 32 + (c & 3) * 8 : out_col - tn * GN + c * 8));
             const uint32_t w4[4] = {q.x, q.y, q.z, q.w};
 #pragma unroll
             for (int e = 0; e < 4; ++e) {
-              v[c8 * 8 + 2 * e] += __uint_as_float(w4[e] << 16);
-              v[c8 * 8 + 2 * e + 1] += __uint_as_float(w4[e] & 0xffff0000u);
+              v[c * 8 + 2 * e] += __uint_as_float(w4[e] << 16);
+              v[c * 8 + 2 * e + 1] += __uint_as_float(w4[e] & 0xffff0000u);
             }
           }
         }
-        if (rp) {   // warp-uniform: rows past M are rotated too (t stays a valid table row) and clipped by the store
-          const float* cr = p.cosT + (int64_t)t * p.slab;
-          const float* sr = p.sinT + (int64_t)t * p.slab;
-          if (p.slab == 64) {
-            // pairs (d, d+32) live in this block
-            // each thread reads its own table row: 16-byte loads (a row is 256 B, 16-byte aligned)
+        if (tb.rope[sb]) {   // pairs (d, d + slab/2) are v[j], v[32 + j].  Warp-uniform: rows past M are clipped by the store
 #pragma unroll
-            for (int j4 = 0; j4 < 8; ++j4) {
-              const float4 c4 = cs4[j4];
-              const float4 s4 = sn4[j4];
-              const float cc[4] = {c4.x, c4.y, c4.z, c4.w}, ss[4] = {s4.x, s4.y, s4.z, s4.w};
+          for (int j4 = 0; j4 < 8; ++j4) {
+            const float cc[4] = {cs4[j4].x, cs4[j4].y, cs4[j4].z, cs4[j4].w}, ss[4] = {sn4[j4].x, sn4[j4].y, sn4[j4].z, sn4[j4].w};
 #pragma unroll
-              for (int e = 0; e < 4; ++e) {
-                const int j = j4 * 4 + e;
-                const float x1 = v[j], x2 = v[32 + j];
-                v[j] = x1 * cc[e] - x2 * ss[e];
-                v[32 + j] = x2 * cc[e] + x1 * ss[e];
-              }
-            }
-          } else {
-            // slab 128: partner block is the other 64-column block of the same tile
-            const int pu = (u ^ 1) & (SUBS - 1);   // (a rotated 128-row slab never meets one-block tiles)
-            uint32_t q0[32], q1[32];
-            tmem_ld32(tsrc + pu * 64, q0);
-            tmem_ld32(tsrc + pu * 64 + 32, q1);
-            tmem_ld_wait();
-            const __nv_bfloat16* bp = p.bias[w] ? reinterpret_cast<const __nv_bfloat16*>(p.bias[w]) + tb.row0[tn * SUBS + pu] : nullptr;
-#pragma unroll
-            for (int j4 = 0; j4 < 16; ++j4) {
-              const float4 c4 = reinterpret_cast<const float4*>(cr + in_slab)[j4];
-              const float4 s4 = reinterpret_cast<const float4*>(sr + in_slab)[j4];
-              const float cc[4] = {c4.x, c4.y, c4.z, c4.w}, ss[4] = {s4.x, s4.y, s4.z, s4.w};
-#pragma unroll
-              for (int e = 0; e < 4; ++e) {
-                const int j = j4 * 4 + e;
-                float o = __uint_as_float(j < 32 ? q0[j] : q1[j - 32]);
-                if (bp) o += __bfloat162float(bp[j]);
-                // first half: x1*c - x2*s ; second half: x2*c + x1*s
-                v[j] = (in_slab == 0) ? (v[j] * cc[e] - o * ss[e]) : (v[j] * cc[e] + o * ss[e]);
-              }
+            for (int e = 0; e < 4; ++e) {
+              const int j = j4 * 4 + e;
+              const float x1 = v[j], x2 = v[32 + j];
+              v[j] = x1 * cc[e] - x2 * ss[e];
+              v[32 + j] = x2 * cc[e] + x1 * ss[e];
             }
           }
+        }
+        // a group has one staging block: its last store has read it by now, the accumulator's way to here hid the wait
+        if (!p.residual_tma) {
+          if (chief) tma_store_wait_read0();
+          named_bar_sync(bar_id, bar_n);
         }
         // bf16 pack -> swizzled staging: 16-byte chunk c of row r lands at chunk (c ^ (r & 7))
-        uint8_t* dst = out_stage + ob * (OUT_BYTES / 2) + row * 128;
 #pragma unroll
         for (int c = 0; c < 8; ++c) {
           uint4 q;
@@ -439,24 +475,23 @@ indexed_gemm_kernel(const __grid_constant__ CUtensorMap mapX, const __grid_const
           q.y = pack_bf16(v[c * 8 + 2], v[c * 8 + 3]);
           q.z = pack_bf16(v[c * 8 + 4], v[c * 8 + 5]);
           q.w = pack_bf16(v[c * 8 + 6], v[c * 8 + 7]);
-          *reinterpret_cast<uint4*>(dst + ((c ^ (row & 7)) << 4)) = q;
+          uint8_t* dst = (both ? out_stage + (c >> 2) * (OUT_BYTES / 2) : stg) + row * 128;
+          const int ch = both ? grp * 4 + (c & 3) : c;
+          *reinterpret_cast<uint4*>(dst + ((ch ^ (row & 7)) << 4)) = q;
         }
         fence_proxy_async_smem();
-        named_bar_sync(1, 128);
-        if (etid == 0) {
-          tma_store_2d(&mapO, out_stage + ob * (OUT_BYTES / 2), out_col, tm * C::ROWS + rank * GM);
+        named_bar_sync(bar_id, bar_n);
+        if (chief) {
+          tma_store_2d(&mapO, stg, out_col, tm * C::ROWS + rank * GM);
           tma_store_commit();
+          if (p.residual_tma) {
+            tma_store_wait_read0();
+            ask_residual(tile, st + 1);
+          }
         }
       }
-      // accumulator buffer can be overwritten by the MMA warp
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) {
-        if constexpr (PAIR) mbar_arrive_cluster(cluster_addr_of(&sl->acc_empty[buf], 0));   // the even CTA's MMA warp waits
-        else mbar_arrive(&sl->acc_empty[buf]);
-      }
     }
-    if (etid == 0) tma_store_wait_all();
+    if (chief) tma_store_wait_all();
   }
   tc_fence_before();
   __syncthreads();
@@ -468,10 +503,18 @@ indexed_gemm_kernel(const __grid_constant__ CUtensorMap mapX, const __grid_const
   }
 }
 
+// Column tiles whose weights are walked together: groups of equal width of at most 32 MB, a quarter of the L2 (its two
+// halves may hold a line each).
+int columns_together(int tiles_n, int tile_cols, int K) {
+  const int64_t bytes = (int64_t)tiles_n * tile_cols * K * 2;
+  const int groups = (int)std::min<int64_t>(tiles_n, (bytes + (32 << 20) - 1) / (32 << 20));
+  return (tiles_n + groups - 1) / groups;
+}
+
 bool aligned16(const void* p) { return ((uintptr_t)p & 15) == 0; }
 
 template <int SUBS>
-int launch_single(const CUtensorMap& mx, const CUtensorMap* mw, const CUtensorMap& mo, GemmParams p, const SubTable& tb,
+int launch_single(const CUtensorMap& mx, const CUtensorMap* mw, const CUtensorMap& mo, const CUtensorMap& mr, GemmParams p, const SubTable& tb,
                   cudaStream_t st) {
   using C = GCfg<false, SUBS>;
   constexpr size_t smem = 1024 + C::STAGES * C::STAGE_BYTES + OUT_BYTES + sizeof(SmemLayout);
@@ -479,9 +522,10 @@ int launch_single(const CUtensorMap& mx, const CUtensorMap* mw, const CUtensorMa
   static PerDeviceOnce smem_once;
   if (int rc = ensure_dyn_smem(indexed_gemm_kernel<false, SUBS>, (int)smem, smem_once)) return rc;
   p.tiles_n = (p.N + C::GN - 1) / C::GN;
+  p.group_n = columns_together(p.tiles_n, C::GN, p.K);
   const int grid = std::min(device_sm_count(), p.tiles_m * p.tiles_n);
   return launch_pdl("indexed_gemm_kernel", indexed_gemm_kernel<false, SUBS>, dim3(grid), GEMM_THREADS, smem, st, 1, mx, mw[0], mw[1],
-                    mw[2], mw[3], mo, p, tb);
+                    mw[2], mw[3], mo, mr, p, tb);
 }
 
 }  // namespace
@@ -510,7 +554,7 @@ int launch_gemm_sm100(const SafIndexedLinearArgs& a, cudaStream_t st, int32_t* z
   }
   if (!saf_device_supported()) return SAF_ERR_UNSUPPORTED;
 
-  CUtensorMap mx, mw[4], mo;
+  CUtensorMap mx, mw[4], mo, mr;
   int rc;
   {
     uint64_t dims[2] = {(uint64_t)a.C, (uint64_t)a.M};
@@ -531,6 +575,14 @@ int launch_gemm_sm100(const SafIndexedLinearArgs& a, cudaStream_t st, int32_t* z
     uint64_t strides[2] = {0, (uint64_t)a.ldo * 2};
     uint32_t box[2] = {64, GM};
     if ((rc = make_tensor_map_bf16(&mo, a.out, 2, dims, strides, box, false))) return rc;
+  }
+  const bool residual_tma = a.residual && !a.rope_cos && a.act != SAF_ACT_SWIGLU;
+  mr = mo;
+  if (residual_tma) {
+    uint64_t dims[2] = {(uint64_t)N, (uint64_t)a.M};
+    uint64_t strides[2] = {0, (uint64_t)a.ldr * 2};
+    uint32_t box[2] = {64, GM};
+    if ((rc = make_tensor_map_bf16(&mr, a.residual, 2, dims, strides, box, false))) return rc;
   }
   SubTable tb;
   memset(&tb, 0, sizeof(tb));
@@ -567,6 +619,8 @@ int launch_gemm_sm100(const SafIndexedLinearArgs& a, cudaStream_t st, int32_t* z
   p.act = a.act;
   p.residual = reinterpret_cast<const __nv_bfloat16*>(a.residual);
   p.ldr = a.ldr;
+  p.residual_tma = residual_tma ? 1 : 0;
+  p.runs = a.rope_cos && !halves ? 1 : 0;
   p.halves = halves ? 1 : 0;
   p.zero2 = zero2;
   p.weights_early = weights_early ? 1 : 0;
@@ -584,6 +638,7 @@ int launch_gemm_sm100(const SafIndexedLinearArgs& a, cudaStream_t st, int32_t* z
     if ((rc = ensure_dyn_smem(kernel, (int)smem_p, smem_once_p))) return rc;
     p.tiles_m = (a.M + C::ROWS - 1) / C::ROWS;
     p.tiles_n = (N + C::GN - 1) / C::GN;
+    p.group_n = columns_together(p.tiles_n, C::GN, p.K);
     // pairs that can be resident at once (an SM without a free neighbour in its GPC stays out)
     static std::atomic<int> pairs_cache[SAF_MAX_DEVICES];
     const int dev = current_device();
@@ -612,15 +667,15 @@ int launch_gemm_sm100(const SafIndexedLinearArgs& a, cudaStream_t st, int32_t* z
     }
     pairs = std::min(pairs, p.tiles_m * p.tiles_n);
     if ((rc = launch_pdl("indexed_gemm_kernel<pair>", kernel, dim3(2 * pairs), GEMM_THREADS, smem_p, st, 2, mx, mw[0], mw[1], mw[2], mw[3],
-                         mo, p, tb)))
+                         mo, mr, p, tb)))
       return rc;
   } else {
     const bool together = a.act == SAF_ACT_SWIGLU || (!halves && a.slab == 128 && a.slab_rope);
     p.tiles_m = (a.M + GM - 1) / GM;
     switch (pick_subs(p.tiles_m, N, (a.C + GK - 1) / GK, together ? 2 : 1)) {
-      case 1: rc = launch_single<1>(mx, mw, mo, p, tb, st); break;
-      case 2: rc = launch_single<2>(mx, mw, mo, p, tb, st); break;
-      default: rc = launch_single<4>(mx, mw, mo, p, tb, st); break;
+      case 1: rc = launch_single<1>(mx, mw, mo, mr, p, tb, st); break;
+      case 2: rc = launch_single<2>(mx, mw, mo, mr, p, tb, st); break;
+      default: rc = launch_single<4>(mx, mw, mo, mr, p, tb, st); break;
     }
     if (rc) return rc;
   }

@@ -113,6 +113,10 @@ __device__ __forceinline__ void fence_proxy_async_smem() {
 // ---------------------------------------------------------------------------
 // TMA (cp.async.bulk.tensor), loads complete on an mbarrier, stores use bulk groups
 // ---------------------------------------------------------------------------
+// a tile on its way into L2
+__device__ __forceinline__ void tma_prefetch_2d(const CUtensorMap* m, int x, int y) {
+  asm volatile("cp.async.bulk.prefetch.tensor.2d.L2.global.tile [%0, {%1, %2}];" ::"l"(m), "r"(x), "r"(y) : "memory");
+}
 __device__ __forceinline__ void tma_prefetch_desc(const CUtensorMap* m) {
   asm volatile("prefetch.tensormap [%0];" ::"l"(m) : "memory");
 }
@@ -150,6 +154,7 @@ __device__ __forceinline__ void tma_store_4d(const CUtensorMap* m, const void* s
 }
 __device__ __forceinline__ void tma_store_commit() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
 __device__ __forceinline__ void tma_store_wait_all() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
+__device__ __forceinline__ void tma_store_wait_read0() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); }
 __device__ __forceinline__ void tma_store_wait_read1() {   // at most one store group still reading smem
   asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
 }
