@@ -17,7 +17,7 @@
 //               once per row of tiles, before the accumulator is waited for, so their latency hides behind the MMAs.
 //               With K = 768 a tile's products take 6144 cycles; one group of four warps needed longer than that for
 //               a GELU or (by far) a rotation of 128-row slabs, whose 64 cos and 64 sin values it had to read anew for
-//               every tile: 65536 x 1536 -> 1664, 128-row slabs, 692 -> 453 us; 65536 x 768 -> 1920, 64-row, 209 -> 180.
+//               every tile: 65536 x 1536 -> 1664, 128-row slabs, 692 -> 322 us; 65536 x 768 -> 1920, 64-row, 209 -> 190.
 //               A residual comes by TMA into the block's own staging place, fetched into L2 while the products run:
 //               65536 x 768 -> 768 with residual 125 -> 90 us (row by row from global memory before).
 // Large products run the same kernel as CTA PAIRS (template parameter PAIR, a cluster of two): one 256x256 tile per
@@ -352,14 +352,32 @@ indexed_gemm_kernel(const __grid_constant__ CUtensorMap mapX, const __grid_const
       const int m = tm * C::ROWS + rank * GM + row;
       if (p.cosT && !p.halves && tm != tm_held) {
         tm_held = tm;
-        const int64_t at = (int64_t)(p.T > 0 ? m % p.T : 0) * p.slab + (wide ? grp * 32 : 0);   // (the tables repeat per half)
-        const float4* cr4 = reinterpret_cast<const float4*>(p.cosT + at);
-        const float4* sr4 = reinterpret_cast<const float4*>(p.sinT + at);
+        // 32 values of 128 table rows (the tables repeat per half), whole 128-byte pieces of 4 rows per load, handed to
+        // the threads of the rows through the group's staging block.  (A thread reading its own row touched 32 lines per
+        // load: 8192 cycles of the load path for the two groups, more than the products of a narrow tile.)
+        const int l = tid & 127;
 #pragma unroll
-        for (int j4 = 0; j4 < 8; ++j4) {
-          cs4[j4] = cr4[j4];
-          sn4[j4] = sr4[j4];
+        for (int q = 0; q < 8; ++q) {
+          const int mr = tm * C::ROWS + rank * GM + (l >> 3) + 16 * q;
+          const int64_t at = (int64_t)(p.T > 0 ? mr % p.T : 0) * p.slab + (wide ? grp * 32 : 0) + (l & 7) * 4;
+          cs4[q] = *reinterpret_cast<const float4*>(p.cosT + at);
+          sn4[q] = *reinterpret_cast<const float4*>(p.sinT + at);
         }
+        if (chief) tma_store_wait_read0();
+        named_bar_sync(1 + grp, 128);
+        auto own_row = [&](float4 (&x)[8]) {
+#pragma unroll
+          for (int q = 0; q < 8; ++q) {
+            const int r = (l >> 3) + 16 * q;
+            *reinterpret_cast<float4*>(stg + r * 128 + (((l & 7) ^ (r & 7)) << 4)) = x[q];
+          }
+          named_bar_sync(1 + grp, 128);
+#pragma unroll
+          for (int c = 0; c < 8; ++c) x[c] = *reinterpret_cast<const float4*>(stg + row * 128 + ((c ^ (row & 7)) << 4));
+          named_bar_sync(1 + grp, 128);
+        };
+        own_row(cs4);
+        own_row(sn4);
       }
       const uint32_t tsrc = tmem + ((uint32_t)(quad * 32) << 16) + buf * GN;
       // gated MLP: blocks come in (gate, up) pairs, a group takes a pair and produces 64 output columns
