@@ -114,6 +114,8 @@ indexed_gemm_bwd_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_c
   if (warp == 0) {
     if (lane == 0) {
       tma_prefetch_desc(&mapA);
+      pdl_wait();
+      pdl_trigger();
       uint32_t it = 0;
       bool ok = true;
       for (int tile = blockIdx.x; tile < total_tiles && ok; tile += gridDim.x) {
@@ -189,6 +191,7 @@ indexed_gemm_bwd_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_c
       __syncwarp();
     }
   } else {
+    pdl_wait();
     const int quad = warp & 3;
     const int row = quad * 32 + lane;
     const int etid = tid - 64;
@@ -347,9 +350,8 @@ int launch_mode(const CUtensorMap& ma, const CUtensorMap& mb, const CUtensorMap*
   static PerDeviceOnce smem_once;
   if (int rc = ensure_dyn_smem(indexed_gemm_bwd_kernel<MODE, F32OUT>, (int)smem, smem_once)) return rc;
   const int grid = std::min(sm_count, p.tiles_m * p.tiles_n * std::max(1, p.splits));
-  indexed_gemm_bwd_kernel<MODE, F32OUT><<<grid, BGEMM_THREADS, smem, st>>>(ma, mb, mw[0], mw[1], mw[2], mw[3], mo, p, tb);
-  count_launch();
-  return check_launch(MODE == MODE_DX ? "indexed_gemm_bwd_kernel<dx>" : "indexed_gemm_bwd_kernel<dw>");
+  return launch_pdl(MODE == MODE_DX ? "indexed_gemm_bwd_kernel<dx>" : "indexed_gemm_bwd_kernel<dw>", indexed_gemm_bwd_kernel<MODE, F32OUT>,
+                    dim3(grid), BGEMM_THREADS, smem, st, 1, ma, mb, mw[0], mw[1], mw[2], mw[3], mo, p, tb);
 }
 
 }  // namespace
@@ -430,6 +432,8 @@ struct FinishParams {
 // column per thread and row, consecutive threads along the row.
 __global__ void __launch_bounds__(FIN_THREADS) dw_finish_kernel(const __grid_constant__ FinishParams p,
                                                                 const __grid_constant__ FinishTable tb) {
+  pdl_wait();
+  pdl_trigger();
   const int run = blockIdx.y;
   int w = 0;
   while (w + 1 < p.n && run >= p.run0[w + 1]) ++w;
@@ -535,9 +539,7 @@ int launch_gemm_bwd_dw_full_sm100(const SafIndexedLinearArgs& a, const void* dou
   fp.f32 = f32_out ? 1 : 0;
   const int per_run = (32 * fp.C4 + FIN_THREADS - 1) / FIN_THREADS;
   const dim3 grid((unsigned)std::min(per_run, std::max(1, 8 * device_sm_count() / runs)), (unsigned)runs);
-  dw_finish_kernel<<<grid, FIN_THREADS, 0, st>>>(fp, ft);
-  count_launch();
-  return check_launch("dw_finish_kernel");
+  return launch_pdl("dw_finish_kernel", dw_finish_kernel, grid, FIN_THREADS, 0, st, 1, fp, ft);
 }
 
 }  // namespace saf

@@ -372,6 +372,8 @@ __global__ void __launch_bounds__(256) rope_slabs_vec_kernel(__nv_bfloat16* __re
                                                              int slab, int Tlen, const float* __restrict__ cosT,
                                                              const float* __restrict__ sinT,
                                                              const __grid_constant__ SlabTable tb, float sgn) {
+  pdl_wait();
+  pdl_trigger();
   const int half = slab >> 1, per_slab = half >> 3;
   const int64_t total = (int64_t)M * n_slabs * per_slab;
   for (int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; idx < total; idx += (int64_t)gridDim.x * blockDim.x) {
@@ -546,7 +548,8 @@ int launch_rope_slabs(void* x, int64_t ld, int M, int n_slabs, int slab, int T, 
   if (vec) {
     const int64_t tv = (int64_t)M * n_slabs * (slab / 16);
     const int bv = (int)std::min<int64_t>((tv + 255) / 256, 148 * 32);
-    rope_slabs_vec_kernel<<<bv, 256, 0, st>>>(reinterpret_cast<__nv_bfloat16*>(x), ld, M, n_slabs, slab, T, cosT, sinT, tb, sgn);
+    return launch_pdl("rope_slabs_kernel", rope_slabs_vec_kernel, dim3(bv), 256, 0, st, 1, reinterpret_cast<__nv_bfloat16*>(x), ld, M,
+                      n_slabs, slab, T, cosT, sinT, tb, sgn);
   } else if (dtype == SAF_F32)
     rope_slabs_kernel<float><<<blocks, 256, 0, st>>>(reinterpret_cast<float*>(x), ld, M, n_slabs, slab, T, cosT, sinT, tb, sgn);
   else
