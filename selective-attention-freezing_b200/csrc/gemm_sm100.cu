@@ -40,7 +40,7 @@ constexpr int MAX_STAGES = 8;
 // and HALF of the weight tile (two 64-row blocks), so the operand traffic per SM drops from 96 to 64 bytes per clock at
 // the full MMA rate -- what one SM can pull from L2 -- and a stage shrinks to 32 KB (6 stages instead of 4).
 // SUBS: 64-column blocks of a tile.  4 (128x256 tiles, 96 B/clk of operand traffic per SM at the full MMA rate) is the form
-// for products with tiles to spare; 2 and 1 cut a small product into enough tiles to occupy the SMs (pick_subs).
+// for products with tiles to spare; 2 and 1 cut a small product into enough tiles to occupy the SMs (pick_form).
 template <bool PAIR, int SUBS>
 struct GCfg {
   static constexpr int GN = SUBS * 64;                                 // columns of a tile
@@ -83,24 +83,31 @@ struct GemmParams {
   int32_t* zero2;                // two ints this launch clears for the next one on the stream (a tile queue), or null
 };
 
-// Width of a single-CTA tile, in 64-column blocks.  With few rows the 256-column tiles leave most SMs idle (777 rows of
-// a 12 x 64 layer: 21 to 84 tiles on 148 SMs, 18 us a product), so the narrower form that finishes first is taken: waves
-// of tiles, each KB K steps at the pace of its MMA (256 columns 128 cycles, 128: 64, 64: 48, bound by the A operand's
-// shared-memory reads; four per step) plus its blocks' way out.  `least`: blocks that belong together (a 128-row
-// rotated slab, a gate/up pair).
-int pick_subs(int tiles_m, int N, int KB, int least) {
+// Form of a product: 64-column blocks of a single-CTA tile (1, 2, 4), or PAIR_FORM for 256 x 256 tiles of CTA pairs.
+// A form takes fixed + waves x K steps x step: the fixed part is launch, first loads and the last tile's way out, a step is
+// bound by the operands from L2 (24 / 32 / 48 KB an SM per step of a 1-, 2-, 4-block tile, 32 KB for a pair's 256 x 256).
+// Fitted to each form's times over 128 to 8192 rows, K 256 to 3072, N 256 to 17920 on a B200, where the form it takes
+// is within 8 % of the best one.  In us, pair / 4 / 2 / 1 blocks: 777 x 768 -> 3072 10.4 / 11.0 / 12.1 / 13.3, 777 x 3072
+// -> 768 21.4 / 27.1 / 19.7 / 15.8, 777 x 2048 -> 5120 28.4 / 21.4 / 27.7 / 38.1, 3001 x 768 -> 768 9.7 / 11.0 / 8.7 /
+// 10.2, 3001 x 1536 -> 3840 33.0 / 42.1 / 49.0 / 69.3, 8192 x 2048 -> 5120 122 / 150 / 211 / 301.
+// `least`: blocks that belong together (a 128-row rotated slab, a gate/up pair).
+constexpr int PAIR_FORM = 8;
+int pick_form(int M, int N, int KB, int least, int pairs) {
   const int sms = device_sm_count();
+  const int rows = (M + GM - 1) / GM, pair_rows = (M + 2 * GM - 1) / (2 * GM);
   int best = 4;
   double best_t = 1e30;
-  for (int subs = 4; subs >= least; subs >>= 1) {
-    const int tiles = tiles_m * ((N / 64 + subs - 1) / subs);
-    const double step = subs == 4 ? 512.0 : (subs == 2 ? 256.0 : 192.0);
-    const double t = (double)((tiles + sms - 1) / sms) * KB * step + 1200.0 * subs;
+  auto consider = [&](int form, int64_t tiles, int units, double fixed, double step) {
+    const double t = fixed + (double)((tiles + units - 1) / units) * KB * step;
     if (t < best_t) {
       best_t = t;
-      best = subs;
+      best = form;
     }
-  }
+  };
+  if (N >= 256 && pairs > 0) consider(PAIR_FORM, (int64_t)pair_rows * ((N + 255) / 256), pairs, 4.9, 0.40);
+  consider(4, (int64_t)rows * ((N + 255) / 256), sms, 4.9, 0.53);
+  if (least <= 2) consider(2, (int64_t)rows * ((N + 127) / 128), sms, 3.6, 0.38);
+  if (least <= 1) consider(1, (int64_t)rows * (N / 64), sms, 3.1, 0.27);
   return best;
 }
 
@@ -531,6 +538,44 @@ int columns_together(int tiles_n, int tile_cols, int K) {
 
 bool aligned16(const void* p) { return ((uintptr_t)p & 15) == 0; }
 
+constexpr size_t PAIR_SMEM = 1024 + GCfg<true, 4>::STAGES * GCfg<true, 4>::STAGE_BYTES + OUT_BYTES + sizeof(SmemLayout);
+static_assert(PAIR_SMEM <= 227 * 1024, "pair kernel shared memory");
+
+// CTA pairs that can be resident at once (an SM without a free neighbour in its GPC stays out), after the pair kernel
+// has its shared memory
+int resident_pairs(cudaStream_t st, int* out) {
+  auto kernel = indexed_gemm_kernel<true, 4>;
+  static PerDeviceOnce smem_once;
+  if (int rc = ensure_dyn_smem(kernel, (int)PAIR_SMEM, smem_once)) return rc;
+  static std::atomic<int> cache[SAF_MAX_DEVICES];
+  const int dev = current_device();
+  int pairs = (dev >= 0 && dev < SAF_MAX_DEVICES) ? cache[dev].load(std::memory_order_acquire) : 0;
+  if (pairs <= 0) {
+    cudaLaunchConfig_t cfg;
+    memset(&cfg, 0, sizeof(cfg));
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = 2;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    cfg.blockDim = dim3(GEMM_THREADS);
+    cfg.dynamicSmemBytes = PAIR_SMEM;
+    cfg.stream = st;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    cfg.gridDim = dim3(device_sm_count() & ~1);
+    int n = 0;
+    if (cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) != cudaSuccess || n <= 0) {
+      cudaGetLastError();
+      n = device_sm_count() / 2;
+    }
+    pairs = n;
+    if (dev >= 0 && dev < SAF_MAX_DEVICES) cache[dev].store(pairs, std::memory_order_release);
+  }
+  *out = pairs;
+  return SAF_OK;
+}
+
 template <int SUBS>
 int launch_single(const CUtensorMap& mx, const CUtensorMap* mw, const CUtensorMap& mo, const CUtensorMap& mr, GemmParams p, const SubTable& tb,
                   cudaStream_t st) {
@@ -643,54 +688,24 @@ int launch_gemm_sm100(const SafIndexedLinearArgs& a, cudaStream_t st, int32_t* z
   p.zero2 = zero2;
   p.weights_early = weights_early ? 1 : 0;
 
-  const int sm_count = device_sm_count();
-  // CTA pairs on 256-row tiles when the product is large enough to fill the machine with them
+  const bool together = a.act == SAF_ACT_SWIGLU || (!halves && a.slab == 128 && a.slab_rope);
   const char* pair_env = getenv("SAF_B200_GEMM_PAIR");
   const bool pair_off = pair_env && pair_env[0] == '0' && pair_env[1] == 0;
-  if (!pair_off && a.M >= 2 * GM * 32 && N >= 256) {
+  int pairs = 0;
+  if (!pair_off && N >= 256 && (rc = resident_pairs(st, &pairs))) return rc;
+  const int form = pick_form(a.M, N, (a.C + GK - 1) / GK, together ? 2 : 1, pairs);
+  if (form == PAIR_FORM) {
     using C = GCfg<true, 4>;
-    constexpr size_t smem_p = 1024 + C::STAGES * C::STAGE_BYTES + OUT_BYTES + sizeof(SmemLayout);
-    static_assert(smem_p <= 227 * 1024, "pair kernel shared memory");
-    auto kernel = indexed_gemm_kernel<true, 4>;
-    static PerDeviceOnce smem_once_p;
-    if ((rc = ensure_dyn_smem(kernel, (int)smem_p, smem_once_p))) return rc;
     p.tiles_m = (a.M + C::ROWS - 1) / C::ROWS;
     p.tiles_n = (N + C::GN - 1) / C::GN;
     p.group_n = columns_together(p.tiles_n, C::GN, p.K);
-    // pairs that can be resident at once (an SM without a free neighbour in its GPC stays out)
-    static std::atomic<int> pairs_cache[SAF_MAX_DEVICES];
-    const int dev = current_device();
-    int pairs = (dev >= 0 && dev < SAF_MAX_DEVICES) ? pairs_cache[dev].load(std::memory_order_acquire) : 0;
-    if (pairs <= 0) {
-      cudaLaunchConfig_t cfg;
-      memset(&cfg, 0, sizeof(cfg));
-      cudaLaunchAttribute attr[1];
-      attr[0].id = cudaLaunchAttributeClusterDimension;
-      attr[0].val.clusterDim.x = 2;
-      attr[0].val.clusterDim.y = 1;
-      attr[0].val.clusterDim.z = 1;
-      cfg.blockDim = dim3(GEMM_THREADS);
-      cfg.dynamicSmemBytes = smem_p;
-      cfg.stream = st;
-      cfg.attrs = attr;
-      cfg.numAttrs = 1;
-      cfg.gridDim = dim3(sm_count & ~1);
-      int n = 0;
-      if (cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) != cudaSuccess || n <= 0) {
-        cudaGetLastError();
-        n = sm_count / 2;
-      }
-      pairs = n;
-      if (dev >= 0 && dev < SAF_MAX_DEVICES) pairs_cache[dev].store(pairs, std::memory_order_release);
-    }
     pairs = std::min(pairs, p.tiles_m * p.tiles_n);
-    if ((rc = launch_pdl("indexed_gemm_kernel<pair>", kernel, dim3(2 * pairs), GEMM_THREADS, smem_p, st, 2, mx, mw[0], mw[1], mw[2], mw[3],
+    if ((rc = launch_pdl("indexed_gemm_kernel<pair>", indexed_gemm_kernel<true, 4>, dim3(2 * pairs), GEMM_THREADS, PAIR_SMEM, st, 2, mx, mw[0], mw[1], mw[2], mw[3],
                          mo, mr, p, tb)))
       return rc;
   } else {
-    const bool together = a.act == SAF_ACT_SWIGLU || (!halves && a.slab == 128 && a.slab_rope);
     p.tiles_m = (a.M + GM - 1) / GM;
-    switch (pick_subs(p.tiles_m, N, (a.C + GK - 1) / GK, together ? 2 : 1)) {
+    switch (form) {
       case 1: rc = launch_single<1>(mx, mw, mo, mr, p, tb, st); break;
       case 2: rc = launch_single<2>(mx, mw, mo, mr, p, tb, st); break;
       default: rc = launch_single<4>(mx, mw, mo, mr, p, tb, st); break;

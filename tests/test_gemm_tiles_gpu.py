@@ -15,7 +15,7 @@ def rel(a, r):
     return ((a.double() - r.double()).norm() / r.double().norm()).item()
 
 
-@pytest.mark.parametrize("M", [1, 300, 8193, 8500])
+@pytest.mark.parametrize("M", [1, 300, 1500, 3001, 8193, 8500])
 @pytest.mark.parametrize("K,N", [(4096, 4608), (192, 192), (64, 832), (8192, 2240)])
 @pytest.mark.parametrize("residual", [False, True])
 def test_linear_tiles(M, K, N, residual):
