@@ -263,6 +263,11 @@ class SafCausalSelfAttention(nn.Module):
         super()._load_from_state_dict(state_dict, prefix, *args, **kwargs)
         self._fz_dirty = True
 
+    def __setstate__(self, state):
+        super().__setstate__(state)
+        if "_plan" not in state:              # a module saved before the cache held a layer plan
+            self._fz_dirty = True
+
     def _refresh_freeze_cache(self):
         """Per-freeze-set caches; the only place with host syncs (nanogpt/model.py:846-898)."""
         frozen = self.dyn_frozen

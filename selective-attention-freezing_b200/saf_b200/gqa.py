@@ -85,6 +85,11 @@ class SafGqaAttention(nn.Module):
         self._plan = None
         self._rope_key = None
 
+    def __setstate__(self, state):
+        super().__setstate__(state)
+        if "_states" not in state:            # a module saved before it kept its head states and plan
+            self._states, self._plan = self.frozen_mask_i32.tolist(), None
+
     # ---- freeze state -----------------------------------------------------------------------
     def set_frozen(self, dense=(), patterns=None, decomposed=(), decomp=None, sink_decay=(), sd_params=None):
         """Install the frozen heads of this layer.  dense: heads frozen on stored (T, T) patterns, `patterns`

@@ -18,9 +18,11 @@ MAX_BLOCKS = 160          # 64-row blocks of one backward product
 
 
 class LayerPlan:
-    """What a freeze set fixes on the host: head states and slots, and the argument struct with them filled in."""
+    """What a freeze set fixes on the host: head states and slots, and the argument struct with them filled in.  The
+    struct points into this plan's own arrays, so a copied or unpickled plan is built anew from what made it."""
 
     def __init__(self, states, live, head_dim, width, n_kv=0):
+        self._made_of = (list(states), list(live), head_dim, width, n_kv)
         H, U = len(states), len(live)
         self.H, self.U, self.hd, self.C, self.n_kv = H, U, head_dim, width, n_kv
         self._states = (C.c_int32 * H)(*states)
@@ -36,6 +38,9 @@ class LayerPlan:
         t.frozen_host = self._states
         self._template = bytes(a)
         self._sizes = {}
+
+    def __reduce__(self):
+        return LayerPlan, self._made_of
 
     def width(self):
         return (self.U + 2 * self.n_kv if self.n_kv else 2 * self.U + self.H) * self.hd
