@@ -406,6 +406,7 @@ class SafCausalSelfAttention(nn.Module):
         if call is not None:
             if torch.is_grad_enabled() and residual is not None:
                 return residual + _layer.attention_layer(self._plan, x, **call)
+            residual = None if residual is None else residual.to(torch.bfloat16)
             return _layer.attention_layer(self._plan, x, residual=residual, **call)
         rp = self._rope_f32(rope, T, x.device)
         dec = (self.dyn_alpha, self.dyn_rho, self.dyn_z) if self._dec_any else (None, None, None)

@@ -231,18 +231,28 @@ def _bf16_rows(x):
     return x2.contiguous() if x2.stride(0) % 8 or x2.data_ptr() % 16 else x2
 
 
+def _residual_rows(residual, tokens, width):
+    """`residual` as the output projection reads it; its map covers tokens x width whatever the tensor holds."""
+    r2 = ops._as_2d(residual)
+    if r2.shape != (tokens, width) or r2.dtype != torch.bfloat16:
+        raise ValueError("residual must match the output")
+    return _bf16_rows(r2)
+
+
 def attention_layer(plan, x, weights, rope, frozen, hidx, *, kvidx=None, sink_decay=None, patt=None, pidx=None,
                     decomposed=(None, None, None), learn=None, biases=None, residual=None, measure=None):
     """x (B, T, C) -> bf16 (B, T, C).  weights: q, k, v, o; decomposed: (alpha, rho, z) buffers; learn: (alpha, rho)
     parameters that receive gradients (decomposed then holds their detached values and current normalisers);
     measure: called with the rotated q, k of the live heads.  Biases and residual go with inference."""
     grad = torch.is_grad_enabled() and (x.requires_grad or learn is not None or any(w.requires_grad for w in weights))
+    if residual is not None:
+        residual = _residual_rows(residual, x.shape[0] * x.shape[1], plan.C)
     c = _Call(x.shape[0], x.shape[1], _rows(x.detach()), weights, int(grad), rope, frozen, hidx, kvidx, sink_decay, patt, pidx,
               decomposed)
     if grad:
         ap, rp = learn if learn is not None else (None, None)
         return _LayerFunction.apply(x, *weights, ap, rp, plan, c, measure)
-    out, work, sz = _forward(plan, c, biases, None if residual is None else _bf16_rows(residual))
+    out, work, sz = _forward(plan, c, biases, residual)
     if measure is not None:
         q, k, _, _ = projection_views(plan, work, sz, c.B, c.T)
         measure(q, k)
