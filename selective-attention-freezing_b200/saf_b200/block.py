@@ -81,6 +81,6 @@ class SafBlock(nn.Module):
             return None
         n1, n2 = (self.ln_1.weight, self.ln_1.bias), (self.ln_2.weight, self.ln_2.bias)
         w = (mlp.c_fc.weight, None, mlp.c_fc.bias, mlp.c_proj.weight, mlp.c_proj.bias)
-        if not _layer.block_usable(m._plan, x, (*call["weights"], *n1, *n2, *w), w[0].shape[0], False):
+        if not _layer.block_usable(m._plan, x, call, n1, n2, w, False):
             return None
         return _layer.block(m._plan, x, call, n1, n2, w, 1e-5)

@@ -239,10 +239,9 @@ class SafQwenBlock(nn.Module):
             if call is not None:
                 n1, n2 = self.input_layernorm, self.post_attention_layernorm
                 w = (mlp.gate_proj.weight, mlp.up_proj.weight, None, mlp.down_proj.weight, None)
-                used = (*call["weights"], *call.get("biases", ()), n1.weight, n2.weight, *w)
-                if n1.variance_epsilon == n2.variance_epsilon and _layer.block_usable(m._plan, x, used, w[0].shape[0], True):
-                    return _layer.block(m._plan, x, call, (n1.weight, None), (n2.weight, None), w, n1.variance_epsilon,
-                                        rms=True, gated=True)
+                norms = (n1.weight, None), (n2.weight, None)
+                if n1.variance_epsilon == n2.variance_epsilon and _layer.block_usable(m._plan, x, call, *norms, w, True):
+                    return _layer.block(m._plan, x, call, *norms, w, n1.variance_epsilon, rms=True, gated=True)
         x = self.self_attn(self.input_layernorm(x), position_embeddings, residual=x)
         return self.mlp(self.post_attention_layernorm(x), residual=x)
 

@@ -22,3 +22,45 @@ def test_residual_of_another_shape_or_dtype_is_refused(residual):
     i = torch.zeros(H, dtype=torch.int32)
     with torch.no_grad(), pytest.raises(ValueError, match="residual must match"):
         attention_layer(plan(), x, [x] * 4, None, i, i, residual=residual)
+
+
+def good(n_kv=0, dtype=torch.bfloat16):
+    p = plan(n_kv)
+    return p, torch.zeros(2, 8, p.C, dtype=dtype), [torch.zeros(s, dtype=dtype) for s in p.weight_shapes]
+
+
+@pytest.mark.parametrize("n_kv", [0, 1])
+@pytest.mark.parametrize("training", [False, True])
+def test_layer_entry_takes_three_dimensions_and_the_plans_shapes(n_kv, training):
+    from saf_b200.layer import usable
+    p, x, w = good(n_kv)
+    assert usable(p, x, w, training)
+    for other in (x[0], x[None], x[..., :64], torch.zeros(2, 8, 192, dtype=x.dtype), x[:0], x.half()):
+        assert not usable(p, other, w, training)
+    for i in range(4):
+        rows, cols = w[i].shape
+        for other in (torch.zeros(rows - 64, cols, dtype=x.dtype), torch.zeros(rows, cols + 64, dtype=x.dtype), w[i].float(),
+                      torch.zeros(cols, rows * 2, dtype=x.dtype).t()[:rows]):
+            assert not usable(p, x, w[:i] + [other] + w[i + 1:], training)
+
+
+@pytest.mark.parametrize("gated", [False, True])
+def test_block_entry_takes_the_plans_widths_only(gated):
+    from saf_b200.layer import block_usable
+    p, x, w = good()
+    hidden = 256
+
+    def t(*shape, dtype=torch.bfloat16):
+        return torch.zeros(shape, dtype=dtype)
+
+    parts = dict(call=dict(weights=w, biases=[t(s[0]) for s in p.weight_shapes]), norm1=[t(p.C), t(p.C)], norm2=[t(p.C), None],
+                 mlp=[t(hidden, p.C), t(hidden, p.C) if gated else None, t(hidden), t(p.C, hidden), t(p.C)], gated=gated)
+    assert block_usable(p, x, **parts)
+    for name, i, other in [("norm1", 0, t(p.C + 8)), ("norm1", 1, t(1)), ("norm2", 0, t(p.C, dtype=torch.float32)),
+                           ("mlp", 0, t(hidden, p.C + 64)), ("mlp", 2, t(8)), ("mlp", 3, t(p.C, hidden + 64)),
+                           ("mlp", 3, t(p.C - 64, hidden)), ("mlp", 4, t(8)), ("mlp", 3, t(hidden, p.C).t())]:
+        part = list(parts[name])
+        part[i] = other
+        assert not block_usable(p, x, **{**parts, name: part})
+    assert not block_usable(p, x, **{**parts, "call": dict(weights=w, biases=[t(8)] + parts["call"]["biases"][1:])})
+    assert not block_usable(p, x, **{**parts, "call": dict(weights=[v.float() for v in w])})
