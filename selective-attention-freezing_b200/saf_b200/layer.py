@@ -76,7 +76,7 @@ class LayerPlan:
             t.SD = c.alpha.shape[1]
             t.dec_dtype = ops._dt(c.alpha)
         a.x_dtype, a.w_dtype, a.train = _DT[x.dtype], _DT[c.w[0].dtype], c.train
-        a.x, a.ldx = x.data_ptr(), x.stride(0)
+        a.x, a.ldx = x.data_ptr(), _ld(x)
         a.wq, a.wk, a.wv, a.wo = [w.data_ptr() for w in c.w]
         if c.rope is not None:
             a.rope_cos, a.rope_sin = c.rope[0].data_ptr(), c.rope[1].data_ptr()
@@ -119,10 +119,18 @@ def usable(plan, x, weights, training):
 
 
 def _rows(x):
+    """x as rows the library reads by TMA: 16-byte aligned, a whole number of 16-byte pieces and at least a row apart (an
+    expanded tensor's rows are not); fp32 rows follow each other."""
     x2 = ops._as_2d(x)
-    if x.dtype == torch.float32:
-        return x2.contiguous()
-    return x2 if x2.stride(0) % 8 == 0 else x2.contiguous()
+    step, C = _ld(x2), x2.shape[1]
+    if x2.data_ptr() % 16 or (step != C if x2.dtype == torch.float32 else step % 8 or step < C):
+        return x2.clone(memory_format=torch.contiguous_format)     # (.contiguous() keeps a misaligned contiguous tensor)
+    return x2
+
+
+def _ld(x2):
+    """Row stride of a matrix; torch reports anything for a single row."""
+    return x2.stride(0) if x2.shape[0] > 1 else x2.shape[1]
 
 
 def _blob(n, device):
@@ -141,7 +149,7 @@ def _forward(plan, c, biases=None, residual=None):
     if biases is not None:
         a.bq, a.bk, a.bv, a.bo = [None if b is None else b.data_ptr() for b in biases]
     if residual is not None:
-        a.residual, a.ldr = residual.data_ptr(), residual.stride(0)
+        a.residual, a.ldr = residual.data_ptr(), _ld(residual)
     events = ops.attention_event_pair()
     if events is not None:
         a.event_before, a.event_after = events
@@ -189,11 +197,7 @@ class _LayerFunction(torch.autograd.Function):
         B, T = ctx.bt
         dev = dout.device
         need = ctx.needs_input_grad
-        d2 = ops._as_2d(dout)
-        if d2.dtype != torch.bfloat16:
-            d2 = d2.to(torch.bfloat16)
-        if d2.stride(0) % 8 or d2.data_ptr() % 16:
-            d2 = d2.contiguous()
+        d2 = _bf16_rows(dout)
         x_shape, x_dtype = ctx.x_like
         # a converted tensor is read from the workspace; its argument only tells the dtype and layout
         x_arg = x2 if x2 is not None else work.view(torch.float32)[:plan.C].view(1, plan.C)
@@ -204,7 +208,7 @@ class _LayerFunction(torch.autograd.Function):
         g.struct_size = C.sizeof(SafAttnLayerBwdArgs)
         g.fwd = plan.args(c)
         g.fwd.work, g.fwd.work_bytes = work.data_ptr(), sz[0]
-        g.dout, g.lddo = d2.data_ptr(), d2.stride(0)
+        g.dout, g.lddo = d2.data_ptr(), _ld(d2)
         scratch = _blob(sz[1], dev)
         g.work, g.work_bytes = scratch.data_ptr(), sz[1]
         dx, dw = None, [None] * 4
@@ -230,10 +234,7 @@ class _LayerFunction(torch.autograd.Function):
 
 
 def _bf16_rows(x):
-    x2 = ops._as_2d(x)
-    if x2.dtype != torch.bfloat16:
-        x2 = x2.to(torch.bfloat16)
-    return x2.contiguous() if x2.stride(0) % 8 or x2.data_ptr() % 16 else x2
+    return _rows(x if x.dtype == torch.bfloat16 else x.to(torch.bfloat16))
 
 
 def _residual_rows(residual, tokens, width):

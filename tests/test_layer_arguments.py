@@ -64,3 +64,21 @@ def test_block_entry_takes_the_plans_widths_only(gated):
         assert not block_usable(p, x, **{**parts, name: part})
     assert not block_usable(p, x, **{**parts, "call": dict(weights=w, biases=[t(8)] + parts["call"]["biases"][1:])})
     assert not block_usable(p, x, **{**parts, "call": dict(weights=[v.float() for v in w])})
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+def test_rows_reach_the_library_aligned_and_a_row_apart(dtype):
+    from saf_b200.layer import _ld, _rows
+    C = 64
+    flat = torch.arange(40 * C + 8, dtype=torch.float32).to(dtype)
+    wide = torch.arange(6 * (C + 8), dtype=torch.float32).to(dtype).view(6, C + 8)
+    odd = torch.arange(6 * (C + 1), dtype=torch.float32).to(dtype).view(6, C + 1)
+    for x in (flat[:6 * C].view(2, 3, C), flat[1:1 + 6 * C].view(2, 3, C), flat[8:8 + 6 * C].view(2, 3, C),
+              wide[:, :C], wide[:, 8:], odd[:, :C], flat[:C].expand(2, 3, C), flat[:2 * C].view(2, 1, C).expand(2, 3, C),
+              flat[:32 * C].as_strided((6, C), (8, 1)), flat[:C].as_strided((1, 1, C), (1, 1, 1)), flat[1:1 + C].view(1, 1, C),
+              flat[:6 * C].view(2, C, 3).transpose(1, 2)):
+        r = _rows(x)
+        assert torch.equal(r, x.reshape(-1, C)) and r.data_ptr() % 16 == 0 and r.stride(1) == 1
+        assert _ld(r) >= C and _ld(r) * r.element_size() % 16 == 0 and (dtype == torch.bfloat16 or _ld(r) == C)
+    kept = wide[:, 8:] if dtype == torch.bfloat16 else flat[:6 * C].view(6, C)
+    assert _rows(kept).data_ptr() == kept.data_ptr()
