@@ -639,11 +639,12 @@ int launch_gemm_sm100(const SafIndexedLinearArgs& a, cudaStream_t st, int32_t* z
     uint32_t box[2] = {64, GM};
     if ((rc = make_tensor_map_bf16(&mo, a.out, 2, dims, strides, box, false))) return rc;
   }
-  const bool residual_tma = a.residual && !a.rope_cos && a.act != SAF_ACT_SWIGLU;
+  // (a residual whose rows overlap, such as one row for all, has no tensor map: it is read row by row)
+  const bool residual_tma = a.residual && !a.rope_cos && a.act != SAF_ACT_SWIGLU && (a.ldr >= N || a.M == 1);
   mr = mo;
   if (residual_tma) {
     uint64_t dims[2] = {(uint64_t)N, (uint64_t)a.M};
-    uint64_t strides[2] = {0, (uint64_t)a.ldr * 2};
+    uint64_t strides[2] = {0, (uint64_t)std::max<int64_t>(a.ldr, N) * 2};     // (M == 1: any stride)
     uint32_t box[2] = {64, GM};
     if ((rc = make_tensor_map_bf16(&mr, a.residual, 2, dims, strides, box, false))) return rc;
   }
