@@ -357,7 +357,7 @@ indexed_gemm_kernel(const __grid_constant__ CUtensorMap mapX, const __grid_const
       const int nsub = min(SUBS, (p.N - tn * GN) / 64);
       const int buf = lt & 1;
       const int m = tm * C::ROWS + rank * GM + row;
-      if (p.cosT && !p.halves && tm != tm_held) {
+      if (p.cosT && tm != tm_held) {
         tm_held = tm;
         // 32 values of 128 table rows (the tables repeat per half), whole 128-byte pieces of 4 rows per load, handed to
         // the threads of the rows through the group's staging block.  (A thread reading its own row touched 32 lines per
@@ -616,6 +616,10 @@ int launch_gemm_sm100(const SafIndexedLinearArgs& a, cudaStream_t st, int32_t* z
     if (a.ldw[w] % 8 || (a.cdw[w] != 0 && a.cdw[w] != 1) || !aligned16(a.weights[w])) return SAF_ERR_UNSUPPORTED;
   }
   if (!saf_device_supported()) return SAF_ERR_UNSUPPORTED;
+  // Tables count only when some slab rotates: the form of the tiles and the epilogue's way through a 128-row slab (both
+  // groups on one pair of blocks) have to follow from the same fact.
+  bool rotates = false;
+  for (int g = 0; g < a.n_slabs && a.slab_rope; ++g) rotates |= a.slab_rope[g] != 0;
 
   CUtensorMap mx, mw[4], mo, mr;
   int rc;
@@ -640,7 +644,7 @@ int launch_gemm_sm100(const SafIndexedLinearArgs& a, cudaStream_t st, int32_t* z
     if ((rc = make_tensor_map_bf16(&mo, a.out, 2, dims, strides, box, false))) return rc;
   }
   // (a residual whose rows overlap, such as one row for all, has no tensor map: it is read row by row)
-  const bool residual_tma = a.residual && !a.rope_cos && a.act != SAF_ACT_SWIGLU && (a.ldr >= N || a.M == 1);
+  const bool residual_tma = a.residual && !rotates && a.act != SAF_ACT_SWIGLU && (a.ldr >= N || a.M == 1);
   mr = mo;
   if (residual_tma) {
     uint64_t dims[2] = {(uint64_t)N, (uint64_t)a.M};
@@ -650,7 +654,6 @@ int launch_gemm_sm100(const SafIndexedLinearArgs& a, cudaStream_t st, int32_t* z
   }
   SubTable tb;
   memset(&tb, 0, sizeof(tb));
-  bool rope_after = false;
   if (halves) {
     for (int hb = 0; hb < N / 32; ++hb) {          // 32-column runs of the output, two per block
       const int g = (hb * 32) / a.slab, r = (hb * 32) % a.slab;
@@ -662,8 +665,6 @@ int launch_gemm_sm100(const SafIndexedLinearArgs& a, cudaStream_t st, int32_t* z
         tb.weight[hb >> 1] = (uint8_t)a.slab_weight[g];
       }
     }
-    if (a.slab_rope)
-      for (int g = 0; g < a.n_slabs; ++g) rope_after |= a.slab_rope[g] != 0;
   } else {
     const int per = a.slab / 64;
     for (int g = 0; g < a.n_slabs; ++g)
@@ -677,19 +678,19 @@ int launch_gemm_sm100(const SafIndexedLinearArgs& a, cudaStream_t st, int32_t* z
   memset(&p, 0, sizeof(p));
   p.M = a.M; p.N = N; p.K = a.C; p.T = a.T; p.slab = a.slab;
   for (int w = 0; w < a.n_weights; ++w) p.bias[w] = a.biases[w];
-  p.cosT = a.rope_cos;
+  p.cosT = rotates && !halves ? a.rope_cos : nullptr;     // halves: rotated by a launch of its own, below
   p.sinT = a.rope_sin;
   p.status = a.status;
   p.act = a.act;
   p.residual = reinterpret_cast<const __nv_bfloat16*>(a.residual);
   p.ldr = a.ldr;
   p.residual_tma = residual_tma ? 1 : 0;
-  p.runs = a.rope_cos && !halves ? 1 : 0;
+  p.runs = p.cosT ? 1 : 0;
   p.halves = halves ? 1 : 0;
   p.zero2 = zero2;
   p.weights_early = weights_early ? 1 : 0;
 
-  const bool together = a.act == SAF_ACT_SWIGLU || (!halves && a.slab == 128 && a.slab_rope);
+  const bool together = a.act == SAF_ACT_SWIGLU || (a.slab == 128 && p.cosT);
   const char* pair_env = getenv("SAF_B200_GEMM_PAIR");
   const bool pair_off = pair_env && pair_env[0] == '0' && pair_env[1] == 0;
   int pairs = 0;
@@ -713,7 +714,7 @@ int launch_gemm_sm100(const SafIndexedLinearArgs& a, cudaStream_t st, int32_t* z
     }
     if (rc) return rc;
   }
-  if (rope_after)
+  if (halves && rotates)
     return launch_rope_slabs(a.out, a.ldo, a.M, a.n_slabs, a.slab, a.T, a.slab_rope, a.rope_cos, a.rope_sin, a.dtype, 0, st);
   return SAF_OK;
 }

@@ -26,3 +26,30 @@ def test_residual_rows_that_overlap(M, N):
     x, w = rand(M, 128, seed=M), rand(N, 128, seed=N, scale=0.05)
     for res in (rand(N, seed=1).expand(M, N), rand(M * 8 + N, seed=2).as_strided((M, N), (8, 1))):
         assert torch.equal(ops.linear_act(x, w, None, residual=res), ops.linear_act(x, w, None, residual=res.contiguous().clone()))
+
+
+@pytest.mark.parametrize("M", [1, 130, 3001])
+@pytest.mark.parametrize("slab", [64, 128])
+@pytest.mark.parametrize("slab_rope", [None, 0, 1])
+def test_tables_without_a_slab_to_rotate(M, slab, slab_rope):
+    """128-row slabs with cos / sin tables and no rotation asked for, at sizes whose tiles hold one 64-row block; and with it,
+    where they hold whole slabs."""
+    from saf_b200 import ops
+    from saf_b200._cabi import lib
+    K, n = 128, 3
+    x, w = rand(M, K, seed=M), rand(n * slab, K, seed=slab, scale=0.05)
+    ang = torch.rand(M, slab // 2, device="cuda", generator=torch.Generator(device="cuda").manual_seed(3)).repeat(1, 2) * 6
+    cos, sin = ang.cos().contiguous(), ang.sin().contiguous()
+    keep = []
+    rope = None if slab_rope is None else [slab_rope] * n
+    a = ops._lin_args(x, [w], None, slab, [0] * n, [slab * i for i in range(n)], keep, rope=(cos, sin), T=M, slab_rope=rope)
+    a.rope_cos, a.rope_sin = cos.data_ptr(), sin.data_ptr()
+    out = torch.empty(M, n * slab, dtype=torch.bfloat16, device="cuda")
+    a.out, a.ldo = out.data_ptr(), n * slab
+    ops._call(x, lib.saf_indexed_linear_fwd, C.byref(a))
+    ref = (x.float() @ w.float().t()).view(M, n, slab)
+    if slab_rope:
+        turned = torch.cat([-ref[..., slab // 2:], ref[..., :slab // 2]], dim=-1)
+        ref = ref * cos[:, None] + turned * sin[:, None]
+    assert rel(out, ref.reshape(M, -1)) <= REL
+    ops.device_status()
