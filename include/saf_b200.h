@@ -190,7 +190,9 @@ typedef struct SafIndexedLinearArgs {
   const int32_t* slab_weight; /* HOST (n_slabs,) weight index of slab g            */
   const int32_t* slab_row0;   /* HOST (n_slabs,) first weight row of slab g        */
   const int32_t* slab_rope;   /* HOST (n_slabs,) or null: rotate this slab         */
-  const float* rope_cos;      /* device (T, slab) fp32                             */
+  const float* rope_cos;      /* device (T, slab) fp32; bf16 calls on slabs other than
+                                 128 rows take the second half of a row as a
+                                 repetition of the first                           */
   const float* rope_sin;
   void* out;                  /* (M, n_slabs*slab) row-major, row stride ldo       */
   int64_t ldo;

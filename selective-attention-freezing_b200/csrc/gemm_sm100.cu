@@ -330,13 +330,16 @@ indexed_gemm_kernel(const __grid_constant__ CUtensorMap mapX, const __grid_const
     const bool chief = (tid & 127) == 0;        // loads and stores its group's blocks
     const bool swiglu = p.act == SAF_ACT_SWIGLU;
     // a rotated 128-row slab is two blocks: group g rotates columns 32g .. 32g+31 of the first with those of the second,
-    // so that a thread needs 32 cos and 32 sin values of its row (held over the row's tiles), and both fill both blocks
+    // so that a thread needs 32 cos and 32 sin values of its row (held over the row's tiles), and both fill both blocks.
+    // The second half of a table row repeats the first in every rotary embedding; a block of 128 rows where it does not
+    // is noticed as the values arrive, and reads its second halves where it needs them
     const bool wide = p.slab == 128 && p.cosT;
     const int bar_id = wide ? 3 : 1 + grp, bar_n = wide ? 256 : 128;
     uint8_t* stg = out_stage + grp * (OUT_BYTES / 2);
     uint32_t lt = 0;
     int tm_held = -1;                           // row tile whose cos / sin values the registers hold
     float4 cs4[8], sn4[8];
+    bool halves_differ = false;
     // the residual block of this group's first output block at or behind (tile, step), into its free staging block
     uint32_t n_res = 0;
     auto ask_residual = [&](int tile, int st) {
@@ -363,15 +366,21 @@ indexed_gemm_kernel(const __grid_constant__ CUtensorMap mapX, const __grid_const
         // the threads of the rows through the group's staging block.  (A thread reading its own row touched 32 lines per
         // load: 8192 cycles of the load path for the two groups, more than the products of a narrow tile.)
         const int l = tid & 127;
+        bool differ = false;
 #pragma unroll
         for (int q = 0; q < 8; ++q) {
           const int mr = tm * C::ROWS + rank * GM + (l >> 3) + 16 * q;
           const int64_t at = (int64_t)(p.T > 0 ? mr % p.T : 0) * p.slab + (wide ? grp * 32 : 0) + (l & 7) * 4;
           cs4[q] = *reinterpret_cast<const float4*>(p.cosT + at);
           sn4[q] = *reinterpret_cast<const float4*>(p.sinT + at);
+          if (wide) {
+            const float4 c2 = *reinterpret_cast<const float4*>(p.cosT + at + 64), s2 = *reinterpret_cast<const float4*>(p.sinT + at + 64);
+            differ |= c2.x != cs4[q].x || c2.y != cs4[q].y || c2.z != cs4[q].z || c2.w != cs4[q].w || s2.x != sn4[q].x ||
+                      s2.y != sn4[q].y || s2.z != sn4[q].z || s2.w != sn4[q].w;
+          }
         }
         if (chief) tma_store_wait_read0();
-        named_bar_sync(1 + grp, 128);
+        halves_differ = named_bar_or(1 + grp, 128, differ);
         auto own_row = [&](float4 (&x)[8]) {
 #pragma unroll
           for (int q = 0; q < 8; ++q) {
@@ -478,12 +487,19 @@ indexed_gemm_kernel(const __grid_constant__ CUtensorMap mapX, const __grid_const
 #pragma unroll
           for (int j4 = 0; j4 < 8; ++j4) {
             const float cc[4] = {cs4[j4].x, cs4[j4].y, cs4[j4].z, cs4[j4].w}, ss[4] = {sn4[j4].x, sn4[j4].y, sn4[j4].z, sn4[j4].w};
+            float4 c2 = cs4[j4], s2 = sn4[j4];
+            if (halves_differ) {
+              const int64_t at = (int64_t)(p.T > 0 ? m % p.T : 0) * p.slab + 64 + grp * 32 + j4 * 4;
+              c2 = *reinterpret_cast<const float4*>(p.cosT + at);
+              s2 = *reinterpret_cast<const float4*>(p.sinT + at);
+            }
+            const float cc2[4] = {c2.x, c2.y, c2.z, c2.w}, ss2[4] = {s2.x, s2.y, s2.z, s2.w};
 #pragma unroll
             for (int e = 0; e < 4; ++e) {
               const int j = j4 * 4 + e;
               const float x1 = v[j], x2 = v[32 + j];
               v[j] = x1 * cc[e] - x2 * ss[e];
-              v[32 + j] = x2 * cc[e] + x1 * ss[e];
+              v[32 + j] = x2 * cc2[e] + x1 * ss2[e];
             }
           }
         }

@@ -53,3 +53,20 @@ def test_tables_without_a_slab_to_rotate(M, slab, slab_rope):
         ref = ref * cos[:, None] + turned * sin[:, None]
     assert rel(out, ref.reshape(M, -1)) <= REL
     ops.device_status()
+
+
+@pytest.mark.parametrize("M,T", [(1, 1), (200, 50), (4500, 900)])
+def test_tables_whose_halves_differ(M, T):
+    """128-row slabs honour both halves of a table row, in the rows where they differ and in those where they do not."""
+    from saf_b200 import ops
+    hd, heads, live = 128, 3, [0, 2]
+    x = rand(M, 384, seed=M)
+    w = [rand(384, 384, seed=i, scale=0.05) for i in range(3)]
+    ang = torch.rand(T, hd, device="cuda", generator=torch.Generator(device="cuda").manual_seed(T)) * 6
+    ang[T // 2:, hd // 2:] = ang[T // 2:, :hd // 2]
+    cos, sin = ang.cos().contiguous(), ang.sin().contiguous()
+    y = ops.qkv_projection(x, *w, live, hd, rope=(cos, sin), T=T).view(M, -1, hd)
+    full = [(x.float() @ wi.float().t()).view(M, heads, hd) for wi in w]
+    row = torch.arange(M, device="cuda") % T
+    rot = [t[:, live] * cos[row][:, None] + torch.cat([-t[:, live, hd // 2:], t[:, live, :hd // 2]], -1) * sin[row][:, None] for t in full[:2]]
+    assert rel(y, torch.cat([*rot, full[2]], dim=1)) <= REL
