@@ -336,12 +336,15 @@ attn_stats_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constan
     bool ok = true;
     float w = 0.f, cw = 0.f;                        // weights of the merge: nb / (c0 + nb), c0 nb / (c0 + nb)
     double cwd = 0.0;
-    for (int t = blockIdx.x; t < total && ok; t += gridDim.x, ++n) {
+    // (a warp whose wait ran out keeps walking its tiles, doing nothing but its part of flush_head's barriers: the others
+    // end on their own limits instead of waiting there for it)
+    for (int t = blockIdx.x; t < total; t += gridDim.x, ++n) {
       const AsTile x = as_decode<LOGITS>(p, t);
       if (!LOGITS && x.u != cur_u) {
         if (cur_u >= 0) flush_head();
         cur_u = x.u;
       }
+      if (!ok) continue;
       const int gi = x.it * 128 + r;
       const int gj0 = x.jt * AS_COLS + half * 32;
       const bool diag = x.jt * AS_COLS + AS_COLS - 1 > x.it * 128;
@@ -360,7 +363,8 @@ attn_stats_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constan
 #pragma unroll
           for (int b = 0; b < AS_GROUP; ++b) L[b] = Ln[b];
         }
-        if (!mbar_wait(&sh->s_full[k], (g >> 1) & 1) || (gr == 0 && !mbar_wait(&sh->old_full[n & 1], (n >> 1) & 1))) {
+        const bool got = mbar_wait(&sh->s_full[k], (g >> 1) & 1) && (gr > 0 || mbar_wait(&sh->old_full[n & 1], (n >> 1) & 1));
+        if (!__all_sync(0xffffffffu, got)) {
           dev_set_error(p.status, SAF_DEV_TIMEOUT_SOFTMAX, 82);
           ok = false;
           break;
@@ -442,12 +446,12 @@ attn_stats_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constan
           esum += (double)ent * (double)AS_LN2;        // natural log, as the reference's xlogy
         }
       }
-      if (!ok) break;
+      if (!ok) continue;
       fence_proxy_async_smem();
       __syncwarp();
       if (lane == 0) mbar_arrive(&sh->done[n & 1]);
     }
-    if (!LOGITS && ok && cur_u >= 0) flush_head();
+    if (!LOGITS && cur_u >= 0) flush_head();
     if (!LOGITS && p.count_prev == 0) {
       // above the diagonal every probability is zero: the first batch writes the zeros, later ones leave them
       const int64_t rows = (int64_t)p.U * p.T;

@@ -156,6 +156,7 @@ indexed_gemm_bwd_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_c
     const uint32_t sbase = smem_u32(stage_base);
     uint32_t it = 0, lt = 0;
     bool ok = true;
+    pdl_wait();                                 // the limits of the waits below do not run while an earlier kernel does
     for (int tile = blockIdx.x; tile < total_tiles && ok; tile += gridDim.x, ++lt) {
       const int buf = lt & 1;
       if (!mbar_wait(&sl->acc_empty[buf], ((lt >> 1) & 1) ^ 1)) {
@@ -203,7 +204,8 @@ indexed_gemm_bwd_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_c
       const int nsub = min(4, (p.J - tn * BN + 63) / 64);
       const int nrow = (MODE == MODE_DW) ? min(2, p.n_blocks - tm * 2) : 2;
       const int buf = lt & 1;
-      if (!mbar_wait(&sl->acc_full[buf], (lt >> 1) & 1)) {
+      // threads that meet at named barriers leave together: one whose wait ran out takes the others with it
+      if (named_bar_or(1, 128, !mbar_wait(&sl->acc_full[buf], (lt >> 1) & 1))) {
         dev_set_error(p.status, SAF_DEV_TIMEOUT_EPI, 63);
         break;
       }

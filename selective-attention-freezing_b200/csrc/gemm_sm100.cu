@@ -280,6 +280,7 @@ indexed_gemm_kernel(const __grid_constant__ CUtensorMap mapX, const __grid_const
       const uint32_t sbase = smem_u32(stage_base);
       uint32_t it = 0, lt = 0;
       bool ok = true;
+      pdl_wait();                       // the limits of the waits below do not run while an earlier kernel does
       for (int tile = tile_lo; tile < tile_hi && ok; tile += tile_step, ++lt) {
         const int buf = lt & 1;
         if (!mbar_wait(&sl->acc_empty[buf], ((lt >> 1) & 1) ^ 1)) {
@@ -403,9 +404,10 @@ indexed_gemm_kernel(const __grid_constant__ CUtensorMap mapX, const __grid_const
         const bool mine = u < nsub;
         const int out_col = swiglu ? (tn * GN + u * 64) / 2 : tn * GN + u * 64;
         if (st == 0) {
-          if (!mbar_wait(&sl->acc_full[buf], (lt >> 1) & 1)) {
+          // threads that meet at named barriers leave together: one whose wait ran out takes the others with it
+          if (named_bar_or(bar_id, bar_n, !mbar_wait(&sl->acc_full[buf], (lt >> 1) & 1))) {
             dev_set_error(p.status, SAF_DEV_TIMEOUT_EPI, 13);
-            if (p.residual_tma && mine) mbar_wait(&sl->res[grp], n_res & 1);   // its copy is on its way: let it land
+            if (p.residual_tma) mbar_wait(&sl->res[grp], n_res & 1);       // a copy may be on its way: let it land
             tile = tile_hi;
             break;
           }
