@@ -280,6 +280,10 @@ indexed_gemm_kernel(const __grid_constant__ CUtensorMap mapX, const __grid_const
       const uint32_t sbase = smem_u32(stage_base);
       uint32_t it = 0, lt = 0;
       bool ok = true;
+      // K steps of all this unit's tiles.  The last round of stages is not handed back: nobody loads into them again, and in
+      // a pair the hand-back is an arrival that the tensor core makes in both CTAs' shared memory, where another kernel's
+      // CTA may follow as soon as this one is done.
+      const uint32_t steps = tile_lo < tile_hi ? (uint32_t)((tile_hi - tile_lo + tile_step - 1) / tile_step) * KB : 0;
       pdl_wait();                       // the limits of the waits below do not run while an earlier kernel does
       for (int tile = tile_lo; tile < tile_hi && ok; tile += tile_step, ++lt) {
         const int buf = lt & 1;
@@ -310,8 +314,10 @@ indexed_gemm_kernel(const __grid_constant__ CUtensorMap mapX, const __grid_const
               if constexpr (PAIR) umma_ss_pair(d, ad, bd, idesc, (kb | k4) != 0);
               else umma_ss(d, ad, bd, idesc, (kb | k4) != 0);
             }
-            if constexpr (PAIR) umma_commit_pair(&sl->empty[s]);      // frees the stage in both CTAs
-            else umma_commit(&sl->empty[s]);
+            if (it + STAGES < steps) {
+              if constexpr (PAIR) umma_commit_pair(&sl->empty[s]);    // frees the stage in both CTAs
+              else umma_commit(&sl->empty[s]);
+            }
           }
           __syncwarp();
         }
