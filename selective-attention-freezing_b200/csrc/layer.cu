@@ -25,6 +25,8 @@ namespace saf {
 namespace {
 
 constexpr int LAYER_MAX_HEADS = 256;
+constexpr int LAYER_MAX_SLABS = 3 * LAYER_MAX_HEADS;     // of one product: heads of Q, K and V, or 64-row blocks of C
+constexpr int MLP_MAX_BLOCKS = 1024;
 
 int64_t up(int64_t n) { return (n + 255) & ~(int64_t)255; }
 
@@ -109,7 +111,8 @@ int validate_layer(const SafAttnLayerArgs* a) {
   if (t.dtype != SAF_BF16) return fail(SAF_ERR_UNSUPPORTED, "the layer entry computes in bf16");
   if (t.B <= 0 || t.T <= 0 || t.H <= 0 || t.U < 0 || t.U > t.H || t.HD <= 0 || a->C <= 0 || t.HKV < 0)
     return fail(SAF_ERR_INVALID, "bad dimension");
-  if (t.H > LAYER_MAX_HEADS) return fail(SAF_ERR_LIMIT, "more than %d heads", LAYER_MAX_HEADS);
+  if (t.H > LAYER_MAX_HEADS || t.HKV > LAYER_MAX_HEADS) return fail(SAF_ERR_LIMIT, "more than %d heads", LAYER_MAX_HEADS);
+  if (a->C > LAYER_MAX_SLABS * 64) return fail(SAF_ERR_LIMIT, "width %d exceeds the limit of %d", a->C, LAYER_MAX_SLABS * 64);
   if (t.HD % 32 || t.HD > 128 || a->C % 8) return fail(SAF_ERR_UNSUPPORTED, "head_dim %d, width %d", t.HD, a->C);
   if (t.rope || t.force_state >= 0) return fail(SAF_ERR_INVALID, "rope and force_state belong to the attention entry");
   if (!t.frozen || !t.frozen_host) return fail(SAF_ERR_INVALID, "frozen and frozen_host must be non-null");
@@ -135,7 +138,7 @@ SafTensor rows_view(void* base, int64_t first_col, int64_t ld, int T, int hd) { 
 }
 
 struct Slabs {
-  int32_t weight[3 * LAYER_MAX_HEADS], row0[3 * LAYER_MAX_HEADS], rope[3 * LAYER_MAX_HEADS];
+  int32_t weight[LAYER_MAX_SLABS], row0[LAYER_MAX_SLABS], rope[LAYER_MAX_SLABS];
   int n;
 };
 void qkv_slabs(const SafAttnLayerArgs& a, const Dims& d, Slabs* s) {
@@ -396,16 +399,16 @@ int validate_block(const SafBlockArgs* b) {
   if (b->layer.x_dtype != SAF_BF16 || b->layer.w_dtype != SAF_BF16 || b->layer.train)
     return fail(SAF_ERR_UNSUPPORTED, "the block entry is bf16 inference");
   if (b->hidden <= 0 || b->hidden % (b->gated ? 128 : 64) || b->layer.C % 64) return fail(SAF_ERR_UNSUPPORTED, "width %d, hidden %d", b->layer.C, b->hidden);
+  if (b->hidden / 64 * (b->gated ? 2 : 1) > MLP_MAX_BLOCKS) return fail(SAF_ERR_LIMIT, "hidden %d", b->hidden);
   return SAF_OK;
 }
 
 // out = [residual +] act(x W^T + b) over whole matrices in 64-row blocks; gated: blocks of the two weights alternate
 int mlp_linear(const void* x, int M, int K, const void* w0, const void* w1, const void* bias, int N, int act, const void* residual,
                int64_t ldr, void* out, int64_t ldo, int32_t* status, void* stream) {
-  constexpr int MAX = 1024;
-  int32_t weight[MAX], row0[MAX];
+  int32_t weight[MLP_MAX_BLOCKS], row0[MLP_MAX_BLOCKS];
   const int per = w1 ? 2 : 1, n = N / 64 * per;
-  if (n > MAX) return fail(SAF_ERR_LIMIT, "MLP width %d", N);
+  if (n > MLP_MAX_BLOCKS) return fail(SAF_ERR_LIMIT, "MLP width %d", N);
   for (int i = 0; i < n; ++i) {
     weight[i] = w1 ? i & 1 : 0;
     row0[i] = i / per * 64;

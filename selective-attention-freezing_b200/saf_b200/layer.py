@@ -15,6 +15,8 @@ from ._cabi import SafAttnLayerArgs, SafAttnLayerBwdArgs, SafBlockArgs, SafMixed
 _DT = {torch.float32: SAF_F32, torch.bfloat16: SAF_BF16}
 HEAD_DIMS = (64, 96, 128)
 MAX_BLOCKS = 160          # 64-row blocks of one backward product
+MAX_HEADS = 256           # of the library's slab tables; the out projection's hold MAX_WIDTH / 64 blocks
+MAX_WIDTH = 3 * MAX_HEADS * 64
 
 
 class LayerPlan:
@@ -50,7 +52,8 @@ class LayerPlan:
     def shapes_ok(self, training):
         """Sizes the tensor-core products of both directions take."""
         blocks = max(self.width(), self.C) // 64
-        return (self.hd in HEAD_DIMS and self.U > 0 and self.width() % 64 == 0 and self.C % 64 == 0
+        return (self.hd in HEAD_DIMS and 0 < self.U <= self.H <= MAX_HEADS and self.n_kv <= MAX_HEADS
+                and self.C <= MAX_WIDTH and self.width() % 64 == 0 and self.C % 64 == 0
                 and (not training or (blocks <= MAX_BLOCKS and self.H * self.hd % 64 == 0 and self.C + 3 * self.H * self.hd <= 32 * 1024)))
 
     def args(self, c):

@@ -82,3 +82,47 @@ def test_rows_reach_the_library_aligned_and_a_row_apart(dtype):
         assert _ld(r) >= C and _ld(r) * r.element_size() % 16 == 0 and (dtype == torch.bfloat16 or _ld(r) == C)
     kept = wide[:, 8:] if dtype == torch.bfloat16 else flat[:6 * C].view(6, C)
     assert _rows(kept).data_ptr() == kept.data_ptr()
+
+
+def layer_struct(H=2, n_kv=0, width=128):
+    import ctypes as C
+    from saf_b200 import _cabi
+    from saf_b200.layer import LayerPlan
+    p = LayerPlan([0] * H, list(range(H)), HD, width, n_kv=n_kv)
+    a = _cabi.SafAttnLayerArgs.from_buffer_copy(p._template)
+    a.attn.B, a.attn.T = 1, 8
+    a.x_dtype = a.w_dtype = _cabi.SAF_BF16
+    i = (C.c_int32 * H)()
+    a.attn.frozen = C.addressof(i)
+    return a, (p, i)
+
+
+@pytest.mark.parametrize("args,ok", [
+    (dict(H=256, width=16384), True), (dict(H=257, width=16448), False),
+    (dict(n_kv=256), True), (dict(n_kv=257), False), (dict(n_kv=100000), False),
+    (dict(width=768 * 64), True), (dict(width=769 * 64), False), (dict(width=1 << 24), False),
+])
+def test_sizes_beyond_the_layer_entrys_tables_are_refused(args, ok):
+    """Heads, key / value heads and width each fill a table of the entry: refused before anything is written, by the
+    entry and by what decides whether the modules use it."""
+    import ctypes as C
+    from saf_b200 import _cabi
+    a, keep = layer_struct(**args)
+    out = (C.c_int64 * 4)()
+    assert _cabi.lib.saf_attn_layer_workspace(C.byref(a), out) == (_cabi.SAF_OK if ok else _cabi.SAF_ERR_LIMIT)
+    if not ok:
+        assert _cabi.lib.saf_attn_layer_fwd(C.byref(a), None) == _cabi.SAF_ERR_LIMIT
+    assert keep[0].shapes_ok(False) == ok
+
+
+def test_mlp_beyond_the_block_entrys_table_is_refused_before_its_norm_runs():
+    import ctypes as C
+    from saf_b200 import _cabi
+    b = _cabi.SafBlockArgs()
+    b.struct_size = C.sizeof(b)
+    b.layer, keep = layer_struct()
+    n = C.c_int64()
+    for gated, hidden, rc in ((0, 65536, _cabi.SAF_OK), (0, 65536 + 64, _cabi.SAF_ERR_LIMIT), (1, 32768, _cabi.SAF_OK),
+                              (1, 32768 + 128, _cabi.SAF_ERR_LIMIT)):
+        b.gated, b.hidden = gated, hidden
+        assert _cabi.lib.saf_block_workspace(C.byref(b), C.byref(n)) == rc
