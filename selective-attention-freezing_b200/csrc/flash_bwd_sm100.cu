@@ -233,7 +233,7 @@ __device__ __forceinline__ bool bwd_cta_coords(const BwdParams& p, int cta, bool
   const int bh = grp * BWD_HEAD_GROUP + rem % gsize;
   b = bh / p.H;
   h = bh % p.H;
-  const int state = p.force_state >= 0 ? p.force_state : __ldcg(p.frozen + h);
+  const int state = p.force_state >= 0 ? p.force_state : p.frozen[h];
   return state == SAF_LIVE;
 }
 
@@ -276,7 +276,7 @@ flash_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_con
                       const __grid_constant__ BwdParams p) {
   using C = BwdCfg<HD>;
   pdl_wait();
-  pdl_trigger();          // the dQ tiles, which need nothing of this kernel, may start as its last CTAs leave SMs idle
+  pdl_trigger();
   if ((int)blockIdx.x < p.scan_slots) {
     // ---- reverse scan of a structured frozen head: one slot per (batch, head, 64-column slice)
     constexpr int PER = HD / SCAN_COLS;
@@ -592,17 +592,11 @@ __global__ void __launch_bounds__(BWD_THREADS, 1)
 flash_bwd_dq_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant__ CUtensorMap mapK,
                     const __grid_constant__ CUtensorMap mapV, const __grid_constant__ CUtensorMap mapdO,
                     const __grid_constant__ CUtensorMap mapdQ, const __grid_constant__ BwdParams p) {
-  // Started beside the dK / dV kernel, whose CTAs have all passed their own wait for the kernels before it: everything read
-  // here is complete (and read past the L1, which nothing has cleared since).  The CTA waits for the dK / dV kernel only
-  // before it ends, so that whatever follows this launch follows both.  Its longest tiles come first, so the wait is over by
-  // then.  12 x 64, T = 1024, B = 8, with the other launches of the backward overlapping the same way: 316 -> 293 us a pass.
+  pdl_wait();
   using C = BwdCfg<HD>;
   int b, h, it;
-  if (!bwd_cta_coords(p, (int)blockIdx.x, false, b, h, it)) {
-    pdl_wait();
-    return;
-  }
-  const int hq = p.hidx ? __ldcg(p.hidx + h) : h;
+  if (!bwd_cta_coords(p, (int)blockIdx.x, false, b, h, it)) return;
+  const int hq = p.hidx ? p.hidx[h] : h;
   const int n = it + 1;                    // key tiles 0 .. it
   const int i0 = it * 128;
 
@@ -721,8 +715,8 @@ flash_bwd_dq_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_const
     const int row = i0 + r;
     float lse_r = INFINITY, dl_r = 0.f;            // +inf: P = 0 for rows past T
     if (row < p.T) {
-      lse_r = __ldcg(p.lse + (int64_t)b * p.lse_s[0] + (int64_t)h * p.lse_s[1] + (int64_t)row * p.lse_s[2]);
-      dl_r = __ldcg(p.delta + (int64_t)b * p.delta_s[0] + (int64_t)h * p.delta_s[1] + (int64_t)row * p.delta_s[2]);
+      lse_r = p.lse[(int64_t)b * p.lse_s[0] + (int64_t)h * p.lse_s[1] + (int64_t)row * p.lse_s[2]];
+      dl_r = p.delta[(int64_t)b * p.delta_s[0] + (int64_t)h * p.delta_s[1] + (int64_t)row * p.delta_s[2]];
     }
     // (a warp whose wait ran out keeps giving its one arrival per tile on named barrier 2, as in the dK/dV kernel)
     bool ok = true;
@@ -816,7 +810,6 @@ flash_bwd_dq_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_const
   tc_fence_before();
   __syncthreads();
   if (warp == 9) tmem_dealloc(tmem, C::TMEM_COLS);
-  pdl_wait();
 }
 
 // ---------------------------------------------------------------------------------------------
