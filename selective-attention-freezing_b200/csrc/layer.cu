@@ -296,8 +296,10 @@ int saf_attn_layer_fwd(const SafAttnLayerArgs* args, void* stream) {
   go.ldo = a.ldo;
   go.residual = a.residual;
   go.ldr = a.ldr;
-  // (behind the attention launch, which writes no weights)
-  rc = launch_gemm_sm100(go, st, nullptr, true);
+  // The caller's weights may be loaded while the attention launch still runs: it writes none, and whatever did was complete
+  // and flushed before an earlier launch of this call passed its own wait.  Copies this call made itself are not relied on
+  // that way.
+  rc = launch_gemm_sm100(go, st, nullptr, a.w_dtype == SAF_BF16);
   return rc == SAF_ERR_UNSUPPORTED ? saf_indexed_linear_fwd(&go, stream) : rc;
 }
 
