@@ -111,14 +111,22 @@ class _Call:
         self.alpha, self.rho, self.z = decomposed
 
 
+def _plain(t, dtype, shape):
+    """A tensor the library can take by its address and the plan's sizes."""
+    return t.dtype is dtype and t.shape == shape and t.is_contiguous() and t.data_ptr() % 16 == 0
+
+
 def usable(plan, x, weights, training):
     """True when the whole layer can run through the library's layer entry, which takes every size from the plan and the
     first two dimensions of x: other shapes stay with the operators (or are refused there)."""
     dt = weights[0].dtype
-    return (x.dtype in _DT and dt in _DT and x.dim() == 3 and x.shape[2] == plan.C and x.numel() > 0 and plan.shapes_ok(training)
-            and x.data_ptr() % 16 == 0
-            and all(w.dtype == dt and w.shape == s and w.is_contiguous() and w.data_ptr() % 16 == 0
-                    for w, s in zip(weights, plan.weight_shapes)))
+    if not (x.dtype in _DT and dt in _DT and x.dim() == 3 and x.shape[2] == plan.C and x.numel() > 0 and plan.shapes_ok(training)
+            and x.data_ptr() % 16 == 0):
+        return False
+    for w, s in zip(weights, plan.weight_shapes):
+        if not _plain(w, dt, s):
+            return False
+    return True
 
 
 def _rows(x):
@@ -271,13 +279,19 @@ def attention_layer(plan, x, weights, rope, frozen, hidx, *, kvidx=None, sink_de
 def block_usable(plan, x, call, norm1, norm2, mlp, gated):
     """bf16 inference of the whole block: every weight and norm in bf16 and of the plan's width, widths in whole 64-row
     blocks.  Arguments as `block` takes them; `usable` has seen the call's weights."""
-    w_in, w_up, b_in, w_out, b_out = mlp
-    hidden, C = w_in.shape[0], (plan.C,)
-    shapes = ((w_in, (hidden, plan.C)), (w_up, (hidden, plan.C)), (b_in, (hidden,)), (w_out, (plan.C, hidden)), (b_out, C),
-              *((t, C) for t in (*norm1, *norm2)), *((b, s[:1]) for b, s in zip(call.get("biases", ()), plan.weight_shapes)))
-    return (x.dtype == call["weights"][0].dtype == torch.bfloat16 and hidden % (128 if gated else 64) == 0 and hidden // 64 * (2 if gated else 1) <= 288
-            and all(t is None or (t.dtype == torch.bfloat16 and t.shape == s and t.is_contiguous() and t.data_ptr() % 16 == 0)
-                    for t, s in shapes))
+    dt, C, hidden = torch.bfloat16, plan.C, mlp[0].shape[0]
+    if x.dtype is not dt or call["weights"][0].dtype is not dt or hidden % (128 if gated else 64) or hidden // 64 * (2 if gated else 1) > 288:
+        return False
+    for t in (*norm1, *norm2):
+        if t is not None and not _plain(t, dt, (C,)):
+            return False
+    for t, s in zip(mlp, ((hidden, C), (hidden, C), (hidden,), (C, hidden), (C,))):
+        if t is not None and not _plain(t, dt, s):
+            return False
+    for t, s in zip(call.get("biases", ()), plan.weight_shapes):
+        if t is not None and not _plain(t, dt, s[:1]):
+            return False
+    return True
 
 
 def block(plan, x, call, norm1, norm2, mlp, eps, *, rms=False, gated=False):
