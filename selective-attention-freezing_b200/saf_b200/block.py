@@ -72,7 +72,9 @@ class SafBlock(nn.Module):
         if torch.is_grad_enabled() or not x.is_cuda or x.dtype != torch.bfloat16 or torch.is_autocast_enabled("cuda"):
             return None
         m, mlp = self.main_block, self.mlp
-        if m._capture or (self.training and mlp.dropout.p > 0.0):
+        if not _layer.untouched((self.ln_1, LayerNorm), (m, SafCausalSelfAttention), (self.ln_2, LayerNorm), (mlp, MLP)):
+            return None
+        if m._capture or (mlp.training and mlp.dropout.p > 0.0):
             return None
         if m._fz_dirty:
             m._refresh_freeze_cache()

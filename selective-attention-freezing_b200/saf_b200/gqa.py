@@ -234,10 +234,11 @@ class SafQwenBlock(nn.Module):
 
     def forward(self, x, position_embeddings):
         if x.is_cuda and x.dtype == torch.bfloat16 and not torch.is_grad_enabled():
-            m, mlp = self.self_attn, self.mlp
-            call = m._layer_call(x, position_embeddings)
+            m, mlp, n1, n2 = self.self_attn, self.mlp, self.input_layernorm, self.post_attention_layernorm
+            call = None
+            if _layer.untouched((n1, RMSNorm), (m, SafGqaAttention), (n2, RMSNorm), (mlp, GatedMLP)):
+                call = m._layer_call(x, position_embeddings)
             if call is not None:
-                n1, n2 = self.input_layernorm, self.post_attention_layernorm
                 w = (mlp.gate_proj.weight, mlp.up_proj.weight, None, mlp.down_proj.weight, None)
                 norms = (n1.weight, None), (n2.weight, None)
                 if n1.variance_epsilon == n2.variance_epsilon and _layer.block_usable(m._plan, x, call, *norms, w, True):

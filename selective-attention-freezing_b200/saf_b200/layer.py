@@ -276,6 +276,19 @@ def attention_layer(plan, x, weights, rope, frozen, hidx, *, kvidx=None, sink_de
     return out.view(c.B, c.T, plan.C)
 
 
+_HOOKS = torch.nn.modules.module
+
+
+def untouched(*modules):
+    """Whether a block may read these sub-modules' parameters instead of calling them.  modules: (module, class) pairs.  A
+    module of another class (a replaced MLP, a subclass) or with a forward of its own computes something else, and hooks on
+    it, or on all modules, are to be called."""
+    for m, cls in modules:
+        if type(m) is not cls or m._forward_pre_hooks or m._forward_hooks or "forward" in m.__dict__:
+            return False
+    return not (_HOOKS._global_forward_pre_hooks or _HOOKS._global_forward_hooks)
+
+
 def block_usable(plan, x, call, norm1, norm2, mlp, gated):
     """bf16 inference of the whole block: every weight and norm in bf16 and of the plan's width, widths in whole 64-row
     blocks.  Arguments as `block` takes them; `usable` has seen the call's weights."""
