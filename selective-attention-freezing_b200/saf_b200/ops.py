@@ -573,19 +573,15 @@ def _slabs_of(rows, want=None):
     Returns (slab, [row0...]); `want` forces the slab width (every run must be a
     multiple of it).  One device->host copy per distinct index tensor object and version."""
     if want is not None:
-        slab, row0 = _slabs_of(rows)
-        if slab % want and want % slab:
+        _, _, runs = _runs_of(rows)
+        if any(n % want for _, n in runs):
             raise ValueError("rows do not form runs of %d consecutive rows" % want)
-        if slab == want:
-            return slab, row0
-        if slab > want:
-            return want, [r + o for r in row0 for o in range(0, slab, want)]
-        step = want // slab   # merge consecutive blocks of one run
-        merged = row0[::step]
-        for i, r in enumerate(merged):
-            if row0[i * step:(i + 1) * step] != list(range(r, r + want, slab)):
-                raise ValueError("rows do not form runs of %d consecutive rows" % want)
-        return want, merged
+        return want, [first + o for first, n in runs for o in range(0, n, want)]
+    return _runs_of(rows)[:2]
+
+
+def _runs_of(rows):
+    """(slab, [row0...], [(first row, length) of every run]) of `_slabs_of`, cached."""
     hit = _SLAB_CACHE.get(id(rows))
     if hit is not None and hit[0]() is rows and hit[1] == _ver(rows):
         return hit[2]
@@ -606,7 +602,7 @@ def _slabs_of(rows, want=None):
     row0 = []
     for first, n in runs:
         row0.extend(range(first, first + n, slab))
-    out = (slab, row0)
+    out = (slab, row0, runs)
     if len(_SLAB_CACHE) > 1024:
         _SLAB_CACHE.clear()
     _SLAB_CACHE[id(rows)] = (weakref.ref(rows), _ver(rows), out)
