@@ -261,12 +261,14 @@ def attention_layer(plan, x, weights, rope, frozen, hidx, *, kvidx=None, sink_de
     """x (B, T, C) -> bf16 (B, T, C).  weights: q, k, v, o; decomposed: (alpha, rho, z) buffers; learn: (alpha, rho)
     parameters that receive gradients (decomposed then holds their detached values and current normalisers);
     measure: called with the rotated q, k of the live heads.  Biases and residual go with inference."""
-    grad = torch.is_grad_enabled() and (x.requires_grad or learn is not None or any(w.requires_grad for w in weights))
+    enabled = torch.is_grad_enabled()
+    grad = enabled and (x.requires_grad or learn is not None or any(w.requires_grad for w in weights))
     if residual is not None:
         residual = _residual_rows(residual, x.shape[0] * x.shape[1], plan.C)
     c = _Call(x.shape[0], x.shape[1], _rows(x.detach()), weights, int(grad), rope, frozen, hidx, kvidx, sink_decay, patt, pidx,
               decomposed)
-    if grad:
+    # (also when nothing wants a gradient: forward-mode tangents are refused there instead of getting lost)
+    if grad or (enabled and biases is None and residual is None):
         ap, rp = learn if learn is not None else (None, None)
         return _LayerFunction.apply(x, *weights, ap, rp, plan, c, measure)
     out, work, sz = _forward(plan, c, biases, residual)

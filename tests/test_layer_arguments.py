@@ -126,3 +126,17 @@ def test_mlp_beyond_the_block_entrys_table_is_refused_before_its_norm_runs():
                               (1, 32768 + 128, _cabi.SAF_ERR_LIMIT)):
         b.gated, b.hidden = gated, hidden
         assert _cabi.lib.saf_block_workspace(C.byref(b), C.byref(n)) == rc
+
+
+def test_forward_mode_tangents_are_refused(monkeypatch):
+    """As by the operators, whose autograd functions have no forward mode either."""
+    import torch.autograd.forward_ad as fwad
+    from saf_b200 import layer
+    p, x, w = good()
+    monkeypatch.setattr(layer, "_forward", lambda plan, c, *a: (torch.zeros(c.B * c.T, plan.C, dtype=torch.bfloat16), x, (0, 0, 0, 0)))
+    i = torch.zeros(H, dtype=torch.int32)
+    assert layer.attention_layer(p, x, w, None, i, i).shape == x.shape
+    with fwad.dual_level():
+        for args in ((fwad.make_dual(x, torch.ones_like(x)), w), (x, [fwad.make_dual(w[0], torch.ones_like(w[0])), *w[1:]])):
+            with pytest.raises(RuntimeError):
+                layer.attention_layer(p, *args, None, i, i)
