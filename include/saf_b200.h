@@ -402,6 +402,8 @@ typedef struct SafBlockArgs {
   const void *b_in;         /* (hidden,) or null                                      */
   const void* w_out;        /* (C, hidden)                                            */
   const void* b_out;        /* (C,) or null                                           */
+  int32_t keep_projection;  /* 1: the projection and the attention output stay in the workspace, at the offsets of
+                               saf_attn_layer_workspace().  0: the MLP's hidden rows take their place               */
 } SafBlockArgs;
 int saf_block_workspace(const SafBlockArgs* args, int64_t* bytes);
 int saf_block_fwd(const SafBlockArgs* args, void* stream);

@@ -375,20 +375,21 @@ int saf_attn_layer_bwd(const SafAttnLayerBwdArgs* args, void* stream) {
 // ---- the transformer block around the layer (inference) ----------------------------------------------------------------
 namespace {
 
-struct BlockLayout {
-  int64_t layer, normed, x1, hidden, total;
+struct BlockLayout {       // (the layer's workspace comes first)
+  int64_t normed, x1, hidden, total;
 };
 BlockLayout block_layout(const SafBlockArgs& b) {
   const Dims d = dims_of(b.layer);
   BlockLayout l;
-  l.layer = 0;
-  int64_t at = up(fwd_layout(b.layer, d).total);
+  // The layer's part is read for the last time by its output projection, two launches before the first write of the MLP's
+  // hidden rows, which may lie there.
+  const int64_t layer = up(fwd_layout(b.layer, d).total), hidden = up(d.tok * b.hidden * 2);
+  l.hidden = b.keep_projection ? layer : 0;
+  int64_t at = b.keep_projection ? layer + hidden : std::max(layer, hidden);
   l.normed = at;
   at += up(d.tok * d.C * 2);
   l.x1 = at;
   at += up(d.tok * d.C * 2);
-  l.hidden = at;
-  at += up(d.tok * b.hidden * 2);
   l.total = at;
   return l;
 }
@@ -471,7 +472,6 @@ int saf_block_fwd(const SafBlockArgs* args, void* stream) {
   a.ldr = b.layer.ldx;
   a.out = x1;
   a.ldo = d.C;
-  a.work_bytes = l.normed;
   a.after_library_launch = 1;       // the norm, which writes no weights
   if ((rc = saf_attn_layer_fwd(&a, stream))) return rc;
   if ((rc = launch_layernorm(x1, d.C, b.n2_w, b.n2_b, normed, d.C, M, d.C, b.eps, SAF_BF16, b.rms, st))) return rc;

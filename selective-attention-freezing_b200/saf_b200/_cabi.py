@@ -119,6 +119,7 @@ class SafBlockArgs(C.Structure):
         ("layer", SafAttnLayerArgs),
         ("n1_w", C.c_void_p), ("n1_b", C.c_void_p), ("n2_w", C.c_void_p), ("n2_b", C.c_void_p),
         ("w_in", C.c_void_p), ("w_up", C.c_void_p), ("b_in", C.c_void_p), ("w_out", C.c_void_p), ("b_out", C.c_void_p),
+        ("keep_projection", C.c_int32),
     ]
 
 

@@ -326,7 +326,8 @@ def block(plan, x, call, norm1, norm2, mlp, eps, *, rms=False, gated=False):
     sz = plan.sizes(a)
     tok, Cw = c.B * c.T, plan.C
     dev = x.device
-    key = ("block", c.B, c.T, g.hidden)
+    g.keep_projection = int(measure is not None)
+    key = ("block", c.B, c.T, g.hidden, g.keep_projection)
     n = plan._sizes.get(key)
     if n is None:
         g.layer = a

@@ -104,3 +104,22 @@ def test_an_input_of_other_dimensions_is_refused(build):
         for other in (x[0], x[None]):
             with pytest.raises(ValueError):
                 b(other, rope)
+
+
+@pytest.mark.gpu
+def test_statistics_of_a_fused_block_are_those_of_its_layer():
+    """The accumulators read q and k after the block's last launch."""
+    from saf_b200.capture import AttentionMoments, LogitMoments
+    b, names, rope, x = make(dense_block, "cuda")
+    with torch.inference_mode():
+        y = b(x, rope)
+        got = []
+        for fused in (True, False):
+            a, l = AttentionMoments(3, T, "cuda"), LogitMoments(3, T, "cuda", with_var=True)
+            b.main_block.set_statistics(a, l)
+            z = b(x, rope) if fused else b.main_block(b.ln_1(x), rope=rope)
+            b.main_block.set_statistics(None)
+            got.append([a.mean, a.head_m2, a.neg_entropy, l.mean, l.m2])
+            assert not fused or torch.equal(z, y)
+    for u, v in zip(*got):
+        assert ((u.double() - v.double()).norm() / v.double().norm().clamp_min(1e-30)).item() <= 1e-6

@@ -140,3 +140,40 @@ def test_forward_mode_tangents_are_refused(monkeypatch):
         for args in ((fwad.make_dual(x, torch.ones_like(x)), w), (x, [fwad.make_dual(w[0], torch.ones_like(w[0])), *w[1:]])):
             with pytest.raises(RuntimeError):
                 layer.attention_layer(p, *args, None, i, i)
+
+
+def test_layer_structs_match_the_header(tmp_path):
+    import ctypes as C
+    import os
+    import subprocess
+    from saf_b200 import _cabi
+    include = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "include")
+    names = ("SafAttnLayerArgs", "SafAttnLayerBwdArgs", "SafBlockArgs")
+    prog = tmp_path / "sz.c"
+    prog.write_text('#include <stdio.h>\n#include "saf_b200.h"\nint main(){%s return 0;}\n'
+                    % "".join('printf("%%zu\\n",sizeof(%s));' % n for n in names))
+    exe = tmp_path / "sz"
+    subprocess.check_call(["gcc", "-I", include, str(prog), "-o", str(exe)])
+    assert [int(v) for v in subprocess.check_output([str(exe)]).split()] == [C.sizeof(getattr(_cabi, n)) for n in names]
+
+
+def test_hidden_rows_of_a_block_lie_where_the_attention_was():
+    """The block's workspace holds no more than what lives at one time: normed and x1 beside the larger of the layer's part
+    and the hidden rows; all of it only when the projection is kept."""
+    import ctypes as C
+    from saf_b200 import _cabi
+    b = _cabi.SafBlockArgs()
+    b.struct_size = C.sizeof(b)
+    b.layer, keep = layer_struct(width=128)
+    B, T = 4, 512
+    b.layer.attn.B, b.layer.attn.T = B, T
+    part, n = (C.c_int64 * 4)(), C.c_int64()
+    assert _cabi.lib.saf_attn_layer_workspace(C.byref(b.layer), part) == 0
+    rows = B * T * 128 * 2
+    for hidden in (64, 128, 512, 4096):
+        b.hidden = hidden
+        got = []
+        for b.keep_projection in (0, 1):
+            assert _cabi.lib.saf_block_workspace(C.byref(b), C.byref(n)) == 0
+            got.append(n.value)
+        assert got == [2 * rows + max(part[0], B * T * hidden * 2), 2 * rows + part[0] + B * T * hidden * 2]
