@@ -70,3 +70,18 @@ def test_tables_whose_halves_differ(M, T):
     row = torch.arange(M, device="cuda") % T
     rot = [t[:, live] * cos[row][:, None] + torch.cat([-t[:, live, hd // 2:], t[:, live, :hd // 2]], -1) * sin[row][:, None] for t in full[:2]]
     assert rel(y, torch.cat([*rot, full[2]], dim=1)) <= REL
+
+
+@pytest.mark.parametrize("M", [1, 300, 1500, 8193, 8500])
+@pytest.mark.parametrize("K,N", [(192, 192), (64, 832), (1024, 2240)])
+@pytest.mark.parametrize("residual", [False, True])
+def test_every_row_of_every_block(M, K, N, residual):
+    """Per row and 64-column block, so that one wrong block of a ragged last row tile shows: each value is rounded to bf16
+    once, 2^-9 of it at most, so the norm over a block differs by no more than 2^-9 of it; as much again for fp32 sums."""
+    from saf_b200 import ops
+    x, w = rand(M, K, seed=M), rand(N, K, seed=N, scale=0.05)
+    res = rand(M, N, seed=7) if residual else None
+    y = ops.linear_act(x, w, None, residual=res).double().view(M, -1, 64)
+    ref = x.double() @ w.double().t()
+    ref = (ref + res.double() if residual else ref).view(M, -1, 64)
+    assert ((y - ref).norm(dim=-1) / ref.norm(dim=-1)).max().item() <= REL
