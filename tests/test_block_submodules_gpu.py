@@ -22,7 +22,6 @@ def grouped_block():
     from saf_b200.gqa import SafQwenBlock
     b = SafQwenBlock(SimpleNamespace(hidden_size=256, num_attention_heads=4, num_key_value_heads=2, head_dim=64, attention_bias=True,
                                      intermediate_size=512))
-    b.self_attn.set_frozen(sink_decay=[1], sd_params=([0.2], [0.9]))
     return b, ("input_layernorm", "self_attn", "post_attention_layernorm", "mlp"), rope_tables(64, T)
 
 
@@ -30,7 +29,10 @@ def make(build, device):
     torch.manual_seed(0)
     b, names, rope = build()
     x = torch.randn(2, T, 256).to(device, torch.bfloat16)
-    return b.to(device, torch.bfloat16).eval(), names, tuple(t.to(device) for t in rope), x
+    b = b.to(device, torch.bfloat16).eval()
+    if build is grouped_block:                  # (its structured heads' numbers are fp32: after the cast)
+        b.self_attn.set_frozen(sink_decay=[1], sd_params=([0.2], [0.9]))
+    return b, names, tuple(t.to(device) for t in rope), x
 
 
 class OtherMLP(nn.Module):
