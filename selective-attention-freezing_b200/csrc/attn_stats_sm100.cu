@@ -25,7 +25,7 @@
 //   warp 8: TMA producer ([Q_b tile | K_b tile] ring), warp 9: MMA issuer
 //   warps 10-11: running tiles in and out: one thread with TMA, or (T not a multiple of 4: rows do not start on 16-byte
 //                boundaries) both warps with 4-byte cp.async and coalesced stores
-// Every wait is bounded; on expiry the kernel records a code in *status and falls through.
+// Every mbarrier wait is bounded; on expiry the kernel records a code in *status and falls through.
 #include <type_traits>
 
 #include "saf_internal.h"

@@ -17,7 +17,7 @@
 //               then the epilogue: TMEM -> bf16 -> swizzled staging -> TMA store
 // Work per stage: 2 * NB * 128 * 64 * head_dim MACs against 32 KB of pattern read from HBM: at head_dim 64
 // that is ~1500 tensor cycles per 32 KB per SM, i.e. the kernel sits at the HBM roofline of the pattern.
-// All waits are bounded.
+// All mbarrier waits are bounded.
 #pragma once
 #include "saf_internal.h"
 #include "sm100_prims.cuh"

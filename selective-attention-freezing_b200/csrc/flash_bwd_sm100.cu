@@ -23,7 +23,7 @@
 // first 64 columns of the tile they read (see operand_columns_read); the TS MMA takes K step ks from
 // columns 8 ks.
 // The sm_scale factor of dS is applied once to the finished dK / dQ accumulators.
-// Every wait is bounded; on expiry the kernel records a code in *status and falls through.
+// Every mbarrier wait is bounded; on expiry the kernel records a code in *status and falls through.
 #include "saf_internal.h"
 #include "dense_pv_body.cuh"
 #include "scan_body.cuh"

@@ -10,7 +10,7 @@
 //       the finished 128 x 256 tile is stored through the weight-gradient maps, 64 rows at a time, at the
 //       rows the two blocks own (the reference zero-fills and index_copy_'s a dense product instead).
 // Same persistent, warp-specialised CTA as the forward GEMM: warp 0 TMA, warp 1 MMA issuer, warps 2-5
-// epilogue; 128x256 tiles, K step 64, 4 stages, two TMEM accumulators.  All waits are bounded.
+// epilogue; 128x256 tiles, K step 64, 4 stages, two TMEM accumulators.  All mbarrier waits are bounded.
 //
 // A training layer keeps fp32 master weights and an fp32 residual stream, so both products also exist with an fp32
 // result (F32OUT: the accumulator leaves the kernel unrounded, 32 columns per 16 KB staging block), and DW can be

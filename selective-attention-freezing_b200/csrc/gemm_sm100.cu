@@ -22,7 +22,7 @@
 //               65536 x 768 -> 768 with residual 125 -> 90 us (row by row from global memory before).
 // Large products run the same kernel as CTA PAIRS (template parameter PAIR, a cluster of two): one 256x256 tile per
 // pair through tcgen05.mma.cta_group::2, each CTA loading its 128 rows of x and half of the weight tile (see GCfg).
-// All waits are bounded; a wait that runs out sets *status and the CTA drains.
+// All mbarrier waits are bounded; a wait that runs out sets *status and the CTA drains.
 #include <algorithm>
 #include <atomic>
 

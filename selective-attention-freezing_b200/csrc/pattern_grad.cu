@@ -11,7 +11,7 @@
 //                 delta_i comes from a small pre-pass (one warp per row)
 //     warp 16: TMA producer (dO_i ring), warp 17: MMA issuer
 //   generic kernel (any dtype / head_dim): 32x32 tile pairs on the CUDA cores, fp32 throughout.
-// Every wait is bounded; on expiry the kernel records a code in *status and falls through.
+// Every mbarrier wait is bounded; on expiry the kernel records a code in *status and falls through.
 #include "saf_internal.h"
 #include "sm100_prims.cuh"
 

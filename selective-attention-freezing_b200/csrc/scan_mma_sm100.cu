@@ -33,7 +33,7 @@
 //                             of row 127 publishes the block's end state before anything else, so the serial chain
 //                             from block to block is 64 fused multiply-adds long and the two warpgroups overlap
 //                             otherwise.
-// Every wait is bounded.
+// Every mbarrier wait is bounded.
 #include <algorithm>
 
 #include "saf_internal.h"

@@ -202,8 +202,9 @@ class _LayerFunction(torch.autograd.Function):
     @staticmethod
     @torch.autograd.function.once_differentiable
     def backward(ctx, dout):
-        work, x2, wq, wk, wv, wo, patt, pidx, alpha, rho, z, cos, sin, frozen, hidx = ctx.saved_tensors[:15]
-        sink_decay = ctx.saved_tensors[15:] or None
+        saved = ctx.saved_tensors          # once: a checkpointed layer unpacks what it recomputed a single time
+        work, x2, wq, wk, wv, wo, patt, pidx, alpha, rho, z, cos, sin, frozen, hidx = saved[:15]
+        sink_decay = saved[15:] or None
         plan, sz = ctx.plan, ctx.sz
         B, T = ctx.bt
         dev = dout.device

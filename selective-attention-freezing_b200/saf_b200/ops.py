@@ -695,9 +695,10 @@ class _RowSlicedLinearN(torch.autograd.Function):
 
     @staticmethod
     def backward(ctx, dout):
-        x, rows = ctx.saved_tensors[:2]
+        saved = ctx.saved_tensors          # once: a checkpointed layer unpacks what it recomputed a single time
+        x, rows = saved[:2]
         nw = ctx.nw
-        weights = list(ctx.saved_tensors[2:2 + nw])
+        weights = list(saved[2:2 + nw])
         slab, row0 = _slabs_of(rows, want=ctx.rope[1] if ctx.rope is not None else None)
         n_per = len(row0)
         sw = [i for i in range(nw) for _ in range(n_per)]
@@ -706,7 +707,7 @@ class _RowSlicedLinearN(torch.autograd.Function):
         x2 = _as_2d(x)
         if ctx.rope is not None:
             # gradient w.r.t. the un-rotated projection: adjoint rotation of a private copy
-            cos, sin = ctx.saved_tensors[2 + nw:4 + nw]
+            cos, sin = saved[2 + nw:4 + nw]
             dout2 = dout2.clone() if dout2.data_ptr() == dout.data_ptr() else dout2
             _call(x, lib.saf_rope_slabs, dout2.data_ptr(), dout2.stride(0), dout2.shape[0], len(sr), slab, ctx.rope[0],
                                      None, cos.data_ptr(), sin.data_ptr(), _dt(dout2), 1)

@@ -85,3 +85,16 @@ def test_the_same_gradients_whichever_way_the_graph_is_kept(dtype):
     for other in ([plain[0], *first], [plain[0], *again], again_from_file, moved, aside):
         for a, b in zip(plain, other):
             assert torch.equal(a, b)
+
+
+def test_checkpointed_fp32_layer():
+    """The operators' own backward, which an fp32 layer walks."""
+    m, rope, _, g = build(4, 64, 200, [1], 9, torch.float32)
+    x = torch.randn(1, 200, 256, generator=g).cuda()
+    dy = torch.randn(1, 200, 256, generator=g).cuda()
+    got = []
+    for run in (lambda t: m(t, rope=rope), lambda t: checkpoint(lambda u: m(u, rope=rope), t, use_reentrant=False)):
+        xx = x.clone().requires_grad_(True)
+        got.append(torch.autograd.grad(run(xx), [xx, *m.parameters()], dy))
+    for a, b in zip(*got):
+        assert torch.equal(a, b)
