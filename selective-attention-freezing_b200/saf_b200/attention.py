@@ -375,8 +375,9 @@ class SafCausalSelfAttention(nn.Module):
         if act_dt != torch.bfloat16 or not self._live or (self.dropout > 0.0 and self.training):
             return None
         grad = torch.is_grad_enabled()
-        w = (self.q_proj.weight, self.k_proj.weight, self.v_proj.weight, self.c_proj.weight)
-        bias = self.q_proj.bias is not None
+        q_proj = self.q_proj
+        w = (q_proj.weight, self.k_proj.weight, self.v_proj.weight, self.c_proj.weight)
+        bias = q_proj.bias is not None
         # without autocast, training wants x and the weights in one dtype (the separate operators say so)
         mixed = grad and w[0].dtype != x.dtype and not torch.is_autocast_enabled("cuda")
         if (grad and bias) or mixed or not _layer.usable(self._plan, x, w, grad):

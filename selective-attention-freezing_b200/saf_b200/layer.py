@@ -119,8 +119,8 @@ def _plain(t, dtype, shape):
 def usable(plan, x, weights, training):
     """True when the whole layer can run through the library's layer entry, which takes every size from the plan and the
     first two dimensions of x: other shapes stay with the operators (or are refused there)."""
-    dt = weights[0].dtype
-    if not (x.dtype in _DT and dt in _DT and x.dim() == 3 and x.shape[2] == plan.C and x.numel() > 0 and plan.shapes_ok(training)
+    dt, shape = weights[0].dtype, x.shape
+    if not (x.dtype in _DT and dt in _DT and len(shape) == 3 and shape[2] == plan.C and x.numel() > 0 and plan.shapes_ok(training)
             and x.data_ptr() % 16 == 0):
         return False
     for w, s in zip(weights, plan.weight_shapes):
@@ -132,6 +132,8 @@ def usable(plan, x, weights, training):
 def _rows(x):
     """x as rows the library reads by TMA: 16-byte aligned, a whole number of 16-byte pieces and at least a row apart (an
     expanded tensor's rows are not); fp32 rows follow each other."""
+    if x.is_contiguous() and x.data_ptr() % 16 == 0:
+        return x
     x2 = ops._as_2d(x)
     step, C = _ld(x2), x2.shape[1]
     if x2.data_ptr() % 16 or (step != C if x2.dtype == torch.float32 else step % 8 or step < C):
@@ -139,9 +141,9 @@ def _rows(x):
     return x2
 
 
-def _ld(x2):
-    """Row stride of a matrix; torch reports anything for a single row."""
-    return x2.stride(0) if x2.shape[0] > 1 else x2.shape[1]
+def _ld(x):
+    """Row stride of a contiguous tensor or a matrix (torch reports any stride for a single row)."""
+    return x.shape[-1] if x.is_contiguous() else x.stride(0)
 
 
 def _blob(n, device):
@@ -313,18 +315,15 @@ def block_usable(plan, x, call, norm1, norm2, mlp, gated):
 def block(plan, x, call, norm1, norm2, mlp, eps, *, rms=False, gated=False):
     """One pre-norm block, x (B, T, C) bf16 -> (B, T, C), in one library call.  call: the keyword arguments of
     `attention_layer`; norm: (weight, bias); mlp: (w_in, w_up, b_in, w_out, b_out)."""
-    kw = dict(call)
-    weights, rope, frozen, hidx = kw.pop("weights"), kw.pop("rope"), kw.pop("frozen"), kw.pop("hidx")
-    biases, measure = kw.pop("biases", None), kw.pop("measure", None)
-    kw.pop("learn", None)
-    c = _Call(x.shape[0], x.shape[1], _bf16_rows(x), weights, 0, rope, frozen, hidx, **kw)
+    biases, measure = call.get("biases"), call.get("measure")
+    c = _Call(x.shape[0], x.shape[1], _bf16_rows(x), call["weights"], 0, call["rope"], call["frozen"], call["hidx"], call.get("kvidx"),
+              call.get("sink_decay"), call.get("patt"), call.get("pidx"), call.get("decomposed", (None, None, None)))
     g = SafBlockArgs()
     g.struct_size = C.sizeof(SafBlockArgs)
     g.rms, g.gated, g.hidden, g.eps = int(rms), int(gated), mlp[0].shape[0], eps
     a = plan.args(c)
     if biases is not None:
         a.bq, a.bk, a.bv, a.bo = [None if b is None else b.data_ptr() for b in biases]
-    sz = plan.sizes(a)
     tok, Cw = c.B * c.T, plan.C
     dev = x.device
     g.keep_projection = int(measure is not None)
@@ -334,6 +333,8 @@ def block(plan, x, call, norm1, norm2, mlp, eps, *, rms=False, gated=False):
         g.layer = a
         out = C.c_int64()
         check(lib.saf_block_workspace(C.byref(g), C.byref(out)))
+        if len(plan._sizes) >= 64:
+            plan._sizes.clear()
         n = plan._sizes[key] = out.value
     work = _blob(n, dev)
     out = torch.empty((tok, Cw), dtype=torch.bfloat16, device=dev)
@@ -347,6 +348,6 @@ def block(plan, x, call, norm1, norm2, mlp, eps, *, rms=False, gated=False):
     g.w_in, g.w_up, g.b_in, g.w_out, g.b_out = [None if t is None else t.data_ptr() for t in mlp]
     ops._call(c.x, lib.saf_block_fwd, C.byref(g))
     if measure is not None:
-        q, k, _, _ = projection_views(plan, work, sz, c.B, c.T)
+        q, k, _, _ = projection_views(plan, work, plan.sizes(a), c.B, c.T)
         measure(q, k)
     return out.view(c.B, c.T, Cw)
