@@ -17,9 +17,9 @@
 //               once per row of tiles, before the accumulator is waited for, so their latency hides behind the MMAs.
 //               With K = 768 a tile's products take 6144 cycles; one group of four warps needed longer than that for
 //               a GELU or (by far) a rotation of 128-row slabs, whose 64 cos and 64 sin values it had to read anew for
-//               every tile: 65536 x 1536 -> 1664, 128-row slabs, 692 -> 322 us; 65536 x 768 -> 1920, 64-row, 209 -> 190.
+//               every tile: 65536 x 1536 -> 1664, 128-row slabs, 692 -> 333 us; 65536 x 768 -> 1920, 64-row, 209 -> 175.
 //               A residual comes by TMA into the block's own staging place, fetched into L2 while the products run:
-//               65536 x 768 -> 768 with residual 125 -> 90 us (row by row from global memory before).
+//               65536 x 768 -> 768 with residual 125 -> 86 us (row by row from global memory before).
 // Large products run the same kernel as CTA PAIRS (template parameter PAIR, a cluster of two): one 256x256 tile per
 // pair through tcgen05.mma.cta_group::2, each CTA loading its 128 rows of x and half of the weight tile (see GCfg).
 // All mbarrier waits are bounded; a wait that runs out sets *status and the CTA drains.
@@ -165,7 +165,8 @@ indexed_gemm_kernel(const __grid_constant__ CUtensorMap mapX, const __grid_const
   // K = 8960 that is 340 MB, and x comes from memory once per column tile.  65536 x 8960 -> 1536 with that order and its
   // sibling 1536 -> 2 x 8960 2372 us on average, now 1882.)  A rotated product keeps the runs: its epilogue holds the
   // row's cos / sin values over the run, and reading them anew for every tile cost more than x from memory
-  // (65536 x 768 -> 1920: 180 us with runs, 260 without; at 128-row slabs no difference).
+  // (65536 x 768 -> 1920, before the tables were read as whole lines: 180 us with runs, 260 without; at 128-row slabs no
+  // difference).
   const int tile_lo = p.runs ? (int)((int64_t)unit * total_tiles / n_units) : unit;
   const int tile_hi = p.runs ? (int)((int64_t)(unit + 1) * total_tiles / n_units) : total_tiles;
   const int tile_step = p.runs ? 1 : n_units;

@@ -12,9 +12,9 @@
 //             its Q and K slabs;  dx = d[QKV] W and dW = d[QKV]^T x as ONE product each, fp32 when the tensor is fp32
 //
 // (nanogpt/model.py:946-1077, the cheap path of the reference's module.)  Measured on a B200, forward and backward of one
-// training layer under bf16 autocast: 12 x 64, T = 1024, B = 8 1.2-1.5 ms (41 launches, host-bound) -> 0.33 ms (14
-// launches); 16 x 128, T = 8192, B = 2 4.16 -> 3.55 ms (0.8 ms of it were fills, copies, conversions and additions);
-// one inference layer of 4 x 64, T = 512, B = 2 163 -> 41 us.
+// training layer under bf16 autocast: 12 x 64, T = 1024, B = 8 1.2-1.5 ms (41 launches, host-bound) -> 0.30 ms (14
+// launches); 16 x 128, T = 8192, B = 2 4.16 -> 3.43 ms (0.8 ms of it were fills, copies, conversions and additions);
+// one inference layer of 4 x 64, T = 512, B = 2 163 -> 39 us.
 #include <string.h>
 
 #include <algorithm>
