@@ -98,3 +98,71 @@ def test_checkpointed_fp32_layer():
         got.append(torch.autograd.grad(run(xx), [xx, *m.parameters()], dy))
     for a, b in zip(*got):
         assert torch.equal(a, b)
+
+
+def test_inference_and_training_captured_into_graphs():
+    """Replays follow the inputs and weights in place, as eager calls do."""
+    from saf_b200.block import SafBlock
+    m, rope, _, g = build(4, 64, 300, [2], 4, torch.float32)
+    cfg = SimpleNamespace(n_embd=256, n_head=4, block_size=300, bias=False, dropout=0.0, position_encoding="rope")
+    b = SafBlock(cfg)
+    b.main_block.freeze_heads_sink_decay([1], [0.2], [0.9])
+    b = b.cuda().bfloat16().eval()
+    x = torch.randn(2, 300, 256, generator=g).cuda().requires_grad_(True)
+    xb = x.detach().bfloat16()
+    dy = torch.randn(2, 300, 256, generator=g).cuda().bfloat16()
+
+    def infer():
+        with torch.inference_mode(False), torch.no_grad():
+            return [b(b(xb, rope=rope), rope=rope)]
+
+    def train():
+        with torch.autocast("cuda", dtype=torch.bfloat16):
+            y = m(x, rope=rope)
+        return [y.detach(), *torch.autograd.grad(y, [x, *m.parameters()], dy)]
+
+    for fn in (infer, train):
+        s = torch.cuda.Stream()
+        s.wait_stream(torch.cuda.current_stream())
+        with torch.cuda.stream(s):
+            fn()
+        torch.cuda.current_stream().wait_stream(s)
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph):
+            static = fn()
+        for _ in range(3):
+            with torch.no_grad():
+                x.copy_(torch.randn(x.shape, generator=g))
+                xb.copy_(x)
+                m.q_proj.weight.mul_(1.25)
+                b.mlp.c_fc.weight.mul_(0.75)
+                b.main_block.c_proj.weight.mul_(1.25)
+            graph.replay()
+            graph.replay()
+            got = [t.clone() for t in static]
+            for u, v in zip(got, fn()):
+                assert torch.equal(u, v)
+
+
+def test_two_threads_with_streams_of_their_own():
+    import threading
+    m, rope, _, g = build(4, 64, 500, [1], 12, torch.float32)
+    xs = [torch.randn(2, 500, 256, generator=g).cuda() for _ in range(2)]
+    dy = torch.randn(2, 500, 256, generator=g).cuda().bfloat16()
+    want = [one_pass(m, x, rope, dy) for x in xs]
+    torch.cuda.synchronize()
+    bad = []
+
+    def work(i):
+        with torch.cuda.stream(torch.cuda.Stream()):
+            for _ in range(10):
+                got = one_pass(m, xs[i], rope, dy)
+                bad.extend(k for k, (a, b) in enumerate(zip(got, want[i])) if not torch.equal(a, b))
+        torch.cuda.synchronize()
+
+    threads = [threading.Thread(target=work, args=(i,)) for i in range(2)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not bad
