@@ -13,8 +13,8 @@
 //
 // (nanogpt/model.py:946-1077, the cheap path of the reference's module.)  Measured on a B200, forward and backward of one
 // training layer under bf16 autocast: 12 x 64, T = 1024, B = 8 1.2-1.5 ms (41 launches, host-bound) -> 0.30 ms (14
-// launches); 16 x 128, T = 8192, B = 2 4.16 -> 3.43 ms (0.8 ms of it were fills, copies, conversions and additions);
-// one inference layer of 4 x 64, T = 512, B = 2 163 -> 39 us.
+// launches); 16 x 128, T = 8192, B = 2 4.16 -> 3.36 ms (0.8 ms of it were fills, copies, conversions and additions);
+// one inference layer of 4 x 64, T = 512, B = 2 163 -> 41 us.
 #include <string.h>
 
 #include <algorithm>
