@@ -81,10 +81,19 @@ int make_tensor_map(CUtensorMap* out, CUtensorMapDataType type, const void* base
     es[i] = 1;
     if (i > 0) s[i - 1] = strides_bytes[i];
   }
-  CUresult r = enc(out, type, (cuuint32_t)rank, const_cast<void*>(base), d, s, b, es,
-                   CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
-                   l2_256 ? CU_TENSOR_MAP_L2_PROMOTION_L2_256B : CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
-                   CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  auto encode = [&] {
+    return enc(out, type, (cuuint32_t)rank, const_cast<void*>(base), d, s, b, es, CU_TENSOR_MAP_INTERLEAVE_NONE,
+               CU_TENSOR_MAP_SWIZZLE_128B, l2_256 ? CU_TENSOR_MAP_L2_PROMOTION_L2_256B : CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+               CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  };
+  CUresult r = encode();
+  if (r == CUDA_ERROR_INVALID_CONTEXT) {
+    // A thread that has made no runtime call yet (the autograd engine's, a new one of the caller's) has no context for this
+    // driver call; selecting its device gives it the primary one.
+    int dev = 0;
+    if (cudaGetDevice(&dev) == cudaSuccess && cudaSetDevice(dev) == cudaSuccess) r = encode();
+    else cudaGetLastError();
+  }
   if (r != CUDA_SUCCESS) return fail(SAF_ERR_CUDA, "cuTensorMapEncodeTiled failed with CUresult %d", (int)r);
   return SAF_OK;
 }

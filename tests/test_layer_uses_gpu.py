@@ -166,3 +166,44 @@ def test_two_threads_with_streams_of_their_own():
     for t in threads:
         t.join()
     assert not bad
+
+
+@pytest.mark.parametrize("what", ["layer", "block", "backward"])
+def test_the_first_cuda_call_of_a_thread(what):
+    """Nothing on the thread has given it a context: the allocator serves from its cache and no torch kernel runs before."""
+    import subprocess
+    import sys
+    import os
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    code = """
+import sys, threading
+sys.path[:0] = [%r, %r]
+import torch
+from types import SimpleNamespace
+from saf_b200.block import SafBlock
+torch.manual_seed(0)
+b = SafBlock(SimpleNamespace(n_embd=256, n_head=4, block_size=64, bias=False, dropout=0.0, position_encoding="none"))
+b = b.cuda().bfloat16().eval()
+m, x = b.main_block, torch.randn(2, 64, 256).cuda().bfloat16().requires_grad_(True)
+dy = torch.randn(2, 64, 256).cuda().bfloat16()
+keep = []
+def once():
+    if %r == "backward":
+        y = m(x)
+        torch.empty(1 << 26, dtype=torch.uint8, device="cuda")       # what the backward allocates comes from this block
+        torch.cuda.synchronize()
+        keep.append(torch.autograd.grad(y, [x, *m.parameters()], dy)[0])
+    else:
+        with torch.inference_mode():
+            keep.append(b(x) if %r == "block" else m(x))
+if %r == "backward":
+    once()                                                           # the engine's thread, on its first call
+else:
+    once(); once()
+    keep.pop()                                                       # its output and workspace are free again
+    torch.cuda.synchronize()
+    t = threading.Thread(target=once); t.start(); t.join()
+    assert len(keep) == 2 and torch.equal(keep[0], keep[1])
+assert torch.isfinite(keep[-1].float()).all()
+""" % (root, os.path.join(root, "selective-attention-freezing_b200"), what, what, what)
+    subprocess.run([sys.executable, "-c", code], check=True, timeout=180)
