@@ -1,4 +1,4 @@
-// CUDA-core indexed linear (fp32 accumulate): forward for fp32 / shapes the
+// CUDA-core indexed linear (fp32 accumulate): forward for rows that are not whole 16-byte pieces / shapes the
 // tensor-core GEMM does not take, and both backward products.  Weight rows are
 // addressed in place through the slab table; no gathered weight copy exists
 // (the reference builds one per call, kernel/indexed_linear.py:93).
@@ -8,34 +8,14 @@
 //   dw  : dW[n][c]   = sum_m dout[m,n] x[m,c], db[n] = sum_m dout[m,n]   (:50-55, 110-121)
 // where n = g*slab + r addresses row (row0[g] + r) of weight matrix slab_weight[g].
 // Also: the freeze-time row normaliser of decomposed patterns (kernel/fused_attn.py:101-116).
+#include "linear_tables.cuh"
 #include "saf_internal.h"
 #include "sm100_prims.cuh"
 
 namespace saf {
 namespace {
 
-constexpr int MAX_SLABS = 2048;
-struct SlabTable {
-  int32_t row0[MAX_SLABS];
-  uint8_t weight[MAX_SLABS];
-  uint8_t rope[MAX_SLABS];
-};
-struct WeightSet {
-  const void* w[SAF_MAX_WEIGHTS];
-  const void* b[SAF_MAX_WEIGHTS];
-  int64_t ldw[SAF_MAX_WEIGHTS];
-  int64_t cdw[SAF_MAX_WEIGHTS];
-};
-
 constexpr int TM = 64, TN = 64, TK = 16, GNT = 256;
-
-// pointer to element (row n of the selection, column c)
-template <typename T>
-__device__ __forceinline__ const T* welem(const WeightSet& ws, const SlabTable& tb, int n, int slab, int c) {
-  const int g = n / slab, r = n - g * slab;
-  const int w = tb.weight[g];
-  return reinterpret_cast<const T*>(ws.w[w]) + (int64_t)(tb.row0[g] + r) * ws.ldw[w] + (int64_t)c * ws.cdw[w];
-}
 
 __device__ __forceinline__ void mma_tile(const float (*As)[TM + 1], const float (*Bs)[TN + 1], int ty, int tx,
                                          float (&acc)[4][4]) {
@@ -136,176 +116,6 @@ __global__ void __launch_bounds__(GNT) linear_generic_kernel(const T* __restrict
   }
 }
 
-// ---- fp32, 16-byte rows ----------------------------------------------------------------------------------------------
-// Bound by the FMA pipe once shared memory keeps up: a thread owns 8 x 8 outputs and reads its operands as float4 along
-// whichever index they store contiguously, 16 reads for 256 FMAs (the any-shape kernel above: 8 for 16).  An operand
-// stays in its own layout, K-contiguous rows (stride 36: 8 neighbouring rows' float4 reads hit all banks once) or
-// row-contiguous K slices, so cp.async brings every tile and nothing is transposed.  Training products of one narrow
-// layer are only 64 to 400 tiles of 64 x 64, so a CTA is four groups of 64 threads that each take a quarter of every K
-// slice and add their sums at the end: four times the warps in flight for the same tiles, and shorter chains of sums.
-// 2048 x 768 x 768 on a B200: forward 217 -> 82 us, dx 209 -> 84, dW 380 -> 68.
-constexpr int FK = 32, FGROUPS = 4, FKG = FK / FGROUPS, FLD = FK + 4, FSTAGES = 3, FRED = 68;
-
-// acc[i][j] = element (frag_row(i), frag_row(j)) of the group's tile
-template <bool KC>
-__device__ __forceinline__ int frag_at(int t, int i) { return KC ? t + 8 * i : t * 4 + (i & 3) + 32 * (i >> 2); }
-__device__ __forceinline__ float f4c(const float4& v, int e) { return e == 0 ? v.x : (e == 1 ? v.y : (e == 2 ? v.z : v.w)); }
-
-template <int MODE>
-__global__ void __launch_bounds__(GNT, 2) linear_f32_kernel(const float* __restrict__ A, int64_t lda, const float* __restrict__ X,
-                                                            int64_t ldx, float* __restrict__ Cout, int64_t ldc, int M, int C,
-                                                            int N, int slab, const __grid_constant__ WeightSet ws,
-                                                            const __grid_constant__ SlabTable tb) {
-  constexpr bool A_KC = MODE != 2, B_KC = MODE == 0;
-  constexpr int A_F = A_KC ? TM * FLD : FK * TM, B_F = B_KC ? TN * FLD : FK * TN;
-  extern __shared__ __align__(16) float lin_smem[];
-  const int tid = threadIdx.x, kg = tid >> 6, ty = (tid & 63) >> 3, tx = tid & 7;
-  const int I = (MODE == 2) ? N : M;
-  const int J = (MODE == 0) ? N : C;
-  const int K = (MODE == 0) ? C : (MODE == 1 ? N : M);
-  const int i0 = blockIdx.y * TM, j0 = blockIdx.x * TN;
-  // MODE 0: the weight rows this thread copies pieces of
-  const float* wrow[2] = {nullptr, nullptr};
-  if constexpr (MODE == 0) {
-#pragma unroll
-    for (int q = 0; q < 2; ++q) {
-      const int j = j0 + ((tid + q * GNT) >> 3);
-      if (j < J) wrow[q] = welem<float>(ws, tb, j, slab, 0);
-    }
-  }
-  auto load = [&](int kt, int s) {
-    float* as = lin_smem + s * (A_F + B_F);
-    float* bs = as + A_F;
-    const int k0 = kt * FK;
-    const float* wk = nullptr;                 // MODE 1: row k0 of the selection (slabs are whole 32-row runs)
-    int64_t wld = 0;
-    if constexpr (MODE == 1) {
-      wk = welem<float>(ws, tb, k0, slab, 0);
-      wld = ws.ldw[tb.weight[k0 / slab]];
-    }
-#pragma unroll
-    for (int q = 0; q < 2; ++q) {
-      const int idx = tid + q * GNT;
-      const int r = idx >> 3, rc = (idx & 7) * 4;      // K-contiguous: row, first k
-      const int kk = idx >> 4, kc = (idx & 15) * 4;    // K slices: k, first row
-      if constexpr (A_KC) {
-        const bool ok = i0 + r < I && k0 + rc < K;
-        cp_async16_zfill(as + r * FLD + rc, ok ? A + (int64_t)(i0 + r) * lda + k0 + rc : A, ok);
-      } else {
-        const bool ok = i0 + kc < I && k0 + kk < K;
-        cp_async16_zfill(as + kk * TM + kc, ok ? A + (int64_t)(k0 + kk) * lda + i0 + kc : A, ok);
-      }
-      if constexpr (MODE == 0) {
-        const bool ok = wrow[q] && k0 + rc < K;
-        cp_async16_zfill(bs + r * FLD + rc, ok ? wrow[q] + k0 + rc : A, ok);
-      } else if constexpr (MODE == 1) {
-        const bool ok = j0 + kc < J;
-        cp_async16_zfill(bs + kk * TN + kc, ok ? wk + kk * wld + j0 + kc : A, ok);
-      } else {
-        const bool ok = j0 + kc < J && k0 + kk < K;
-        cp_async16_zfill(bs + kk * TN + kc, ok ? X + (int64_t)(k0 + kk) * ldx + j0 + kc : A, ok);
-      }
-    }
-  };
-  float acc[8][8];
-#pragma unroll
-  for (int i = 0; i < 8; ++i)
-#pragma unroll
-    for (int j = 0; j < 8; ++j) acc[i][j] = 0.f;
-  const int KT = (K + FK - 1) / FK;
-#pragma unroll
-  for (int s = 0; s < FSTAGES - 1; ++s) {
-    if (s < KT) load(s, s);
-    cp_async_commit();
-  }
-  for (int kt = 0; kt < KT; ++kt) {
-    cp_async_wait<FSTAGES - 2>();
-    __syncthreads();
-    if (kt + FSTAGES - 1 < KT) load(kt + FSTAGES - 1, (kt + FSTAGES - 1) % FSTAGES);
-    cp_async_commit();
-    const float* as = lin_smem + (kt % FSTAGES) * (A_F + B_F);
-    const float* bs = as + A_F;
-    if constexpr (A_KC && B_KC) {
-#pragma unroll
-      for (int h = 0; h < FKG; h += 4) {
-        float4 b[8];
-#pragma unroll
-        for (int j = 0; j < 8; ++j) b[j] = *reinterpret_cast<const float4*>(bs + (tx + 8 * j) * FLD + kg * FKG + h);
-#pragma unroll
-        for (int i = 0; i < 8; ++i) {
-          const float4 a = *reinterpret_cast<const float4*>(as + (ty + 8 * i) * FLD + kg * FKG + h);
-#pragma unroll
-          for (int e = 0; e < 4; ++e)
-#pragma unroll
-            for (int j = 0; j < 8; ++j) acc[i][j] = fmaf(f4c(a, e), f4c(b[j], e), acc[i][j]);
-        }
-      }
-    } else {
-#pragma unroll
-      for (int h = 0; h < FKG; h += 4) {
-        float4 ak[8];
-        if constexpr (A_KC) {
-#pragma unroll
-          for (int i = 0; i < 8; ++i) ak[i] = *reinterpret_cast<const float4*>(as + (ty + 8 * i) * FLD + kg * FKG + h);
-        }
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          const int k = kg * FKG + h + e;
-          const float4 b0 = *reinterpret_cast<const float4*>(bs + k * TN + tx * 4);
-          const float4 b1 = *reinterpret_cast<const float4*>(bs + k * TN + 32 + tx * 4);
-          float4 a0, a1;
-          if constexpr (!A_KC) {
-            a0 = *reinterpret_cast<const float4*>(as + k * TM + ty * 4);
-            a1 = *reinterpret_cast<const float4*>(as + k * TM + 32 + ty * 4);
-          }
-#pragma unroll
-          for (int i = 0; i < 8; ++i) {
-            float av;
-            if constexpr (A_KC) av = f4c(ak[i], e);
-            else av = f4c(i < 4 ? a0 : a1, i & 3);
-#pragma unroll
-            for (int j = 0; j < 8; ++j) acc[i][j] = fmaf(av, f4c(j < 4 ? b0 : b1, j & 3), acc[i][j]);
-          }
-        }
-      }
-    }
-  }
-  // ---- the groups' sums, added in order
-  cp_async_wait<0>();
-  __syncthreads();
-  float* red = lin_smem + kg * TM * FRED;
-#pragma unroll
-  for (int i = 0; i < 8; ++i)
-#pragma unroll
-    for (int j = 0; j < 8; ++j) red[frag_at<A_KC>(ty, i) * FRED + frag_at<B_KC>(tx, j)] = acc[i][j];
-  __syncthreads();
-#pragma unroll
-  for (int q = 0; q < TM * TN / 4 / GNT; ++q) {
-    const int idx = tid + q * GNT, r = idx >> 4, c = (idx & 15) * 4;
-    const int ii = i0 + r, jj = j0 + c;
-    if (ii >= I || jj >= J) continue;
-    float4 v = *reinterpret_cast<const float4*>(lin_smem + r * FRED + c);
-#pragma unroll
-    for (int g = 1; g < FGROUPS; ++g) {
-      const float4 t = *reinterpret_cast<const float4*>(lin_smem + (g * TM + r) * FRED + c);
-      v.x += t.x; v.y += t.y; v.z += t.z; v.w += t.w;
-    }
-    const float* bias = nullptr;
-    if constexpr (MODE == 0) {
-      const int g = jj / slab;
-      const float* b = reinterpret_cast<const float*>(ws.b[tb.weight[g]]);
-      if (b) bias = b + tb.row0[g] + (jj - g * slab);
-    } else if constexpr (MODE == 1) {
-      if (X) bias = X + jj;                    // optional bias over the output columns
-    }
-    if (bias) {
-      v.x += bias[0]; v.y += bias[1]; v.z += bias[2]; v.w += bias[3];
-    }
-    float* dst = MODE == 2 ? const_cast<float*>(welem<float>(ws, tb, ii, slab, jj)) : Cout + (int64_t)ii * ldc + jj;
-    *reinterpret_cast<float4*>(dst) = v;
-  }
-}
-
 // Whether every row the product touches is made of whole 16-byte pieces and a 32-deep K slice stays inside one slab.
 // A: the left operand (x, or dout in the backward); Cout is null for the weight gradient.
 bool f32_rows_ok(const SafIndexedLinearArgs& a, const void* A, int64_t lda, const void* X, int64_t ldx, const void* Cout, int64_t ldc) {
@@ -314,19 +124,6 @@ bool f32_rows_ok(const SafIndexedLinearArgs& a, const void* A, int64_t lda, cons
   for (int w = 0; w < a.n_weights; ++w)
     if (!ok(a.weights[w], a.ldw[w]) || (a.cdw[w] != 0 && a.cdw[w] != 1)) return false;
   return true;
-}
-
-template <int MODE>
-int launch_linear_f32(dim3 grid, const void* A, int64_t lda, const void* X, int64_t ldx, void* Cout, int64_t ldc, const SafIndexedLinearArgs& a,
-                      const WeightSet& ws, const SlabTable& tb, cudaStream_t st) {
-  constexpr int A_F = MODE != 2 ? TM * FLD : FK * TM, B_F = MODE == 0 ? TN * FLD : FK * TN;
-  constexpr int smem = 4 * (FSTAGES * (A_F + B_F) > FGROUPS * TM * FRED ? FSTAGES * (A_F + B_F) : FGROUPS * TM * FRED);
-  static PerDeviceOnce once;
-  if (int rc = ensure_dyn_smem(linear_f32_kernel<MODE>, smem, once)) return rc;
-  linear_f32_kernel<MODE><<<grid, GNT, smem, st>>>(reinterpret_cast<const float*>(A), lda, reinterpret_cast<const float*>(X), ldx,
-                                                   reinterpret_cast<float*>(Cout), ldc, a.M, a.C, a.n_slabs * a.slab, a.slab, ws, tb);
-  count_launch();
-  return check_launch("linear_f32_kernel");
 }
 
 // db[n] = sum_m dout[m, n], scattered to bias rows
@@ -435,7 +232,7 @@ int gemm_generic_typed(const SafIndexedLinearArgs& a, int mode, const void* dout
   if (mode == 0) {
     dim3 grid((N + TN - 1) / TN, (a.M + TM - 1) / TM);
     if (f32 && f32_rows_ok(a, a.x, a.ldx, nullptr, 0, a.out, a.ldo)) {
-      if ((rc = launch_linear_f32<0>(grid, a.x, a.ldx, nullptr, 0, a.out, a.ldo, a, ws, tb, st))) return rc;
+      if ((rc = launch_linear_f32(0, a.x, a.ldx, nullptr, 0, a.out, a.ldo, a, ws, tb, st))) return rc;
     } else {
       linear_generic_kernel<T, 0><<<grid, GNT, 0, st>>>(reinterpret_cast<const T*>(a.x), a.ldx, nullptr, 0,
                                                         reinterpret_cast<T*>(a.out), a.ldo, a.M, a.C, N, a.slab, ws, tb);
@@ -455,7 +252,7 @@ int gemm_generic_typed(const SafIndexedLinearArgs& a, int mode, const void* dout
   } else if (mode == 1) {
     dim3 grid((a.C + TN - 1) / TN, (a.M + TM - 1) / TM);
     if (f32 && f32_rows_ok(a, dout, lddo, nullptr, 0, dx, lddx))
-      return launch_linear_f32<1>(grid, dout, lddo, bias, 0, dx, lddx, a, ws, tb, st);
+      return launch_linear_f32(1, dout, lddo, bias, 0, dx, lddx, a, ws, tb, st);
     linear_generic_kernel<T, 1><<<grid, GNT, 0, st>>>(reinterpret_cast<const T*>(dout), lddo,
                                                       reinterpret_cast<const T*>(bias), 0,
                                                       reinterpret_cast<T*>(dx), lddx, a.M, a.C, N, a.slab, ws, tb);
@@ -464,7 +261,7 @@ int gemm_generic_typed(const SafIndexedLinearArgs& a, int mode, const void* dout
   } else {
     dim3 grid((a.C + TN - 1) / TN, (N + TM - 1) / TM);
     if (f32 && f32_rows_ok(a, dout, lddo, a.x, a.ldx, nullptr, 0)) {
-      if ((rc = launch_linear_f32<2>(grid, dout, lddo, a.x, a.ldx, nullptr, 0, a, ws, tb, st))) return rc;
+      if ((rc = launch_linear_f32(2, dout, lddo, a.x, a.ldx, nullptr, 0, a, ws, tb, st))) return rc;
     } else {
       linear_generic_kernel<T, 2><<<grid, GNT, 0, st>>>(reinterpret_cast<const T*>(dout), lddo,
                                                         reinterpret_cast<const T*>(a.x), a.ldx, nullptr, 0, a.M, a.C, N,
