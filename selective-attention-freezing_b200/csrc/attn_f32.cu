@@ -1,287 +1,560 @@
-// fp32 attention of the live heads at head_dim 64: forward, dK / dV and dQ on the CUDA cores in true fp32.
+// fp32 attention of the live heads at head_dim 64 on the tensor cores: forward, dK / dV and dQ.
 //
-// What bounds it: the FMA pipe (the tensor cores have no fp32 product), so everything else has to stay out of its way.  The
-// any-type kernels beside this file read two operands from shared memory for every two FMAs and spend their time there.
-// Here a thread owns 8 x 4 outputs of a 64 x 64 tile and reads its operands as float4 along the contraction index, or
-// along the output columns where the operand is stored that way: 12 16-byte reads for 128 FMAs.  Every operand is used
-// in the layout it has in memory (rows of 64 floats), so tiles arrive by cp.async and nothing is transposed.  Rows of a
-// probability tile are written and read by the same half-warp: no block-wide barrier between the two products.
+// Every fp32 operand, probabilities and score gradients included, is split into three bf16 parts (split_bf16.cuh) and a
+// product is the sum of the six part products that reach 2^-24 of it, as in the fp32 projections (linear_f32_sm100.cu).
+// The leading part product of a 64-deep step is taken out of tensor memory after the step and added in fp32 with
+// rounding; the five small ones have an accumulator of their own.  Exponentials, row maxima and row sums are fp32.
 //
-//   forward  CTA = 64 query rows, walks the key tiles; K of the next tile loads under softmax and P V, V under Q K^T
-//   dK / dV  CTA = 64 keys, S^T = K Q^T and dP^T = V dO^T, then dV += P^T dO, dK += dS^T Q
-//   dQ       CTA = 64 query rows, S, dP, dQ += dS K
-// 9 live heads, T = 1024, B = 2 on a B200: forward 365 -> 151 us, dK / dV 581 -> 246, dQ 389 -> 192.
+//   forward  CTA = 128 query rows, walks 64-key tiles:     S = Q K^T,                       O   += P V
+//   dK / dV  CTA = 128 keys, walks 64-row query tiles:     S = K Q^T, dP = V dO^T,          dV  += P^T dO, dK += dS^T Q
+//   dQ       CTA = 128 query rows, walks 64-key tiles:     S = Q K^T, dP = dO V^T,          dQ  += dS K
+// All three have the same skeleton: one or two resident operands of 128 rows, two streamed ones of 64 rows a step.
+//   warps 0-7   read fp32 rows one step ahead, split them into shared memory
+//   warps 8-23  four threads per row, 16 columns each: scores out of TMEM, probabilities / score gradients back into the
+//               columns the same thread has read, as A operands; they also keep the outputs in registers
+//   warp 24     issues (25-27 complete the warpgroup that hands registers to the others)
+//
+// What bounds it: the 24 to 48 part products of a step, 128 x 64 x 16 at 48 cycles from shared memory and 32 from tensor
+// memory (two thirds of the time of the longest walks), and the row tiles' unequal walks.  9 heads, T = 1024, B = 2 on a B200,
+// before (fp32 FMAs, 64 x 64 tiles) and now: forward 119 -> 33 us, backward 397 -> 78; relative error against 64 bits 3.3e-7 ->
+// 1.6e-7 (y), 4.5e-7 -> 3.0e-7 (dq), 7.9e-7 -> 3.2e-7 (dk), 8.0e-7 -> 2.6e-7 (dv).  Two threads per row instead of four:
+// 41 and 196 us; each step's products one after the other: 164.
+//
 // The same split as the reference (kernel/fused_attn.py:228-289, 415-481, 483-540): no atomics, fixed order of sums.
+// What the parts cannot carry shows in the results (infinities, NaN, a tile of nothing but tiny values): such a tile is
+// computed again with fp32 FMAs, row by row.
+#include <string.h>
+
 #include "head_index.cuh"
 #include "saf_internal.h"
-#include "sm100_prims.cuh"
+#include "split_bf16.cuh"
+
 
 namespace saf {
 namespace {
 
-constexpr int FB = 64;          // rows, keys and columns of a tile
-constexpr int FHD = 64;
-constexpr int FLD = 68;         // row stride of operand tiles: float4 reads of 8 neighbouring rows hit all banks once
-constexpr int FLP = 80;         // row stride of probability tiles: the two rows a warp writes lie 16 banks apart
-constexpr int FNT = 128;
+constexpr int AR = 128, AX = 64, AHD = 64;      // resident rows, streamed rows, head width
+constexpr int APROD = 256, ACOMP = 512, ATHREADS = APROD + ACOMP + 128;
+constexpr int AISSUER = (APROD + ACOMP) / 32;
+constexpr int RES_PART = 2 * SBLK, RES = 3 * RES_PART;        // a resident operand: 48 KB
+constexpr int STR = 3 * SBLK, ASTAGE = 2 * STR;               // a streamed one, a stage of two
 constexpr float F_LOG2E = 1.4426950408889634f;
-constexpr int TILE_F = FB * FLD, PROB_F = FB * FLP;
+enum { A_FWD = 0, A_DKDV = 1, A_DQ = 2 };
 
-// rows row0 .. row0+63 of one head -> dst[r * FLD + d]; rows from T on are zero
-__device__ __forceinline__ void f32_tile(float* dst, const float* base, int64_t s_row, int row0, int T) {
-#pragma unroll
-  for (int q = 0; q < FB * FHD / 4 / FNT; ++q) {
-    const int idx = threadIdx.x + q * FNT, r = idx >> 4, c = (idx & 15) * 4;
-    const bool ok = row0 + r < T;
-    cp_async16_zfill(dst + r * FLD + c, ok ? base + (int64_t)(row0 + r) * s_row + c : base, ok);
-  }
-}
-
-__device__ __forceinline__ float4 ld4(const float* p) { return *reinterpret_cast<const float4*>(p); }
-__device__ __forceinline__ float comp(const float4& v, int e) { return e == 0 ? v.x : (e == 1 ? v.y : (e == 2 ? v.z : v.w)); }
-
-// s[i][j] = sum_d A[ty + 8i][d] B[tx + 16j][d]
-__device__ __forceinline__ void f32_dot(const float* A, const float* B, int ty, int tx, float (&s)[8][4]) {
-#pragma unroll
-  for (int i = 0; i < 8; ++i)
-#pragma unroll
-    for (int j = 0; j < 4; ++j) s[i][j] = 0.f;
-#pragma unroll 4
-  for (int d = 0; d < FHD; d += 4) {
-    float4 b[4];
-#pragma unroll
-    for (int j = 0; j < 4; ++j) b[j] = ld4(B + (tx + 16 * j) * FLD + d);
-#pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      const float4 a = ld4(A + (ty + 8 * i) * FLD + d);
-#pragma unroll
-      for (int e = 0; e < 4; ++e)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) s[i][j] = fmaf(comp(a, e), comp(b[j], e), s[i][j]);
-    }
-  }
-}
-
-// acc[i][c] += sum_k P[ty + 8i][k] B[k][4 tx + c]
-__device__ __forceinline__ void f32_acc(const float* P, const float* B, int ty, int tx, float (&acc)[8][4]) {
-#pragma unroll 2
-  for (int k = 0; k < FB; k += 4) {
-    float4 b[4];
-#pragma unroll
-    for (int e = 0; e < 4; ++e) b[e] = ld4(B + (k + e) * FLD + tx * 4);
-#pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      const float4 p = ld4(P + (ty + 8 * i) * FLP + k);
-#pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        acc[i][0] = fmaf(comp(p, e), b[e].x, acc[i][0]);
-        acc[i][1] = fmaf(comp(p, e), b[e].y, acc[i][1]);
-        acc[i][2] = fmaf(comp(p, e), b[e].z, acc[i][2]);
-        acc[i][3] = fmaf(comp(p, e), b[e].w, acc[i][3]);
-      }
-    }
-  }
-}
+template <int MODE>
+struct AttnShape {
+  static constexpr int NRES = MODE == A_FWD ? 1 : 2, STAGES = MODE == A_FWD ? 3 : 2;
+  struct Ctrl {
+    uint64_t full[STAGES], empty[STAGES], res_full, s_full[2], dp_full, p_full, ds_full, acc_full[2];
+    uint32_t tmem_base;
+    alignas(16) float lse[STAGES][AX], delta[STAGES][AX];   // dK / dV: of the streamed query rows
+    float mx[2][4][AR];                         // forward: row maxima, row sums of the four quarters
+  };
+  static constexpr int SMEM = 1024 + NRES * RES + STAGES * ASTAGE + (int)sizeof(Ctrl);
+};
+// TMEM columns: every accumulator is 64 columns of the leading product and 64 of the small ones.  The forward alternates its
+// scores between T_S and T_DP and its output between T_ACC1 and T_ACC2, dQ its scores between T_S and T_ACC2
+constexpr uint32_t T_S = 0, T_DP = 128, T_ACC1 = 256, T_ACC2 = 384;
 
 __device__ __forceinline__ const float* f32_head(const SafTensor& t, int b, int h) {
   return reinterpret_cast<const float*>(t.ptr) + (int64_t)b * t.stride[0] + (int64_t)h * t.stride[1];
 }
-__device__ __forceinline__ void f32_store(const SafTensor& t, int b, int h, int row, int tx, const float (&v)[4], float f) {
-  float* p = reinterpret_cast<float*>(t.ptr) + (int64_t)b * t.stride[0] + (int64_t)h * t.stride[1] + (int64_t)row * t.stride[2];
-  *reinterpret_cast<float4*>(p + tx * 4) = make_float4(v[0] * f, v[1] * f, v[2] * f, v[3] * f);
+
+// The six part products of one 16-deep step, k4; A in shared memory or, as it was put back, in tensor memory.  The parts of
+// an operand lie RES_PART / SBLK bytes apart: one descriptor, advanced by constants.
+__device__ __forceinline__ void six_ss(uint32_t d, uint64_t a, uint64_t b, int k4, uint32_t idesc) {
+  const uint32_t o = k4 * 32;
+  auto pa = [&](int u) { return umma_desc_advance(a, u * RES_PART + o); };
+  auto pb = [&](int u) { return umma_desc_advance(b, u * SBLK + o); };
+  umma_ss(d, pa(0), pb(0), idesc, k4 > 0);
+  umma_ss(d + 64, pa(0), pb(1), idesc, k4 > 0);
+  umma_ss(d + 64, pa(1), pb(0), idesc, 1);
+  umma_ss(d + 64, pa(0), pb(2), idesc, 1);
+  umma_ss(d + 64, pa(1), pb(1), idesc, 1);
+  umma_ss(d + 64, pa(2), pb(0), idesc, 1);
+}
+// `at`: the 64 leading columns of the region that held the scores; step k4's parts lie where its thread read them
+__device__ __forceinline__ void six_ts(uint32_t d, uint32_t at, uint64_t b, int k4, uint32_t idesc, bool first_small) {
+  const uint32_t a0 = at + 16 * k4, a1 = a0 + 8, a2 = a0 + 64, o = k4 * 2048;
+  auto pb = [&](int u) { return umma_desc_advance(b, u * SBLK + o); };
+  umma_ts(d, a0, pb(0), idesc, k4 > 0);
+  umma_ts(d + 64, a0, pb(1), idesc, !first_small);
+  umma_ts(d + 64, a1, pb(0), idesc, 1);
+  umma_ts(d + 64, a0, pb(2), idesc, 1);
+  umma_ts(d + 64, a1, pb(1), idesc, 1);
+  umma_ts(d + 64, a2, pb(0), idesc, 1);
 }
 
-// grid (B * H, row tiles): the longest tiles of all heads first
-__global__ void __launch_bounds__(FNT, 3) f32_fwd_kernel(const __grid_constant__ SafMixedAttnArgs a) {
-  extern __shared__ __align__(16) float f32_smem[];
-  const HeadIdx hx = head_index(a, blockIdx.x);
-  if (hx.state != SAF_LIVE) return;
-  const int mt = gridDim.y - 1 - blockIdx.y, i0 = mt * FB, T = a.T;
-  float *Qs = f32_smem, *Ks = Qs + TILE_F, *Vs = Ks + TILE_F, *Ps = Vs + TILE_F;
-  const int tid = threadIdx.x, ty = tid >> 4, tx = tid & 15;
-  const float *qb = f32_head(a.q, hx.b, hx.hq), *kb = f32_head(a.k, hx.b, hx.hk), *vb = f32_head(a.v, hx.b, hx.hv);
-  f32_tile(Qs, qb, a.q.stride[2], i0, T);
-  f32_tile(Ks, kb, a.k.stride[2], 0, T);
-  cp_async_commit();
-  f32_tile(Vs, vb, a.v.stride[2], 0, T);
-  cp_async_commit();
-  float acc[8][4], m[8], l[8];
+// 16 columns of an accumulator pair, added
+__device__ __forceinline__ void tmem_sum16(uint32_t at, float (&v)[16]) {
+  uint32_t x[16], y[16];
+  tmem_ld16(at, x);
+  tmem_ld16(at + 64, y);
+  tmem_ld_wait();
 #pragma unroll
-  for (int i = 0; i < 8; ++i) {
-    m[i] = -INFINITY;
-    l[i] = 0.f;
+  for (int j = 0; j < 16; ++j) v[j] = __uint_as_float(x[j]) + __uint_as_float(y[j]);
+}
+// 16 values -> their parts, in the columns `at`.. the thread read them from
+__device__ __forceinline__ void tmem_parts16(uint32_t at, const float (&v)[16]) {
+  uint32_t w[3][8];
 #pragma unroll
-    for (int c = 0; c < 4; ++c) acc[i][c] = 0.f;
+  for (int j = 0; j < 8; ++j) {
+    uint32_t q[3];
+    split2(v[2 * j], v[2 * j + 1], q);
+#pragma unroll
+    for (int u = 0; u < 3; ++u) w[u][j] = q[u];
   }
-  const float scale = a.sm_scale * F_LOG2E;
-  for (int jt = 0; jt <= mt; ++jt) {
-    const int j0 = jt * FB;
-    cp_async_wait<1>();                       // Q, K of this tile; V may still be on its way
-    __syncthreads();
-    float s[8][4];
-    f32_dot(Qs, Ks, ty, tx, s);
-    __syncthreads();                          // K is read
-    if (jt < mt) f32_tile(Ks, kb, a.k.stride[2], j0 + FB, T);
-    cp_async_commit();
-#pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      const int r = ty + 8 * i;
-      float mx = -INFINITY;
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const bool ok = jt < mt || (tx + 16 * j <= r && j0 + tx + 16 * j < T);
-        s[i][j] = ok ? s[i][j] * scale : -INFINITY;
-        mx = fmaxf(mx, s[i][j]);
-      }
-#pragma unroll
-      for (int off = 8; off; off >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, off));
-      const float m_new = fmaxf(m[i], mx), m_safe = (m_new == -INFINITY) ? 0.f : m_new;
-      const float f = (m[i] == -INFINITY) ? 0.f : exp2f(m[i] - m_safe);
-      float sum = 0.f;
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const float p = exp2f(s[i][j] - m_safe);
-        Ps[r * FLP + tx + 16 * j] = p;
-        sum += p;
-      }
-      l[i] = l[i] * f + sum;                  // this thread's columns; added over the row at the end
-      m[i] = m_new;
-#pragma unroll
-      for (int c = 0; c < 4; ++c) acc[i][c] *= f;
-    }
-    cp_async_wait<1>();                       // V of this tile; the next K may still be on its way
-    __syncthreads();
-    f32_acc(Ps, Vs, ty, tx, acc);
-    __syncthreads();                          // V is read
-    if (jt < mt) f32_tile(Vs, vb, a.v.stride[2], j0 + FB, T);
-    cp_async_commit();
-  }
-  cp_async_wait<0>();
-#pragma unroll
-  for (int i = 0; i < 8; ++i) {
-#pragma unroll
-    for (int off = 8; off; off >>= 1) l[i] += __shfl_xor_sync(0xffffffffu, l[i], off);
-    const int t = i0 + ty + 8 * i;
-    if (t >= T) continue;
-    const float ls = l[i] == 0.f ? 1.f : l[i];
-    f32_store(a.out, hx.b, hx.h, t, tx, acc[i], 1.f / ls);
-    if (a.lse.ptr && tx == 0)
-      reinterpret_cast<float*>(a.lse.ptr)[(int64_t)hx.b * a.lse.stride[0] + (int64_t)hx.h * a.lse.stride[1] + (int64_t)t * a.lse.stride[2]] =
-          ((m[i] == -INFINITY) ? 0.f : m[i]) + log2f(ls);
-  }
+  tmem_st8(at, w[0]);
+  tmem_st8(at + 8, w[1]);
+  tmem_st8(at + 64, w[2]);
 }
 
-__global__ void __launch_bounds__(FNT, 2) f32_dkdv_kernel(const __grid_constant__ SafMixedAttnBwdArgs g) {
-  extern __shared__ __align__(16) float f32_smem[];
+__device__ __forceinline__ float row_dot(const float* x, const float* y) {
+  float s = 0.f;
+#pragma unroll 1
+  for (int d = 0; d < AHD; d += 4) {
+    const float4 a = *reinterpret_cast<const float4*>(x + d), b = *reinterpret_cast<const float4*>(y + d);
+    s = fmaf(a.x, b.x, s);
+    s = fmaf(a.y, b.y, s);
+    s = fmaf(a.z, b.z, s);
+    s = fmaf(a.w, b.w, s);
+  }
+  return s;
+}
+__device__ __forceinline__ void axpy16(float f, const float* x, float (&acc)[16]) {
+#pragma unroll
+  for (int c = 0; c < 16; c += 4) {
+    const float4 v = *reinterpret_cast<const float4*>(x + c);
+    acc[c] = fmaf(f, v.x, acc[c]);
+    acc[c + 1] = fmaf(f, v.y, acc[c + 1]);
+    acc[c + 2] = fmaf(f, v.z, acc[c + 2]);
+    acc[c + 3] = fmaf(f, v.w, acc[c + 3]);
+  }
+}
+__device__ __forceinline__ void store16(const SafTensor& t, int b, int h, int row, int col, const float (&v)[16], float f) {
+  float* p = reinterpret_cast<float*>(t.ptr) + (int64_t)b * t.stride[0] + (int64_t)h * t.stride[1] + (int64_t)row * t.stride[2] + col;
+#pragma unroll
+  for (int c = 0; c < 16; c += 4) *reinterpret_cast<float4*>(p + c) = make_float4(v[c] * f, v[c + 1] * f, v[c + 2] * f, v[c + 3] * f);
+}
+
+// the row tile with the `rank`-th longest walk of one (batch, head)
+template <int MODE>
+__device__ __forceinline__ void attn_f32_tile(const SafMixedAttnBwdArgs& g, int rank, int tiles) {
+  using S = AttnShape<MODE>;
   const SafMixedAttnArgs& a = g.fwd;
+  extern __shared__ uint8_t attn_smem[];
+  uint8_t* smem = (uint8_t*)(((uintptr_t)attn_smem + 1023) & ~(uintptr_t)1023);
+  uint8_t* stages = smem + S::NRES * RES;
+  typename S::Ctrl* sl = reinterpret_cast<typename S::Ctrl*>(stages + S::STAGES * ASTAGE);
   const HeadIdx hx = head_index(a, blockIdx.x);
   if (hx.state != SAF_LIVE) return;
-  const int j0 = blockIdx.y * FB, T = a.T;
-  float *Ks = f32_smem, *Vs = Ks + TILE_F, *Qs = Vs + TILE_F, *Ds = Qs + TILE_F, *Pt = Ds + TILE_F, *St = Pt + PROB_F;
-  const int tid = threadIdx.x, ty = tid >> 4, tx = tid & 15;
-  const float *qb = f32_head(a.q, hx.b, hx.hq), *dob = f32_head(g.dout, hx.b, hx.h);
-  f32_tile(Ks, f32_head(a.k, hx.b, hx.hk), a.k.stride[2], j0, T);
-  f32_tile(Vs, f32_head(a.v, hx.b, hx.hv), a.v.stride[2], j0, T);
-  float dk[8][4], dv[8][4];
-#pragma unroll
-  for (int i = 0; i < 8; ++i)
-#pragma unroll
-    for (int c = 0; c < 4; ++c) dk[i][c] = dv[i][c] = 0.f;
-  const float scale = a.sm_scale * F_LOG2E;
-  const float* lse = f32_head(a.lse, hx.b, hx.h);
-  const float* del = f32_head(g.delta, hx.b, hx.h);
-  for (int i0 = j0; i0 < T; i0 += FB) {
-    f32_tile(Qs, qb, a.q.stride[2], i0, T);
-    f32_tile(Ds, dob, g.dout.stride[2], i0, T);
-    cp_async_commit();
-    float L[4], dl[4];                        // of query rows tx + 16 j
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const int q = i0 + tx + 16 * j;
-      L[j] = q < T ? lse[(int64_t)q * a.lse.stride[2]] : 0.f;
-      dl[j] = q < T ? del[(int64_t)q * g.delta.stride[2]] : 0.f;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, T = a.T;
+  const int r0 = (MODE == A_DKDV ? rank : tiles - 1 - rank) * AR;     // first resident row
+  // streamed tiles: keys up to the last row's, or queries from the first key's on
+  const int x0 = MODE == A_DKDV ? r0 / AX : 0, xt = (T + AX - 1) / AX;
+  const int x1 = MODE == A_DKDV ? xt : min(xt, (r0 + AR) / AX);
+
+  if (tid == 0) {
+    for (int s = 0; s < S::STAGES; ++s) {
+      mbar_init(&sl->full[s], APROD / 32);
+      mbar_init(&sl->empty[s], 1);
     }
-    cp_async_wait<0>();
-    __syncthreads();
-    float s[8][4], dp[8][4];
-    f32_dot(Ks, Qs, ty, tx, s);
-    f32_dot(Vs, Ds, ty, tx, dp);
+    mbar_init(&sl->res_full, APROD / 32);
+    for (int b = 0; b < 2; ++b) {
+      mbar_init(&sl->s_full[b], 1);
+      mbar_init(&sl->acc_full[b], 1);
+    }
+    mbar_init(&sl->dp_full, 1);
+    mbar_init(&sl->p_full, ACOMP / 32);
+    mbar_init(&sl->ds_full, ACOMP / 32);
+    fence_mbar_init();
+  }
+  if (warp == AISSUER) {
+    tmem_alloc(&sl->tmem_base, 512);
+    tmem_relinquish();
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem = sl->tmem_base;
+
+  if (warp < APROD / 32) {
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 56;");
+    const int row = tid >> 4, c4 = (tid & 15) * 4;           // 16 bytes of a row, 16 rows apart
+    const uint32_t off = row * 128 + ((((tid & 15) >> 1) ^ (row & 7)) << 4) + (tid & 1) * 8;
+    // the resident operands, block by block
+    {
+      const SafTensor& t0 = MODE == A_DKDV ? a.k : a.q;
+      const SafTensor& t1 = MODE == A_DKDV ? a.v : g.dout;
+      const float* p0 = f32_head(t0, hx.b, MODE == A_DKDV ? hx.hk : hx.hq) + c4;
+      const float* p1 = S::NRES == 2 ? f32_head(t1, hx.b, MODE == A_DKDV ? hx.hv : hx.h) + c4 : nullptr;
+#pragma unroll 1
+      for (int n = 0; n < 2 * S::NRES; ++n) {
+        const int o = n >> 1, blk = n & 1;
+        const float* src = o ? p1 : p0;
+        const int64_t ld = (o ? t1 : t0).stride[2];
+        float4 v[4];
 #pragma unroll
-    for (int i = 0; i < 8; ++i)
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const int c = ty + 8 * i, r = tx + 16 * j;
-        float p = 0.f, ds = 0.f;
-        if (i0 + r < T && j0 + c <= i0 + r) {
-          p = exp2f(s[i][j] * scale - L[j]);
-          ds = p * (dp[i][j] - dl[j]) * a.sm_scale;
+        for (int q = 0; q < 4; ++q) {
+          const int t = r0 + blk * 64 + q * 16 + row;
+          v[q] = ld4_or_0(src + (int64_t)t * ld, t < T);
         }
-        Pt[c * FLP + r] = p;
-        St[c * FLP + r] = ds;
-      }
-    __syncwarp();
-    f32_acc(Pt, Ds, ty, tx, dv);
-    f32_acc(St, Qs, ty, tx, dk);
-    __syncthreads();
-  }
 #pragma unroll
-  for (int i = 0; i < 8; ++i) {
-    const int t = j0 + ty + 8 * i;
-    if (t >= T) continue;
-    f32_store(g.dv, hx.b, hx.hv, t, tx, dv[i], 1.f);
-    f32_store(g.dk, hx.b, hx.hk, t, tx, dk[i], 1.f);
+        for (int q = 0; q < 4; ++q) split_store(smem + o * RES + blk * SBLK + q * 2048 + off, RES_PART, v[q]);
+      }
+    }
+    fence_proxy_async_smem();
+    __syncwarp();
+    if (lane == 0) mbar_arrive(&sl->res_full);
+    const SafTensor& s0 = MODE == A_DKDV ? a.q : a.k;
+    const SafTensor& s1 = MODE == A_DKDV ? g.dout : a.v;
+    const float* p0 = f32_head(s0, hx.b, MODE == A_DKDV ? hx.hq : hx.hk) + c4;
+    const float* p1 = f32_head(s1, hx.b, MODE == A_DKDV ? hx.h : hx.hv) + c4;
+    const float* lse = MODE == A_DKDV ? f32_head(a.lse, hx.b, hx.h) : nullptr;
+    const float* del = MODE == A_DKDV ? f32_head(g.delta, hx.b, hx.h) : nullptr;
+    float4 v[2][4];
+    float stat = 0.f;
+    auto load = [&](int o, int xi) {
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        const int t = xi * AX + q * 16 + row;
+        v[o][q] = ld4_or_0((o ? p1 : p0) + (int64_t)t * (o ? s1 : s0).stride[2], t < T);
+      }
+      if (MODE == A_DKDV && o == 1 && tid < 2 * AX) {
+        const int t = xi * AX + (tid & (AX - 1));
+        stat = t < T ? (tid < AX ? lse[(int64_t)t * a.lse.stride[2]] : del[(int64_t)t * g.delta.stride[2]]) : 0.f;
+      }
+    };
+    if (x0 < x1) {
+      load(0, x0);
+      load(1, x0);
+    }
+    for (int xi = x0; xi < x1; ++xi) {
+      const int it = xi - x0, s = it % S::STAGES;
+      if (!mbar_wait(&sl->empty[s], ((it / S::STAGES) & 1) ^ 1)) {
+        dev_set_error(a.status, SAF_DEV_TIMEOUT_TMA, 75);
+        break;
+      }
+      uint8_t* st = stages + s * ASTAGE + off;
+#pragma unroll
+      for (int o = 0; o < 2; ++o) {
+#pragma unroll
+        for (int q = 0; q < 4; ++q) split_store(st + o * STR + q * 2048, SBLK, v[o][q]);
+        if (MODE == A_DKDV && o == 1 && tid < 2 * AX) (tid < AX ? sl->lse : sl->delta)[s][tid & (AX - 1)] = stat;
+        if (xi + 1 < x1) load(o, xi + 1);
+      }
+      fence_proxy_async_smem();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&sl->full[s]);
+    }
+  } else if (warp >= AISSUER) {
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 40;");
+    if (warp == AISSUER) {
+      const bool leader = elect_one();
+      const uint32_t id_k = umma_idesc_bf16(AR, AX, 0, 0), id_mn = umma_idesc_bf16(AR, AHD, 0, 1);
+      const uint32_t sb = smem_u32(smem), xb = smem_u32(stages);
+      // products of the resident operand o with streamed tile `it`, into `d`
+      auto scores = [&](int o, int it, uint32_t d, uint64_t* done) {
+        const uint64_t ad = umma_smem_desc_sw128(sb + o * RES, 16, 1024);
+        const uint64_t bd = umma_smem_desc_sw128(xb + (it % S::STAGES) * ASTAGE + o * STR, 16, 1024);
+        if (leader) {
+#pragma unroll
+          for (int k4 = 0; k4 < 4; ++k4) six_ss(d, ad, bd, k4, id_k);
+          umma_commit(done);
+        }
+        __syncwarp();
+      };
+      // products of the parts in region `at` with the rows of streamed operand o, into `d`; a step's leading product starts
+      // again, the small ones go on unless `fresh`
+      auto apply = [&](uint32_t at, int o, int it, uint32_t d, bool fresh) {
+        const uint64_t bd = umma_smem_desc_sw128(xb + (it % S::STAGES) * ASTAGE + o * STR, SBLK, 1024);
+        if (leader) {
+#pragma unroll
+          for (int k4 = 0; k4 < 4; ++k4) six_ts(d, at, bd, k4, id_mn, fresh && k4 == 0);
+        }
+      };
+      auto commit = [&](uint64_t* bar) {
+        if (leader) umma_commit(bar);
+        __syncwarp();
+      };
+      auto wait = [&](uint64_t* bar, int phase, int site) {
+        if (mbar_wait(bar, phase & 1)) {
+          tc_fence_after();
+          return true;
+        }
+        dev_set_error(a.status, SAF_DEV_TIMEOUT_MMA, site);
+        return false;
+      };
+      auto stage_full = [&](int it) { return wait(&sl->full[it % S::STAGES], it / S::STAGES, 76); };
+      const int n = x1 - x0;
+      bool ok = wait(&sl->res_full, 0, 77);
+      // Instructions of one thread run in order: a region is free for the next product once the last one that reads it has
+      // been issued and its readers in the compute warps have arrived.
+      if constexpr (MODE == A_FWD) {
+        for (int it = 0; it < 2 && it < n && ok; ++it)
+          if ((ok = stage_full(it))) scores(0, it, tmem + it * 128, &sl->s_full[it]);
+        for (int it = 0; it < n && ok; ++it) {
+          if (!(ok = wait(&sl->p_full, it, 78))) break;
+          apply(tmem + (it & 1) * 128, 1, it, tmem + T_ACC1 + (it & 1) * 128, true);
+          commit(&sl->empty[it % S::STAGES]);
+          commit(&sl->acc_full[it & 1]);
+          if (it + 2 < n && (ok = stage_full(it + 2))) scores(0, it + 2, tmem + (it & 1) * 128, &sl->s_full[it & 1]);
+        }
+      } else if constexpr (MODE == A_DKDV) {
+        // dV of a step and S of the next run while the compute warps make dS; dK and the next dP while they make P
+        if (n > 0 && ok && (ok = stage_full(0))) {
+          scores(0, 0, tmem + T_S, &sl->s_full[0]);
+          scores(1, 0, tmem + T_DP, &sl->dp_full);
+        }
+        for (int it = 0; it < n && ok; ++it) {
+          if (!(ok = wait(&sl->p_full, it, 78))) break;
+          apply(tmem + T_S, 1, it, tmem + T_ACC1, it == 0);
+          if (it + 1 < n) {
+            if (!(ok = stage_full(it + 1))) break;
+            scores(0, it + 1, tmem + T_S, &sl->s_full[0]);
+          }
+          if (!(ok = wait(&sl->ds_full, it, 74))) break;
+          apply(tmem + T_DP, 0, it, tmem + T_ACC2, it == 0);
+          commit(&sl->empty[it % S::STAGES]);
+          if (it + 1 < n) scores(1, it + 1, tmem + T_DP, &sl->dp_full);
+          else commit(&sl->acc_full[0]);
+        }
+      } else {
+        // S of the next step, in the other of two regions, is ready before a step's dS; its dP runs while they make P
+        constexpr uint32_t T_S2[2] = {T_S, T_ACC2};
+        if (n > 0 && ok && (ok = stage_full(0))) {
+          scores(0, 0, tmem + T_S, &sl->s_full[0]);
+          scores(1, 0, tmem + T_DP, &sl->dp_full);
+        }
+        for (int it = 0; it < n && ok; ++it) {
+          if (it + 1 < n) {
+            if (!(ok = stage_full(it + 1))) break;
+            scores(0, it + 1, tmem + T_S2[(it + 1) & 1], &sl->s_full[(it + 1) & 1]);
+          }
+          if (!(ok = wait(&sl->ds_full, it, 74))) break;
+          apply(tmem + T_DP, 0, it, tmem + T_ACC1, it == 0);
+          commit(&sl->empty[it % S::STAGES]);
+          if (it + 1 < n) scores(1, it + 1, tmem + T_DP, &sl->dp_full);
+          else commit(&sl->acc_full[0]);
+        }
+      }
+    }
+  } else {
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 88;");
+    const int quad = warp & 3, part = (warp - APROD / 32) >> 2, row = quad * 32 + lane, col = part * 16;
+    const int t = r0 + row;                                   // this thread's query (dK / dV: key)
+    const uint32_t lanes = tmem + ((uint32_t)(quad * 32) << 16) + col;
+    const float scale = a.sm_scale * F_LOG2E;
+    float acc1[16], acc2[16];
+#pragma unroll
+    for (int c = 0; c < 16; ++c) acc1[c] = acc2[c] = 0.f;
+    float m = -INFINITY, l = 0.f, L = 0.f, dl = 0.f;
+    if (MODE == A_DQ && t < T) {
+      L = f32_head(a.lse, hx.b, hx.h)[(int64_t)t * a.lse.stride[2]];
+      dl = f32_head(g.delta, hx.b, hx.h)[(int64_t)t * g.delta.stride[2]];
+    }
+    const int n = x1 - x0;
+    // the leading product of the step before (forward: and the small ones, which a new row maximum scales as well)
+    auto drain = [&](uint32_t at, float (&acc)[16], bool small) {
+      uint32_t x[16];
+      tmem_ld16(lanes + at, x);
+      tmem_ld_wait();
+#pragma unroll
+      for (int j = 0; j < 16; ++j) acc[j] += __uint_as_float(x[j]);
+      if (small) {
+        tmem_ld16(lanes + at + 64, x);
+        tmem_ld_wait();
+#pragma unroll
+        for (int j = 0; j < 16; ++j) acc[j] += __uint_as_float(x[j]);
+      }
+    };
+    auto hand_over = [&](uint64_t* bar) {
+      tmem_st_wait();
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(bar);
+    };
+    auto wait = [&](uint64_t* bar, int phase, int site) {
+      const bool in_time = mbar_wait(bar, phase & 1);
+      if (!in_time) dev_set_error(a.status, SAF_DEV_TIMEOUT_SOFTMAX, site);
+      tc_fence_after();
+      return in_time;
+    };
+    bool ok = true;
+    for (int it = 0; it < n; ++it) {
+      const int xb = (x0 + it) * AX + col;                    // this thread's first streamed row
+      const uint32_t sat = lanes + (MODE == A_FWD ? (it & 1) * 128 : (MODE == A_DQ && (it & 1) ? T_ACC2 : T_S));
+      ok = MODE == A_DKDV ? wait(&sl->s_full[0], it, 79) : wait(&sl->s_full[it & 1], it >> 1, 79);
+      if (MODE != A_FWD && !ok) break;                        // (the forward leaves at the vote, where the row's threads meet)
+      const bool edge = MODE == A_DKDV ? xb < r0 + AR || xb + 16 > T : xb + 15 > r0;       // some scores may be masked
+      float s[16];
+      tmem_sum16(sat, s);
+      if constexpr (MODE == A_FWD) {
+        float mx = -INFINITY;
+#pragma unroll
+        for (int j = 0; j < 16; ++j) s[j] *= scale;
+        if (edge) {
+#pragma unroll
+          for (int j = 0; j < 16; ++j)
+            if (xb + j > t || xb + j >= T) s[j] = -INFINITY;
+        }
+#pragma unroll
+        for (int j = 0; j < 16; ++j) mx = fmaxf(mx, s[j]);
+        sl->mx[it & 1][part][row] = mx;
+        if (named_bar_or(1, ACOMP, !ok)) {
+          ok = false;
+          break;
+        }
+        mx = fmaxf(fmaxf(sl->mx[it & 1][0][row], sl->mx[it & 1][1][row]), fmaxf(sl->mx[it & 1][2][row], sl->mx[it & 1][3][row]));
+        const float m_new = fmaxf(m, mx), m_safe = (m_new == -INFINITY) ? 0.f : m_new;
+        const float f = (m == -INFINITY) ? 0.f : exp2f(m - m_safe);
+        float sum = 0.f;
+#pragma unroll
+        for (int j = 0; j < 16; ++j) {
+          s[j] = exp2f(s[j] - m_safe);
+          sum += s[j];
+        }
+        tmem_parts16(sat, s);
+        hand_over(&sl->p_full);
+        l = l * f + sum;                                      // this thread's columns; added over the row at the end
+        m = m_new;
+        // the step before, from the other accumulator, under this one's product
+        if (it > 0) {
+          ok = wait(&sl->acc_full[(it - 1) & 1], (it - 1) >> 1, 80);
+          drain(T_ACC1 + ((it - 1) & 1) * 128, acc1, true);
+          tc_fence_before();                                  // (ordered before the next hand-over)
+        }
+#pragma unroll
+        for (int c = 0; c < 16; ++c) acc1[c] *= f;
+      } else {
+        const int st = it % S::STAGES;
+        // (the row statistics beside the tile)
+        if (MODE == A_DKDV && !(ok = wait(&sl->full[st], it / S::STAGES, 82))) break;
+#pragma unroll
+        for (int j = 0; j < 16; j += 4) {
+          const float4 Lj = MODE == A_DKDV ? *reinterpret_cast<const float4*>(&sl->lse[st][col + j]) : make_float4(L, L, L, L);
+          s[j] = exp2f(s[j] * scale - Lj.x);
+          s[j + 1] = exp2f(s[j + 1] * scale - Lj.y);
+          s[j + 2] = exp2f(s[j + 2] * scale - Lj.z);
+          s[j + 3] = exp2f(s[j + 3] * scale - Lj.w);
+        }
+        if (edge) {
+#pragma unroll
+          for (int j = 0; j < 16; ++j) {
+            const int x = xb + j;
+            if (MODE == A_DKDV ? x >= T || t > x : t >= T || x > t) s[j] = 0.f;
+          }
+        }
+        if constexpr (MODE == A_DKDV) {
+          tmem_parts16(sat, s);
+          if (it > 0) drain(T_ACC1, acc1, false);             // (S was issued after the dV of the step before)
+          hand_over(&sl->p_full);
+        }
+        if (!(ok = wait(&sl->dp_full, it, 83))) break;
+        float ds[16];
+        tmem_sum16(lanes + T_DP, ds);
+#pragma unroll
+        for (int j = 0; j < 16; j += 4) {
+          const float4 dj = MODE == A_DKDV ? *reinterpret_cast<const float4*>(&sl->delta[st][col + j]) : make_float4(dl, dl, dl, dl);
+          ds[j] = s[j] * (ds[j] - dj.x) * a.sm_scale;
+          ds[j + 1] = s[j + 1] * (ds[j + 1] - dj.y) * a.sm_scale;
+          ds[j + 2] = s[j + 2] * (ds[j + 2] - dj.z) * a.sm_scale;
+          ds[j + 3] = s[j + 3] * (ds[j + 3] - dj.w) * a.sm_scale;
+        }
+        tmem_parts16(lanes + T_DP, ds);
+        // (dP was issued after the dK / dQ of the step before)
+        if (it > 0) drain(MODE == A_DKDV ? T_ACC2 : T_ACC1, MODE == A_DKDV ? acc2 : acc1, false);
+        hand_over(&sl->ds_full);
+      }
+    }
+    if (n > 0 && ok) {
+      const int b = MODE == A_FWD ? (n - 1) & 1 : 0;
+      ok = wait(&sl->acc_full[b], MODE == A_FWD ? (n - 1) >> 1 : 0, 81);
+      drain(T_ACC1 + b * 128, acc1, true);
+      if constexpr (MODE == A_DKDV) drain(T_ACC2, acc2, true);
+    }
+    float top = 0.f;
+    bool odd = false;
+#pragma unroll
+    for (int c = 0; c < 16; ++c) {
+      odd |= !(fabsf(acc1[c]) < INFINITY) || !(fabsf(acc2[c]) < INFINITY);
+      top = fmaxf(top, fmaxf(fabsf(acc1[c]), fabsf(acc2[c])));
+    }
+    if (MODE == A_FWD) {
+      odd |= !(l < INFINITY);
+      sl->mx[0][part][row] = l;       // (the last step's maxima were read before its p_full; the vote orders the rest)
+    }
+    // nothing but tiny values in the whole tile, or something that is not finite: once more in plain fp32
+    const bool some = named_bar_or(1, ACOMP, top > 0.f), big = named_bar_or(1, ACOMP, top >= SPLIT_TINY);
+    odd = named_bar_or(1, ACOMP, odd) || (some && !big);
+    if (MODE == A_FWD) l = (sl->mx[0][0][row] + sl->mx[0][1][row]) + (sl->mx[0][2][row] + sl->mx[0][3][row]);
+    if (odd && t < T) {
+      const float *qb = f32_head(a.q, hx.b, hx.hq), *kb = f32_head(a.k, hx.b, hx.hk), *vb = f32_head(a.v, hx.b, hx.hv);
+      const float* dob = MODE == A_FWD ? nullptr : f32_head(g.dout, hx.b, hx.h);
+#pragma unroll
+      for (int c = 0; c < 16; ++c) acc1[c] = acc2[c] = 0.f;
+      m = -INFINITY;
+      l = 0.f;
+      const int lo = MODE == A_DKDV ? t : 0, hi = MODE == A_DKDV ? T : t + 1;
+      for (int x = lo; x < hi; ++x) {
+        const int qi = MODE == A_DKDV ? x : t, ki = MODE == A_DKDV ? t : x;
+        const float s = row_dot(qb + (int64_t)qi * a.q.stride[2], kb + (int64_t)ki * a.k.stride[2]) * scale;
+        if constexpr (MODE == A_FWD) {
+          const float m_new = fmaxf(m, s), m_safe = (m_new == -INFINITY) ? 0.f : m_new;
+          const float f = (m == -INFINITY) ? 0.f : exp2f(m - m_safe), p = exp2f(s - m_safe);
+          l = l * f + p;
+          m = m_new;
+#pragma unroll
+          for (int c = 0; c < 16; ++c) acc1[c] *= f;
+          axpy16(p, vb + (int64_t)ki * a.v.stride[2] + col, acc1);
+        } else {
+          const float* dor = dob + (int64_t)qi * g.dout.stride[2];
+          const float Lx = f32_head(a.lse, hx.b, hx.h)[(int64_t)qi * a.lse.stride[2]];
+          const float dx = f32_head(g.delta, hx.b, hx.h)[(int64_t)qi * g.delta.stride[2]];
+          const float p = exp2f(s - Lx);
+          const float ds = p * (row_dot(dor, vb + (int64_t)ki * a.v.stride[2]) - dx) * a.sm_scale;
+          if constexpr (MODE == A_DKDV) {
+            axpy16(p, dor + col, acc1);
+            axpy16(ds, qb + (int64_t)qi * a.q.stride[2] + col, acc2);
+          } else {
+            axpy16(ds, kb + (int64_t)ki * a.k.stride[2] + col, acc1);
+          }
+        }
+      }
+    }
+    if (t < T) {
+      if constexpr (MODE == A_FWD) {
+        const float ls = l == 0.f ? 1.f : l;
+        store16(a.out, hx.b, hx.h, t, col, acc1, 1.f / ls);
+        if (a.lse.ptr && part == 0)
+          reinterpret_cast<float*>(a.lse.ptr)[(int64_t)hx.b * a.lse.stride[0] + (int64_t)hx.h * a.lse.stride[1] + (int64_t)t * a.lse.stride[2]] =
+              ((m == -INFINITY) ? 0.f : m) + log2f(ls);
+      } else if constexpr (MODE == A_DKDV) {
+        store16(g.dv, hx.b, hx.hv, t, col, acc1, 1.f);
+        store16(g.dk, hx.b, hx.hk, t, col, acc2, 1.f);
+      } else {
+        store16(g.dq, hx.b, hx.hq, t, col, acc1, 1.f);
+      }
+    }
   }
+  tc_fence_before();
+  __syncthreads();
+  if (warp == AISSUER) tmem_dealloc(tmem, 512);
 }
 
-__global__ void __launch_bounds__(FNT, 2) f32_dq_kernel(const __grid_constant__ SafMixedAttnBwdArgs g) {
-  extern __shared__ __align__(16) float f32_smem[];
-  const SafMixedAttnArgs& a = g.fwd;
-  const HeadIdx hx = head_index(a, blockIdx.x);
-  if (hx.state != SAF_LIVE) return;
-  const int mt = gridDim.y - 1 - blockIdx.y, i0 = mt * FB, T = a.T;
-  float *Qs = f32_smem, *Ds = Qs + TILE_F, *Ks = Ds + TILE_F, *Vs = Ks + TILE_F, *Ss = Vs + TILE_F;
-  const int tid = threadIdx.x, ty = tid >> 4, tx = tid & 15;
-  const float *kb = f32_head(a.k, hx.b, hx.hk), *vb = f32_head(a.v, hx.b, hx.hv);
-  f32_tile(Qs, f32_head(a.q, hx.b, hx.hq), a.q.stride[2], i0, T);
-  f32_tile(Ds, f32_head(g.dout, hx.b, hx.h), g.dout.stride[2], i0, T);
-  float dq[8][4], L[8], dl[8];
-  const float* lse = f32_head(a.lse, hx.b, hx.h);
-  const float* del = f32_head(g.delta, hx.b, hx.h);
-#pragma unroll
-  for (int i = 0; i < 8; ++i) {
-    const int q = i0 + ty + 8 * i;
-    L[i] = q < T ? lse[(int64_t)q * a.lse.stride[2]] : 0.f;
-    dl[i] = q < T ? del[(int64_t)q * g.delta.stride[2]] : 0.f;
-#pragma unroll
-    for (int c = 0; c < 4; ++c) dq[i][c] = 0.f;
-  }
-  const float scale = a.sm_scale * F_LOG2E;
-  for (int jt = 0; jt <= mt; ++jt) {
-    const int j0 = jt * FB;
-    f32_tile(Ks, kb, a.k.stride[2], j0, T);
-    f32_tile(Vs, vb, a.v.stride[2], j0, T);
-    cp_async_commit();
-    cp_async_wait<0>();
-    __syncthreads();
-    float s[8][4], dp[8][4];
-    f32_dot(Qs, Ks, ty, tx, s);
-    f32_dot(Ds, Vs, ty, tx, dp);
-#pragma unroll
-    for (int i = 0; i < 8; ++i)
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const int r = ty + 8 * i, c = tx + 16 * j;
-        float ds = 0.f;
-        if (i0 + r < T && j0 + c <= i0 + r) ds = exp2f(s[i][j] * scale - L[i]) * (dp[i][j] - dl[i]) * a.sm_scale;
-        Ss[r * FLP + c] = ds;
-      }
-    __syncwarp();
-    f32_acc(Ss, Ks, ty, tx, dq);
-    __syncthreads();
-  }
-#pragma unroll
-  for (int i = 0; i < 8; ++i)
-    if (i0 + ty + 8 * i < T) f32_store(g.dq, hx.b, hx.hq, i0 + ty + 8 * i, tx, dq[i], 1.f);
+// grid (B * H, row tiles): the longest walks of all heads first
+__global__ void __launch_bounds__(ATHREADS, 1) attn_f32_fwd_kernel(const __grid_constant__ SafMixedAttnBwdArgs g) {
+  pdl_wait();
+  pdl_trigger();
+  attn_f32_tile<A_FWD>(g, blockIdx.y, gridDim.y);
+}
+// grid (B * H, 2 x row tiles): dK / dV and dQ tiles of one length take turns.  One launch for both, because a row tile's walk
+// has 2 to 2 tiles' length of steps and a launch of one kind alone ends with most SMs idle
+__global__ void __launch_bounds__(ATHREADS, 1) attn_f32_bwd_kernel(const __grid_constant__ SafMixedAttnBwdArgs g) {
+  pdl_wait();
+  pdl_trigger();
+  if (blockIdx.y & 1) attn_f32_tile<A_DQ>(g, blockIdx.y >> 1, gridDim.y >> 1);
+  else attn_f32_tile<A_DKDV>(g, blockIdx.y >> 1, gridDim.y >> 1);
 }
 
 // 16-byte rows: base, row, head and batch strides (an axis of one element is never stepped over)
@@ -293,7 +566,7 @@ bool f32_rows_ok(const SafTensor& t, int B, int Hn, int T) {
 bool f32_call_ok(const SafMixedAttnArgs& a) {
   const int kv = a.HKV > 0 ? a.HKV : 0;
   // (grid.y holds the row tiles)
-  return a.dtype == SAF_F32 && a.HD == FHD && !a.rope && a.U > 0 && a.T <= 65535 * FB && f32_rows_ok(a.q, a.B, a.U, a.T) &&
+  return a.dtype == SAF_F32 && a.HD == AHD && !a.rope && a.U > 0 && a.T <= 65535 * 64 && f32_rows_ok(a.q, a.B, a.U, a.T) &&
          f32_rows_ok(a.k, a.B, kv ? kv : a.U, a.T) && f32_rows_ok(a.v, a.B, kv ? kv : a.H, a.T) && f32_rows_ok(a.out, a.B, a.H, a.T);
 }
 
@@ -303,12 +576,12 @@ bool f32_call_ok(const SafMixedAttnArgs& a) {
 // with the any-type kernels.
 int launch_attn_f32_fwd(const SafMixedAttnArgs& a, cudaStream_t st) {
   if (!f32_call_ok(a)) return SAF_ERR_UNSUPPORTED;
-  constexpr int smem = (3 * TILE_F + PROB_F) * 4;
+  SafMixedAttnBwdArgs g;
+  memset(&g, 0, sizeof(g));
+  g.fwd = a;
   static PerDeviceOnce once;
-  if (int rc = ensure_dyn_smem(f32_fwd_kernel, smem, once)) return rc;
-  f32_fwd_kernel<<<dim3(a.B * a.H, (a.T + FB - 1) / FB), FNT, smem, st>>>(a);
-  count_launch();
-  return check_launch("f32_fwd_kernel");
+  if (int rc = ensure_dyn_smem(attn_f32_fwd_kernel, AttnShape<A_FWD>::SMEM, once)) return rc;
+  return launch_pdl("attn_f32_fwd_kernel", attn_f32_fwd_kernel, dim3(a.B * a.H, (a.T + AR - 1) / AR), ATHREADS, AttnShape<A_FWD>::SMEM, st, 1, g);
 }
 
 // dK, dV and dQ; delta is filled already
@@ -317,17 +590,11 @@ int launch_attn_f32_bwd(const SafMixedAttnBwdArgs& g, cudaStream_t st) {
   if (!f32_call_ok(a) || a.HKV > 0 || !f32_rows_ok(g.dout, a.B, a.H, a.T) || !f32_rows_ok(g.dv, a.B, a.H, a.T) ||
       !f32_rows_ok(g.dq, a.B, a.U, a.T) || !f32_rows_ok(g.dk, a.B, a.U, a.T))
     return SAF_ERR_UNSUPPORTED;
-  const dim3 grid(a.B * a.H, (a.T + FB - 1) / FB);
-  constexpr int smem_kv = (4 * TILE_F + 2 * PROB_F) * 4, smem_q = (4 * TILE_F + PROB_F) * 4;
-  static PerDeviceOnce once_kv, once_q;
-  if (int rc = ensure_dyn_smem(f32_dkdv_kernel, smem_kv, once_kv)) return rc;
-  if (int rc = ensure_dyn_smem(f32_dq_kernel, smem_q, once_q)) return rc;
-  f32_dkdv_kernel<<<grid, FNT, smem_kv, st>>>(g);
-  count_launch();
-  if (int rc = check_launch("f32_dkdv_kernel")) return rc;
-  f32_dq_kernel<<<grid, FNT, smem_q, st>>>(g);
-  count_launch();
-  return check_launch("f32_dq_kernel");
+  constexpr int smem = AttnShape<A_DKDV>::SMEM;
+  static_assert(smem >= AttnShape<A_DQ>::SMEM, "both kinds of tile fit");
+  static PerDeviceOnce once;
+  if (int rc = ensure_dyn_smem(attn_f32_bwd_kernel, smem, once)) return rc;
+  return launch_pdl("attn_f32_bwd_kernel", attn_f32_bwd_kernel, dim3(a.B * a.H, 2 * ((a.T + AR - 1) / AR)), ATHREADS, smem, st, 1, g);
 }
 
 }  // namespace saf

@@ -27,16 +27,14 @@
 #include <type_traits>
 
 #include "linear_tables.cuh"
-#include "sm100_prims.cuh"
+#include "split_bf16.cuh"
 
 namespace saf {
 namespace {
 
 constexpr int SI = 128, SK = 64;
-constexpr int SBLK = 64 * 64 * 2;              // 64 rows of 64 bf16
 constexpr int SPROD = 512, SEPI = 256, STHREADS = SPROD + SEPI + 128;
 constexpr int ISSUER = (SPROD + SEPI) / 32;
-constexpr float SPLIT_TINY = 1e-28f;
 constexpr int FBK = 32;                        // K slice of the FMA path
 
 template <int BN>
@@ -63,25 +61,6 @@ struct SplitParams {
   int* status;
 };
 
-__device__ __forceinline__ float4 ld4_or_0(const float* p, bool ok) {
-  return ok ? __ldg(reinterpret_cast<const float4*>(p)) : make_float4(0.f, 0.f, 0.f, 0.f);
-}
-// x - h, exact for h = bf16(x): the mixed-precision FMA takes either half of a packed pair without unpacking it
-__device__ __forceinline__ float minus_bf16(float x, uint16_t h) {
-  float r;
-  asm("fma.rn.f32.bf16 %0, %1, %2, %3;" : "=f"(r) : "h"(h), "h"((uint16_t)0xbf80u), "f"(x));
-  return r;
-}
-// two values -> their three parts, packed
-__device__ __forceinline__ void split2(float x, float y, uint32_t (&p)[3]) {
-  p[0] = pack_bf16(x, y);
-  x = minus_bf16(x, (uint16_t)p[0]);
-  y = minus_bf16(y, (uint16_t)(p[0] >> 16));
-  p[1] = pack_bf16(x, y);
-  x = minus_bf16(x, (uint16_t)p[1]);
-  y = minus_bf16(y, (uint16_t)(p[1] >> 16));
-  p[2] = pack_bf16(x, y);
-}
 __device__ __forceinline__ float4 ld_cluster4(uint32_t addr) {
   float4 v;
   asm volatile("ld.shared::cluster.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr) : "memory");
@@ -214,15 +193,7 @@ __global__ void __launch_bounds__(STHREADS, 1) linear_f32_split_kernel(const __g
 #pragma unroll
         for (int b = 0; b < (o ? S::NBJ : 2); ++b)
 #pragma unroll
-          for (int q = 0; q < 2; ++q) {
-            const float4 x = v[2 * o + b][q];
-            uint32_t w0[3], w1[3];
-            split2(x.x, x.y, w0);
-            split2(x.z, x.w, w1);
-#pragma unroll
-            for (int u = 0; u < 3; ++u)
-              *reinterpret_cast<uint2*>(st + o * 3 * S::A_PART + b * SBLK + q * 4096 + u * PART[o]) = make_uint2(w0[u], w1[u]);
-          }
+          for (int q = 0; q < 2; ++q) split_store(st + o * 3 * S::A_PART + b * SBLK + q * 4096, PART[o], v[2 * o + b][q]);
         if (kt + 1 < kt1) load(o, kt + 1);
       }
       fence_proxy_async_smem();

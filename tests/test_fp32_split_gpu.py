@@ -58,3 +58,62 @@ def test_values_the_parts_cannot_carry(what):
             continue
         # plain fp32 sums of up to 300 terms: 8 * 2^-24, as for the FMA kernels
         assert (a.double() - r)[fin].norm() <= 8 * 2.0 ** -24 * r[fin].norm()
+
+
+def causal_attention_64(q, k, v, do, scale):
+    """y, dq, dk, dv in 64 bits, each row from its own keys only: what later keys hold does not reach it."""
+    q, k, v, do = [t.double() for t in (q, k, v, do)]
+    T = q.shape[-2]
+    y, dq, dk, dv = [torch.zeros_like(t) for t in (v, q, k, v)]
+    for i in range(T):
+        qi, ki, vi, di = q[..., i:i + 1, :], k[..., :i + 1, :], v[..., :i + 1, :], do[..., i:i + 1, :]
+        p = ((qi @ ki.transpose(-1, -2)) * scale).softmax(-1)
+        yi = p @ vi
+        y[..., i, :] = yi[..., 0, :]
+        ds = p * (di @ vi.transpose(-1, -2) - (di * yi).sum(-1, keepdim=True)) * scale
+        dq[..., i, :] = (ds @ ki)[..., 0, :]
+        dk[..., :i + 1, :] += ds.transpose(-1, -2) @ qi
+        dv[..., :i + 1, :] += p.transpose(-1, -2) @ di
+    return y, dq, dk, dv
+
+
+def attention(q, k, v, do):
+    from kernel import fused_mixed_attn
+    d = [t.clone().requires_grad_(True) for t in (q, k, v)]
+    y = fused_mixed_attn(*d, None, torch.zeros(q.shape[1], dtype=torch.int32, device="cuda"))
+    y.backward(do)
+    return (y.detach(), *[t.grad for t in d])
+
+
+@pytest.mark.parametrize("sharp", [1.0, 4.0])
+@pytest.mark.parametrize("T", [1, 64, 65, 127, 129, 192, 500])
+def test_attention_against_64_bits(T, sharp):
+    g = torch.Generator(device="cuda").manual_seed(T)
+    q, k, v, do = [torch.randn(2, 2, T, 64, device="cuda", generator=g) for _ in range(4)]
+    q = q * sharp
+    # scores of size 8 sharp round by that times 2^-24 before they are exponentiated; the sums add less.  A single row has no
+    # score gradient: dO.V - dO.O of two equal sums of 64, each off by up to 2^-24 |dO| |V|, then times k or q
+    none = 2 * 2.0 ** -24 * 0.125 * do.norm() * v.norm() * max(k.norm(), q.norm())
+    for i, (a, r) in enumerate(zip(attention(q, k, v, do), causal_attention_64(q, k, v, do, 0.125))):
+        off = (a.double() - r).norm()
+        assert off <= (none if T == 1 and i in (1, 2) else 12 * sharp * 2.0 ** -24 * r.norm())
+
+
+@pytest.mark.parametrize("what", ["v inf", "k -inf", "q nan", "do nan", "do tiny"])
+def test_attention_on_values_the_parts_cannot_carry(what):
+    g = torch.Generator(device="cuda").manual_seed(8)
+    q, k, v, do = [torch.randn(1, 2, 200, 64, device="cuda", generator=g) for _ in range(4)]
+    if what == "v inf": v[0, 1, 70, 3] = float("inf")
+    if what == "k -inf": k[0, 1, 150, 9] = -float("inf")
+    if what == "q nan": q[0, 0, 30, 1] = float("nan")
+    if what == "do nan": do[0, 0, 130, 1] = float("nan")
+    if what == "do tiny": do *= 1e-34
+    for i, (a, r) in enumerate(zip(attention(q, k, v, do), causal_attention_64(q, k, v, do, 0.125))):
+        if what == "v inf" and i == 0:      # infinite where 64 bits are, and nowhere else
+            assert torch.equal(torch.isinf(a), torch.isinf(r.float()))
+        bad = ~torch.isfinite(r)
+        if what == "k -inf" and i:          # 0 * inf in the gradients of rows that give the key no weight
+            continue
+        assert torch.equal(~torch.isfinite(a), bad)
+        # do tiny: dS around 1e-35 has subnormal terms
+        assert (a.double() - r)[~bad].norm() <= (1e-2 if what == "do tiny" else 12 * 2.0 ** -24) * r[~bad].norm()
