@@ -344,27 +344,27 @@ int saf_attention_moments(const SafAttnStatsArgs* args, void* stream);
  * The attention layer as one call per direction: projection of [Q(live) | K(live) | V(all)] (grouped-query:
  * [Q(live) | K | V] of the HKV raw heads) with bias and RoPE, mixed attention, output projection with bias and
  * residual.  Replaces the cheap path of the reference's module (nanogpt/model.py:946-1077) on bf16 tensors; fp32 x or
- * weights are converted inside (autocast), and their gradients come back in fp32.  One caller-owned workspace per
- * direction; the forward's is handed to the backward unchanged.
+ * weights are converted inside (autocast), and their gradients come back in fp32.  With attn.dtype SAF_F32 (x and weights
+ * fp32, no residual) the layer computes in fp32.  One caller-owned workspace per direction; the forward's is handed to the backward unchanged.
  * ------------------------------------------------------------------------- */
 typedef struct SafAttnLayerArgs {
   int32_t struct_size;
   int32_t C;                /* x is (B*T, C)                                          */
   int32_t x_dtype, w_dtype; /* SAF_BF16, or SAF_F32: converted into the workspace     */
   int32_t train;            /* keep what saf_attn_layer_bwd needs                     */
-  SafMixedAttnArgs attn;    /* dtype SAF_BF16, dimensions, head states (frozen_host required), patterns, sm_scale,
+  SafMixedAttnArgs attn;    /* dtype of the computation, dimensions, head states (frozen_host required), patterns, sm_scale,
                                status; q, k, v, out, lse and sched are filled in by the call                    */
   const int32_t* live;      /* HOST (U): head of live slot u                          */
   const void* x;
   int64_t ldx;
   const void *wq, *wk, *wv; /* contiguous (H*HD, C); grouped-query K, V: (HKV*HD, C)  */
   const void* wo;           /* contiguous (C, H*HD)                                   */
-  const void *bq, *bk, *bv, *bo; /* bf16 or null; forward only                        */
+  const void *bq, *bk, *bv, *bo; /* attn.dtype or null; forward only                  */
   const float* rope_cos;    /* device (T, HD) fp32, or both null                      */
   const float* rope_sin;
   const void* residual;     /* bf16 (B*T, C) added to the result, or null             */
   int64_t ldr;
-  void* out;                /* bf16 (B*T, C)                                          */
+  void* out;                /* attn.dtype (B*T, C)                                    */
   int64_t ldo;
   void* work;               /* 256-byte aligned, saf_attn_layer_workspace() bytes     */
   int64_t work_bytes;
@@ -376,13 +376,13 @@ typedef struct SafAttnLayerBwdArgs {
   int32_t struct_size;
   int32_t need_dy;          /* dx and dwq null: still compute the gradient of the attention output          */
   SafAttnLayerArgs fwd;     /* as in the forward call, its workspace included         */
-  const void* dout;         /* bf16 (B*T, C)                                          */
+  const void* dout;         /* attn.dtype (B*T, C)                                    */
   int64_t lddo;
   void* dx;                 /* contiguous (B*T, C) in x_dtype, or null                */
   void *dwq, *dwk, *dwv;    /* like the weights, in w_dtype, every row written; all three or none           */
   void* dwo;                /* or null                                                */
   void* work;               /* 256-byte aligned; starts with the gradient of the attention output,
-                               bf16 (B*T, H*HD)                                       */
+                               attn.dtype (B*T, H*HD)                                 */
   int64_t work_bytes;
 } SafAttnLayerBwdArgs;
 

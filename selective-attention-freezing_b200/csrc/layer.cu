@@ -11,6 +11,8 @@
 //   backward  dY = dout Wo, dWo;  dQ, dK, dV of the attention written into one buffer of that layout;  adjoint RoPE of
 //             its Q and K slabs;  dx = d[QKV] W and dW = d[QKV]^T x as ONE product each, fp32 when the tensor is fp32
 //
+// In fp32 (all tensors fp32) the same sequence with the fp32 products and attention: nothing is converted, the rotation is a
+// launch of its own, dW goes straight to the gradients.
 // (nanogpt/model.py:946-1077, the cheap path of the reference's module.)  Measured on a B200, forward and backward of one
 // training layer under bf16 autocast: 12 x 64, T = 1024, B = 8 1.2-1.5 ms (41 launches, host-bound) -> 0.30 ms (14
 // launches); 16 x 128, T = 8192, B = 2 4.16 -> 3.36 ms (0.8 ms of it were fills, copies, conversions and additions);
@@ -41,6 +43,7 @@ struct BwdLayout {
 struct Dims {
   int B, T, H, U, HD, C, kv, D;     // kv: heads of the K part (V: H or HKV); D: width of the attention output
   int n_q, n_k, n_v;                // heads of the three parts of the projection
+  int es;                           // bytes of an element of the computation: 2, or 4 in fp32
   int64_t tok;
   int width() const { return (n_q + n_k + n_v) * HD; }
 };
@@ -54,6 +57,7 @@ Dims dims_of(const SafAttnLayerArgs& a) {
   d.kv = d.n_k;
   d.D = d.H * d.HD;
   d.tok = (int64_t)d.B * d.T;
+  d.es = dtype_size(a.attn.dtype);
   return d;
 }
 
@@ -69,17 +73,17 @@ FwdLayout fwd_layout(const SafAttnLayerArgs& a, const Dims& d) {
   int64_t at = 256;
   l.sched = 0;
   l.x = at;
-  if (a.x_dtype == SAF_F32) at += up(d.tok * d.C * 2);
+  if (a.x_dtype != a.attn.dtype) at += up(d.tok * d.C * 2);
   for (int i = 0; i < 4; ++i) {
     int r, c;
     weight_shape(a, d, i, &r, &c);
     l.w[i] = at;
-    if (a.w_dtype == SAF_F32) at += up((int64_t)r * c * 2);
+    if (a.w_dtype != a.attn.dtype) at += up((int64_t)r * c * 2);
   }
   l.qkv = at;
-  at += up(d.tok * d.width() * 2);
+  at += up(d.tok * d.width() * d.es);
   l.y = at;
-  at += up(d.tok * d.D * 2);
+  at += up(d.tok * d.D * d.es);
   l.lse = at;
   if (a.train) at += up((int64_t)d.B * d.H * d.T * 4);
   l.total = at;
@@ -90,13 +94,13 @@ BwdLayout bwd_layout(const SafAttnLayerArgs& a, const Dims& d) {
   BwdLayout l;
   int64_t at = 0;
   l.dy = at;
-  at += up(d.tok * d.D * 2);
+  at += up(d.tok * d.D * d.es);
   l.dqkv = at;
-  at += up(d.tok * d.width() * 2);
+  at += up(d.tok * d.width() * d.es);
   l.delta = at;
   at += up((int64_t)d.B * d.H * d.T * 4);
   l.dw = at;                         // the output projection's product is finished before the other one starts
-  at += up(std::max(gemm_dw_workspace_bytes(d.C, d.D, (int)d.tok), gemm_dw_workspace_bytes(d.width(), d.C, (int)d.tok)));
+  if (d.es == 2) at += up(std::max(gemm_dw_workspace_bytes(d.C, d.D, (int)d.tok), gemm_dw_workspace_bytes(d.width(), d.C, (int)d.tok)));
   l.total = at;
   return l;
 }
@@ -108,7 +112,8 @@ int validate_layer(const SafAttnLayerArgs* a) {
                 (int)sizeof(SafAttnLayerArgs));
   const SafMixedAttnArgs& t = a->attn;
   if (t.struct_size != (int32_t)sizeof(SafMixedAttnArgs)) return fail(SAF_ERR_INVALID, "SafMixedAttnArgs size mismatch");
-  if (t.dtype != SAF_BF16) return fail(SAF_ERR_UNSUPPORTED, "the layer entry computes in bf16");
+  if (t.dtype != SAF_BF16 && (t.dtype != SAF_F32 || a->x_dtype != SAF_F32 || a->w_dtype != SAF_F32))
+    return fail(SAF_ERR_UNSUPPORTED, "the layer entry computes in bf16, or in fp32 from fp32 tensors");
   if (t.B <= 0 || t.T <= 0 || t.H <= 0 || t.U < 0 || t.U > t.H || t.HD <= 0 || a->C <= 0 || t.HKV < 0)
     return fail(SAF_ERR_INVALID, "bad dimension");
   if (t.H > LAYER_MAX_HEADS || t.HKV > LAYER_MAX_HEADS) return fail(SAF_ERR_LIMIT, "more than %d heads", LAYER_MAX_HEADS);
@@ -127,9 +132,10 @@ int validate_layer(const SafAttnLayerArgs* a) {
   return SAF_OK;
 }
 
-SafTensor rows_view(void* base, int64_t first_col, int64_t ld, int T, int hd) {   // (B, heads, T, hd) inside token rows
+// (B, heads, T, hd) inside token rows of ld elements of es bytes
+SafTensor rows_view(void* base, int64_t first_col, int64_t ld, int T, int hd, int es) {
   SafTensor v;
-  v.ptr = reinterpret_cast<uint16_t*>(base) + first_col;
+  v.ptr = reinterpret_cast<uint8_t*>(base) + first_col * es;
   v.stride[0] = (int64_t)T * ld;
   v.stride[1] = hd;
   v.stride[2] = ld;
@@ -151,7 +157,7 @@ void qkv_slabs(const SafAttnLayerArgs& a, const Dims& d, Slabs* s) {
 
 // the weights as the products read them: converted copies in the workspace, or the caller's own
 const void* weight_ptr(const SafAttnLayerArgs& a, const FwdLayout& l, int i) {
-  if (a.w_dtype == SAF_F32) return reinterpret_cast<const uint8_t*>(a.work) + l.w[i];
+  if (a.w_dtype != a.attn.dtype) return reinterpret_cast<const uint8_t*>(a.work) + l.w[i];
   const void* w[4] = {a.wq, a.wk, a.wv, a.wo};
   return w[i];
 }
@@ -160,7 +166,7 @@ const void* weight_ptr(const SafAttnLayerArgs& a, const FwdLayout& l, int i) {
 void fill_linear(const SafAttnLayerArgs& a, const Dims& d, const FwdLayout& l, bool out_proj, Slabs* s, SafIndexedLinearArgs* g) {
   memset(g, 0, sizeof(*g));
   g->struct_size = (int32_t)sizeof(*g);
-  g->dtype = SAF_BF16;
+  g->dtype = a.attn.dtype;
   g->M = (int)d.tok;
   g->status = a.attn.status;
   uint8_t* work = reinterpret_cast<uint8_t*>(a.work);
@@ -178,8 +184,9 @@ void fill_linear(const SafAttnLayerArgs& a, const Dims& d, const FwdLayout& l, b
     g->ldw[0] = d.D;
     g->rows_w[0] = d.C;
   } else {
-    g->x = a.x_dtype == SAF_F32 ? work + l.x : a.x;
-    g->ldx = a.x_dtype == SAF_F32 ? d.C : a.ldx;
+    const bool converted = a.x_dtype != a.attn.dtype;
+    g->x = converted ? work + l.x : a.x;
+    g->ldx = converted ? d.C : a.ldx;
     g->C = d.C;
     g->n_weights = 3;
     g->slab = d.HD;
@@ -204,11 +211,11 @@ void attn_views(const SafAttnLayerArgs& a, const Dims& d, const FwdLayout& l, Sa
   *t = a.attn;
   const int64_t W = d.width();
   if (d.U > 0) {
-    t->q = rows_view(work + l.qkv, 0, W, d.T, d.HD);
-    t->k = rows_view(work + l.qkv, (int64_t)d.n_q * d.HD, W, d.T, d.HD);
+    t->q = rows_view(work + l.qkv, 0, W, d.T, d.HD, d.es);
+    t->k = rows_view(work + l.qkv, (int64_t)d.n_q * d.HD, W, d.T, d.HD, d.es);
   }
-  t->v = rows_view(work + l.qkv, (int64_t)(d.n_q + d.n_k) * d.HD, W, d.T, d.HD);
-  t->out = rows_view(work + l.y, 0, d.D, d.T, d.HD);
+  t->v = rows_view(work + l.qkv, (int64_t)(d.n_q + d.n_k) * d.HD, W, d.T, d.HD, d.es);
+  t->out = rows_view(work + l.y, 0, d.D, d.T, d.HD, d.es);
   memset(&t->lse, 0, sizeof(t->lse));
   if (a.train) {
     t->lse.ptr = work + l.lse;
@@ -216,7 +223,7 @@ void attn_views(const SafAttnLayerArgs& a, const Dims& d, const FwdLayout& l, Sa
     t->lse.stride[1] = d.T;
     t->lse.stride[2] = 1;
   }
-  t->sched = d.U > 0 ? reinterpret_cast<int32_t*>(work + l.sched) : nullptr;
+  t->sched = d.U > 0 && d.es == 2 ? reinterpret_cast<int32_t*>(work + l.sched) : nullptr;
 }
 
 }  // namespace
@@ -265,11 +272,12 @@ int saf_attn_layer_fwd(const SafAttnLayerArgs* args, void* stream) {
   uint8_t* work = reinterpret_cast<uint8_t*>(a.work);
   CastSegment seg[MAX_CAST_SEGMENTS];
   int ns = 0;
-  if (a.x_dtype == SAF_F32) {
-    if (a.ldx != d.C) return fail(SAF_ERR_INVALID, "an fp32 x must be contiguous");
+  if (a.x_dtype == SAF_F32 && a.ldx != d.C) return fail(SAF_ERR_INVALID, "an fp32 x must be contiguous");
+  if (d.es == 4 && a.residual) return fail(SAF_ERR_UNSUPPORTED, "the fp32 layer adds no residual");
+  if (a.x_dtype != a.attn.dtype) {
     seg[ns++] = {reinterpret_cast<const float*>(a.x), work + l.x, d.tok * d.C};
   }
-  if (a.w_dtype == SAF_F32) {
+  if (a.w_dtype != a.attn.dtype) {
     const void* w[4] = {a.wq, a.wk, a.wv, a.wo};
     for (int i = 0; i < 4; ++i) {
       int r, c;
@@ -320,7 +328,7 @@ int saf_attn_layer_bwd(const SafAttnLayerBwdArgs* args, void* stream) {
     return fail(SAF_ERR_INVALID, "null pointer or workspace too small");
   cudaStream_t st = (cudaStream_t)stream;
   uint8_t* bw = reinterpret_cast<uint8_t*>(args->work);
-  const bool w32 = a.w_dtype == SAF_F32, x32 = a.x_dtype == SAF_F32;
+  const bool f32 = d.es == 4, w32 = a.w_dtype == SAF_F32, x32 = a.x_dtype == SAF_F32;
   float* ws = reinterpret_cast<float*>(bw + b.dw);
   const int64_t ws_bytes = b.total - b.dw;
   Slabs s, so;
@@ -329,11 +337,14 @@ int saf_attn_layer_bwd(const SafAttnLayerBwdArgs* args, void* stream) {
   fill_linear(a, d, l, true, &so, &go);
   if ((rc = validate_linear_args(&g)) || (rc = validate_linear_args(&go))) return rc;
   // ---- output projection: dY and dWo
-  if ((rc = launch_gemm_bwd_dx_sm100(go, args->dout, args->lddo, bw + b.dy, d.D, nullptr, false, st))) return rc;
+  rc = f32 ? launch_gemm_bwd_dx(go, args->dout, args->lddo, bw + b.dy, d.D, nullptr, st)
+           : launch_gemm_bwd_dx_sm100(go, args->dout, args->lddo, bw + b.dy, d.D, nullptr, false, st);
+  if (rc) return rc;
   if (args->dwo) {
     SafIndexedLinearArgs gw = go;
     gw.weights[0] = args->dwo;
-    if ((rc = launch_gemm_bwd_dw_full_sm100(gw, args->dout, args->lddo, ws, ws_bytes, w32, st))) return rc;
+    rc = f32 ? launch_gemm_bwd_dw(gw, args->dout, args->lddo, st) : launch_gemm_bwd_dw_full_sm100(gw, args->dout, args->lddo, ws, ws_bytes, w32, st);
+    if (rc) return rc;
   }
   if (!args->dx && !args->dwq && !args->need_dy) return SAF_OK;
   // ---- attention: every gradient lands in one buffer of the projection's layout
@@ -343,12 +354,12 @@ int saf_attn_layer_bwd(const SafAttnLayerBwdArgs* args, void* stream) {
   attn_views(a, d, l, &m.fwd);
   m.fwd.sched = nullptr;
   const int64_t W = d.width();
-  m.dout = rows_view(bw + b.dy, 0, d.D, d.T, d.HD);
+  m.dout = rows_view(bw + b.dy, 0, d.D, d.T, d.HD, d.es);
   if (d.U > 0) {
-    m.dq = rows_view(bw + b.dqkv, 0, W, d.T, d.HD);
-    m.dk = rows_view(bw + b.dqkv, (int64_t)d.n_q * d.HD, W, d.T, d.HD);
+    m.dq = rows_view(bw + b.dqkv, 0, W, d.T, d.HD, d.es);
+    m.dk = rows_view(bw + b.dqkv, (int64_t)d.n_q * d.HD, W, d.T, d.HD, d.es);
   }
-  m.dv = rows_view(bw + b.dqkv, (int64_t)(d.n_q + d.n_k) * d.HD, W, d.T, d.HD);
+  m.dv = rows_view(bw + b.dqkv, (int64_t)(d.n_q + d.n_k) * d.HD, W, d.T, d.HD, d.es);
   m.delta.ptr = bw + b.delta;
   m.delta.stride[0] = (int64_t)d.H * d.T;
   m.delta.stride[1] = d.T;
@@ -356,15 +367,26 @@ int saf_attn_layer_bwd(const SafAttnLayerBwdArgs* args, void* stream) {
   if (!args->dx && !args->dwq) return SAF_OK;
   if ((rc = saf_mixed_attn_bwd(&m, stream))) return rc;
   if (a.rope_cos && d.U > 0 &&
-      (rc = launch_rope_slabs(bw + b.dqkv, W, (int)d.tok, d.n_q + d.n_k, d.HD, d.T, nullptr, a.rope_cos, a.rope_sin, SAF_BF16, 1, st)))
+      (rc = launch_rope_slabs(bw + b.dqkv, W, (int)d.tok, d.n_q + d.n_k, d.HD, d.T, nullptr, a.rope_cos, a.rope_sin, a.attn.dtype, 1, st)))
     return rc;
   // ---- projection: dx and the three weight gradients, one product each
-  if (args->dx && (rc = launch_gemm_bwd_dx_sm100(g, bw + b.dqkv, W, args->dx, d.C, nullptr, x32, st))) return rc;
+  if (args->dx) {
+    rc = f32 ? launch_gemm_bwd_dx(g, bw + b.dqkv, W, args->dx, d.C, nullptr, st)
+             : launch_gemm_bwd_dx_sm100(g, bw + b.dqkv, W, args->dx, d.C, nullptr, x32, st);
+    if (rc) return rc;
+  }
   if (args->dwq) {
     SafIndexedLinearArgs gw = g;
     gw.weights[0] = args->dwq;
     gw.weights[1] = args->dwk;
     gw.weights[2] = args->dwv;
+    if (f32) {
+      // rows of frozen heads belong to no slab of the product: exactly zero
+      const size_t bytes = (size_t)d.D * d.C * 4;
+      if (d.U < d.H && (cudaMemsetAsync(args->dwq, 0, bytes, st) != cudaSuccess || cudaMemsetAsync(args->dwk, 0, bytes, st) != cudaSuccess))
+        return fail(SAF_ERR_CUDA, "cudaMemsetAsync");
+      return launch_gemm_bwd_dw(gw, bw + b.dqkv, W, st);
+    }
     if ((rc = launch_gemm_bwd_dw_full_sm100(gw, bw + b.dqkv, W, ws, ws_bytes, w32, st))) return rc;
   }
   return SAF_OK;
@@ -399,7 +421,7 @@ int validate_block(const SafBlockArgs* b) {
   if (b->struct_size != (int32_t)sizeof(SafBlockArgs))
     return fail(SAF_ERR_INVALID, "SafBlockArgs size mismatch: caller %d, library %d", b->struct_size, (int)sizeof(SafBlockArgs));
   if (int rc = validate_layer(&b->layer)) return rc;
-  if (b->layer.x_dtype != SAF_BF16 || b->layer.w_dtype != SAF_BF16 || b->layer.train)
+  if (b->layer.attn.dtype != SAF_BF16 || b->layer.x_dtype != SAF_BF16 || b->layer.w_dtype != SAF_BF16 || b->layer.train)
     return fail(SAF_ERR_UNSUPPORTED, "the block entry is bf16 inference");
   if (b->hidden <= 0 || b->hidden % (b->gated ? 128 : 64) || b->layer.C % 64) return fail(SAF_ERR_UNSUPPORTED, "width %d, hidden %d", b->layer.C, b->hidden);
   if (b->hidden / 64 * (b->gated ? 2 : 1) > MLP_MAX_BLOCKS) return fail(SAF_ERR_LIMIT, "hidden %d", b->hidden);

@@ -369,14 +369,16 @@ class SafCausalSelfAttention(nn.Module):
         return patt, None
 
     def _layer_call(self, x, rope):
-        """Arguments of `layer.attention_layer` for this call, or None when the layer runs operator by operator: fp32,
-        head widths the tensor-core kernels do not take, attention dropout, bias gradients."""
+        """Arguments of `layer.attention_layer` for this call, or None when the layer runs operator by operator: head widths
+        the tensor-core kernels do not take, attention dropout, bias gradients, fp32 from anything but fp32 tensors."""
         act_dt = torch.get_autocast_dtype("cuda") if torch.is_autocast_enabled("cuda") else x.dtype
-        if act_dt != torch.bfloat16 or not self._live or (self.dropout > 0.0 and self.training):
+        if act_dt not in (torch.bfloat16, torch.float32) or not self._live or (self.dropout > 0.0 and self.training):
             return None
         grad = torch.is_grad_enabled()
         q_proj = self.q_proj
         w = (q_proj.weight, self.k_proj.weight, self.v_proj.weight, self.c_proj.weight)
+        if act_dt == torch.float32 and (x.dtype != act_dt or w[0].dtype != act_dt):
+            return None
         bias = q_proj.bias is not None
         # without autocast, training wants x and the weights in one dtype (the separate operators say so)
         mixed = grad and w[0].dtype != x.dtype and not torch.is_autocast_enabled("cuda")
@@ -384,7 +386,7 @@ class SafCausalSelfAttention(nn.Module):
             return None
         T = x.shape[1]
         call = dict(weights=w, rope=self._rope_f32(rope, T, x.device), frozen=self._fz_mask_i32, hidx=self._hidx_i32,
-                    sink_decay=self._sd)
+                    sink_decay=self._sd, dtype=act_dt)
         if 1 in self._states:
             call["patt"], call["pidx"] = self._patterns(act_dt)
         if self._dec_any:
@@ -405,7 +407,7 @@ class SafCausalSelfAttention(nn.Module):
         nh, hd = self.n_head, self.head_dim
         call = self._layer_call(x, rope)
         if call is not None:
-            if torch.is_grad_enabled() and residual is not None:
+            if residual is not None and (torch.is_grad_enabled() or call["dtype"] != torch.bfloat16):
                 return residual + _layer.attention_layer(self._plan, x, **call)
             residual = None if residual is None else residual.to(torch.bfloat16)
             return _layer.attention_layer(self._plan, x, residual=residual, **call)
@@ -436,7 +438,7 @@ class SafCausalSelfAttention(nn.Module):
                 return ops.linear_act(y, cw, cb, residual=residual.to(act_dt))   # residual add in the GEMM epilogue
             out = ops.linear_rows(y, cw, cb, self._all_rows)
             return out if residual is None else residual + out
-        # training / fp32: live-only Q,K projection with exact-zero frozen rows in the weight gradient; v_proj and
+        # training / fp32, operator by operator: live-only Q,K projection with exact-zero frozen rows in the weight gradient; v_proj and
         # c_proj run on the library's own forward / dx / dW GEMMs too (all rows selected)
         v = ops.linear_rows(x, self.v_proj.weight, self.v_proj.bias, self._all_rows).view(B, T, nh, hd).transpose(1, 2)
         if nuf == 0:

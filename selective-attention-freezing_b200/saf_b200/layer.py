@@ -61,6 +61,7 @@ class LayerPlan:
         a = SafAttnLayerArgs.from_buffer_copy(self._template)
         t = a.attn
         x = c.x
+        t.dtype = _DT[c.dt]
         t.B, t.T = c.B, c.T
         t.status = ops._status_ptr(x.device)
         t.frozen, t.hidx = c.frozen.data_ptr(), c.hidx.data_ptr()
@@ -88,7 +89,7 @@ class LayerPlan:
     def sizes(self, a):
         """(forward bytes, backward bytes, offset of the projection, offset of the attention output)."""
         t = a.attn
-        key = (t.B, t.T, a.x_dtype, a.w_dtype, a.train)
+        key = (t.B, t.T, t.dtype, a.x_dtype, a.w_dtype, a.train)
         got = self._sizes.get(key)
         if got is None:
             out = (C.c_int64 * 4)()
@@ -100,12 +101,13 @@ class LayerPlan:
 
 
 class _Call:
-    """Tensors of one layer call, in the form the library reads them."""
-    __slots__ = ("B", "T", "x", "w", "train", "rope", "frozen", "hidx", "kvidx", "sink_decay", "patt", "pidx", "alpha", "rho", "z")
+    """Tensors of one layer call, in the form the library reads them; dt is the dtype of the computation."""
+    __slots__ = ("B", "T", "x", "w", "train", "rope", "frozen", "hidx", "kvidx", "sink_decay", "patt", "pidx", "alpha", "rho", "z",
+                 "dt")
 
     def __init__(self, B, T, x, w, train, rope, frozen, hidx, kvidx=None, sink_decay=None, patt=None, pidx=None,
-                 decomposed=(None, None, None)):
-        self.B, self.T, self.x, self.w, self.train, self.rope = B, T, x, w, train, rope
+                 decomposed=(None, None, None), dt=torch.bfloat16):
+        self.B, self.T, self.x, self.w, self.train, self.rope, self.dt = B, T, x, w, train, rope, dt
         self.frozen, self.hidx, self.kvidx, self.sink_decay = frozen, hidx, kvidx, sink_decay
         self.patt, self.pidx = patt, pidx
         self.alpha, self.rho, self.z = decomposed
@@ -151,12 +153,12 @@ def _blob(n, device):
 
 
 def _forward(plan, c, biases=None, residual=None):
-    """Enqueues the layer; returns (out (tokens, C) bf16, workspace, sizes)."""
+    """Enqueues the layer; returns (out (tokens, C), workspace, sizes)."""
     a = plan.args(c)
     sz = plan.sizes(a)
     dev = c.x.device
     work = _blob(sz[0], dev)
-    out = torch.empty((c.B * c.T, plan.C), dtype=torch.bfloat16, device=dev)
+    out = torch.empty((c.B * c.T, plan.C), dtype=c.dt, device=dev)
     a.out, a.ldo = out.data_ptr(), plan.C
     a.work, a.work_bytes = work.data_ptr(), sz[0]
     if biases is not None:
@@ -170,13 +172,13 @@ def _forward(plan, c, biases=None, residual=None):
     return out, work, sz
 
 
-def projection_views(plan, work, sz, B, T):
+def projection_views(plan, work, sz, B, T, dt=torch.bfloat16):
     """q, k, v (B, heads, T, hd) and the attention output y inside a forward workspace."""
-    W, hd = plan.width(), plan.hd
+    W, hd, es = plan.width(), plan.hd, dt.itemsize
     n = B * T * W
-    qkv = work[sz[2]:sz[2] + 2 * n].view(torch.bfloat16).view(B, T, W // hd, hd)
+    qkv = work[sz[2]:sz[2] + es * n].view(dt).view(B, T, W // hd, hd)
     nk = plan.n_kv or plan.U
-    y = work[sz[3]:sz[3] + 2 * B * T * plan.H * hd].view(torch.bfloat16).view(B, T, plan.H, hd)
+    y = work[sz[3]:sz[3] + es * B * T * plan.H * hd].view(dt).view(B, T, plan.H, hd)
     q, k, v = qkv[:, :, :plan.U], qkv[:, :, plan.U:plan.U + nk], qkv[:, :, plan.U + nk:]
     return q.transpose(1, 2), k.transpose(1, 2), v.transpose(1, 2), y.transpose(1, 2)
 
@@ -188,12 +190,12 @@ class _LayerFunction(torch.autograd.Function):
     def forward(ctx, x, wq, wk, wv, wo, alpha_p, rho_p, plan, c, measure):
         out, work, sz = _forward(plan, c)
         if measure is not None:
-            q, k, _, _ = projection_views(plan, work, sz, c.B, c.T)
+            q, k, _, _ = projection_views(plan, work, sz, c.B, c.T, c.dt)
             measure(q, k)
-        ctx.plan, ctx.sz, ctx.bt = plan, sz, (c.B, c.T)
-        ctx.x_like, ctx.w_cast = (x.shape, x.dtype), wq.dtype != torch.bfloat16
+        ctx.plan, ctx.sz, ctx.bt, ctx.dt = plan, sz, (c.B, c.T), c.dt
+        ctx.x_like, ctx.w_cast = (x.shape, x.dtype), wq.dtype != c.dt
         # (converted tensors live in the workspace: the originals are not needed again)
-        kept = [work, c.x if x.dtype == torch.bfloat16 else None]
+        kept = [work, c.x if x.dtype == c.dt else None]
         kept += [None] * 4 if ctx.w_cast else [wq, wk, wv, wo]
         kept += [c.patt, c.pidx, c.alpha, c.rho, c.z, *(c.rope or (None, None))]
         ctx.save_for_backward(*kept, c.frozen, c.hidx, *(c.sink_decay or ()))
@@ -211,13 +213,13 @@ class _LayerFunction(torch.autograd.Function):
         B, T = ctx.bt
         dev = dout.device
         need = ctx.needs_input_grad
-        d2 = _bf16_rows(dout)
+        d2 = _bf16_rows(dout) if ctx.dt == torch.bfloat16 else _rows(dout)
         x_shape, x_dtype = ctx.x_like
         # a converted tensor is read from the workspace; its argument only tells the dtype and layout
         x_arg = x2 if x2 is not None else work.view(torch.float32)[:plan.C].view(1, plan.C)
         w_arg = [wq, wk, wv, wo] if wq is not None else [work.view(torch.float32)] * 4
         c = _Call(B, T, x_arg, w_arg, 1, (cos, sin) if cos is not None else None, frozen, hidx, None, sink_decay, patt, pidx,
-                  (alpha, rho, z))
+                  (alpha, rho, z), ctx.dt)
         g = SafAttnLayerBwdArgs()
         g.struct_size = C.sizeof(SafAttnLayerBwdArgs)
         g.fwd = plan.args(c)
@@ -241,8 +243,8 @@ class _LayerFunction(torch.autograd.Function):
         da = dr = None
         if ctx.learns:
             from .trainable_patterns import pattern_param_grad
-            _, _, v, y = projection_views(plan, work, sz, B, T)
-            dy = scratch[:2 * B * T * plan.H * plan.hd].view(torch.bfloat16).view(B, T, plan.H, plan.hd).transpose(1, 2)
+            _, _, v, y = projection_views(plan, work, sz, B, T, ctx.dt)
+            dy = scratch[:ctx.dt.itemsize * B * T * plan.H * plan.hd].view(ctx.dt).view(B, T, plan.H, plan.hd).transpose(1, 2)
             da, dr = pattern_param_grad(dy, y, v, alpha, rho, z, frozen)
         return (dx, *[t if need[1 + i] else None for i, t in enumerate(dw)], da, dr, None, None, None)
 
@@ -260,23 +262,24 @@ def _residual_rows(residual, tokens, width):
 
 
 def attention_layer(plan, x, weights, rope, frozen, hidx, *, kvidx=None, sink_decay=None, patt=None, pidx=None,
-                    decomposed=(None, None, None), learn=None, biases=None, residual=None, measure=None):
-    """x (B, T, C) -> bf16 (B, T, C).  weights: q, k, v, o; decomposed: (alpha, rho, z) buffers; learn: (alpha, rho)
-    parameters that receive gradients (decomposed then holds their detached values and current normalisers);
-    measure: called with the rotated q, k of the live heads.  Biases and residual go with inference."""
+                    decomposed=(None, None, None), learn=None, biases=None, residual=None, measure=None, dtype=torch.bfloat16):
+    """x (B, T, C) -> (B, T, C) in `dtype`, the dtype of the computation: bf16, or fp32 with everything in fp32.  weights:
+    q, k, v, o; decomposed: (alpha, rho, z) buffers; learn: (alpha, rho) parameters that receive gradients (decomposed then
+    holds their detached values and current normalisers); measure: called with the rotated q, k of the live heads.  Biases
+    and residual go with inference, the residual with bf16."""
     enabled = torch.is_grad_enabled()
     grad = enabled and (x.requires_grad or learn is not None or any(w.requires_grad for w in weights))
     if residual is not None:
         residual = _residual_rows(residual, x.shape[0] * x.shape[1], plan.C)
     c = _Call(x.shape[0], x.shape[1], _rows(x.detach()), weights, int(grad), rope, frozen, hidx, kvidx, sink_decay, patt, pidx,
-              decomposed)
+              decomposed, dtype)
     # (also when nothing wants a gradient: forward-mode tangents are refused there instead of getting lost)
     if grad or (enabled and biases is None and residual is None):
         ap, rp = learn if learn is not None else (None, None)
         return _LayerFunction.apply(x, *weights, ap, rp, plan, c, measure)
     out, work, sz = _forward(plan, c, biases, residual)
     if measure is not None:
-        q, k, _, _ = projection_views(plan, work, sz, c.B, c.T)
+        q, k, _, _ = projection_views(plan, work, sz, c.B, c.T, c.dt)
         measure(q, k)
     return out.view(c.B, c.T, plan.C)
 
