@@ -93,6 +93,10 @@ struct Cfg {
 
 // ring depth of the tensor-core scan when it runs in a scan slot of these launches: what their shared memory holds
 constexpr int SCAN_ROLE_STAGES = 8;
+// shortest sequence whose structured heads take the tensor-core scan: below it the register scan, one 64-column slice after
+// the other, is as fast
+template <int HD>
+constexpr int SCAN_MMA_MIN_T = HD == 64 ? 4 * MB : 1;
 static_assert(ms_smem_bytes(SCAN_ROLE_STAGES) <= Cfg<64>::SMEM_BYTES && ms_smem_bytes(SCAN_ROLE_STAGES) <= Cfg<64>::SMEM_PERSIST &&
                   ms_smem_bytes(SCAN_ROLE_STAGES) <= Cfg<128>::SMEM_BYTES && ms_smem_bytes(SCAN_ROLE_STAGES) <= Cfg<128>::SMEM_PERSIST,
               "the scan role must fit the launches' dynamic shared memory");
@@ -190,8 +194,9 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant
     if (state == SAF_SINK_DECAY && p.has_scan) {
       {
         // the whole sequence as 128-row Toeplitz products on the tensor core, one 64-column slice after the other
-        // (about a third of the time of the register scan, so the SM joins the live tiles that much earlier)
-        if (p.T >= 4 * MB && p.scan.HD == HD) {
+        // (about a third of the time of the register scan, so the SM joins the live tiles that much earlier); head width 96
+        // as well, whose second slice the tensor maps clip
+        if (p.T >= SCAN_MMA_MIN_T<HD>) {
           extern __shared__ uint8_t scan_smem_raw[];
           MsParams mp;
           mp.a = p.scan;
@@ -747,8 +752,9 @@ flash_fwd_persistent_kernel(const __grid_constant__ CUtensorMap mapQ, const __gr
     if (state == SAF_SINK_DECAY && p.has_scan) {
       {
         // the whole sequence as 128-row Toeplitz products on the tensor core, one 64-column slice after the other
-        // (about a third of the time of the register scan, so the SM joins the live tiles that much earlier)
-        if (p.T >= 4 * MB && p.scan.HD == HD) {
+        // (about a third of the time of the register scan, so the SM joins the live tiles that much earlier); head width 96
+        // as well, whose second slice the tensor maps clip
+        if (p.T >= SCAN_MMA_MIN_T<HD>) {
           extern __shared__ uint8_t scan_smem_raw[];
           MsParams mp;
           mp.a = p.scan;

@@ -155,7 +155,7 @@ __device__ __forceinline__ void sink_decay_apply_mma_cta(const CUtensorMap& mapV
       if (p.use_stash && wg == 0) carry_in = *scan_stash<__nv_bfloat16>(const_cast<__nv_bfloat16*>(ob0), a.so[2], p_lo, et);
       const __nv_bfloat16* v0 = reinterpret_cast<const __nv_bfloat16*>(a.in) + (int64_t)b * a.si[0] + (int64_t)hin * a.si[1] +
                                 (int64_t)(col0 + sl * SCAN_COLS + et);
-      v_first = __bfloat162float(*v0);
+      if (col0 + sl * SCAN_COLS + et < a.HD) v_first = __bfloat162float(*v0);      // (a width of 96 ends inside a slice)
     }
     // Toeplitz operand in TMEM, row `lrow`, column k = the bf16 pair (L[2k], L[2k+1]): its bf16 head from warpgroup 0
     // and the bf16 remainder from warpgroup 1
