@@ -283,7 +283,14 @@ flash_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_con
     const int bh = blockIdx.x / PER, col0 = (blockIdx.x % PER) * SCAN_COLS;
     const int sb = bh / p.H, sh = bh % p.H;
     const int state = p.force_state >= 0 ? p.force_state : p.frozen[sh];
-    if (state == SAF_SINK_DECAY && threadIdx.x < SCAN_NT) {
+    // (its eight warps take the registers of the third warpgroup: at the launch's 168 the scan spilled, and set the time of
+    // launches of few heads -- 9 live + 3 structured heads, T = 3001, B = 1: width 96 86 -> 60 us, 128 77 -> 61, 64 67 -> 58)
+    if (threadIdx.x >= SCAN_NT) {
+      breg_dec<56>();
+      return;
+    }
+    breg_inc<224>();
+    if (state == SAF_SINK_DECAY) {
       extern __shared__ uint8_t scan_smem_raw[];
       float* scratch = reinterpret_cast<float*>(((uintptr_t)scan_smem_raw + 1023) & ~(uintptr_t)1023);
       sink_decay_scan_cta<__nv_bfloat16, true, 0, true>(p.scan, sb, sh, col0, 0, -1, scratch);
