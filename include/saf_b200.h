@@ -269,6 +269,10 @@ int saf_decomposed_logz(const float* alpha, const float* rho, float* z, int32_t 
  * ------------------------------------------------------------------------- */
 int saf_pattern_normalisers(const float* alpha, const float* rho, float* z, int32_t H, int32_t S, int32_t T,
                             void* stream);
+/* The same for the heads whose state (device int32 (H,)) is SAF_DECOMP, the only ones whose z is read; the others' rows are
+ * set to zero. */
+int saf_pattern_normalisers_of(const float* alpha, const float* rho, float* z, const int32_t* states, int32_t H, int32_t S,
+                               int32_t T, void* stream);
 
 typedef struct SafPatternGradArgs {
   int32_t struct_size; /* sizeof(SafPatternGradArgs), checked                        */

@@ -458,7 +458,7 @@ int saf_decomposed_logz(const float* alpha, const float* rho, float* z, int32_t 
   if (H < 0 || S < 0) return fail(SAF_ERR_INVALID, "negative dimension");
   if (H == 0 || S == 0) return SAF_OK;
   if (!alpha || !rho || !z) return fail(SAF_ERR_INVALID, "null pointer");
-  return launch_logz(alpha, rho, z, H, S, S, (cudaStream_t)stream);
+  return launch_logz(alpha, rho, z, nullptr, H, S, S, (cudaStream_t)stream);
 }
 
 int saf_pattern_normalisers(const float* alpha, const float* rho, float* z, int32_t H, int32_t S, int32_t T,
@@ -467,7 +467,16 @@ int saf_pattern_normalisers(const float* alpha, const float* rho, float* z, int3
   if (T > S) return fail(SAF_ERR_INVALID, "pattern normalisers: T > S");
   if (H == 0 || S == 0) return SAF_OK;
   if (!alpha || !rho || !z) return fail(SAF_ERR_INVALID, "null pointer");
-  return launch_logz(alpha, rho, z, H, S, T, (cudaStream_t)stream);
+  return launch_logz(alpha, rho, z, nullptr, H, S, T, (cudaStream_t)stream);
+}
+
+int saf_pattern_normalisers_of(const float* alpha, const float* rho, float* z, const int32_t* states, int32_t H, int32_t S,
+                               int32_t T, void* stream) {
+  if (H < 0 || S < 0 || T < 0) return fail(SAF_ERR_INVALID, "negative dimension");
+  if (T > S) return fail(SAF_ERR_INVALID, "pattern normalisers: T > S");
+  if (H == 0 || S == 0) return SAF_OK;
+  if (!alpha || !rho || !z || !states) return fail(SAF_ERR_INVALID, "null pointer");
+  return launch_logz(alpha, rho, z, states, H, S, T, (cudaStream_t)stream);
 }
 
 int saf_pattern_param_grad(const SafPatternGradArgs* a, void* stream) {

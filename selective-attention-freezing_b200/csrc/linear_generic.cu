@@ -282,18 +282,19 @@ int gemm_generic_typed(const SafIndexedLinearArgs& a, int mode, const void* dout
 
 // z[h,i] = logsumexp_{j<=i}(alpha[h,j] + rho[h,i-j]); one warp per row
 __global__ void logz_kernel(const float* __restrict__ alpha, const float* __restrict__ rho, float* __restrict__ z,
-                            int H, int S, int rows) {
+                            const int32_t* __restrict__ states, int H, int S, int rows) {
   const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
   if (warp >= H * S) return;
   const int h = warp / S, i = warp - h * S;
-  if (i >= rows) {
+  if (i >= rows || (states && states[h] != SAF_DECOMP)) {
     if (lane == 0) z[(int64_t)h * S + i] = 0.f;
     return;
   }
   const float* al = alpha + (int64_t)h * S;
   const float* rh = rho + (int64_t)h * S;
   // the row's maximum first, then the sum against it: short chains instead of one that rescales as it goes
-  // (12 heads, 2048 rows: 55 -> 42 us, now bound by the instructions of 25 M expf).
+  // (12 heads, 2048 rows: 55 -> 42 us, now bound by the instructions of 25 M expf; of a layer with 3 decomposed heads only
+  // theirs are computed)
   // Entries that are -inf or NaN take no part.
   float mx[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
   int j = lane;
@@ -359,10 +360,10 @@ int launch_rope_slabs(void* x, int64_t ld, int M, int n_slabs, int slab, int T, 
   count_launch();
   return check_launch("rope_slabs_kernel");
 }
-int launch_logz(const float* alpha, const float* rho, float* z, int H, int S, int rows, cudaStream_t st) {
+int launch_logz(const float* alpha, const float* rho, float* z, const int32_t* states, int H, int S, int rows, cudaStream_t st) {
   const int64_t warps = (int64_t)H * S;
   const int64_t blocks = (warps * 32 + 255) / 256;
-  logz_kernel<<<(unsigned)blocks, 256, 0, st>>>(alpha, rho, z, H, S, rows);
+  logz_kernel<<<(unsigned)blocks, 256, 0, st>>>(alpha, rho, z, states, H, S, rows);
   count_launch();
   return check_launch("logz_kernel");
 }

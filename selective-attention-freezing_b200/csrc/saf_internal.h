@@ -153,7 +153,8 @@ struct CastSegment {
 constexpr int MAX_CAST_SEGMENTS = 6;
 int launch_cast_bf16(const CastSegment* seg, int n, cudaStream_t st);   // fp32 -> bf16, all segments in one launch
 int validate_linear_args(const SafIndexedLinearArgs* a);
-int launch_logz(const float* alpha, const float* rho, float* z, int H, int S, int rows, cudaStream_t st);   // rows >= `rows` get 0
+// rows >= `rows` get 0, and with `states` all rows of heads that are not decomposed
+int launch_logz(const float* alpha, const float* rho, float* z, const int32_t* states, int H, int S, int rows, cudaStream_t st);
 int launch_pattern_grad(const SafPatternGradArgs& a, cudaStream_t st);
 int launch_attn_stats_sm100(const SafAttnStatsArgs& a, cudaStream_t st);
 

@@ -131,7 +131,7 @@ EXPORTS = (
     "saf_mixed_attn_fwd", "saf_mixed_attn_bwd", "saf_mixed_attn_bwd_static", "saf_frozen_pv_fwd", "saf_frozen_pv_bwd",
     "saf_indexed_linear_fwd", "saf_indexed_linear_bwd_dx", "saf_indexed_linear_bwd_dw",
     "saf_decomposed_logz", "saf_rope_slabs", "saf_layernorm_fwd", "saf_rmsnorm_fwd",
-    "saf_pattern_normalisers", "saf_pattern_param_grad", "saf_attention_moments",
+    "saf_pattern_normalisers", "saf_pattern_normalisers_of", "saf_pattern_param_grad", "saf_attention_moments",
     "saf_attn_layer_workspace", "saf_attn_layer_fwd", "saf_attn_layer_bwd",
     "saf_block_workspace", "saf_block_fwd",
     "saf_selftest_wait_timeout", "saf_selftest_per_device_once", "saf_selftest_mma_rate",
@@ -180,6 +180,9 @@ def _load():
     lib.saf_pattern_normalisers.argtypes = [C.c_void_p, C.c_void_p, C.c_void_p, C.c_int32, C.c_int32, C.c_int32,
                                             C.c_void_p]
     lib.saf_pattern_normalisers.restype = C.c_int
+    lib.saf_pattern_normalisers_of.argtypes = [C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p, C.c_int32, C.c_int32, C.c_int32,
+                                               C.c_void_p]
+    lib.saf_pattern_normalisers_of.restype = C.c_int
     lib.saf_rope_slabs.argtypes = [C.c_void_p, C.c_int64, C.c_int32, C.c_int32, C.c_int32, C.c_int32,
                                    C.POINTER(C.c_int32), C.c_void_p, C.c_void_p, C.c_int32, C.c_int32, C.c_void_p]
     lib.saf_rope_slabs.restype = C.c_int

@@ -394,7 +394,7 @@ class SafCausalSelfAttention(nn.Module):
             if grad and (dec[0].requires_grad or dec[1].requires_grad):
                 from . import trainable_patterns as tp
                 call["learn"] = dec[:2]
-                dec = (dec[0].detach(), dec[1].detach(), tp.current_normalisers(dec[0], dec[1], T))
+                dec = (dec[0].detach(), dec[1].detach(), tp.current_normalisers(dec[0], dec[1], T, self._fz_mask_i32))
             call["decomposed"] = dec
         if bias:
             call["biases"] = [m.bias.to(act_dt) for m in (self.q_proj, self.k_proj, self.v_proj, self.c_proj)]

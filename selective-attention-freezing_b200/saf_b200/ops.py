@@ -443,7 +443,7 @@ def fused_mixed_attn(q, k, v, patt, frozen, hidx=None, pidx=None,
             raise NotImplementedError("trainable patterns with kvidx (GQA) are not implemented")
         from . import trainable_patterns as _tp
         alpha_p, rho_p = alpha, rho
-        z = _tp.current_normalisers(alpha, rho, v.shape[-2])
+        z = _tp.current_normalisers(alpha, rho, v.shape[-2], frozen)
         alpha, rho = alpha.detach(), rho.detach()
     if alpha is not None and z is None:
         z = decomposed_logz(alpha, rho)

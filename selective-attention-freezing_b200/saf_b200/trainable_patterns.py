@@ -20,15 +20,19 @@ from . import ops
 
 
 @torch.no_grad()
-def normalisers(alpha, rho, length):
+def normalisers(alpha, rho, length, states=None):
     """z[h,i] = logsumexp_{j<=i}(alpha[h,j] + rho[h,i-j]) for i < length, 0 beyond
-    (supplement/trainable_pattern_kernels.py:62-66).  alpha, rho (H, S); returns (H, S) like alpha."""
+    (supplement/trainable_pattern_kernels.py:62-66).  alpha, rho (H, S); returns (H, S) like alpha.  states: (H,) int32
+    head states; heads that are not decomposed, whose z nothing reads, then get zeros."""
     ops._require_cuda(alpha, "alpha")
     H, S = alpha.shape
     a = alpha.detach().float().contiguous()
     r = rho.detach().float().contiguous()
     z = torch.empty_like(a)
-    ops._call(a, lib.saf_pattern_normalisers, a.data_ptr(), r.data_ptr(), z.data_ptr(), H, S, int(length))
+    if states is None:
+        ops._call(a, lib.saf_pattern_normalisers, a.data_ptr(), r.data_ptr(), z.data_ptr(), H, S, int(length))
+    else:
+        ops._call(a, lib.saf_pattern_normalisers_of, a.data_ptr(), r.data_ptr(), z.data_ptr(), states.data_ptr(), H, S, int(length))
     return z.to(alpha.dtype)
 
 
@@ -96,17 +100,17 @@ def clear_pattern_cache():
     _Z_CACHE.clear()
 
 
-def current_normalisers(alpha, rho, length):
-    """`normalisers`, cached per (alpha, rho) version like the reference's dispatch cache
+def current_normalisers(alpha, rho, length, states=None):
+    """`normalisers`, cached per (alpha, rho, states) version like the reference's dispatch cache
     (supplement/trainable_patterns.py:66-80).  Optimizers that update parameters without touching the
     version counter must call `clear_pattern_cache()` after each step (`attach_optimizer` does)."""
     key = id(alpha)
-    sig = (ops._ver(alpha), ops._ver(rho), int(length), alpha.device)
+    sig = (ops._ver(alpha), ops._ver(rho), int(length), alpha.device, None if states is None else ops._ver(states))
     hit = _Z_CACHE.get(key)
-    if hit is not None and hit[0] is alpha and hit[1] == sig:
+    if hit is not None and hit[0] is alpha and hit[1] == sig and hit[3] is states:
         return hit[2]
-    z = normalisers(alpha, rho, length)
-    _Z_CACHE[key] = (alpha, sig, z)
+    z = normalisers(alpha, rho, length, states)
+    _Z_CACHE[key] = (alpha, sig, z, states)
     return z
 
 
