@@ -314,6 +314,8 @@ int saf_pattern_param_grad(const SafPatternGradArgs* args, void* stream);
  * saf_mixed_attn_fwd writes it.  bf16 q, k with head_dim 64 / 128 (tensor-core kernel);
  * anything else returns SAF_ERR_UNSUPPORTED.
  *
+ * quantity == SAF_STATS_LSE only fills lse (then an output) from q and k; mean and the rest are not used.
+ *
  * quantity == SAF_STATS_LOGITS measures the raw scores instead, lg = q k^T * sm_scale
  * over the whole square (nothing masked), as the priors that sample logits want them
  * (`_last_logits`, nanogpt/model.py:828-831; dynamic_freeze.py:721-737):
@@ -326,6 +328,7 @@ int saf_pattern_param_grad(const SafPatternGradArgs* args, void* stream);
  * ------------------------------------------------------------------------- */
 #define SAF_STATS_PROBS 0
 #define SAF_STATS_LOGITS 1
+#define SAF_STATS_LSE 2
 typedef struct SafAttnStatsArgs {
   int32_t struct_size; /* sizeof(SafAttnStatsArgs), checked */
   int32_t dtype;       /* SafDType of q, k */
@@ -338,7 +341,7 @@ typedef struct SafAttnStatsArgs {
   double* head_m2;
   double* neg_entropy;
   int32_t* status;     /* optional device int32, as in SafMixedAttnArgs */
-  int32_t quantity;    /* SAF_STATS_PROBS or SAF_STATS_LOGITS */
+  int32_t quantity;    /* SAF_STATS_PROBS, SAF_STATS_LOGITS or SAF_STATS_LSE */
   float* cell_m2;      /* SAF_STATS_LOGITS: optional (U, T, T) fp32 centred squares per cell, 16-byte aligned */
 } SafAttnStatsArgs;
 

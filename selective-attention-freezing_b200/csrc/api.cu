@@ -507,9 +507,9 @@ int saf_attention_moments(const SafAttnStatsArgs* a, void* stream) {
   memset(&x, 0, sizeof(x));
   memcpy(&x, a, (size_t)a->struct_size);
   if (x.B < 0 || x.U < 0 || x.T < 0 || x.HD <= 0 || x.count_prev < 0) return fail(SAF_ERR_INVALID, "bad dimension");
-  if (x.quantity != SAF_STATS_PROBS && x.quantity != SAF_STATS_LOGITS) return fail(SAF_ERR_INVALID, "unknown quantity %d", x.quantity);
+  if (x.quantity != SAF_STATS_PROBS && x.quantity != SAF_STATS_LOGITS && x.quantity != SAF_STATS_LSE) return fail(SAF_ERR_INVALID, "unknown quantity %d", x.quantity);
   if (x.B == 0 || x.U == 0 || x.T == 0) return SAF_OK;
-  if (!x.q.ptr || !x.k.ptr || !x.mean) return fail(SAF_ERR_INVALID, "null pointer");
+  if (!x.q.ptr || !x.k.ptr || (x.quantity == SAF_STATS_LSE ? !x.lse.ptr : !x.mean)) return fail(SAF_ERR_INVALID, "null pointer");
   if (x.quantity == SAF_STATS_PROBS && (!x.lse.ptr || !x.head_m2 || !x.neg_entropy)) return fail(SAF_ERR_INVALID, "null pointer");
   if (x.quantity == SAF_STATS_PROBS && x.cell_m2) return fail(SAF_ERR_INVALID, "cell_m2 goes with SAF_STATS_LOGITS");
   return launch_attn_stats_sm100(x, (cudaStream_t)stream);

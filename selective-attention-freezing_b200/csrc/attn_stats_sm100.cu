@@ -526,6 +526,10 @@ int launch_attn_stats_sm100(const SafAttnStatsArgs& a, cudaStream_t st) {
   if (a.dtype != SAF_BF16 || (a.HD != 64 && a.HD != 128)) return fail(SAF_ERR_UNSUPPORTED, "attention statistics: bf16 with head_dim 64 or 128 only");
   if (!tma_rows_ok(a.q) || !tma_rows_ok(a.k))
     return fail(SAF_ERR_UNSUPPORTED, "attention statistics: q, k need 16-byte aligned rows and unit last stride");
+  if (a.quantity == SAF_STATS_LSE) {
+    if (!saf_device_supported()) return fail(SAF_ERR_UNSUPPORTED, "attention statistics need an sm_100 device");
+    return launch_row_lse_sm100(a, st);
+  }
   if ((uintptr_t)a.mean & 15) return fail(SAF_ERR_INVALID, "attention statistics: mean must be 16-byte aligned");
   if (!saf_device_supported()) return fail(SAF_ERR_UNSUPPORTED, "attention statistics need an sm_100 device");
   if ((uintptr_t)a.cell_m2 & 15) return fail(SAF_ERR_INVALID, "attention statistics: cell_m2 must be 16-byte aligned");

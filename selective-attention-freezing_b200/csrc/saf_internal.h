@@ -157,6 +157,7 @@ int validate_linear_args(const SafIndexedLinearArgs* a);
 int launch_logz(const float* alpha, const float* rho, float* z, const int32_t* states, int H, int S, int rows, cudaStream_t st);
 int launch_pattern_grad(const SafPatternGradArgs& a, cudaStream_t st);
 int launch_attn_stats_sm100(const SafAttnStatsArgs& a, cudaStream_t st);
+int launch_row_lse_sm100(const SafAttnStatsArgs& a, cudaStream_t st);
 
 // TMA descriptor encode through the driver entry point (no link-time libcuda dependency)
 typedef CUresult (*TensorMapEncodeFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,

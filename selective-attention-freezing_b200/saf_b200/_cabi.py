@@ -123,7 +123,7 @@ class SafBlockArgs(C.Structure):
     ]
 
 
-STATS_PROBS, STATS_LOGITS = 0, 1
+STATS_PROBS, STATS_LOGITS, STATS_LSE = 0, 1, 2
 ACT_NONE, ACT_GELU, ACT_SWIGLU = 0, 1, 2
 
 EXPORTS = (

@@ -18,19 +18,22 @@ import math
 import torch
 
 from . import ops
-from ._cabi import STATS_LOGITS, SafAttnStatsArgs, SafMixedAttnArgs, lib
+from ._cabi import STATS_LOGITS, STATS_LSE, SafAttnStatsArgs, lib
 
 
 def _row_lse(q, k, sm_scale):
-    """(B, U, T) fp32 log2-domain log-sum-exp of the causal scores, from the mixed-attention forward run with every
-    head live (k stands in for v; the output is scratch)."""
+    """(B, U, T) fp32 log2-domain log-sum-exp of the causal scores."""
     B, U, T, HD = q.shape
-    out = torch.empty((B, U, T, HD), device=q.device, dtype=q.dtype)
     lse = torch.empty((B, U, T), device=q.device, dtype=torch.float32)
-    live = torch.zeros(U, dtype=torch.int32, device=q.device)
-    a, keep = SafMixedAttnArgs(), []
-    ops._fill_mixed(a, q, k, k, out, lse, None, None, None, None, live, None, None, None, sm_scale, None, None, keep)
-    ops._call(q, lib.saf_mixed_attn_fwd, C.byref(a))
+    a = SafAttnStatsArgs()
+    a.struct_size = C.sizeof(SafAttnStatsArgs)
+    a.dtype = ops._dt(q)
+    a.B, a.U, a.T, a.HD = B, U, T, HD
+    a.sm_scale = float(sm_scale)
+    a.q, a.k, a.lse = ops._st(q), ops._st(k), ops._st(lse)
+    a.status = ops._status_ptr(q.device)
+    a.quantity = STATS_LSE
+    ops._call(q, lib.saf_attention_moments, C.byref(a))
     return lse
 
 
