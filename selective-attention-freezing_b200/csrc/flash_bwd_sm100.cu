@@ -30,11 +30,13 @@
 #include "sm100_prims.cuh"
 #include <string.h>
 
+#include <algorithm>
+
 namespace saf {
 namespace {
 
 constexpr int BWD_THREADS = 384;
-constexpr int BWD_HEAD_GROUP = 8;
+constexpr int BWD_MAX_LIST = 256;
 constexpr float LOG2E_B = 1.4426950408889634f;
 
 #ifdef SAF_BWD_TRACE
@@ -66,6 +68,10 @@ struct BwdCfg {
 
 struct BwdParams {
   int B, H, T, n_tiles, force_state;
+  int head_group;                       // (batch, head) pairs whose tiles are dealt out together, the longest walks first
+  // heads with walks: the live ones where the host knows them, else all H, each CTA looking its head's state up
+  int n_heads, listed;
+  uint8_t heads[BWD_MAX_LIST];
   float scale_log2, sm_scale;
   const int32_t* frozen;
   const int32_t* hidx;
@@ -222,17 +228,16 @@ __device__ __forceinline__ void stage_cols(uint8_t* stage, const uint32_t (&o)[3
 // CTA -> (batch, head, tile), heads in groups so CTAs in flight share their streamed tiles in L2,
 // heaviest tiles first inside a group.  Returns false when the CTA has nothing to do.
 __device__ __forceinline__ bool bwd_cta_coords(const BwdParams& p, int cta, bool heavy_is_low, int& b, int& h, int& tile) {
-  const int bh_count = p.B * p.H;
-  const int per_group = BWD_HEAD_GROUP * p.n_tiles;
+  const int per_group = p.head_group * p.n_tiles;
   const int grp = cta / per_group;
-  const int gsize = min(BWD_HEAD_GROUP, bh_count - grp * BWD_HEAD_GROUP);
+  const int gsize = min(p.head_group, p.B * p.n_heads - grp * p.head_group);      // (only the last group is smaller)
   const int rem = cta - grp * per_group;
-  if (rem >= gsize * p.n_tiles) return false;
   const int t = rem / gsize;
   tile = heavy_is_low ? t : p.n_tiles - 1 - t;
-  const int bh = grp * BWD_HEAD_GROUP + rem % gsize;
-  b = bh / p.H;
-  h = bh % p.H;
+  const int bh = grp * p.head_group + rem % gsize;
+  b = bh / p.n_heads;
+  h = bh % p.n_heads;
+  if (p.listed) h = p.heads[h];
   const int state = p.force_state >= 0 ? p.force_state : p.frozen[h];
   return state == SAF_LIVE;
 }
@@ -967,9 +972,25 @@ int bwd_launch_typed(const SafMixedAttnBwdArgs& g, bool live, bool* dense_done, 
   static PerDeviceOnce smem_once_dkdv, smem_once_dq;
   if ((rc = ensure_dyn_smem(flash_bwd_dkdv_kernel<HD>, BwdCfg<HD>::SMEM_BYTES, smem_once_dkdv))) return rc;
   if ((rc = ensure_dyn_smem(flash_bwd_dq_kernel<HD>, BwdCfg<HD>::SMEM_BYTES_DQ, smem_once_dq))) return rc;
-  const int bh = a.B * a.H;
-  const int groups = (bh + BWD_HEAD_GROUP - 1) / BWD_HEAD_GROUP;
-  const unsigned grid = live ? (unsigned)(groups * BWD_HEAD_GROUP * p.n_tiles) : 0u;
+  p.n_heads = a.H;
+  if (a.frozen_host && a.force_state < 0 && a.H <= BWD_MAX_LIST) {
+    p.listed = 1;
+    p.n_heads = 0;
+    for (int hh = 0; hh < a.H; ++hh)
+      if (a.frozen_host[hh] == SAF_LIVE) p.heads[p.n_heads++] = (uint8_t)hh;
+  }
+  // All heads in one group as far as Q, K, V and dO of a group fit half of the L2, else even groups: a launch ends with the
+  // shortest walks of its last group, so a small last group, whose longest walks start late, leaves SMs idle.  (Groups of 8
+  // before.  dK / dV and dQ of 12 live heads, T = 3001,
+  // B = 1: width 64 71 + 46 -> 53 + 35 us, 96 92 + 56 -> 66 + 44, 128 91 + 58 -> 73 + 45; 9 live heads x 64, T = 1024, B = 8:
+  // 66 + 41 -> 62 + 36.)
+  const int bh = a.B * p.n_heads;
+  const int64_t total_bytes = (int64_t)bh * a.T * a.HD * 8;
+  const int groups = (int)std::min<int64_t>(bh, std::max<int64_t>(1, (total_bytes + (64 << 20) - 1) / (64 << 20)));
+  p.head_group = bh > 0 ? (bh + groups - 1) / groups : 1;
+  const int64_t ctas = live ? (int64_t)bh * p.n_tiles : 0;
+  if (ctas > 0x3fffffff) return fail(SAF_ERR_LIMIT, "backward: too many tiles");
+  const unsigned grid = (unsigned)ctas;
   if (grid + p.scan_slots + p.dense_slots == 0) return SAF_ERR_UNSUPPORTED;
   if ((rc = launch_pdl("flash_bwd_dkdv_kernel", flash_bwd_dkdv_kernel<HD>, dim3(grid + p.scan_slots + p.dense_slots), BWD_THREADS,
                        BwdCfg<HD>::SMEM_BYTES, st, 1, mq, mk, mv, mdo, mdk, mdv, mp64, mdo64, p)))
