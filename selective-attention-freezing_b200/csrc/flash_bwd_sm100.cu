@@ -59,7 +59,9 @@ struct BwdCfg {
   static constexpr int ND = (HD == 64) ? 3 : 2;
   static constexpr int KS = 3;                        // dQ kernel: K ring (a K tile lives until its dQ product)
   static constexpr int VS = (HD == 64) ? 3 : 2;       // dQ kernel: V ring (a V tile is done after its dP product)
-  static constexpr int SMEM_DKDV = 1024 + 2 * TILE_BYTES + (NQ + ND) * TILE_BYTES + 256 + 1040;
+  // lse and delta of the current query tile: two buffers where shared memory has room, one barrier a tile then does
+  static constexpr int VEC_BUFS = (HD == 64) ? 2 : 1;
+  static constexpr int SMEM_DKDV = 1024 + 2 * TILE_BYTES + (NQ + ND) * TILE_BYTES + 256 + VEC_BUFS * 1024;
   // the dK/dV launch also hosts the dense-pattern dV role, which brings its own ring
   static constexpr int SMEM_BYTES = SMEM_DKDV > DpCfg<HD>::SMEM_BYTES ? SMEM_DKDV : DpCfg<HD>::SMEM_BYTES;
   static constexpr int SMEM_BYTES_DQ = 1024 + 2 * TILE_BYTES + (KS + VS) * TILE_BYTES + 512;
@@ -108,7 +110,7 @@ __device__ __forceinline__ float ex2b(float x) {
   return y;
 }
 #ifndef SAF_BWD_POLY_PER_8
-#define SAF_BWD_POLY_PER_8 4        // of every 8 exponentials, this many run on the FMA pipe
+#define SAF_BWD_POLY_PER_8 2        // of every 8 exponentials, this many run on the FMA pipe (4: 1 to 2 % slower, 0: dQ 5 %)
 #endif
 // 2^x on the FMA/ALU pipes for x <= 0 (clamped at -126): round to nearest integer with the magic-number
 // add, cubic minimax on the fraction, exponent added as an integer shift.  Relative error ~1e-4.
@@ -164,6 +166,13 @@ __device__ __forceinline__ void operand_columns_wait(int half, int id) {
     named_bar_sync(id, 256);
     tc_fence_after();
   }
+}
+// this warp's part of the operand is in tensor memory: one arrival
+__device__ __forceinline__ void operand_written(uint64_t* bar, int tid) {
+  tmem_st_wait();
+  tc_fence_before();
+  __syncwarp();
+  if ((tid & 31) == 0) mbar_arrive(bar);
 }
 // two fp32 -> packed bf16x2
 __device__ __forceinline__ uint32_t bpack(float lo, float hi) {
@@ -255,8 +264,8 @@ __device__ __forceinline__ void bwd_setup(BwdBars* bars, int tid, int warp) {
     mbar_init(&bars->s_full[0], 1);
     mbar_init(&bars->s_full[1], 1);
     mbar_init(&bars->dp_full, 1);
-    mbar_init(&bars->p_full, 256);
-    mbar_init(&bars->ds_full, 256);
+    mbar_init(&bars->p_full, 8);              // one arrival per compute warp
+    mbar_init(&bars->ds_full, 8);
     mbar_init(&bars->acc_full, 1);
     fence_mbar_init();
   }
@@ -321,11 +330,14 @@ flash_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_con
   uint8_t* ring = smem + 2 * C::TILE_BYTES;           // stage s: [Q_i | dO_i]
   uint8_t* ringdO = ring + C::NQ * C::TILE_BYTES;       // `ring` is the Q ring
   BwdBars* bars = reinterpret_cast<BwdBars*>(ringdO + C::ND * C::TILE_BYTES);
-  BwdVectors* vec = reinterpret_cast<BwdVectors*>(reinterpret_cast<uint8_t*>(bars) + 256);
+  BwdVectors* vecs = reinterpret_cast<BwdVectors*>(reinterpret_cast<uint8_t*>(bars) + 256);
   const int tid = threadIdx.x, warp = tid >> 5;
   bwd_setup<HD>(bars, tid, warp);
   const uint32_t tmem = bars->tmem_base;
-  constexpr uint32_t COL_S = 0, COL_DP = 128, COL_DV = 256, COL_DK = 256 + HD;
+  // At head_dim 64 tensor memory has room for a second buffer of scores: S^T of the next query tile is there before P^T and
+  // dS^T of this one are done
+  constexpr uint32_t COL_S = 0, COL_DP = 128, COL_DV = 256, COL_DK = 256 + HD, COL_S2 = 384;
+  constexpr bool TWO_S = HD == 64;
 #ifdef SAF_BWD_TRACE
   const bool trace_on = (b == 0 && h == 0 && jt == 0) && (tid == 0 || tid == 9 * 32);
   const bool wtrace_on = (b == 0 && h == 0 && jt == 0) && (tid & 31) == 0 && tid < 256;
@@ -370,23 +382,39 @@ flash_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_con
       const uint32_t aK = smem_u32(sK), aV = smem_u32(sV), aR = smem_u32(ring), aRd = smem_u32(ringdO);
       bool ok = mbar_wait(&bars->res_full, 0);
       if (!ok) dev_set_error(p.status, SAF_DEV_TIMEOUT_MMA, 41);
+      // S^T of query tile i (in its buffer), dP^T of query tile i
+      auto issue_scores = [&](int i) -> bool {
+        const int s = i % C::NQ;
+        if (!mbar_wait(&bars->ring_full[s], (i / C::NQ) & 1)) {
+          dev_set_error(p.status, SAF_DEV_TIMEOUT_MMA, 44);
+          return false;
+        }
+        tc_fence_after();
+        if (leader) {
+          issue_ss<HD>(tmem + (TWO_S && (i & 1) ? COL_S2 : COL_S), aK, aR + s * C::TILE_BYTES, idesc_s);
+          umma_commit(&bars->s_full[TWO_S ? i & 1 : 0]);
+        }
+        __syncwarp();
+        return true;
+      };
+      auto issue_dp = [&](int i) -> bool {
+        const int sd = i % C::ND;
+        if (!mbar_wait(&bars->v_full[sd], (i / C::ND) & 1)) {
+          dev_set_error(p.status, SAF_DEV_TIMEOUT_MMA, 59);
+          return false;
+        }
+        tc_fence_after();
+        if (leader) {
+          issue_ss<HD>(tmem + COL_DP, aV, aRd + sd * C::TILE_BYTES, idesc_s);
+          umma_commit(&bars->dp_full);
+        }
+        __syncwarp();
+        return true;
+      };
+      if (ok) ok = issue_scores(0) && issue_dp(0);
+      if (TWO_S && ok && n > 1) ok = issue_scores(1);
       for (int i = 0; i < n && ok; ++i) {
         const int s = i % C::NQ, sd = i % C::ND;
-        const uint32_t aQ = aR + s * C::TILE_BYTES, adO = aRd + sd * C::TILE_BYTES;
-        if (i == 0) {
-          if (!mbar_wait(&bars->ring_full[0], 0) || !mbar_wait(&bars->v_full[0], 0)) {
-            dev_set_error(p.status, SAF_DEV_TIMEOUT_MMA, 42);
-            break;
-          }
-          tc_fence_after();
-          if (leader) {
-            issue_ss<HD>(tmem + COL_S, aK, aQ, idesc_s);
-            umma_commit(&bars->s_full[0]);
-            issue_ss<HD>(tmem + COL_DP, aV, adO, idesc_s);
-            umma_commit(&bars->dp_full);
-          }
-          __syncwarp();
-        }
         if (!mbar_wait(&bars->p_full, i & 1)) {
           dev_set_error(p.status, SAF_DEV_TIMEOUT_MMA, 43);
           break;
@@ -394,26 +422,14 @@ flash_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_con
         tc_fence_after();
         TRACE(0, 4, i);   // issuer saw p_full
         if (leader) {
-          issue_ts<HD>(tmem + COL_DV, tmem + COL_S, adO, idesc_o, i > 0);
+          issue_ts<HD>(tmem + COL_DV, tmem + (TWO_S && (i & 1) ? COL_S2 : COL_S), aRd + sd * C::TILE_BYTES, idesc_o, i > 0);
           umma_commit(&bars->v_empty[sd]);                // dO_i is not read again
         }
         __syncwarp();
         TRACE(0, 6, i);   // dV issued
-        const int s2 = (i + 1) % C::NQ, sd2 = (i + 1) % C::ND;
-        const uint32_t aQ2 = aR + s2 * C::TILE_BYTES, adO2 = aRd + sd2 * C::TILE_BYTES;
-        if (i + 1 < n) {
-          if (!mbar_wait(&bars->ring_full[s2], ((i + 1) / C::NQ) & 1)) {
-            dev_set_error(p.status, SAF_DEV_TIMEOUT_MMA, 44);
-            break;
-          }
-          tc_fence_after();
-          if (leader) {
-            issue_ss<HD>(tmem + COL_S, aK, aQ2, idesc_s);   // ordered behind the dV product that read P^T
-            umma_commit(&bars->s_full[0]);
-          }
-          __syncwarp();
-          TRACE(0, 7, i);   // next S^T issued
-        }
+        const int next = i + (TWO_S ? 2 : 1);
+        if (next < n && !(ok = issue_scores(next))) break;  // ordered behind the dV product that read P^T
+        TRACE(0, 7, i);   // next S^T issued
         if (!mbar_wait(&bars->ds_full, i & 1)) {
           dev_set_error(p.status, SAF_DEV_TIMEOUT_MMA, 45);
           break;
@@ -421,22 +437,11 @@ flash_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_con
         tc_fence_after();
         TRACE(0, 5, i);   // issuer saw ds_full
         if (leader) {
-          issue_ts<HD>(tmem + COL_DK, tmem + COL_DP, aQ, idesc_o, i > 0);
+          issue_ts<HD>(tmem + COL_DK, tmem + COL_DP, aR + s * C::TILE_BYTES, idesc_o, i > 0);
           umma_commit(&bars->ring_empty[s]);              // Q_i is not read again
         }
         __syncwarp();
-        if (i + 1 < n) {
-          if (!mbar_wait(&bars->v_full[sd2], ((i + 1) / C::ND) & 1)) {
-            dev_set_error(p.status, SAF_DEV_TIMEOUT_MMA, 59);
-            break;
-          }
-          tc_fence_after();
-          if (leader) {
-            issue_ss<HD>(tmem + COL_DP, aV, adO2, idesc_s);  // ordered behind the dK product that read dS^T
-            umma_commit(&bars->dp_full);
-          }
-          __syncwarp();
-        }
+        if (i + 1 < n) ok = issue_dp(i + 1);              // ordered behind the dK product that read dS^T
       }
       if (leader) umma_commit(&bars->acc_full);
       __syncwarp();
@@ -448,7 +453,7 @@ flash_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_con
     const int r = tid & 127;                       // key row of the tile
     const int cb = half * 64;                      // first query column of this group
     const uint32_t lane_base = (uint32_t)((warp & 3) * 32) << 16;
-    const uint32_t tS = tmem + lane_base + COL_S, tdP = tmem + lane_base + COL_DP;
+    const uint32_t tdP = tmem + lane_base + COL_DP;
     const float sc = p.scale_log2;
     const float* lse_g = p.lse + (int64_t)b * p.lse_s[0] + (int64_t)h * p.lse_s[1];
     const float* dl_g = p.delta + (int64_t)b * p.delta_s[0] + (int64_t)h * p.delta_s[1];
@@ -459,25 +464,27 @@ flash_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_con
     };
     float nxt = fetch(jt);
     // A warp whose wait ran out (decided for the whole warp) stops working but keeps taking part, one-way, in the
-    // named barriers of every remaining tile -- two arrivals on barrier 1, one each on 2 and 3 per tile, as a working
+    // named barriers of every remaining tile -- those on barrier 1 (one or two) and one each on 2 and 3, as a working
     // warp gives -- so the other warps never block on it; they run into their own limits because P^T / dS^T stay
     // incomplete, and all meet again at the epilogue's barrier.
     bool ok = true;
     for (int i = 0; i < n; ++i) {
       if (!ok) {
-        named_bar_arrive(1, 256);
+        if constexpr (C::VEC_BUFS == 1) named_bar_arrive(1, 256);
         named_bar_arrive(1, 256);
         named_bar_arrive(2, 256);
         named_bar_arrive(3, 256);
         continue;
       }
-      named_bar_sync(1, 256);                 // the previous tile's readers are done with the vectors
+      BwdVectors* vec = vecs + (C::VEC_BUFS == 2 ? i & 1 : 0);
+      if constexpr (C::VEC_BUFS == 1) named_bar_sync(1, 256);   // the previous tile's readers are done with the vectors
       if (tid < 128) vec->lse[r] = nxt;
       else vec->dl[r] = nxt;
       named_bar_sync(1, 256);
       if (i + 1 < n) nxt = fetch(jt + i + 1);
       // ---- P^T
-      if (!__all_sync(0xffffffffu, mbar_wait(&bars->s_full[0], i & 1))) {
+      const uint32_t tS = tmem + lane_base + (TWO_S && (i & 1) ? COL_S2 : COL_S);
+      if (!__all_sync(0xffffffffu, TWO_S ? mbar_wait(&bars->s_full[i & 1], (i >> 1) & 1) : mbar_wait(&bars->s_full[0], i & 1))) {
         dev_set_error(p.status, SAF_DEV_TIMEOUT_SOFTMAX, 46);
         ok = false;
         named_bar_arrive(2, 256);
@@ -519,9 +526,7 @@ flash_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_con
           tmem_st16(tS + half * 32 + ch * 16, pk);
         }
       }
-      tmem_st_wait();
-      tc_fence_before();
-      mbar_arrive(&bars->p_full);
+      operand_written(&bars->p_full, tid);
       TRACE(0, 1, i);   // P^T handed over
       WTRACE(0, i);
       // ---- dS^T
@@ -557,9 +562,7 @@ flash_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_con
           tmem_st16(tdP + half * 32 + ch * 16, pk);
         }
       }
-      tmem_st_wait();
-      tc_fence_before();
-      mbar_arrive(&bars->ds_full);
+      operand_written(&bars->ds_full, tid);
       TRACE(0, 3, i);   // dS^T handed over
       WTRACE(1, i);
     }
@@ -793,9 +796,7 @@ flash_bwd_dq_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_const
           tmem_st16(tdP + half * 32 + ch * 16, pk);
         }
       }
-      tmem_st_wait();
-      tc_fence_before();
-      mbar_arrive(&bars->ds_full);
+      operand_written(&bars->ds_full, tid);
       TRACE(1, 3, j);
     }
     if (ok && !mbar_wait(&bars->acc_full, 0)) {
