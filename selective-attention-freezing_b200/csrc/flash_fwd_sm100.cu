@@ -102,6 +102,7 @@ static_assert(ms_smem_bytes(SCAN_ROLE_STAGES) <= Cfg<64>::SMEM_BYTES && ms_smem_
               "the scan role must fit the launches' dynamic shared memory");
 
 struct FlashParams {
+  int head_group;            // persistent kernel: (batch, live head) pairs whose items the queue holds together
   int B, H, T, HKV, force_state, n_pairs;
   float scale_log2;
   const int32_t* frozen;
@@ -713,12 +714,12 @@ struct TileGeom {
 
 __device__ __forceinline__ TileGeom decode_item(const FlashParams& p, int li) {
   TileGeom g;
-  const int per_group = HEAD_GROUP * p.n_pairs;
+  const int per_group = p.head_group * p.n_pairs;
   const int grp = li / per_group;
-  const int gsize = min(HEAD_GROUP, p.B * p.U - grp * HEAD_GROUP);
+  const int gsize = min(p.head_group, p.B * p.U - grp * p.head_group);
   const int rem = li - grp * per_group;
   g.mp = p.n_pairs - 1 - rem / gsize;
-  const int bu = grp * HEAD_GROUP + rem % gsize;
+  const int bu = grp * p.head_group + rem % gsize;
   g.b = bu / p.U;
   g.h = p.live_head[bu % p.U];
   g.row0 = g.mp * 2 * FM;
@@ -1325,6 +1326,12 @@ int launch_typed(const SafMixedAttnArgs& a, uint32_t want, cudaStream_t st) {
     p.sched = a.sched;
     p.U = a.U;
     p.n_items = a.B * a.U * p.n_pairs;
+    // The queue hands out the row pairs of a group of (batch, head) pairs, the longest first, then the next group's: as many
+    // pairs in a group as K and V of half the L2 hold, evenly, because the launch ends with its last group's shortest
+    // items.  (Groups of 8 before, the last one with what was left over.)
+    const int64_t kv_bytes = (int64_t)a.B * (a.HKV > 0 ? a.HKV : a.U) * a.T * a.HD * 4;
+    const int groups = (int)std::min<int64_t>(a.B * a.U, std::max<int64_t>(1, (kv_bytes + (64 << 20) - 1) / (64 << 20)));
+    p.head_group = (a.B * a.U + groups - 1) / groups;
     p.lead = bh + p.dense_slots;
     static PerDeviceOnce smem_once_p;
     if ((rc = ensure_dyn_smem(flash_fwd_persistent_kernel<HD>, Cfg<HD>::SMEM_PERSIST, smem_once_p))) return rc;
