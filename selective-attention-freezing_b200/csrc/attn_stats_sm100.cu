@@ -371,11 +371,15 @@ attn_stats_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constan
         }
         tc_fence_after();
         if constexpr (!LOGITS) row_lse(gr + 1 < n_groups ? t : t + gridDim.x, gr + 1 < n_groups ? gr + 1 : 0, Ln);
-        float ent = 0.f;                              // sum p log2 p of this thread's cells
+        float2 ent2 = make_float2(0.f, 0.f);          // sum p log2 p of this thread's cells
         double corr = 0.0;
-        // compiled per number of samples: with a test of nb in front of every sample the cells' chains run one by one
-        auto cells = [&](auto nb_c) {
+        // Two cells at a time on packed pairs: the samples' mean, then the squares about it -- sums instead of a chain of
+        // updates.  Compiled per number of samples and for tiles the diagonal crosses.
+        auto cells = [&](auto nb_c, auto diag_c) {
           constexpr int NB = decltype(nb_c)::value;
+          constexpr bool DIAG = decltype(diag_c)::value;
+          const float2 f2 = make_float2(LOGITS ? p.scale : sc, LOGITS ? p.scale : sc), inv2 = make_float2(1.f / NB, 1.f / NB);
+          const float2 w2 = make_float2(w, w);
 #pragma unroll
           for (int c16 = 0; c16 < 2; ++c16) {
             uint32_t d[NB][16];
@@ -387,63 +391,78 @@ attn_stats_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constan
             for (int c4 = 0; c4 < 4; ++c4) {
               float4* mp = reinterpret_cast<float4*>(mrow + (((c16 * 4 + c4) ^ (r & 7)) << 4));
               float4* qp = reinterpret_cast<float4*>(reinterpret_cast<uint8_t*>(mp) + AS_STATE);
-              float mm[4], m2[4];
+              float2 mm[2], m2[2];
 #pragma unroll
-              for (int e = 0; e < 4; ++e) {
-                const int c = c4 * 4 + e;
-                mm[e] = m2[e] = 0.f;
+              for (int e = 0; e < 2; ++e) {
+                const int c = c4 * 4 + 2 * e;
+                float2 pe[NB], sum = make_float2(0.f, 0.f);
 #pragma unroll
                 for (int b = 0; b < NB; ++b) {
-                  float pe;
+                  const float2 v = make_float2(__uint_as_float(d[b][c]), __uint_as_float(d[b][c + 1]));
                   if constexpr (LOGITS) {
-                    pe = __uint_as_float(d[b][c]) * p.scale;                     // the raw score
+                    pe[b] = __fmul2_rn(v, f2);                                   // the raw scores
                   } else {
-                    float xl = fmaf(__uint_as_float(d[b][c]), sc, -L[b]);        // log2 of the probability
-                    if (diag && gj0 + c16 * 16 + c > gi) xl = -INFINITY;         // causal mask
-                    pe = as_ex2(xl);
-                    ent = fmaf(pe, fmaxf(xl, -200.f), ent);                      // p = 0 there, so the clamp only avoids 0 * inf
+                    float2 x2 = __ffma2_rn(v, f2, make_float2(-L[b], -L[b]));    // log2 of the probabilities
+                    if constexpr (DIAG) {                                        // causal mask
+                      if (gj0 + c16 * 16 + c > gi) x2.x = -INFINITY;
+                      if (gj0 + c16 * 16 + c + 1 > gi) x2.y = -INFINITY;
+                    }
+                    pe[b] = make_float2(as_ex2(x2.x), as_ex2(x2.y));
+                    // (p = 0 there, so the clamp only avoids 0 * inf)
+                    ent2 = __ffma2_rn(pe[b], make_float2(fmaxf(x2.x, -200.f), fmaxf(x2.y, -200.f)), ent2);
                   }
-                  // Welford update of the samples' mean and centred sum of squares
-                  const float dlt = pe - mm[e];
-                  mm[e] = fmaf(dlt, 1.f / (float)(b + 1), mm[e]);
-                  m2[e] = fmaf(dlt, pe - mm[e], m2[e]);
+                  sum = b == 0 ? pe[0] : __fadd2_rn(sum, pe[b]);
+                }
+                mm[e] = NB == 1 ? sum : __fmul2_rn(sum, inv2);
+                m2[e] = make_float2(0.f, 0.f);
+                if constexpr (NB > 1) {
+#pragma unroll
+                  for (int b = 0; b < NB; ++b) {
+                    const float2 dlt = __fadd2_rn(pe[b], make_float2(-mm[e].x, -mm[e].y));
+                    m2[e] = __ffma2_rn(dlt, dlt, m2[e]);
+                  }
                 }
               }
-              if constexpr (!LOGITS) m2sum += (double)(m2[0] + m2[1]) + (double)(m2[2] + m2[3]);
-              if (c0 > 0) {                               // Chan merge into the running cell
+              if constexpr (!LOGITS) m2sum += (double)(m2[0].x + m2[0].y) + (double)(m2[1].x + m2[1].y);
+              if (c0 > 0) {                               // Chan merge into the running cells
                 const float4 old = *mp;
-                const float ov[4] = {old.x, old.y, old.z, old.w};
-                float o2[4] = {0.f, 0.f, 0.f, 0.f}, cs = 0.f;
+                const float2 ov[2] = {make_float2(old.x, old.y), make_float2(old.z, old.w)};
+                float2 o2[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)}, cs = make_float2(0.f, 0.f);
                 if (has_m2) {
                   const float4 q = *qp;
-                  o2[0] = q.x; o2[1] = q.y; o2[2] = q.z; o2[3] = q.w;
+                  o2[0] = make_float2(q.x, q.y);
+                  o2[1] = make_float2(q.z, q.w);
                 }
 #pragma unroll
-                for (int e = 0; e < 4; ++e) {
-                  const float dlt = mm[e] - ov[e];
-                  mm[e] = fmaf(dlt, w, ov[e]);
-                  if constexpr (LOGITS) m2[e] += fmaf(dlt * dlt, cw, o2[e]);
-                  else cs = fmaf(dlt, dlt, cs);
+                for (int e = 0; e < 2; ++e) {
+                  const float2 dlt = __fadd2_rn(mm[e], make_float2(-ov[e].x, -ov[e].y));
+                  mm[e] = __ffma2_rn(dlt, w2, ov[e]);
+                  if constexpr (LOGITS) m2[e] = __fadd2_rn(m2[e], __ffma2_rn(__fmul2_rn(dlt, dlt), make_float2(cw, cw), o2[e]));
+                  else cs = __ffma2_rn(dlt, dlt, cs);
                 }
-                if constexpr (!LOGITS) corr += (double)cs;
+                if constexpr (!LOGITS) corr += (double)(cs.x + cs.y);
               }
-              *mp = make_float4(mm[0], mm[1], mm[2], mm[3]);
-              if (has_m2) *qp = make_float4(m2[0], m2[1], m2[2], m2[3]);
+              *mp = make_float4(mm[0].x, mm[0].y, mm[1].x, mm[1].y);
+              if (has_m2) *qp = make_float4(m2[0].x, m2[0].y, m2[1].x, m2[1].y);
             }
           }
         };
-        switch (nb) {
-          case 1: cells(std::integral_constant<int, 1>{}); break;
-          case 2: cells(std::integral_constant<int, 2>{}); break;
-          case 3: cells(std::integral_constant<int, 3>{}); break;
-          default: cells(std::integral_constant<int, AS_GROUP>{});
-        }
+        auto by_count = [&](auto diag_c) {
+          switch (nb) {
+            case 1: cells(std::integral_constant<int, 1>{}, diag_c); break;
+            case 2: cells(std::integral_constant<int, 2>{}, diag_c); break;
+            case 3: cells(std::integral_constant<int, 3>{}, diag_c); break;
+            default: cells(std::integral_constant<int, AS_GROUP>{}, diag_c);
+          }
+        };
+        if (!LOGITS && diag) by_count(std::integral_constant<bool, !LOGITS>{});
+        else by_count(std::false_type{});
         tc_fence_before();
         __syncwarp();
         if (lane == 0) mbar_arrive(&sh->s_empty[k]);
         if constexpr (!LOGITS) {
           m2sum += corr * cwd;
-          esum += (double)ent * (double)AS_LN2;        // natural log, as the reference's xlogy
+          esum += (double)(ent2.x + ent2.y) * (double)AS_LN2;        // natural log, as the reference's xlogy
         }
       }
       if (!ok) continue;
