@@ -52,6 +52,7 @@ struct BlockTable {
 struct BwdGemmParams {
   int I, J, KB;              // output rows, output columns, K steps of 64
   int tiles_m, tiles_n;
+  int subs;                  // 64-column blocks of a tile: 2, 3 or 4
   int n_blocks;              // selected 64-row blocks
   const void* bias;          // DX only: bf16 over the J output columns, or null
   int* status;
@@ -90,6 +91,7 @@ indexed_gemm_bwd_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_c
     kb1 = (int)((int64_t)p.KB * (sp + 1) / splits);
   };
   const CUtensorMap* wm[4] = {&mapW0, &mapW1, &mapW2, &mapW3};
+  const int bn = p.subs * 64;                                // columns of a tile
 
   if (tid == 0) {
     for (int s = 0; s < NSTG; ++s) {
@@ -121,7 +123,7 @@ indexed_gemm_bwd_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_c
       for (int tile = blockIdx.x; tile < total_tiles && ok; tile += gridDim.x) {
         int tm, tn, sp, kb0, kb1;
         unit(tile, tm, tn, sp, kb0, kb1);
-        const int nsub = min(4, (p.J - tn * BN + 63) / 64);                      // 64-column blocks of B
+        const int nsub = min(p.subs, (p.J - tn * bn + 63) / 64);                      // 64-column blocks of B
         const int nrow = (MODE == MODE_DW) ? min(2, p.n_blocks - tm * 2) : 2;    // 64-feature blocks of A
         for (int kb = kb0; kb < kb1; ++kb, ++it) {
           const int s = it % NSTG;
@@ -136,23 +138,23 @@ indexed_gemm_bwd_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_c
             mbar_expect_tx(&sl->full[s], BA_BYTES + nsub * ATOM);
             tma_load_2d(a, &mapA, &sl->full[s], kb * BK, tm * BM);               // dout[m tile, block kb]
             for (int u = 0; u < nsub; ++u) {
-              tma_load_2d(b + u * ATOM, wm[tb.weight[kb]], &sl->full[s], tn * BN + u * 64, tb.row0[kb]);
+              tma_load_2d(b + u * ATOM, wm[tb.weight[kb]], &sl->full[s], tn * bn + u * 64, tb.row0[kb]);
               if (p.halves)
-                tma_load_2d(b + u * ATOM + ATOM / 2, wm[tb.weightb[kb]], &sl->full[s], tn * BN + u * 64, tb.row0b[kb]);
+                tma_load_2d(b + u * ATOM + ATOM / 2, wm[tb.weightb[kb]], &sl->full[s], tn * bn + u * 64, tb.row0b[kb]);
             }
           } else {
             mbar_expect_tx(&sl->full[s], (nrow + nsub) * ATOM);
             for (int u = 0; u < nrow; ++u)
               tma_load_2d(a + u * ATOM, &mapA, &sl->full[s], (tm * 2 + u) * 64, kb * BK);   // dout[token block, features]
             for (int u = 0; u < nsub; ++u)
-              tma_load_2d(b + u * ATOM, &mapB, &sl->full[s], tn * BN + u * 64, kb * BK);    // x[token block, columns]
+              tma_load_2d(b + u * ATOM, &mapB, &sl->full[s], tn * bn + u * 64, kb * BK);    // x[token block, columns]
           }
         }
       }
     }
   } else if (warp == 1) {
     const bool leader = elect_one();
-    const uint32_t idesc = umma_idesc_bf16(BM, BN, MODE == MODE_DW ? 1 : 0, 1);
+    const uint32_t idesc = umma_idesc_bf16(BM, bn, MODE == MODE_DW ? 1 : 0, 1);
     const uint32_t sbase = smem_u32(stage_base);
     uint32_t it = 0, lt = 0;
     bool ok = true;
@@ -201,7 +203,7 @@ indexed_gemm_bwd_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_c
     for (int tile = blockIdx.x; tile < total_tiles; tile += gridDim.x, ++lt) {
       int tm, tn, sp, kb0, kb1;
       unit(tile, tm, tn, sp, kb0, kb1);
-      const int nsub = min(4, (p.J - tn * BN + 63) / 64);
+      const int nsub = min(p.subs, (p.J - tn * bn + 63) / 64);
       const int nrow = (MODE == MODE_DW) ? min(2, p.n_blocks - tm * 2) : 2;
       const int buf = lt & 1;
       // threads that meet at named barriers leave together: one whose wait ran out takes the others with it
@@ -213,7 +215,7 @@ indexed_gemm_bwd_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_c
       const uint32_t tsrc = tmem + ((uint32_t)(quad * 32) << 16) + buf * BN;
       if constexpr (F32OUT) {
         const int orow = (MODE == MODE_DW) ? sp * p.split_rows + tm * BM : tm * BM;
-        const int n32 = min(2 * nsub, (p.J - tn * BN + 31) / 32);
+        const int n32 = min(2 * nsub, (p.J - tn * bn + 31) / 32);
         for (int u = 0; u < n32; ++u) {             // 32 fp32 columns: 128-byte rows, 16 KB
           const int ob = (n_out++) & 1;
           if (etid == 0) tma_store_wait_read1();
@@ -228,7 +230,7 @@ indexed_gemm_bwd_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_c
           fence_proxy_async_smem();
           named_bar_sync(1, 128);
           if (etid == 0) {
-            tma_store_2d(&mapO, out_stage + ob * (BOUT_BYTES / 2), tn * BN + u * 32, orow);
+            tma_store_2d(&mapO, out_stage + ob * (BOUT_BYTES / 2), tn * bn + u * 32, orow);
             tma_store_commit();
           }
         }
@@ -249,10 +251,10 @@ indexed_gemm_bwd_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_c
           v[32 + j] = __uint_as_float(r1[j]);
         }
         if (MODE == MODE_DX && p.bias) {
-          const __nv_bfloat16* bp = reinterpret_cast<const __nv_bfloat16*>(p.bias) + tn * BN + u * 64;
+          const __nv_bfloat16* bp = reinterpret_cast<const __nv_bfloat16*>(p.bias) + tn * bn + u * 64;
 #pragma unroll
           for (int j = 0; j < 64; ++j)
-            if (tn * BN + u * 64 + j < p.J) v[j] += __bfloat162float(bp[j]);
+            if (tn * bn + u * 64 + j < p.J) v[j] += __bfloat162float(bp[j]);
         }
         uint8_t* dst = out_stage + ob * (BOUT_BYTES / 2) + row * 128;
 #pragma unroll
@@ -269,12 +271,12 @@ indexed_gemm_bwd_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_c
         if (etid == 0) {
           const uint8_t* src = out_stage + ob * (BOUT_BYTES / 2);
           if (MODE == MODE_DX) {
-            tma_store_2d(&mapO, src, tn * BN + u * 64, tm * BM);
+            tma_store_2d(&mapO, src, tn * bn + u * 64, tm * BM);
           } else {
             for (int hb = 0; hb < nrow; ++hb) {
               const int sb = tm * 2 + hb;
-              tma_store_2d(wm[tb.weight[sb]], src + hb * ATOM, tn * BN + u * 64, tb.row0[sb]);
-              if (p.halves) tma_store_2d(wm[tb.weightb[sb]], src + hb * ATOM + ATOM / 2, tn * BN + u * 64, tb.row0b[sb]);
+              tma_store_2d(wm[tb.weight[sb]], src + hb * ATOM, tn * bn + u * 64, tb.row0[sb]);
+              if (p.halves) tma_store_2d(wm[tb.weightb[sb]], src + hb * ATOM + ATOM / 2, tn * bn + u * 64, tb.row0b[sb]);
             }
           }
           tma_store_commit();
@@ -356,6 +358,25 @@ int launch_mode(const CUtensorMap& ma, const CUtensorMap& mb, const CUtensorMap*
                     dim3(grid), BGEMM_THREADS, smem, st, 1, ma, mb, mw[0], mw[1], mw[2], mw[3], mo, p, tb);
 }
 
+// Columns of a dx tile, in 64-column blocks, by the time the waves should take, in cycles: a K step is bound by its
+// operands' way from L2 (16 KB of dout and 8 KB of weights per block).  A last wave that is nearly empty costs as much as a
+// full one.  Measured with 256, 192 and 128 columns: 8192 rows, 1920 -> 768 29.0, 26.2 and 32.7 us (192 tiles, 256, 384 on 148
+// SMs), 768 -> 768 14.1, 12.9, 15.7; 1024 rows, 1920 -> 768 15.6, 13.7, 12.5; 3001 rows, 3840 -> 1536 29.9, 47, 43.
+int dx_subs(int tiles_m, int C, int KB) {
+  const int sms = device_sm_count();
+  int best = 4;
+  double cost = 1e30;
+  for (int s = 4; s >= 2; --s) {
+    const int64_t tiles = (int64_t)tiles_m * ((C + s * 64 - 1) / (s * 64));
+    const double t = (double)((tiles + sms - 1) / sms) * (KB * (445.0 + 110.0 * s) + 1000.0 + 300.0 * s);
+    if (t < cost) {
+      cost = t;
+      best = s;
+    }
+  }
+  return best;
+}
+
 }  // namespace
 
 int launch_gemm_bwd_dx_sm100(const SafIndexedLinearArgs& a, const void* dout, int64_t lddo, void* dx, int64_t lddx,
@@ -380,7 +401,8 @@ int launch_gemm_bwd_dx_sm100(const SafIndexedLinearArgs& a, const void* dout, in
   p.halves = is_halves(a) ? 1 : 0;
   p.I = a.M; p.J = a.C; p.KB = N / 64; p.n_blocks = N / 64;
   p.tiles_m = (a.M + BM - 1) / BM;
-  p.tiles_n = (a.C + BN - 1) / BN;
+  p.subs = dx_subs(p.tiles_m, a.C, p.KB);
+  p.tiles_n = (a.C + p.subs * 64 - 1) / (p.subs * 64);
   p.bias = bias;
   p.status = a.status;
   if (f32_out) return launch_mode<MODE_DX, true>(ma, ma, mw, mo, p, tb, st);
@@ -408,6 +430,7 @@ int launch_gemm_bwd_dw_sm100(const SafIndexedLinearArgs& a, const void* dout, in
   p.halves = is_halves(a) ? 1 : 0;
   p.I = N; p.J = a.C; p.KB = (a.M + BK - 1) / BK; p.n_blocks = N / 64;
   p.tiles_m = (p.n_blocks + 1) / 2;
+  p.subs = 4;
   p.tiles_n = (a.C + BN - 1) / BN;
   p.status = a.status;
   return launch_mode<MODE_DW>(ma, mb, mw, ma, p, tb, st);
@@ -527,6 +550,7 @@ int launch_gemm_bwd_dw_full_sm100(const SafIndexedLinearArgs& a, const void* dou
   memset(&p, 0, sizeof(p));
   p.I = N; p.J = a.C; p.KB = (a.M + BK - 1) / BK; p.n_blocks = N / 64;
   p.tiles_m = (p.n_blocks + 1) / 2;
+  p.subs = 4;
   p.tiles_n = (a.C + BN - 1) / BN;
   p.splits = d.splits;
   p.split_rows = d.split_rows;
