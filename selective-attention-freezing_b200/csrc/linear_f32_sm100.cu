@@ -402,7 +402,8 @@ SplitForm pick_split_form(int mode, int I, int J, int KT) {
       if (s > 1 && (mode == 0 || KT < 2 * s)) break;
       const int64_t room = s == 4 ? sms * 9 / 10 / 4 * 4 : sms / s * s;       // clusters of four leave SMs over
       const double waves = (double)((tiles * s + room - 1) / room);
-      const double t = waves * (6600.0 + (s > 1 ? 1500.0 : 0.0) + ((KT + s - 1) / s) * (bn == 128 ? 2800.0 : 2100.0));
+      const double fixed = s == 1 ? 6000.0 : (s == 2 ? 12000.0 : 14600.0);
+      const double t = waves * (fixed + ((KT + s - 1) / s) * (bn == 128 ? 2800.0 : 2100.0));
       if (t < cost) {
         cost = t;
         best = {bn, s};

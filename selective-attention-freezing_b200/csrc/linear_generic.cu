@@ -164,6 +164,28 @@ __global__ void rope_slabs_kernel(T* __restrict__ out, int64_t ldo, int M, int n
   }
 }
 
+// fp32, 16-byte accesses: one thread rotates 4 pairs of one slab of one row (2048 rows of 18 heads x 64: 10.5 -> 5 us)
+__global__ void __launch_bounds__(256) rope_slabs_f32x4_kernel(float* __restrict__ out, int64_t ldo, uint32_t total, uint32_t n_slabs,
+                                                               uint32_t slab, uint32_t Tlen, const float* __restrict__ cosT,
+                                                               const float* __restrict__ sinT, const __grid_constant__ SlabTable tb, float sgn) {
+  pdl_wait();
+  pdl_trigger();
+  const uint32_t half = slab >> 1, per_slab = half >> 2;
+  for (uint32_t idx = blockIdx.x * blockDim.x + threadIdx.x; idx < total; idx += gridDim.x * blockDim.x) {
+    const uint32_t q = idx / per_slab, d = (idx - q * per_slab) * 4, m = q / n_slabs, g = q - m * n_slabs;
+    if (!tb.rope[g]) continue;
+    float* p = out + (int64_t)m * ldo + (int64_t)g * slab + d;
+    const int64_t at = (int64_t)(m % Tlen) * slab + d;
+    const float4 x1 = *reinterpret_cast<const float4*>(p), x2 = *reinterpret_cast<const float4*>(p + half);
+    const float4 c1 = *reinterpret_cast<const float4*>(cosT + at), c2 = *reinterpret_cast<const float4*>(cosT + at + half);
+    const float4 s1 = *reinterpret_cast<const float4*>(sinT + at), s2 = *reinterpret_cast<const float4*>(sinT + at + half);
+    *reinterpret_cast<float4*>(p) = make_float4(x1.x * c1.x - x2.x * (sgn * s1.x), x1.y * c1.y - x2.y * (sgn * s1.y),
+                                                x1.z * c1.z - x2.z * (sgn * s1.z), x1.w * c1.w - x2.w * (sgn * s1.w));
+    *reinterpret_cast<float4*>(p + half) = make_float4(x2.x * c2.x + x1.x * (sgn * s2.x), x2.y * c2.y + x1.y * (sgn * s2.y),
+                                                       x2.z * c2.z + x1.z * (sgn * s2.z), x2.w * c2.w + x1.w * (sgn * s2.w));
+  }
+}
+
 // bf16, 16-byte accesses: one thread rotates 8 pairs (d .. d+7, d+half .. d+half+7) of one slab of one row
 __global__ void __launch_bounds__(256) rope_slabs_vec_kernel(__nv_bfloat16* __restrict__ out, int64_t ldo, int M, int n_slabs,
                                                              int slab, int Tlen, const float* __restrict__ cosT,
@@ -200,6 +222,20 @@ __global__ void __launch_bounds__(256) rope_slabs_vec_kernel(__nv_bfloat16* __re
     *reinterpret_cast<uint4*>(p) = make_uint4(lw[0], lw[1], lw[2], lw[3]);
     *reinterpret_cast<uint4*>(p + half) = make_uint4(hw[0], hw[1], hw[2], hw[3]);
   }
+}
+
+// fp32 rows in place; rows, tables and slabs of whole 16-byte pieces go four pairs at a time
+int rope_f32(float* x, int64_t ld, int M, int n_slabs, int slab, int T, const float* cosT, const float* sinT, const SlabTable& tb, float sgn,
+             cudaStream_t st) {
+  const int64_t pairs = (int64_t)M * n_slabs * (slab / 2);
+  if (slab % 8 == 0 && ld % 4 == 0 && !(((uintptr_t)x | (uintptr_t)cosT | (uintptr_t)sinT) & 15) && pairs / 4 <= 0x7fffffff) {
+    const int blocks = (int)std::min<int64_t>((pairs / 4 + 255) / 256, 148 * 32);
+    return launch_pdl("rope_slabs_kernel", rope_slabs_f32x4_kernel, dim3(blocks), 256, 0, st, 1, x, ld, (uint32_t)(pairs / 4), (uint32_t)n_slabs,
+                      (uint32_t)slab, (uint32_t)T, cosT, sinT, tb, sgn);
+  }
+  rope_slabs_kernel<float><<<(int)std::min<int64_t>((pairs + 255) / 256, 148 * 16), 256, 0, st>>>(x, ld, M, n_slabs, slab, T, cosT, sinT, tb, sgn);
+  count_launch();
+  return check_launch("rope_slabs_kernel");
 }
 
 int fill_tables(const SafIndexedLinearArgs& a, WeightSet* ws, SlabTable* tb) {
@@ -241,6 +277,8 @@ int gemm_generic_typed(const SafIndexedLinearArgs& a, int mode, const void* dout
     }
     bool any_rope = false;
     for (int g = 0; g < a.n_slabs; ++g) any_rope |= tb.rope[g] != 0;
+    if (any_rope && f32)
+      return rope_f32(reinterpret_cast<float*>(a.out), a.ldo, a.M, a.n_slabs, a.slab, a.T, a.rope_cos, a.rope_sin, tb, 1.f, st);
     if (any_rope) {
       const int64_t total = (int64_t)a.M * a.n_slabs * (a.slab / 2);
       const int blocks = (int)std::min<int64_t>((total + 255) / 256, 148 * 16);
@@ -352,10 +390,9 @@ int launch_rope_slabs(void* x, int64_t ld, int M, int n_slabs, int slab, int T, 
     const int bv = (int)std::min<int64_t>((tv + 255) / 256, 148 * 32);
     return launch_pdl("rope_slabs_kernel", rope_slabs_vec_kernel, dim3(bv), 256, 0, st, 1, reinterpret_cast<__nv_bfloat16*>(x), ld, M,
                       n_slabs, slab, T, cosT, sinT, tb, sgn);
-  } else if (dtype == SAF_F32)
-    rope_slabs_kernel<float><<<blocks, 256, 0, st>>>(reinterpret_cast<float*>(x), ld, M, n_slabs, slab, T, cosT, sinT, tb, sgn);
-  else
-    rope_slabs_kernel<__nv_bfloat16><<<blocks, 256, 0, st>>>(reinterpret_cast<__nv_bfloat16*>(x), ld, M, n_slabs, slab, T,
+  }
+  if (dtype == SAF_F32) return rope_f32(reinterpret_cast<float*>(x), ld, M, n_slabs, slab, T, cosT, sinT, tb, sgn, st);
+  rope_slabs_kernel<__nv_bfloat16><<<blocks, 256, 0, st>>>(reinterpret_cast<__nv_bfloat16*>(x), ld, M, n_slabs, slab, T,
                                                             cosT, sinT, tb, sgn);
   count_launch();
   return check_launch("rope_slabs_kernel");
