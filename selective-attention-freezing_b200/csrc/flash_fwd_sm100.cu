@@ -695,10 +695,13 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant
 //               tile through its own 16 KB buffer (64 columns at a time), so Q is never held back by a store
 // Score tiles of an item are produced in the order (0,0) (1,0) (0,1) (1,1) ... with the extra diagonal step
 // of tile 1 last, so every index of the running counter is a real tile and barrier phases follow from it.
+// s_full is kept per query tile: a warpgroup whose tile an item does not have (the last row pair of an odd number of row
+// tiles) is handed the next item while the other one still works, more than one phase of a shared barrier ahead of it, and
+// a wait by parity cannot tell that phase from the one before.
 struct PersistBars {
   uint64_t q_full[2], q_free[2];
   uint64_t k_full[4], k_empty[4], v_full[4], v_empty[4];
-  uint64_t s_full[3], p_full[3], buf_free[3];
+  uint64_t s_full[2][3], p_full[3], buf_free[3];
   uint64_t o_free[2];
   uint64_t w_full[2], w_empty[2];
   volatile int32_t work[2];
@@ -804,7 +807,8 @@ flash_fwd_persistent_kernel(const __grid_constant__ CUtensorMap mapQ, const __gr
       mbar_init(&bars->v_empty[s], 1);
     }
     for (int i = 0; i < 3; ++i) {
-      mbar_init(&bars->s_full[i], 1);
+      mbar_init(&bars->s_full[0][i], 1);
+      mbar_init(&bars->s_full[1][i], 1);
       mbar_init(&bars->p_full[i], 128);
       mbar_init(&bars->buf_free[i], 1);
     }
@@ -962,7 +966,7 @@ flash_fwd_persistent_kernel(const __grid_constant__ CUtensorMap mapQ, const __gr
               const uint32_t off = (ks >> 2) * 16384 + (ks & 3) * 32;
               umma_ss(d, umma_desc_advance(dq, off), umma_desc_advance(dk, off), idesc_s, ks > 0);
             }
-            umma_commit(&bars->s_full[buf]);
+            umma_commit(&bars->s_full[t][buf]);
             if (t == 1 || !g.act1) umma_commit(&bars->k_empty[ks_]);   // last reader of K_j
             if (!C::STAGE_IN_Q && j == (t ? g.nkv1 : g.nkv0) - 1) umma_commit(&bars->q_free[t]);   // last reader of Q_t
           }
@@ -1038,7 +1042,7 @@ flash_fwd_persistent_kernel(const __grid_constant__ CUtensorMap mapQ, const __gr
     const uint32_t tO = tmem + lane_base + C::O_COL + t * HD;
     const float sc = p.scale_log2;
     const bool warp_lead = (tid & 31) == 0;
-    uint32_t g_base = 0;
+    uint32_t g_base = 0, s_phase = 0;      // s_phase: one bit per score buffer, the parity of this tile's next use of it
     bool ok = true;
     for (int n = 0; ok; ++n) {
       const int it = fetch(n, warp_lead);
@@ -1055,11 +1059,12 @@ flash_fwd_persistent_kernel(const __grid_constant__ CUtensorMap mapQ, const __gr
           const uint32_t gi = g_base + (g.act1 ? ((t == 1 && j == g.nkv0) ? 2 * g.nkv0 : 2 * j + t) : j);
           const uint32_t buf = gi % C::NBUF, bph = (gi / C::NBUF) & 1;
           const uint32_t tS = tmem + lane_base + buf * FN;
-          if (!mbar_wait(&bars->s_full[buf], bph)) {
+          if (!mbar_wait(&bars->s_full[t][buf], (s_phase >> buf) & 1)) {
             dev_set_error(p.status, SAF_DEV_TIMEOUT_SOFTMAX, 54);
             ok = false;
             break;
           }
+          s_phase ^= 1u << buf;
           tc_fence_after();
           uint32_t s[4][32];
 #pragma unroll
