@@ -266,6 +266,12 @@ int saf_mixed_attn_fwd(const SafMixedAttnArgs* args, void* stream) {
     if (rc == SAF_OK) todo &= ~handled;
     else if (rc != SAF_ERR_UNSUPPORTED) return rc;
   }
+  if (todo & 1u) {                  // fp32: live heads, and the structured ones beside them
+    const uint32_t scan = todo & (1u << SAF_SINK_DECAY);
+    rc = launch_attn_f32_fwd(a, scan != 0, st);
+    if (rc == SAF_OK) todo &= ~(1u | scan);
+    else if (rc != SAF_ERR_UNSUPPORTED) return rc;
+  }
   if (todo & (1u << SAF_SINK_DECAY)) {
     if ((rc = launch_scan_fwd(a, st))) return rc;
     todo &= ~(1u << SAF_SINK_DECAY);
@@ -302,7 +308,7 @@ int saf_mixed_attn_bwd(const SafMixedAttnBwdArgs* args, void* stream) {
     if (rc == SAF_OK) todo &= ~handled;
     else if (rc != SAF_ERR_UNSUPPORTED) return rc;
   }
-  if (todo & (1u << SAF_SINK_DECAY)) {
+  if ((todo & (1u << SAF_SINK_DECAY)) && !((todo & 1u) && attn_f32_bwd_ok(*args))) {   // (else a role of the fp32 launch)
     if ((rc = launch_scan_bwd(*args, st))) return rc;
     todo &= ~(1u << SAF_SINK_DECAY);
   }

@@ -27,6 +27,7 @@
 
 #include "head_index.cuh"
 #include "saf_internal.h"
+#include "scan_body.cuh"
 #include "split_bf16.cuh"
 
 
@@ -542,17 +543,49 @@ __device__ __forceinline__ void attn_f32_tile(const SafMixedAttnBwdArgs& g, int 
   if (warp == AISSUER) tmem_dealloc(tmem, 512);
 }
 
+// A structured head's CTA of the first row of the grid runs its scan, a sequential chain that ends long before the longest
+// walks (launched on their own before: 17 us forward, 26 backward of the layer's 394 at T = 1024; now 366).  256 x 168 + 640 x 24 registers <= 896 x 72;
+// the warps without work leave before the others take theirs, so that the compiler sees one path with the larger share.
+__device__ __forceinline__ bool attn_f32_scan_head(const SafMixedAttnArgs& a, const ScanArgs& sc) {
+  return blockIdx.y == 0 && sc.in != nullptr && head_index(a, blockIdx.x).state == SAF_SINK_DECAY;
+}
+template <bool BWD>
+__device__ __forceinline__ void attn_f32_scan(const SafMixedAttnArgs& a, const ScanArgs& sc) {
+  asm volatile("setmaxnreg.inc.sync.aligned.u32 168;");
+  extern __shared__ uint8_t attn_smem[];
+  const int b = blockIdx.x / a.H, h = blockIdx.x % a.H;
+  sink_decay_scan_cta<float, BWD, 0, true>(sc, b, h, 0, 0, -1, reinterpret_cast<float*>(attn_smem));
+}
+
 // grid (B * H, row tiles): the longest walks of all heads first
-__global__ void __launch_bounds__(ATHREADS, 1) attn_f32_fwd_kernel(const __grid_constant__ SafMixedAttnBwdArgs g) {
+__global__ void __launch_bounds__(ATHREADS, 1) attn_f32_fwd_kernel(const __grid_constant__ SafMixedAttnBwdArgs g,
+                                                                   const __grid_constant__ ScanArgs sc) {
   pdl_wait();
   pdl_trigger();
+  if (attn_f32_scan_head(g.fwd, sc)) {
+    if (threadIdx.x >= SCAN_NT) {
+      asm volatile("setmaxnreg.dec.sync.aligned.u32 24;");
+      return;
+    }
+    attn_f32_scan<false>(g.fwd, sc);
+    return;
+  }
   attn_f32_tile<A_FWD>(g, blockIdx.y, gridDim.y);
 }
 // grid (B * H, 2 x row tiles): dK / dV and dQ tiles of one length take turns.  One launch for both, because a row tile's walk
 // has 2 to 2 tiles' length of steps and a launch of one kind alone ends with most SMs idle
-__global__ void __launch_bounds__(ATHREADS, 1) attn_f32_bwd_kernel(const __grid_constant__ SafMixedAttnBwdArgs g) {
+__global__ void __launch_bounds__(ATHREADS, 1) attn_f32_bwd_kernel(const __grid_constant__ SafMixedAttnBwdArgs g,
+                                                                   const __grid_constant__ ScanArgs sc) {
   pdl_wait();
   pdl_trigger();
+  if (attn_f32_scan_head(g.fwd, sc)) {
+    if (threadIdx.x >= SCAN_NT) {
+      asm volatile("setmaxnreg.dec.sync.aligned.u32 24;");
+      return;
+    }
+    attn_f32_scan<true>(g.fwd, sc);
+    return;
+  }
   if (blockIdx.y & 1) attn_f32_tile<A_DQ>(g, blockIdx.y >> 1, gridDim.y >> 1);
   else attn_f32_tile<A_DKDV>(g, blockIdx.y >> 1, gridDim.y >> 1);
 }
@@ -574,27 +607,33 @@ bool f32_call_ok(const SafMixedAttnArgs& a) {
 
 // The live heads of an fp32 call whose rows are whole 16-byte pieces and come rotated already; everything else stays
 // with the any-type kernels.
-int launch_attn_f32_fwd(const SafMixedAttnArgs& a, cudaStream_t st) {
+int launch_attn_f32_fwd(const SafMixedAttnArgs& a, bool scan, cudaStream_t st) {
   if (!f32_call_ok(a)) return SAF_ERR_UNSUPPORTED;
   SafMixedAttnBwdArgs g;
   memset(&g, 0, sizeof(g));
   g.fwd = a;
   static PerDeviceOnce once;
   if (int rc = ensure_dyn_smem(attn_f32_fwd_kernel, AttnShape<A_FWD>::SMEM, once)) return rc;
-  return launch_pdl("attn_f32_fwd_kernel", attn_f32_fwd_kernel, dim3(a.B * a.H, (a.T + AR - 1) / AR), ATHREADS, AttnShape<A_FWD>::SMEM, st, 1, g);
+  return launch_pdl("attn_f32_fwd_kernel", attn_f32_fwd_kernel, dim3(a.B * a.H, (a.T + AR - 1) / AR), ATHREADS, AttnShape<A_FWD>::SMEM, st, 1, g,
+                    scan ? scan_args_fwd(a) : ScanArgs{});
+}
+
+bool attn_f32_bwd_ok(const SafMixedAttnBwdArgs& g) {
+  const SafMixedAttnArgs& a = g.fwd;
+  return f32_call_ok(a) && a.HKV == 0 && f32_rows_ok(g.dout, a.B, a.H, a.T) && f32_rows_ok(g.dv, a.B, a.H, a.T) &&
+         f32_rows_ok(g.dq, a.B, a.U, a.T) && f32_rows_ok(g.dk, a.B, a.U, a.T);
 }
 
 // dK, dV and dQ; delta is filled already
-int launch_attn_f32_bwd(const SafMixedAttnBwdArgs& g, cudaStream_t st) {
+int launch_attn_f32_bwd(const SafMixedAttnBwdArgs& g, bool scan, cudaStream_t st) {
   const SafMixedAttnArgs& a = g.fwd;
-  if (!f32_call_ok(a) || a.HKV > 0 || !f32_rows_ok(g.dout, a.B, a.H, a.T) || !f32_rows_ok(g.dv, a.B, a.H, a.T) ||
-      !f32_rows_ok(g.dq, a.B, a.U, a.T) || !f32_rows_ok(g.dk, a.B, a.U, a.T))
-    return SAF_ERR_UNSUPPORTED;
+  if (!attn_f32_bwd_ok(g)) return SAF_ERR_UNSUPPORTED;
   constexpr int smem = AttnShape<A_DKDV>::SMEM;
   static_assert(smem >= AttnShape<A_DQ>::SMEM, "both kinds of tile fit");
   static PerDeviceOnce once;
   if (int rc = ensure_dyn_smem(attn_f32_bwd_kernel, smem, once)) return rc;
-  return launch_pdl("attn_f32_bwd_kernel", attn_f32_bwd_kernel, dim3(a.B * a.H, 2 * ((a.T + AR - 1) / AR)), ATHREADS, smem, st, 1, g);
+  return launch_pdl("attn_f32_bwd_kernel", attn_f32_bwd_kernel, dim3(a.B * a.H, 2 * ((a.T + AR - 1) / AR)), ATHREADS, smem, st, 1, g,
+                    scan ? scan_args_bwd(g) : ScanArgs{});
 }
 
 }  // namespace saf

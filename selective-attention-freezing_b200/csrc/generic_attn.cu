@@ -556,10 +556,11 @@ int bwd_typed(const SafMixedAttnBwdArgs& g, uint32_t mask, cudaStream_t st) {
     generic_delta_kernel<T><<<gd, NT, 0, st>>>(g);
     count_launch();
     if ((rc = check_launch("generic_delta_kernel"))) return rc;
-    rc = launch_attn_f32_bwd(g, st);
+    const uint32_t scan = mask & (1u << SAF_SINK_DECAY);
+    rc = launch_attn_f32_bwd(g, scan != 0, st);
     if (rc == SAF_OK) {
       any_live = false;
-      mask &= ~1u;
+      mask &= ~(1u | scan);
     } else if (rc != SAF_ERR_UNSUPPORTED) {
       return rc;
     }
@@ -588,12 +589,6 @@ int bwd_typed(const SafMixedAttnBwdArgs& g, uint32_t mask, cudaStream_t st) {
 int launch_generic_fwd(const SafMixedAttnArgs& a, uint32_t states_mask, cudaStream_t st) {
   if (a.HD > 128) return fail(SAF_ERR_UNSUPPORTED, "head_dim %d > 128", a.HD);
   if (a.T == 0 || a.B == 0 || a.H == 0) return SAF_OK;
-  if (states_mask & 1u) {
-    const int rc = launch_attn_f32_fwd(a, st);
-    if (rc == SAF_OK) states_mask &= ~1u;
-    else if (rc != SAF_ERR_UNSUPPORTED) return rc;
-    if (!states_mask) return SAF_OK;
-  }
   switch (a.dtype) {
     case SAF_F32: return fwd_typed<float>(a, states_mask, st);
     case SAF_BF16: return fwd_typed<__nv_bfloat16>(a, states_mask, st);

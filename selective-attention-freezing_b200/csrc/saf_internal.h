@@ -112,9 +112,11 @@ uint32_t mixed_possible_states(const SafMixedAttnArgs& a);
 // states_mask: bit s set -> heads in state s are processed by this launch
 int launch_generic_fwd(const SafMixedAttnArgs& a, uint32_t states_mask, cudaStream_t st);
 int launch_generic_bwd(const SafMixedAttnBwdArgs& a, uint32_t states_mask, cudaStream_t st);
-// live heads of an fp32 call, head_dim 64; SAF_ERR_UNSUPPORTED when the call does not qualify.  bwd: delta is filled
-int launch_attn_f32_fwd(const SafMixedAttnArgs& a, cudaStream_t st);
-int launch_attn_f32_bwd(const SafMixedAttnBwdArgs& g, cudaStream_t st);
+// live heads of an fp32 call, head_dim 64, and with `scan` its structured heads in the same launch; SAF_ERR_UNSUPPORTED when
+// the call does not qualify.  bwd: delta is filled
+int launch_attn_f32_fwd(const SafMixedAttnArgs& a, bool scan, cudaStream_t st);
+bool attn_f32_bwd_ok(const SafMixedAttnBwdArgs& g);
+int launch_attn_f32_bwd(const SafMixedAttnBwdArgs& g, bool scan, cudaStream_t st);
 int launch_scan_fwd(const SafMixedAttnArgs& a, cudaStream_t st);                       // state 3 heads
 int launch_scan_bwd(const SafMixedAttnBwdArgs& a, cudaStream_t st);                    // state 3 heads: dv
 // state 3 heads, forward, on the tensor core (bf16, head_dim a multiple of 64, long T); SAF_ERR_UNSUPPORTED otherwise

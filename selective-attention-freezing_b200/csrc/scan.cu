@@ -86,12 +86,7 @@ int scan_dispatch(const ScanArgs& s, int dtype, bool bwd, cudaStream_t st) {
 
 }  // namespace
 
-int launch_scan_fwd(const SafMixedAttnArgs& a, cudaStream_t st) {
-  if (!a.sd_alpha || !a.sd_rho) return fail(SAF_ERR_INVALID, "sink-decay heads need sd_alpha and sd_rho");
-  {   // long bf16 sequences: blocks of 128 rows as Toeplitz products on the tensor core
-    const int rc = launch_scan_fwd_mma(a, st);
-    if (rc != SAF_ERR_UNSUPPORTED) return rc;
-  }
+ScanArgs scan_args_fwd(const SafMixedAttnArgs& a) {
   ScanArgs s{};
   s.in = a.v.ptr;
   s.out = a.out.ptr;
@@ -108,12 +103,11 @@ int launch_scan_fwd(const SafMixedAttnArgs& a, cudaStream_t st) {
   s.vec_ok = vec_ok(a.v.ptr, a.v.stride, es) && vec_ok(a.out.ptr, a.out.stride, es);
   if (a.frozen_host && a.force_state < 0)
     for (int h = 0; h < a.H; ++h) s.n_active += a.frozen_host[h] == SAF_SINK_DECAY;
-  return scan_dispatch(s, a.dtype, false, st);
+  return s;
 }
 
-int launch_scan_bwd(const SafMixedAttnBwdArgs& g, cudaStream_t st) {
+ScanArgs scan_args_bwd(const SafMixedAttnBwdArgs& g) {
   const SafMixedAttnArgs& a = g.fwd;
-  if (!a.sd_alpha || !a.sd_rho) return fail(SAF_ERR_INVALID, "sink-decay heads need sd_alpha and sd_rho");
   ScanArgs s{};
   s.in = g.dout.ptr;
   s.out = g.dv.ptr;
@@ -128,6 +122,23 @@ int launch_scan_bwd(const SafMixedAttnBwdArgs& g, cudaStream_t st) {
   s.B = a.B; s.H = a.H; s.T = a.T; s.HD = a.HD; s.force_state = a.force_state; s.HKV = 0;
   const int es = dtype_size(a.dtype);
   s.vec_ok = vec_ok(g.dout.ptr, g.dout.stride, es) && vec_ok(g.dv.ptr, g.dv.stride, es);
+  return s;
+}
+
+int launch_scan_fwd(const SafMixedAttnArgs& a, cudaStream_t st) {
+  if (!a.sd_alpha || !a.sd_rho) return fail(SAF_ERR_INVALID, "sink-decay heads need sd_alpha and sd_rho");
+  {   // long bf16 sequences: blocks of 128 rows as Toeplitz products on the tensor core
+    const int rc = launch_scan_fwd_mma(a, st);
+    if (rc != SAF_ERR_UNSUPPORTED) return rc;
+  }
+  const ScanArgs s = scan_args_fwd(a);
+  return scan_dispatch(s, a.dtype, false, st);
+}
+
+int launch_scan_bwd(const SafMixedAttnBwdArgs& g, cudaStream_t st) {
+  const SafMixedAttnArgs& a = g.fwd;
+  if (!a.sd_alpha || !a.sd_rho) return fail(SAF_ERR_INVALID, "sink-decay heads need sd_alpha and sd_rho");
+  const ScanArgs s = scan_args_bwd(g);
   return scan_dispatch(s, a.dtype, true, st);
 }
 

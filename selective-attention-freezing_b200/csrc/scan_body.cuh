@@ -85,6 +85,10 @@ struct ScanArgs {
   int n_active;        // host hint: heads that are in the structured state (0 = unknown, all H are assumed)
 };
 
+// the scan of a call's structured heads: forward V -> Y, backward dY -> dV (scan.cu)
+ScanArgs scan_args_fwd(const SafMixedAttnArgs& a);
+ScanArgs scan_args_bwd(const SafMixedAttnBwdArgs& g);
+
 // 256-thread barrier that leaves barrier 0 (and any other warps of the CTA) alone
 __device__ __forceinline__ void scan_bar() { asm volatile("bar.sync 15, 256;" ::: "memory"); }
 
