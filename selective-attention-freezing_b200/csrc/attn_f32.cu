@@ -544,8 +544,9 @@ __device__ __forceinline__ void attn_f32_tile(const SafMixedAttnBwdArgs& g, int 
 }
 
 // A structured head's CTA of the first row of the grid runs its scan, a sequential chain that ends long before the longest
-// walks (launched on their own before: 17 us forward, 26 backward of the layer's 394 at T = 1024; now 366).  256 x 168 + 640 x 24 registers <= 896 x 72;
-// the warps without work leave before the others take theirs, so that the compiler sees one path with the larger share.
+// walks (launched on their own before: 17 us forward, 26 backward of the layer's 394 at T = 1024; now 366).  256 x 168 +
+// 640 x 24 registers <= 896 x 72; the warps without work leave before the others take theirs, so that the compiler sees one
+// path with the larger share.
 __device__ __forceinline__ bool attn_f32_scan_head(const SafMixedAttnArgs& a, const ScanArgs& sc) {
   return blockIdx.y == 0 && sc.in != nullptr && head_index(a, blockIdx.x).state == SAF_SINK_DECAY;
 }

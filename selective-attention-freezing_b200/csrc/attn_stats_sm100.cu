@@ -5,7 +5,7 @@
 // (nanogpt/dynamic_freeze.py:96-127 _centered_batch_reduced_moments, :130-143 _merge_reduced_moments,
 // :146-173 _negative_entropy_sum, used by _measure :629-745).  Here a CTA takes one 128 x 64 cell tile of one head
 // at a time: S_b = Q_b K_b^T of up to four samples on tcgen05 into TMEM, then per cell P_b = exp2(S_b scale - lse_b) with
-// the row log-sum-exp of the flash forward, the samples' mean and centred squares (Welford) and the Chan merge into the
+// the row log-sum-exp (row_lse_sm100.cu), the samples' mean and the squares about it, and the Chan merge into the
 // tile of the running mean; the per-head scalars are reduced to one double atomic per CTA and head.
 //
 // LOGITS: the same walk over the raw scores q k^T * sm_scale of the whole square (nothing masked, tiles above the
@@ -19,7 +19,8 @@
 // All samples of a cell are in TMEM at once, so mean and centred squares need no memory at all; more than four samples
 // are merged four at a time into the tile in shared memory.
 // 9 heads, T = 4096, four samples on a B200: raw scores with centred squares 1142 -> 400 us (2.4 GB, 6.0 TB/s),
-// probabilities 373 -> 263 us (the exponentials and Welford chains of 302 M probabilities; their tiles take 90 us).
+// probabilities 373 -> 263 us (302 M probabilities; their tiles alone take 90 us), and 212 us since two cells go through each
+// instruction and a cell's mean and centred squares come from sums over the samples instead of chains of updates.
 //
 //   warps 0-7: two warpgroups x 32 key columns, thread = query row (TMEM lane)
 //   warp 8: TMA producer ([Q_b tile | K_b tile] ring), warp 9: MMA issuer
