@@ -441,12 +441,8 @@ def fused_mixed_attn(q, k, v, patt, frozen, hidx=None, pidx=None,
         # parameter values, the fused call sees detached buffers, and PatternGradient adds their gradients
         if kvidx is not None:
             raise NotImplementedError("trainable patterns with kvidx (GQA) are not implemented")
-        from . import trainable_patterns as _tp
         alpha_p, rho_p = alpha, rho
-        z = _tp.current_normalisers(alpha, rho, v.shape[-2], frozen)
-        alpha, rho = alpha.detach(), rho.detach()
-    if alpha is not None and z is None:
-        z = decomposed_logz(alpha, rho)
+        alpha, rho, z = alpha.detach(), None if rho is None else rho.detach(), None
     if validate:
         assert q.ndim == k.ndim == v.ndim == 4, "q, k, v must be 4-D"
         B, Hv, T, HD = v.shape
@@ -482,16 +478,22 @@ def fused_mixed_attn(q, k, v, patt, frozen, hidx=None, pidx=None,
         else:
             assert states is None or 1 not in states, "dense-frozen heads require patt"
         if alpha is not None:
-            assert rho is not None and alpha.shape == rho.shape == z.shape, \
+            assert rho is not None and alpha.shape == rho.shape and (z is None or z.shape == alpha.shape), \
                 "alpha, rho, and z must have matching (H, S) shapes"
             assert alpha.shape[0] == H and alpha.shape[1] >= T, \
                 "decomposed buffers must have shape (H, S) with S >= T"
-            assert alpha.device == rho.device == z.device == v.device, \
+            assert alpha.device == rho.device == (v if z is None else z).device == v.device, \
                 "decomposed buffers must be on v.device"
         else:
             assert states is None or 2 not in states, "decomposed-frozen heads require alpha/rho/z"
         if sink_decay is None:
             assert states is None or 3 not in states, "sink-decay heads require sink_decay=(a, r)"
+    # (kernels read head states and buffers from here on)
+    if train_patterns:
+        from . import trainable_patterns as _tp
+        z = _tp.current_normalisers(alpha_p, rho_p, v.shape[-2], frozen)
+    elif alpha is not None and z is None:
+        z = decomposed_logz(alpha, rho)
     if (rope is not None and q.dtype == torch.bfloat16 and v.size(-1) in (64, 96, 128) and q.size(1) > 0
             and rope[0].dtype == torch.float32 and rope[0].is_contiguous() and rope[1].is_contiguous()):
         # tensor-core kernels: rotate q, k once into private copies (see _RotatedCopy) and run without in-kernel RoPE

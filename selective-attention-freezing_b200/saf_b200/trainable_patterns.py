@@ -26,6 +26,11 @@ def normalisers(alpha, rho, length, states=None):
     head states; heads that are not decomposed, whose z nothing reads, then get zeros."""
     ops._require_cuda(alpha, "alpha")
     H, S = alpha.shape
+    if states is not None:
+        if states.shape != (H,) or states.dtype != torch.int32 or states.device != alpha.device:
+            raise ValueError("states must be int32 (%d,) on %s, not %s %s on %s"
+                             % (H, alpha.device, states.dtype, tuple(states.shape), states.device))
+        states = states.contiguous()
     a = alpha.detach().float().contiguous()
     r = rho.detach().float().contiguous()
     z = torch.empty_like(a)
