@@ -193,6 +193,12 @@ uint32_t possible_states(const SafMixedAttnArgs& a) {
   return m;
 }
 
+// heads that may be structured are read with both of their parameters, whichever launch takes them
+int sink_decay_given(const SafMixedAttnArgs& a, uint32_t states) {
+  if ((states & (1u << SAF_SINK_DECAY)) && (!a.sd_alpha || !a.sd_rho)) return fail(SAF_ERR_INVALID, "sink-decay heads need sd_alpha and sd_rho");
+  return SAF_OK;
+}
+
 }  // namespace
 
 int validate_mixed_args(const SafMixedAttnArgs* a) { return validate_mixed(a); }
@@ -255,6 +261,7 @@ int saf_mixed_attn_fwd(const SafMixedAttnArgs* args, void* stream) {
   if (a.B == 0 || a.H == 0 || a.T == 0) return SAF_OK;
   cudaStream_t st = (cudaStream_t)stream;
   uint32_t todo = possible_states(a);
+  if ((rc = sink_decay_given(a, todo))) return rc;
   // tensor-core path first; it reports which states it covered
   if (todo == (1u << SAF_SINK_DECAY)) return launch_scan_fwd(a, st);   // scan only: the chunk-parallel scan
   uint32_t handled = 0;
@@ -296,6 +303,7 @@ int saf_mixed_attn_bwd(const SafMixedAttnBwdArgs* args, void* stream) {
   if (args->dout.stride[3] != 1 || args->dv.stride[3] != 1)
     return fail(SAF_ERR_INVALID, "dout and dv need unit stride on head_dim");
   uint32_t todo = possible_states(a);
+  if ((rc = sink_decay_given(a, todo))) return rc;
   if (todo & 1u) {
     if (!args->dq.ptr || !args->dk.ptr || !args->delta.ptr || !a.lse.ptr)
       return fail(SAF_ERR_INVALID, "live heads need dq, dk, delta and lse");

@@ -156,6 +156,28 @@ def test_static_backward_validates_before_it_applies_its_limit():
     assert _cabi.lib.saf_mixed_attn_bwd_static(C.byref(g), None) == _cabi.SAF_ERR_LIMIT
 
 
+@pytest.mark.parametrize("dtype", ["SAF_F32", "SAF_BF16"])
+def test_structured_heads_come_with_both_of_their_parameters(dtype):
+    """Head states the host does not know and one parameter of the structured heads alone: refused in both directions before
+    anything launches."""
+    from saf_b200 import _cabi
+    dummy = (C.c_float * 4096)()
+    at = C.cast(dummy, C.c_void_p).value
+    g = _cabi.SafMixedAttnBwdArgs()
+    g.struct_size = C.sizeof(_cabi.SafMixedAttnBwdArgs)
+    f = g.fwd
+    f.struct_size = C.sizeof(_cabi.SafMixedAttnArgs)
+    f.dtype, f.force_state = getattr(_cabi, dtype), -1
+    f.B, f.H, f.U, f.T, f.HD = 1, 2, 2, 16, 64
+    f.frozen = at
+    for t in (f.q, f.k, f.v, f.out, g.dout, g.dq, g.dk, g.dv, f.lse, g.delta):
+        t.ptr = at
+        t.stride[0], t.stride[1], t.stride[2], t.stride[3] = 2048, 1024, 64, 1
+    f.sd_alpha = at
+    for call, args in ((_cabi.lib.saf_mixed_attn_fwd, f), (_cabi.lib.saf_mixed_attn_bwd, g)):
+        assert call(C.byref(args), None) == _cabi.SAF_ERR_INVALID and "sd_alpha and sd_rho" in _cabi.last_error()
+
+
 def test_fft_normalisers_match_the_direct_ones_and_differentiate():
     """decomposed_logz_fft (the reference's O(T log T) normaliser, nanogpt/dynamic_freeze.py:330-361) equals the
     direct logsumexp the oracle is pinned on (for logit spreads the transform's fp64 round-off can resolve) and its
