@@ -46,7 +46,7 @@ template <int MODE>
 struct AttnShape {
   static constexpr int NRES = MODE == A_FWD ? 1 : 2, STAGES = MODE == A_FWD ? 3 : 2;
   struct Ctrl {
-    uint64_t full[STAGES], empty[STAGES], res_full, s_full[2], dp_full, p_full, ds_full, acc_full[2];
+    uint64_t full[STAGES], empty[STAGES], res_full, s_full[2], dp_full, p_full[2], ds_full, acc_full[2];
     uint32_t tmem_base;
     alignas(16) float lse[STAGES][AX], delta[STAGES][AX];   // dK / dV: of the streamed query rows
     float mx[2][4][AR];                         // forward: row maxima, row sums of the four quarters
@@ -163,10 +163,10 @@ __device__ __forceinline__ void attn_f32_tile(const SafMixedAttnBwdArgs& g, int 
     mbar_init(&sl->res_full, APROD / 32);
     for (int b = 0; b < 2; ++b) {
       mbar_init(&sl->s_full[b], 1);
+      mbar_init(&sl->p_full[b], ACOMP / 32);
       mbar_init(&sl->acc_full[b], 1);
     }
     mbar_init(&sl->dp_full, 1);
-    mbar_init(&sl->p_full, ACOMP / 32);
     mbar_init(&sl->ds_full, ACOMP / 32);
     fence_mbar_init();
   }
@@ -291,11 +291,14 @@ __device__ __forceinline__ void attn_f32_tile(const SafMixedAttnBwdArgs& g, int 
       bool ok = wait(&sl->res_full, 0, 77);
       // Instructions of one thread run in order: a region is free for the next product once the last one that reads it has
       // been issued and its readers in the compute warps have arrived.
+      // A wait by parity tells a phase from the next one only, so a barrier's arrivals for one step must not come before this
+      // warp has seen those for the step before.  The forward's scores are two steps ahead of P: the compute warps can hand
+      // over the next P while P of this step has yet to be seen here, and take turns on two barriers.
       if constexpr (MODE == A_FWD) {
         for (int it = 0; it < 2 && it < n && ok; ++it)
           if ((ok = stage_full(it))) scores(0, it, tmem + it * 128, &sl->s_full[it]);
         for (int it = 0; it < n && ok; ++it) {
-          if (!(ok = wait(&sl->p_full, it, 78))) break;
+          if (!(ok = wait(&sl->p_full[it & 1], it >> 1, 78))) break;
           apply(tmem + (it & 1) * 128, 1, it, tmem + T_ACC1 + (it & 1) * 128, true);
           commit(&sl->empty[it % S::STAGES]);
           commit(&sl->acc_full[it & 1]);
@@ -308,7 +311,7 @@ __device__ __forceinline__ void attn_f32_tile(const SafMixedAttnBwdArgs& g, int 
           scores(1, 0, tmem + T_DP, &sl->dp_full);
         }
         for (int it = 0; it < n && ok; ++it) {
-          if (!(ok = wait(&sl->p_full, it, 78))) break;
+          if (!(ok = wait(&sl->p_full[0], it, 78))) break;
           apply(tmem + T_S, 1, it, tmem + T_ACC1, it == 0);
           if (it + 1 < n) {
             if (!(ok = stage_full(it + 1))) break;
@@ -416,7 +419,7 @@ __device__ __forceinline__ void attn_f32_tile(const SafMixedAttnBwdArgs& g, int 
           sum += s[j];
         }
         tmem_parts16(sat, s);
-        hand_over(&sl->p_full);
+        hand_over(&sl->p_full[it & 1]);
         l = l * f + sum;                                      // this thread's columns; added over the row at the end
         m = m_new;
         // the step before, from the other accumulator, under this one's product
@@ -449,7 +452,7 @@ __device__ __forceinline__ void attn_f32_tile(const SafMixedAttnBwdArgs& g, int 
         if constexpr (MODE == A_DKDV) {
           tmem_parts16(sat, s);
           if (it > 0) drain(T_ACC1, acc1, false);             // (S was issued after the dV of the step before)
-          hand_over(&sl->p_full);
+          hand_over(&sl->p_full[0]);
         }
         if (!(ok = wait(&sl->dp_full, it, 83))) break;
         float ds[16];
