@@ -94,7 +94,7 @@ struct BwdBars {
   uint64_t res_full;                    // the two resident tiles
   uint64_t ring_full[3], ring_empty[3];
   uint64_t v_full[3], v_empty[3];       // dQ kernel: the V ring (ring_* is its K ring)
-  uint64_t s_full[2], dp_full, p_full, ds_full, acc_full;
+  uint64_t s_full[2], dp_full, p_full[2], ds_full, acc_full;
   uint32_t tmem_base;
 };
 static_assert(sizeof(BwdBars) <= 256, "barrier block");
@@ -264,7 +264,8 @@ __device__ __forceinline__ void bwd_setup(BwdBars* bars, int tid, int warp) {
     mbar_init(&bars->s_full[0], 1);
     mbar_init(&bars->s_full[1], 1);
     mbar_init(&bars->dp_full, 1);
-    mbar_init(&bars->p_full, 8);              // one arrival per compute warp
+    mbar_init(&bars->p_full[0], 8);           // one arrival per compute warp
+    mbar_init(&bars->p_full[1], 8);
     mbar_init(&bars->ds_full, 8);
     mbar_init(&bars->acc_full, 1);
     fence_mbar_init();
@@ -335,7 +336,8 @@ flash_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_con
   bwd_setup<HD>(bars, tid, warp);
   const uint32_t tmem = bars->tmem_base;
   // At head_dim 64 tensor memory has room for a second buffer of scores: S^T of the next query tile is there before P^T and
-  // dS^T of this one are done
+  // dS^T of this one are done.  The compute warps may then hand over the next P^T before the issuer has seen this one, two phases
+  // ahead of a wait by parity: the tiles take turns on two barriers
   constexpr uint32_t COL_S = 0, COL_DP = 128, COL_DV = 256, COL_DK = 256 + HD, COL_S2 = 384;
   constexpr bool TWO_S = HD == 64;
 #ifdef SAF_BWD_TRACE
@@ -415,7 +417,7 @@ flash_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_con
       if (TWO_S && ok && n > 1) ok = issue_scores(1);
       for (int i = 0; i < n && ok; ++i) {
         const int s = i % C::NQ, sd = i % C::ND;
-        if (!mbar_wait(&bars->p_full, i & 1)) {
+        if (!(TWO_S ? mbar_wait(&bars->p_full[i & 1], (i >> 1) & 1) : mbar_wait(&bars->p_full[0], i & 1))) {
           dev_set_error(p.status, SAF_DEV_TIMEOUT_MMA, 43);
           break;
         }
@@ -526,7 +528,7 @@ flash_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_con
           tmem_st16(tS + half * 32 + ch * 16, pk);
         }
       }
-      operand_written(&bars->p_full, tid);
+      operand_written(&bars->p_full[TWO_S ? i & 1 : 0], tid);
       TRACE(0, 1, i);   // P^T handed over
       WTRACE(0, i);
       // ---- dS^T

@@ -41,6 +41,35 @@ def fp32_dq(two):                          # A_DQ: S one step ahead, in the othe
     return issuer, warp + [("wait", ("acc", 0), 0)]
 
 
+def bwd_dkdv(scores, two):                 # flash_bwd_sm100.cu: `scores` buffers of S, as many query tiles ahead
+    s = lambda i: (("s", i % scores), i // scores)
+    p = lambda i: (("p", i & 1), i >> 1) if two and scores == 2 else (("p", 0), i)
+    issuer, warp = [("issue", [s(0)[0]]), ("issue", [("dp", 0)])] + ([("issue", [s(1)[0]])] if scores == 2 else []), []
+    for i in range(N):
+        issuer += [("wait", *p(i)), ("issue", [])] + ([("issue", [s(i + scores)[0]])] if i + scores < N else [])
+        issuer += [("wait", ("ds", 0), i), ("issue", [])] + ([("issue", [("dp", 0)])] if i + 1 < N else [])
+        # (row vectors; columns read before they are written over)
+        warp += [("meet",), ("wait", *s(i)), ("meet",), ("arrive", p(i)[0]), ("wait", ("dp", 0), i), ("meet",), ("arrive", ("ds", 0))]
+    return issuer + [("issue", [("acc", 0)])], warp + [("wait", ("acc", 0), 0)]
+
+
+def bwd_dkdv_64(two):
+    return bwd_dkdv(2, two)
+
+
+def bwd_dkdv_128(two):
+    return bwd_dkdv(1, two)
+
+
+def bwd_dq(two):                           # S up to two key tiles ahead, dP one
+    issuer, warp = [("issue", [("s", 0)]), ("issue", [("dp", 0)]), ("issue", [("s", 1)])], []
+    for i in range(N):
+        issuer += [("wait", ("ds", 0), i), ("issue", [])] + ([("issue", [("dp", 0)])] if i + 1 < N else [])
+        issuer += [("issue", [("s", i & 1)])] if i + 2 < N else []
+        warp += [("wait", ("s", i & 1), i >> 1), ("wait", ("dp", 0), i), ("meet",), ("arrive", ("ds", 0))]
+    return issuer + [("issue", [("acc", 0)])], warp + [("wait", ("acc", 0), 0)]
+
+
 def stuck(program, two):
     """A reachable state in which somebody waits for a phase that has gone by, or passes one that has not come."""
     issuer, warp = program(two)
@@ -76,11 +105,11 @@ def stuck(program, two):
     return None
 
 
-@pytest.mark.parametrize("program", [fp32_forward, fp32_dkdv, fp32_dq])
+@pytest.mark.parametrize("program", [fp32_forward, fp32_dkdv, fp32_dq, bwd_dkdv_64, bwd_dkdv_128, bwd_dq])
 def test_no_wait_is_overtaken(program):
     assert stuck(program, True) is None
 
 
-@pytest.mark.parametrize("program", [fp32_forward])
+@pytest.mark.parametrize("program", [fp32_forward, bwd_dkdv_64])
 def test_one_barrier_for_p_is_overtaken_where_scores_run_ahead(program):
     assert stuck(program, False) is not None
