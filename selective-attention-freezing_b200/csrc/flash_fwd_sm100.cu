@@ -94,7 +94,7 @@ struct Cfg {
 // ring depth of the tensor-core scan when it runs in a scan slot of these launches: what their shared memory holds
 constexpr int SCAN_ROLE_STAGES = 8;
 // shortest sequence whose structured heads take the tensor-core scan: below it the register scan, one 64-column slice after
-// the other, is as fast
+// the other, is as fast.  It also runs behind the tensor-core scan where that has met an infinity or a NaN
 template <int HD>
 constexpr int SCAN_MMA_MIN_T = HD == 64 ? 4 * MB : 1;
 static_assert(ms_smem_bytes(SCAN_ROLE_STAGES) <= Cfg<64>::SMEM_BYTES && ms_smem_bytes(SCAN_ROLE_STAGES) <= Cfg<64>::SMEM_PERSIST &&
@@ -180,6 +180,12 @@ __device__ __forceinline__ void load_tile(uint8_t* dst, const CUtensorMap* m, ui
   for (int hh = 0; hh < HD / 64; ++hh) tma_load_4d(dst + hh * 16384, m, bar, hh * 64, row, head, b);
 }
 
+// the whole sequence of a structured head through registers, by the first SCAN_NT threads (a function of its own: inside the
+// kernels its registers spilled, and theirs with them)
+__device__ __noinline__ void register_scan(const ScanArgs& a, int b, int h) {
+  for (int col0 = 0; col0 < a.HD; col0 += SCAN_COLS) sink_decay_scan_cta<__nv_bfloat16, false>(a, b, h, col0);
+}
+
 template <int HD>
 __global__ void __launch_bounds__(FLASH_THREADS, 1)
 flash_fwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant__ CUtensorMap mapK,
@@ -204,12 +210,10 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant
           mp.chunk = (p.T + MB - 1) / MB * MB;
           mp.use_stash = 0;
           mp.status = p.status;
-          sink_decay_apply_mma_cta<SCAN_ROLE_STAGES>(mapV, mapO, mp, b, h, 0, 0, HD / 64, scan_smem_raw);
-          return;
+          if (sink_decay_apply_mma_cta<SCAN_ROLE_STAGES>(mapV, mapO, mp, b, h, 0, 0, HD / 64, scan_smem_raw)) return;
         }
       }
-      if (threadIdx.x < SCAN_NT)
-        for (int col0 = 0; col0 < HD; col0 += SCAN_COLS) sink_decay_scan_cta<__nv_bfloat16, false>(p.scan, b, h, col0);
+      if (threadIdx.x < SCAN_NT) register_scan(p.scan, b, h);
     }
     return;
   }
@@ -765,12 +769,10 @@ flash_fwd_persistent_kernel(const __grid_constant__ CUtensorMap mapQ, const __gr
           mp.chunk = (p.T + MB - 1) / MB * MB;
           mp.use_stash = 0;
           mp.status = p.status;
-          sink_decay_apply_mma_cta<SCAN_ROLE_STAGES>(mapV, mapO, mp, b, h, 0, 0, HD / 64, scan_smem_raw);
-          return;
+          if (sink_decay_apply_mma_cta<SCAN_ROLE_STAGES>(mapV, mapO, mp, b, h, 0, 0, HD / 64, scan_smem_raw)) return;
         }
       }
-      if (threadIdx.x < SCAN_NT)
-        for (int col0 = 0; col0 < HD; col0 += SCAN_COLS) sink_decay_scan_cta<__nv_bfloat16, false>(p.scan, b, h, col0);
+      if (threadIdx.x < SCAN_NT) register_scan(p.scan, b, h);
     }
     return;
   }

@@ -21,9 +21,11 @@ struct MsBars {
   uint32_t tmem_base;
   alignas(16) float carry[4][64];      // carry[n & 3]: the state block n inherits
   alignas(16) float av0[2][64];        // sink term a * v_0 of each column slice
+  alignas(16) float last[2][64];       // the state at the end of each column slice
 };
 // dynamic shared memory of a CTA with a ring of `stages` V tiles
-constexpr int ms_smem_bytes(int stages) { return 1024 + (stages + MS_OUT) * MS_TILE + 2048; }
+constexpr int ms_smem_bytes(int stages) { return 1024 + (stages + MS_OUT) * MS_TILE + 2560; }
+static_assert(sizeof(MsBars) <= 2560, "barrier block");
 static_assert(ms_smem_bytes(MS_MAX_STAGES) <= 227 * 1024, "shared memory limit");
 
 #ifdef SAF_SCAN_TRACE
@@ -45,8 +47,11 @@ struct MsParams {
 // through the same rings: the running block index goes on, the carry restarts at zero at the slice boundary.  Every thread of the CTA must call it (it holds CTA-wide barriers); the first ten warps work, further warps only
 // take part in those barriers.  STAGES V tiles are in flight; `smem_raw` is the CTA's dynamic shared memory, at least
 // ms_smem_bytes(STAGES) bytes.
+// The operand's upper triangle is a product with zero, so an infinity or a NaN in row j of V reaches the rows of its block
+// before j, which must not see it.  It reaches the state at the end of the rows as well: the result, the same for every thread, is
+// false then, and the caller has the register scan write the rows again.
 template <int STAGES>
-__device__ __forceinline__ void sink_decay_apply_mma_cta(const CUtensorMap& mapV, const CUtensorMap& mapY, const MsParams& p,
+__device__ __forceinline__ bool sink_decay_apply_mma_cta(const CUtensorMap& mapV, const CUtensorMap& mapY, const MsParams& p,
                                                          int b, int h, int chunk_idx, int slice, int n_slices, uint8_t* smem_raw) {
   static_assert(STAGES >= 2 && STAGES <= MS_MAX_STAGES, "ring depth");
   constexpr int MS_STAGES = STAGES;
@@ -242,6 +247,13 @@ __device__ __forceinline__ void sink_decay_apply_mma_cta(const CUtensorMap& mapV
           for (int q = 0; q < 8; ++q)
             n4[8 + q] = make_uint4(s1[q * 4] & keep, s1[q * 4 + 1] & keep, s1[q * 4 + 2] & keep, s1[q * 4 + 3] & keep);
           mbar_arrive(&bars->carry_ready[(n + 1) & 3]);
+          if (keep == 0u) {
+            uint4* l4 = reinterpret_cast<uint4*>(bars->last[sl]);
+#pragma unroll
+            for (int q = 0; q < 8; ++q) l4[q] = make_uint4(s0[q * 4], s0[q * 4 + 1], s0[q * 4 + 2], s0[q * 4 + 3]);
+#pragma unroll
+            for (int q = 0; q < 8; ++q) l4[8 + q] = make_uint4(s1[q * 4], s1[q * 4 + 1], s1[q * 4 + 2], s1[q * 4 + 3]);
+          }
           STRACE(7, n);
         }
       }
@@ -286,7 +298,9 @@ __device__ __forceinline__ void sink_decay_apply_mma_cta(const CUtensorMap& mapV
   }
   tc_fence_before();
   __syncthreads();
+  const bool finite = __syncthreads_and(tid >= 64 * n_slices || fabsf(bars->last[0][tid]) < INFINITY);
   if (warp == 1) tmem_dealloc(tmem, 512);
+  return finite;
 }
 
 
