@@ -379,7 +379,8 @@ __device__ __forceinline__ void attn_f32_tile(const SafMixedAttnBwdArgs& g, int 
       if (lane == 0) mbar_arrive(bar);
     };
     auto wait = [&](uint64_t* bar, int phase, int site) {
-      const bool in_time = mbar_wait(bar, phase & 1);
+      // (a lane's limit is its own, and tensor memory is read by whole warps: they leave together)
+      const bool in_time = __all_sync(0xffffffffu, mbar_wait(bar, phase & 1));
       if (!in_time) dev_set_error(a.status, SAF_DEV_TIMEOUT_SOFTMAX, site);
       tc_fence_after();
       return in_time;
@@ -388,7 +389,7 @@ __device__ __forceinline__ void attn_f32_tile(const SafMixedAttnBwdArgs& g, int 
     for (int it = 0; it < n; ++it) {
       const int xb = (x0 + it) * AX + col;                    // this thread's first streamed row
       const uint32_t sat = lanes + (MODE == A_FWD ? (it & 1) * 128 : (MODE == A_DQ && (it & 1) ? T_ACC2 : T_S));
-      ok = MODE == A_DKDV ? wait(&sl->s_full[0], it, 79) : wait(&sl->s_full[it & 1], it >> 1, 79);
+      ok = ok && (MODE == A_DKDV ? wait(&sl->s_full[0], it, 79) : wait(&sl->s_full[it & 1], it >> 1, 79));
       if (MODE != A_FWD && !ok) break;                        // (the forward leaves at the vote, where the row's threads meet)
       const bool edge = MODE == A_DKDV ? xb < r0 + AR || xb + 16 > T : xb + 15 > r0;       // some scores may be masked
       float s[16];

@@ -277,7 +277,7 @@ __global__ void __launch_bounds__(STHREADS, 1) linear_f32_split_kernel(const __g
     bool ok = true;
     for (int h = 0; h < 2 * (kt1 - kt0); ++h) {
       const int b = h & 1;
-      if (!(ok = mbar_wait(&sl->acc_full[b], (h >> 1) & 1))) {
+      if (!(ok = __all_sync(0xffffffffu, mbar_wait(&sl->acc_full[b], (h >> 1) & 1)))) {   // (whole warps read tensor memory)
         dev_set_error(p.status, SAF_DEV_TIMEOUT_EPI, 73);
         break;
       }
