@@ -49,7 +49,7 @@ def test_what_is_not_finite_stays_behind_its_row(hd, T, what, where):
         want[1, 1, :, hd - 5] = True            # the sink
     assert torch.equal(odd, want)
     assert torch.equal(y[0], clean[0]) and torch.equal(y[1, 0], clean[1, 0])
-    # the head's other values come from the scan in registers
+    # the head's other values come from the scan in registers: fp32, then half an ulp of bf16, 2^-8
     fin = ~odd[1, 1]
     assert ((y[1, 1].double() - pattern(T)[1] @ values(hd, T)[1, 3].double()).abs()[fin]
-            <= 1.01 * 2.0 ** -9 * (pattern(T)[1] @ v[1, 3].abs().nan_to_num(0, 0, 0).double())[fin]).all()
+            <= 1.01 * 2.0 ** -8 * (pattern(T)[1] @ v[1, 3].abs().nan_to_num(0, 0, 0).double())[fin]).all()
