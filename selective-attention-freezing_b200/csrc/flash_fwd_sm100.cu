@@ -186,26 +186,6 @@ __device__ __forceinline__ void load_tile(uint8_t* dst, const CUtensorMap* m, ui
 __device__ __noinline__ void scan_again(const ScanArgs& a, int b, int h) {
   for (int col0 = 0; col0 < a.HD; col0 += SCAN_COLS) sink_decay_scan_cta<__nv_bfloat16, false>(a, b, h, col0);
 }
-// The whole sequence of a structured head, by all threads of the CTA.  T >= SCAN_MMA_MIN_T: 128-row Toeplitz products on the
-// tensor core, one 64-column slice after the other (about a third of the time of the register scan, so the SM joins the live tiles
-// that much earlier); head width 96 as well, whose second slice the tensor maps clip.
-template <int HD>
-__device__ __forceinline__ void structured_head(const CUtensorMap& mapV, const CUtensorMap& mapO, const FlashParams& p, int b, int h) {
-  if constexpr (SCAN_MMA_MIN_T<HD> > 1) {
-    if (p.T < SCAN_MMA_MIN_T<HD>) {
-      if (threadIdx.x < SCAN_NT) sink_decay_scan_cta<__nv_bfloat16, false>(p.scan, b, h, 0);
-      return;
-    }
-  }
-  extern __shared__ uint8_t scan_smem_raw[];
-  MsParams mp;
-  mp.a = p.scan;
-  mp.chunk = (p.T + MB - 1) / MB * MB;
-  mp.use_stash = 0;
-  mp.status = p.status;
-  if (!sink_decay_apply_mma_cta<SCAN_ROLE_STAGES>(mapV, mapO, mp, b, h, 0, 0, HD / 64, scan_smem_raw) && threadIdx.x < SCAN_NT)
-    scan_again(p.scan, b, h);
-}
 
 template <int HD>
 __global__ void __launch_bounds__(FLASH_THREADS, 1)
@@ -219,7 +199,27 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant
   if ((int)blockIdx.x < bh_count) {
     const int b = blockIdx.x / p.H, h = blockIdx.x % p.H;
     const int state = p.force_state >= 0 ? p.force_state : p.frozen[h];
-    if (state == SAF_SINK_DECAY && p.has_scan) structured_head<HD>(mapV, mapO, p, b, h);
+    if (state == SAF_SINK_DECAY && p.has_scan) {
+      // the whole sequence as 128-row Toeplitz products on the tensor core, one 64-column slice after the other (about a third
+      // of the time of the register scan, so the SM joins the live tiles that much earlier); head width 96 as well, whose second
+      // slice the tensor maps clip.  (Both scans in place: in a function that is inlined here the launch took 30 us instead of
+      // 28 at T = 1024, B = 8, 12 heads x 64.)
+      if (p.T >= SCAN_MMA_MIN_T<HD>) {
+        extern __shared__ uint8_t scan_smem_raw[];
+        MsParams mp;
+        mp.a = p.scan;
+        mp.chunk = (p.T + MB - 1) / MB * MB;
+        mp.use_stash = 0;
+        mp.status = p.status;
+        if (!sink_decay_apply_mma_cta<SCAN_ROLE_STAGES>(mapV, mapO, mp, b, h, 0, 0, HD / 64, scan_smem_raw) &&
+            threadIdx.x < SCAN_NT)
+          scan_again(p.scan, b, h);
+        return;
+      }
+      if constexpr (SCAN_MMA_MIN_T<HD> > 1) {
+        if (threadIdx.x < SCAN_NT) sink_decay_scan_cta<__nv_bfloat16, false>(p.scan, b, h, 0);
+      }
+    }
     return;
   }
   // ---- dense-stored frozen heads: TMA-staged lower-triangular GEMM, pattern tiles shared by batch rows ---
@@ -762,7 +762,27 @@ flash_fwd_persistent_kernel(const __grid_constant__ CUtensorMap mapQ, const __gr
     pdl_trigger();
     const int b = blockIdx.x / p.H, h = blockIdx.x % p.H;
     const int state = p.force_state >= 0 ? p.force_state : p.frozen[h];
-    if (state == SAF_SINK_DECAY && p.has_scan) structured_head<HD>(mapV, mapO, p, b, h);
+    if (state == SAF_SINK_DECAY && p.has_scan) {
+      // the whole sequence as 128-row Toeplitz products on the tensor core, one 64-column slice after the other (about a third
+      // of the time of the register scan, so the SM joins the live tiles that much earlier); head width 96 as well, whose second
+      // slice the tensor maps clip.  (Both scans in place: in a function that is inlined here the launch took 30 us instead of
+      // 28 at T = 1024, B = 8, 12 heads x 64.)
+      if (p.T >= SCAN_MMA_MIN_T<HD>) {
+        extern __shared__ uint8_t scan_smem_raw[];
+        MsParams mp;
+        mp.a = p.scan;
+        mp.chunk = (p.T + MB - 1) / MB * MB;
+        mp.use_stash = 0;
+        mp.status = p.status;
+        if (!sink_decay_apply_mma_cta<SCAN_ROLE_STAGES>(mapV, mapO, mp, b, h, 0, 0, HD / 64, scan_smem_raw) &&
+            threadIdx.x < SCAN_NT)
+          scan_again(p.scan, b, h);
+        return;
+      }
+      if constexpr (SCAN_MMA_MIN_T<HD> > 1) {
+        if (threadIdx.x < SCAN_NT) sink_decay_scan_cta<__nv_bfloat16, false>(p.scan, b, h, 0);
+      }
+    }
     return;
   }
   if ((int)blockIdx.x < bh_count + p.dense_slots) {   // dense-pattern role
