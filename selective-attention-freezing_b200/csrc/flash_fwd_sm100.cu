@@ -211,7 +211,7 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant
         mp.chunk = (p.T + MB - 1) / MB * MB;
         mp.use_stash = 0;
         mp.status = p.status;
-        if (!sink_decay_apply_mma_cta<SCAN_ROLE_STAGES>(mapV, mapO, mp, b, h, 0, 0, HD / 64, scan_smem_raw) &&
+        if (!sink_decay_apply_mma_cta<SCAN_ROLE_STAGES, HD == 64 ? 2 : 3>(mapV, mapO, mp, b, h, 0, 0, HD / 64, scan_smem_raw) &&
             threadIdx.x < SCAN_NT)
           scan_again(p.scan, b, h);
         return;
@@ -774,7 +774,7 @@ flash_fwd_persistent_kernel(const __grid_constant__ CUtensorMap mapQ, const __gr
         mp.chunk = (p.T + MB - 1) / MB * MB;
         mp.use_stash = 0;
         mp.status = p.status;
-        if (!sink_decay_apply_mma_cta<SCAN_ROLE_STAGES>(mapV, mapO, mp, b, h, 0, 0, HD / 64, scan_smem_raw) &&
+        if (!sink_decay_apply_mma_cta<SCAN_ROLE_STAGES, HD == 64 ? 2 : 3>(mapV, mapO, mp, b, h, 0, 0, HD / 64, scan_smem_raw) &&
             threadIdx.x < SCAN_NT)
           scan_again(p.scan, b, h);
         return;

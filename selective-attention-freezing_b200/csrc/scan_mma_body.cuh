@@ -2,6 +2,8 @@
 // (scan_mma_sm100.cu, which explains the method) and by the mixed-attention launches, whose leading CTAs run it for the
 // structured heads of a call while the other CTAs work on the live heads.
 #pragma once
+#include <type_traits>
+
 #include "saf_internal.h"
 #include "scan_body.cuh"
 #include "sm100_prims.cuh"
@@ -14,7 +16,7 @@ constexpr int MS_TILE = MB * 64 * 2;    // 16 KB: one V tile, one output tile
 constexpr int MS_THREADS = 320;          // TMA warp, MMA warp, two epilogue warpgroups
 constexpr int MS_ACC = 4;               // TMEM accumulators
 constexpr int MS_OUT = 2;               // staging tiles: one per epilogue warpgroup
-constexpr int MS_TL = MS_ACC * 64;      // TMEM column of the Toeplitz operand: bf16 head (64 columns), remainder (64)
+constexpr int MS_TL = MS_ACC * 64;      // TMEM column of the Toeplitz operand: its two or three bf16 parts, 64 columns each
 
 struct MsBars {
   uint64_t full[MS_MAX_STAGES], empty[MS_MAX_STAGES], acc_full[MS_ACC], acc_empty[MS_ACC], carry_ready[4], l_ready;
@@ -50,7 +52,10 @@ struct MsParams {
 // The operand's upper triangle is a product with zero, so an infinity or a NaN in row j of V reaches the rows of its block
 // before j, which must not see it.  It reaches the state at the end of the rows as well: the result, the same for every thread, is
 // false then, and the caller has the register scan write the rows again.
-template <int STAGES>
+// PARTS of the operand: two hold the fp32 weights to 2^-17; three hold them as they are, for calls whose other way is the
+// register scan (their products are added smallest first: results further than their rounding to bf16 from 64 bits are then off by
+// less than 3 * 2^-24 of the row's terms, where two parts are off by up to 30 and the register scan by up to 7).
+template <int STAGES, int PARTS>
 __device__ __forceinline__ bool sink_decay_apply_mma_cta(const CUtensorMap& mapV, const CUtensorMap& mapY, const MsParams& p,
                                                          int b, int h, int chunk_idx, int slice, int n_slices, uint8_t* smem_raw) {
   static_assert(STAGES >= 2 && STAGES <= MS_MAX_STAGES, "ring depth");
@@ -131,11 +136,11 @@ __device__ __forceinline__ bool sink_decay_apply_mma_cta(const CUtensorMap& mapV
       if (leader) {
         STRACE(2, n);
 #pragma unroll
-        for (int part = 0; part < 2; ++part)
+        for (int u = 0; u < PARTS; ++u)
 #pragma unroll
           for (int ks = 0; ks < MB / 16; ++ks)            // 16 rows of V = 8 TMEM columns of packed bf16 pairs
-            umma_ts(d, tmem + MS_TL + part * 64 + ks * 8, umma_smem_desc_sw128(va + ks * 2048, 16384, 1024), idesc,
-                    (part | ks) != 0);
+            umma_ts(d, tmem + MS_TL + (PARTS == 3 ? 2 - u : u) * 64 + ks * 8, umma_smem_desc_sw128(va + ks * 2048, 16384, 1024), idesc,
+                    (u | ks) != 0);
         umma_commit(&bars->empty[s]);
         umma_commit(&bars->acc_full[buf]);
         STRACE(3, n);
@@ -163,8 +168,8 @@ __device__ __forceinline__ bool sink_decay_apply_mma_cta(const CUtensorMap& mapV
       if (col0 + sl * SCAN_COLS + et < a.HD) v_first = __bfloat162float(*v0);      // (a width of 96 ends inside a slice)
     }
     // Toeplitz operand in TMEM, row `lrow`, column k = the bf16 pair (L[2k], L[2k+1]): its bf16 head from warpgroup 0
-    // and the bf16 remainder from warpgroup 1
-    {
+    // and the bf16 remainder from warpgroup 1, or its three parts, the first and the last from warpgroup 0
+    if constexpr (PARTS == 2) {
       uint32_t w0[32], w1[32];
       float val = 1.f;                                      // r^(lrow - j), from the diagonal leftwards
 #pragma unroll
@@ -185,9 +190,45 @@ __device__ __forceinline__ bool sink_decay_apply_mma_cta(const CUtensorMap& mapV
       }
       tmem_st32(tlane + MS_TL + wg * 64, w0);
       tmem_st32(tlane + MS_TL + wg * 64 + 32, w1);
-      tmem_st_wait();
-      tc_fence_before();
+    } else {
+      auto build = [&](auto part_c) {
+        constexpr int PART = decltype(part_c)::value;
+        float val = 1.f;                                    // r^(lrow - j), from the diagonal leftwards
+#pragma unroll
+        for (int half = 1; half >= 0; --half) {
+          uint32_t w[32];
+#pragma unroll
+          for (int k = 31; k >= 0; --k) {
+            const int j = 64 * half + 2 * k;
+            float x0 = 0.f, x1 = 0.f;
+            if (j + 1 <= lrow) {
+              x1 = val;
+              val *= r;
+            }
+            if (j <= lrow) {
+              x0 = val;
+              val *= r;
+            }
+            w[k] = pack_bf16(x0, x1);
+#pragma unroll
+            for (int q = 0; q < PART; ++q) {
+              x0 -= __uint_as_float(w[k] << 16);
+              x1 -= __uint_as_float(w[k] & 0xffff0000u);
+              w[k] = pack_bf16(x0, x1);
+            }
+          }
+          tmem_st32(tlane + MS_TL + PART * 64 + half * 32, w);
+        }
+      };
+      if (wg == 0) {
+        build(std::integral_constant<int, 0>{});
+        build(std::integral_constant<int, 2>{});
+      } else {
+        build(std::integral_constant<int, 1>{});
+      }
     }
+    tmem_st_wait();
+    tc_fence_before();
     if (et < 64 * (wg == 0 ? 1 : n_slices - 1)) {
       if (wg == 0) bars->carry[0][et] = carry_in;
       bars->av0[wg][et] = alpha * v_first;

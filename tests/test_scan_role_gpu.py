@@ -8,7 +8,7 @@ from oracle import saf_oracle as O
 pytestmark = pytest.mark.gpu
 
 SIZES = [(hd, T) for hd in (96, 128) for T in (1, 65, 127, 128, 129, 300, 700)] + [(64, 511), (64, 512), (64, 641)]
-A, R = (0.3, 0.6), (0.98, 0.5)
+A, R = (0.3, 0.6), (0.9, 0.5)
 
 
 def mixed(hd, T, v):
@@ -30,6 +30,18 @@ def values(hd, T):
 
 def pattern(T):
     return O.sink_decay_pattern(torch.tensor(A).double(), torch.tensor(R).double(), T).cuda()
+
+
+@pytest.mark.parametrize("hd,T", SIZES)
+def test_rows_are_64_bit_rows_rounded_once(hd, T):
+    """Each result is the bf16 of something close to the row in 64 bits."""
+    v = values(hd, T)
+    y, p, vd = mixed(hd, T, v), pattern(T), v[:, [0, 3]].double()
+    ref, size = p @ vd, p @ vd.abs()
+    # weights as in fp32 (width 64: to 2^-17); the eight instructions of a block's leading part each truncate their sum by up to
+    # 2^-23 of it, 2^-24 on average
+    off = (128 if hd == 64 else 8) * 2.0 ** -24 * size
+    assert ((ref - off).bfloat16() <= y).all() and (y <= (ref + off).bfloat16()).all()
 
 
 @pytest.mark.parametrize("where", [0, 70, 128, 290, 600])
