@@ -706,11 +706,14 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant
 // of tile 1 last, so every index of the running counter is a real tile and barrier phases follow from it.
 // s_full is kept per query tile: a warpgroup whose tile an item does not have (the last row pair of an odd number of row
 // tiles) is handed the next item while the other one still works, more than one phase of a shared barrier ahead of it, and
-// a wait by parity cannot tell that phase from the one before.
+// a wait by parity cannot tell that phase from the one before.  A tile's score products go through its four barriers in turn (at
+// most three of them are out), so that barrier and phase follow from the warpgroup's own count, and its buffer from step
+// to step: the loop is bound by its instructions, and with a bit per buffer and a division in it the launch took 1547 us where
+// it takes 1511 (9 live heads x 64, T = 16384, B = 4).
 struct PersistBars {
   uint64_t q_full[2], q_free[2];
   uint64_t k_full[4], k_empty[4], v_full[4], v_empty[4];
-  uint64_t s_full[2][3], p_full[3], buf_free[3];
+  uint64_t s_full[2][4], p_full[3], buf_free[3];
   uint64_t o_free[2];
   uint64_t w_full[2], w_empty[2];
   volatile int32_t work[2];
@@ -817,9 +820,8 @@ flash_fwd_persistent_kernel(const __grid_constant__ CUtensorMap mapQ, const __gr
       mbar_init(&bars->v_full[s], 1);
       mbar_init(&bars->v_empty[s], 1);
     }
+    for (int i = 0; i < 8; ++i) mbar_init(&bars->s_full[i >> 2][i & 3], 1);
     for (int i = 0; i < 3; ++i) {
-      mbar_init(&bars->s_full[0][i], 1);
-      mbar_init(&bars->s_full[1][i], 1);
       mbar_init(&bars->p_full[i], 128);
       mbar_init(&bars->buf_free[i], 1);
     }
@@ -927,7 +929,7 @@ flash_fwd_persistent_kernel(const __grid_constant__ CUtensorMap mapQ, const __gr
       // ---------------------------------------------------------- score MMA issuer
       const uint32_t idesc_s = umma_idesc_bf16(FM, FN, 0, 0);
       const uint32_t qaddr0 = smem_u32(sQ), kbase = smem_u32(sK);
-      uint32_t gs = 0, kc = 0, use_q[2] = {0, 0};
+      uint32_t gs = 0, kc = 0, use_q[2] = {0, 0}, use_s[2] = {0, 0};
       bool ok = true;
       for (int n = 0; ok; ++n) {
         const int it = fetch(n, leader);
@@ -977,13 +979,15 @@ flash_fwd_persistent_kernel(const __grid_constant__ CUtensorMap mapQ, const __gr
               const uint32_t off = (ks >> 2) * 16384 + (ks & 3) * 32;
               umma_ss(d, umma_desc_advance(dq, off), umma_desc_advance(dk, off), idesc_s, ks > 0);
             }
-            umma_commit(&bars->s_full[t][buf]);
+            umma_commit(&bars->s_full[t][(use_s[t] + j) & 3]);
             if (t == 1 || !g.act1) umma_commit(&bars->k_empty[ks_]);   // last reader of K_j
             if (!C::STAGE_IN_Q && j == (t ? g.nkv1 : g.nkv0) - 1) umma_commit(&bars->q_free[t]);   // last reader of Q_t
           }
           __syncwarp();
         }
         kc += g.nkv;
+        use_s[0] += g.nkv0;
+        use_s[1] += g.nkv1;
         ++use_q[0];
         if (g.act1) ++use_q[1];
       }
@@ -1053,7 +1057,7 @@ flash_fwd_persistent_kernel(const __grid_constant__ CUtensorMap mapQ, const __gr
     const uint32_t tO = tmem + lane_base + C::O_COL + t * HD;
     const float sc = p.scale_log2;
     const bool warp_lead = (tid & 31) == 0;
-    uint32_t g_base = 0, s_phase = 0;      // s_phase: one bit per score buffer, the parity of this tile's next use of it
+    uint32_t g_base = 0, n_s = 0;          // n_s: score tiles this warpgroup has taken
     bool ok = true;
     for (int n = 0; ok; ++n) {
       const int it = fetch(n, warp_lead);
@@ -1066,16 +1070,17 @@ flash_fwd_persistent_kernel(const __grid_constant__ CUtensorMap mapQ, const __gr
       if (nk > 0) {
         float m_ref = -INFINITY, l = 0.f;
         uint32_t pbuf = 0, pph = 0;
+        // buffer and phase of the running number of this tile's scores, advanced from step to step
+        const uint32_t step = g.act1 ? 2 : 1, gi = g_base + (g.act1 ? t : 0);
+        uint32_t buf = gi % C::NBUF, bph = (gi / C::NBUF) & 1;
         for (int j = 0; j < nk; ++j) {
-          const uint32_t gi = g_base + (g.act1 ? ((t == 1 && j == g.nkv0) ? 2 * g.nkv0 : 2 * j + t) : j);
-          const uint32_t buf = gi % C::NBUF, bph = (gi / C::NBUF) & 1;
           const uint32_t tS = tmem + lane_base + buf * FN;
-          if (!mbar_wait(&bars->s_full[t][buf], (s_phase >> buf) & 1)) {
+          if (!mbar_wait(&bars->s_full[t][n_s & 3], (n_s >> 2) & 1)) {
             dev_set_error(p.status, SAF_DEV_TIMEOUT_SOFTMAX, 54);
             ok = false;
             break;
           }
-          s_phase ^= 1u << buf;
+          ++n_s;
           tc_fence_after();
           uint32_t s[4][32];
 #pragma unroll
@@ -1153,6 +1158,11 @@ flash_fwd_persistent_kernel(const __grid_constant__ CUtensorMap mapQ, const __gr
           mbar_arrive(&bars->p_full[buf]);
           pbuf = buf;
           pph = bph;
+          buf += t && j + 2 == nk ? 1 : step;                  // (the extra diagonal step of tile 1 follows at once)
+          if (buf >= (uint32_t)C::NBUF) {
+            buf -= C::NBUF;
+            bph ^= 1;
+          }
         }
         if (!ok) break;
         // ---- epilogue of tile t: O / l -> bf16 -> the tile's own Q buffer -> TMA store
