@@ -1,5 +1,5 @@
-// fp32 indexed linear on the tensor cores: every operand element is split into three bf16 parts, x = x0 + x1 + x2 exactly
-// (3 x 8 significant bits), and the product is the sum of the six part products that reach 2^-24 of it.
+// fp32 indexed linear on the tensor cores: every operand element is split into three bf16 parts, x = x0 + x1 + x2
+// (split_bf16.cuh), and the product is the sum of the six part products that reach 2^-24 of it.
 //
 // Precision: the tensor core adds into its fp32 accumulator by truncation, and an error of one sign grows with the length
 // of the chain.  So the leading product x0 y0 only runs over 32 of K (two instructions) before the epilogue warps take
@@ -21,8 +21,10 @@
 // distributed shared memory, in the order of the parts (no atomics, no workspace).  The forward is never split: an output
 // then has the same bits whatever other rows and features the call has.
 //
-// What the parts cannot carry shows in the results (infinities, NaN, magnitudes that round to infinity as bf16; values so
-// small that the third part is lost among the subnormals): a tile with such results is computed again with fp32 FMAs.
+// What the parts cannot carry shows in the results: they are not finite, or smaller than what may have been lost of them, which
+// follows from the largest operands (split_bf16.cuh).  A tile with such a result, by its largest operands, is computed again with
+// fp32 FMAs, and the results that are such by the largest elements of their own row and column are taken from there: what
+// a result is depends on these alone.
 #include <algorithm>
 #include <type_traits>
 
@@ -48,6 +50,7 @@ struct SplitShape {
   struct Ctrl {
     uint64_t full[STAGES], empty[STAGES], acc_full[2], acc_empty[2];
     uint32_t tmem_base;
+    uint32_t top, top_j[BN];                   // largest operand of the tile; in the repeat, of a column (fp32 bits)
     const float* brow[BN];                     // forward: the weight rows of the tile's columns, null beyond the last
   };
   static constexpr int SMEM = 1024 + STAGES * STAGE + (int)sizeof(Ctrl);
@@ -97,6 +100,8 @@ __global__ void __launch_bounds__(STHREADS, 1) linear_f32_split_kernel(const __g
     }
     fence_mbar_init();
   }
+  if (tid == 0) sl->top = 0;
+  if (tid < BN) sl->top_j[tid] = 0;
   if constexpr (B_KC) {
     if (tid < BN) sl->brow[tid] = j0 + tid < J ? welem<float>(ws, tb, j0 + tid, p.slab, 0) : nullptr;
   }
@@ -112,7 +117,8 @@ __global__ void __launch_bounds__(STHREADS, 1) linear_f32_split_kernel(const __g
   const uint32_t tmem = sl->tmem_base;
 
   if (warp < SPROD / 32) {
-    asm volatile("setmaxnreg.dec.sync.aligned.u32 64;");
+    // (512 x 64 + 256 x 104 + 128 x 40 registers = 896 x 72; the narrow tile's epilogue holds half as many sums)
+    if constexpr (BN == 128) asm volatile("setmaxnreg.dec.sync.aligned.u32 64;");
     // 16 bytes of a row, 32 rows apart in every block of 64 x 64 elements
     const int row = tid >> 4, c4 = (tid & 15) * 4;
     const uint32_t off = row * 128 + ((((tid & 15) >> 1) ^ (row & 7)) << 4) + (tid & 1) * 8;
@@ -174,6 +180,7 @@ __global__ void __launch_bounds__(STHREADS, 1) linear_f32_split_kernel(const __g
       if (whole && kt * SK + SK <= K) load_as(std::true_type{}, op, kt);
       else load_as(std::false_type{}, op, kt);
     };
+    float top = 0.f;                           // largest operand
     if (kt0 < kt1) {
       load(0, kt0);
       load(1, kt0);
@@ -193,13 +200,19 @@ __global__ void __launch_bounds__(STHREADS, 1) linear_f32_split_kernel(const __g
 #pragma unroll
         for (int b = 0; b < (o ? S::NBJ : 2); ++b)
 #pragma unroll
-          for (int q = 0; q < 2; ++q) split_store(st + o * 3 * S::A_PART + b * SBLK + q * 4096, PART[o], v[2 * o + b][q]);
+          for (int q = 0; q < 2; ++q) {
+            split_store(st + o * 3 * S::A_PART + b * SBLK + q * 4096, PART[o], v[2 * o + b][q]);
+            top = max_abs(top, v[2 * o + b][q]);
+          }
         if (kt + 1 < kt1) load(o, kt + 1);
       }
       fence_proxy_async_smem();
       __syncwarp();
       if (lane == 0) mbar_arrive(&sl->full[s]);
     }
+    const uint32_t m = __reduce_max_sync(0xffffffffu, __float_as_uint(top));
+    if (lane == 0) atomicMax(&sl->top, m);
+    named_bar_arrive(2, SPROD + SEPI);
   } else if (warp >= ISSUER) {
     asm volatile("setmaxnreg.dec.sync.aligned.u32 40;");
     if (warp == ISSUER) {
@@ -253,7 +266,8 @@ __global__ void __launch_bounds__(STHREADS, 1) linear_f32_split_kernel(const __g
     }
     }
   } else {
-    asm volatile("setmaxnreg.inc.sync.aligned.u32 104;");
+    if constexpr (BN == 128) asm volatile("setmaxnreg.inc.sync.aligned.u32 104;");
+    else asm volatile("setmaxnreg.inc.sync.aligned.u32 88;");
     constexpr int CW = BN / 2;                   // columns of a warp
     const int ew = warp - SPROD / 32, row = (warp & 3) * 32 + lane, col = (ew >> 2) * CW;
     const uint32_t tsrc = tmem + ((uint32_t)((warp & 3) * 32) << 16) + col;
@@ -291,23 +305,37 @@ __global__ void __launch_bounds__(STHREADS, 1) linear_f32_split_kernel(const __g
       add(tsrc + 2 * BN);
       add(tsrc + 3 * BN);
     }
-    // An infinity, a NaN or a value that rounds to infinity as bf16 makes its outputs infinite or NaN; a tile of nothing but
-    // tiny values may have lost its third parts among the subnormals.  Both are computed again.
-    float top = 0.f;
-    bool odd = false;
+    named_bar_sync(2, SPROD + SEPI);             // the largest operand is known
+    const float top = __uint_as_float(sl->top), tiny = split_tiny(K, top);
+    const bool zero = top * top < 0x1p-90f;      // all the tile's products may have been lost; else zero is a result like any other
+    auto odd = [&](float v, float tiny) { return !(fabsf(v) < INFINITY) || (fabsf(v) < tiny && (zero || v != 0.f)); };
+    // two operations a result; what they find is looked at again
+    bool any = false;
+    float big = 0.f;
 #pragma unroll
     for (int c = 0; c < CW; ++c) {
-      top = fmaxf(top, fabsf(acc[c]));
-      odd |= !(fabsf(acc[c]) < INFINITY);
+      any |= !(fabsf(acc[c]) >= tiny);
+      big = fmaxf(big, fabsf(acc[c]));
     }
-    odd |= top > 0.f && top < SPLIT_TINY;
-    if (named_bar_or(1, SEPI, odd)) {
-      // plain fp32 over the same K range: slices as [k][row] and [k][column] where the parts were
-      float* as = reinterpret_cast<float*>(smem);
-      float* bs = as + FBK * SI;
-      const int et = tid - SPROD, k1 = min(K, kt1 * SK);
+    any = (any || big == INFINITY) && i0 + row < I;
+    float* dst = reinterpret_cast<float*>(smem) + row * S::LDR + col;
+    auto put = [&](int c) { *reinterpret_cast<float4*>(dst + c) = make_float4(acc[c], acc[c + 1], acc[c + 2], acc[c + 3]); };
 #pragma unroll
-      for (int c = 0; c < CW; ++c) acc[c] = 0.f;
+    for (int c = 0; c < CW; c += 4) put(c);
+    if (any) {
+      any = false;
+#pragma unroll 4
+      for (int c = 0; c < CW; ++c) any |= odd(dst[c], tiny);
+    }
+    if (named_bar_or(1, SEPI, any)) {
+      // plain fp32 over the same K range: slices as [k][row] and [k][column] where the parts were, behind the tile
+      float* as = reinterpret_cast<float*>(smem) + SI * S::LDR;
+      float* bs = as + FBK * SI;
+      float* sum = bs + FBK * BN + row * S::LDR + col;     // of the slices' own sums: short chains, as of the products above
+      const int et = tid - SPROD, k1 = min(K, kt1 * SK);
+      float top_i = 0.f;
+#pragma unroll
+      for (int c = 0; c < CW; c += 4) *reinterpret_cast<float4*>(sum + c) = make_float4(0.f, 0.f, 0.f, 0.f);
       for (int k0 = kt0 * SK; k0 < k1; k0 += FBK) {
         for (int idx = et; idx < FBK * (SI + BN); idx += SEPI) {
           const bool isb = idx >= FBK * SI;
@@ -323,11 +351,15 @@ __global__ void __launch_bounds__(STHREADS, 1) linear_f32_split_kernel(const __g
             }
           }
           (isb ? bs : as)[x] = val;
+          if (isb) atomicMax(&sl->top_j[rr], __float_as_uint(fabsf(val)));
         }
         named_bar_sync(1, SEPI);
         const int kn = min(FBK, k1 - k0);
+#pragma unroll
+        for (int c = 0; c < CW; ++c) acc[c] = 0.f;
         for (int kk = 0; kk < kn; ++kk) {
           const float av = as[kk * SI + row];
+          top_i = fmaxf(top_i, fabsf(av));
 #pragma unroll
           for (int c = 0; c < CW; c += 4) {
             const float4 bv = *reinterpret_cast<const float4*>(bs + kk * BN + col + c);
@@ -337,12 +369,16 @@ __global__ void __launch_bounds__(STHREADS, 1) linear_f32_split_kernel(const __g
             acc[c + 3] = fmaf(av, bv.w, acc[c + 3]);
           }
         }
+#pragma unroll
+        for (int c = 0; c < CW; ++c) sum[c] += acc[c];
         named_bar_sync(1, SEPI);
       }
+#pragma unroll 4
+      for (int c = 0; c < CW; ++c) {
+        const float top_j = __uint_as_float(sl->top_j[col + c]);
+        if (odd(dst[c], split_tiny(K, fmaxf(top_i, top_j)))) dst[c] = sum[c];
+      }
     }
-    float* dst = reinterpret_cast<float*>(smem) + row * S::LDR + col;
-#pragma unroll
-    for (int c = 0; c < CW; c += 4) *reinterpret_cast<float4*>(dst + c) = make_float4(acc[c], acc[c + 1], acc[c + 2], acc[c + 3]);
   }
 
   // ---- the tile lies in shared memory; each CTA of the cluster adds the parts of its share of the rows and stores them

@@ -1,4 +1,6 @@
-// fp32 operands of tensor-core products as three bf16 parts: x = x0 + x1 + x2 exactly (3 x 8 significant bits).
+// fp32 operands of tensor-core products as three bf16 parts: x = x0 + x1 + x2 exactly (3 x 8 significant bits) for every x of
+// 2^-110 and more.  Below that a third part, then a second, falls under bf16's smallest number, 2^-133: the parts are off by up to
+// 2^-134 then.  Infinities, NaN and numbers that round to infinity as bf16 leave NaN in their results.
 #pragma once
 #include "sm100_prims.cuh"
 
@@ -6,8 +8,20 @@ namespace saf {
 
 constexpr int SBLK = 64 * 64 * 2;              // one part of a block: 64 rows of 64 values, 128-byte swizzled rows
 
-// results below this may have lost third parts among the subnormals of bf16
 constexpr float SPLIT_TINY = 1e-28f;
+// A result of n products x y may be off by more than 2^-24 of itself where it is smaller than this: the parts are off by up to
+// 2^-134 for each x and y, times the other one, at most `top`, and the accumulator may have lost up to 2^-126 of each of six part
+// products.  Tested on the results, this needs the largest operand only, and costs the products of 2048 rows 1 %; what the parts
+// leave over of each operand would say the same and cost 12 to 22 %.
+__device__ __forceinline__ float split_tiny(int n, float top) { return n * fmaxf(0x1p-99f, 0x1p-109f * top); }
+
+// the largest magnitude of three; NaN is left out
+__device__ __forceinline__ float max3_abs(float a, float b, float c) {
+  float r;
+  asm("max.abs.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+  return r;
+}
+__device__ __forceinline__ float max_abs(float top, const float4& x) { return max3_abs(max3_abs(top, x.x, x.y), x.z, x.w); }
 
 __device__ __forceinline__ float4 ld4_or_0(const float* p, bool ok) {
   return ok ? __ldg(reinterpret_cast<const float4*>(p)) : make_float4(0.f, 0.f, 0.f, 0.f);

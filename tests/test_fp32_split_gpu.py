@@ -60,6 +60,46 @@ def test_values_the_parts_cannot_carry(what):
         assert (a.double() - r)[fin].norm() <= 8 * 2.0 ** -24 * r[fin].norm()
 
 
+def lines(a, r, dim):
+    """Largest error of a row or column, relative to it."""
+    return ((a.double() - r).norm(dim=dim) / r.norm(dim=dim)).max()
+
+
+# (size of the tiny operands, size of all others they are multiplied with): the parts carry 1e-32 to the last bit, 1e-36 not
+@pytest.mark.parametrize("tiny,large", [(1e-36, 1.0), (1e-36, 1e10), (1e-34, 1e15), (1e-32, 1e10), (3e-20, 1e-14)])
+@pytest.mark.parametrize("what", ["x row", "x column", "w row", "w column", "dy row", "dy column"])
+def test_tiny_rows_and_columns_beside_ordinary_ones(what, tiny, large):
+    g = torch.Generator(device="cuda").manual_seed(6)
+    t = dict(x=torch.randn(300, 256, device="cuda", generator=g), w=torch.randn(192, 256, device="cuda", generator=g),
+             dy=torch.randn(300, 192, device="cuda", generator=g))
+    name, way = what.split()
+    for n in t:
+        if n != name:
+            t[n] *= large
+    at = (70, slice(None)) if way == "row" else (slice(None), 70)
+    t[name][at] *= tiny
+    got, ref = products(t["x"], t["w"], t["dy"], torch.arange(192, device="cuda"))
+    # fp32 sums of up to 300 terms in each row and column
+    for a, r in zip(got, ref):
+        for dim in (0, 1):
+            assert lines(a, r, dim) <= 12 * 2.0 ** -24
+
+
+@pytest.mark.parametrize("size", [1e-36, float("inf"), 3.4e38])
+def test_other_rows_and_features_keep_their_bits(size):
+    from kernel import linear_rows
+    g = torch.Generator(device="cuda").manual_seed(7)
+    x, w = torch.randn(300, 256, device="cuda", generator=g), torch.randn(192, 256, device="cuda", generator=g)
+    rows = torch.arange(192, device="cuda")
+    y = linear_rows(x, w, None, rows)
+    x2, w2 = x.clone(), w.clone()
+    x2[70, 9], w2[3, 200] = size, size
+    y2 = linear_rows(x2, w2, None, rows)
+    keep = torch.ones_like(y, dtype=torch.bool)
+    keep[70], keep[:, 3] = False, False
+    assert torch.equal(y[keep], y2[keep])
+
+
 def causal_attention_64(q, k, v, do, scale):
     """y, dq, dk, dv in 64 bits, each row from its own keys only: what later keys hold does not reach it."""
     q, k, v, do = [t.double() for t in (q, k, v, do)]
