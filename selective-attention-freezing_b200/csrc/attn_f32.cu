@@ -21,8 +21,9 @@
 // 41 and 196 us; each step's products one after the other: 164.
 //
 // The same split as the reference (kernel/fused_attn.py:228-289, 415-481, 483-540): no atomics, fixed order of sums.
-// What the parts cannot carry shows in the results (infinities, NaN, a tile of nothing but tiny values): such a tile is
-// computed again with fp32 FMAs, row by row.
+// What the parts cannot carry shows in the results: they are not finite, or smaller than what may have been lost of them, which
+// follows from the tile's largest operand (split_bf16.cuh).  The thread that holds one computes its 16 columns again with fp32
+// FMAs.
 #include <string.h>
 
 #include "head_index.cuh"
@@ -47,7 +48,7 @@ struct AttnShape {
   static constexpr int NRES = MODE == A_FWD ? 1 : 2, STAGES = MODE == A_FWD ? 3 : 2;
   struct Ctrl {
     uint64_t full[STAGES], empty[STAGES], res_full, s_full[2], dp_full, p_full[2], ds_full, acc_full[2];
-    uint32_t tmem_base;
+    uint32_t tmem_base, top;                    // largest operand (fp32 bits)
     alignas(16) float lse[STAGES][AX], delta[STAGES][AX];   // dK / dV: of the streamed query rows
     float mx[2][4][AR];                         // forward: row maxima, row sums of the four quarters
   };
@@ -156,6 +157,7 @@ __device__ __forceinline__ void attn_f32_tile(const SafMixedAttnBwdArgs& g, int 
   const int x1 = MODE == A_DKDV ? xt : min(xt, (r0 + AR) / AX);
 
   if (tid == 0) {
+    sl->top = 0;
     for (int s = 0; s < S::STAGES; ++s) {
       mbar_init(&sl->full[s], APROD / 32);
       mbar_init(&sl->empty[s], 1);
@@ -183,6 +185,7 @@ __device__ __forceinline__ void attn_f32_tile(const SafMixedAttnBwdArgs& g, int 
     asm volatile("setmaxnreg.dec.sync.aligned.u32 56;");
     const int row = tid >> 4, c4 = (tid & 15) * 4;           // 16 bytes of a row, 16 rows apart
     const uint32_t off = row * 128 + ((((tid & 15) >> 1) ^ (row & 7)) << 4) + (tid & 1) * 8;
+    float top = 0.f;
     // the resident operands, block by block
     {
       const SafTensor& t0 = MODE == A_DKDV ? a.k : a.q;
@@ -201,7 +204,10 @@ __device__ __forceinline__ void attn_f32_tile(const SafMixedAttnBwdArgs& g, int 
           v[q] = ld4_or_0(src + (int64_t)t * ld, t < T);
         }
 #pragma unroll
-        for (int q = 0; q < 4; ++q) split_store(smem + o * RES + blk * SBLK + q * 2048 + off, RES_PART, v[q]);
+        for (int q = 0; q < 4; ++q) {
+          split_store(smem + o * RES + blk * SBLK + q * 2048 + off, RES_PART, v[q]);
+          top = max_abs(top, v[q]);
+        }
       }
     }
     fence_proxy_async_smem();
@@ -240,7 +246,10 @@ __device__ __forceinline__ void attn_f32_tile(const SafMixedAttnBwdArgs& g, int 
 #pragma unroll
       for (int o = 0; o < 2; ++o) {
 #pragma unroll
-        for (int q = 0; q < 4; ++q) split_store(st + o * STR + q * 2048, SBLK, v[o][q]);
+        for (int q = 0; q < 4; ++q) {
+          split_store(st + o * STR + q * 2048, SBLK, v[o][q]);
+          top = max_abs(top, v[o][q]);
+        }
         if (MODE == A_DKDV && o == 1 && tid < 2 * AX) (tid < AX ? sl->lse : sl->delta)[s][tid & (AX - 1)] = stat;
         if (xi + 1 < x1) load(o, xi + 1);
       }
@@ -248,6 +257,9 @@ __device__ __forceinline__ void attn_f32_tile(const SafMixedAttnBwdArgs& g, int 
       __syncwarp();
       if (lane == 0) mbar_arrive(&sl->full[s]);
     }
+    const uint32_t m = __reduce_max_sync(0xffffffffu, __float_as_uint(top));
+    if (lane == 0) atomicMax(&sl->top, m);
+    named_bar_arrive(2, APROD + ACOMP);
   } else if (warp >= AISSUER) {
     asm volatile("setmaxnreg.dec.sync.aligned.u32 40;");
     if (warp == AISSUER) {
@@ -478,21 +490,25 @@ __device__ __forceinline__ void attn_f32_tile(const SafMixedAttnBwdArgs& g, int 
       drain(T_ACC1 + b * 128, acc1, true);
       if constexpr (MODE == A_DKDV) drain(T_ACC2, acc2, true);
     }
-    float top = 0.f;
+    if (MODE == A_FWD) sl->mx[0][part][row] = l;              // (the last step's maxima were read before its p_full)
+    named_bar_sync(2, APROD + ACOMP);                         // row sums and the largest operand are known
+    // dP, a sum of 64 products, is off by that much more, and what it is off by comes times an operand
+    const float top = fmaxf(1.f, __uint_as_float(sl->top)), tiny = split_tiny(64 * AX * n, top) * top;
     bool odd = false;
+    float big = 0.f;
 #pragma unroll
     for (int c = 0; c < 16; ++c) {
-      odd |= !(fabsf(acc1[c]) < INFINITY) || !(fabsf(acc2[c]) < INFINITY);
-      top = fmaxf(top, fmaxf(fabsf(acc1[c]), fabsf(acc2[c])));
+      odd |= !(fabsf(acc1[c]) >= tiny) && acc1[c] != 0.f;
+      big = fmaxf(big, fabsf(acc1[c]));
+      if (MODE == A_DKDV) {
+        odd |= !(fabsf(acc2[c]) >= tiny) && acc2[c] != 0.f;
+        big = fmaxf(big, fabsf(acc2[c]));
+      }
     }
+    odd |= big == INFINITY;
     if (MODE == A_FWD) {
-      odd |= !(l < INFINITY);
-      sl->mx[0][part][row] = l;       // (the last step's maxima were read before its p_full; the vote orders the rest)
+      l = (sl->mx[0][0][row] + sl->mx[0][1][row]) + (sl->mx[0][2][row] + sl->mx[0][3][row]);
     }
-    // nothing but tiny values in the whole tile, or something that is not finite: once more in plain fp32
-    const bool some = named_bar_or(1, ACOMP, top > 0.f), big = named_bar_or(1, ACOMP, top >= SPLIT_TINY);
-    odd = named_bar_or(1, ACOMP, odd) || (some && !big);
-    if (MODE == A_FWD) l = (sl->mx[0][0][row] + sl->mx[0][1][row]) + (sl->mx[0][2][row] + sl->mx[0][3][row]);
     if (odd && t < T) {
       const float *qb = f32_head(a.q, hx.b, hx.hq), *kb = f32_head(a.k, hx.b, hx.hk), *vb = f32_head(a.v, hx.b, hx.hv);
       const float* dob = MODE == A_FWD ? nullptr : f32_head(g.dout, hx.b, hx.h);

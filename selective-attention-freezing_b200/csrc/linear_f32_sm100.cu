@@ -307,7 +307,8 @@ __global__ void __launch_bounds__(STHREADS, 1) linear_f32_split_kernel(const __g
     }
     named_bar_sync(2, SPROD + SEPI);             // the largest operand is known
     const float top = __uint_as_float(sl->top), tiny = split_tiny(K, top);
-    const bool zero = top * top < 0x1p-90f;      // all the tile's products may have been lost; else zero is a result like any other
+    // (zero is a result like any other unless all the tile's products may have been lost)
+    const bool zero = top > 0.f && top * top < 0x1p-90f;
     auto odd = [&](float v, float tiny) { return !(fabsf(v) < INFINITY) || (fabsf(v) < tiny && (zero || v != 0.f)); };
     // two operations a result; what they find is looked at again
     bool any = false;

@@ -8,7 +8,6 @@ namespace saf {
 
 constexpr int SBLK = 64 * 64 * 2;              // one part of a block: 64 rows of 64 values, 128-byte swizzled rows
 
-constexpr float SPLIT_TINY = 1e-28f;
 // A result of n products x y may be off by more than 2^-24 of itself where it is smaller than this: the parts are off by up to
 // 2^-134 for each x and y, times the other one, at most `top`, and the accumulator may have lost up to 2^-126 of each of six part
 // products.  Tested on the results, this needs the largest operand only, and costs the products of 2048 rows 1 %; what the parts

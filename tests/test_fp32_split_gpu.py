@@ -139,7 +139,7 @@ def test_attention_against_64_bits(T, sharp):
         assert off <= (none if T == 1 and i in (1, 2) else 12 * sharp * 2.0 ** -24 * r.norm())
 
 
-@pytest.mark.parametrize("what", ["v inf", "k -inf", "q nan", "do nan", "do tiny"])
+@pytest.mark.parametrize("what", ["v inf", "k -inf", "q nan", "do nan", "do tiny", "do 1e-30"])
 def test_attention_on_values_the_parts_cannot_carry(what):
     g = torch.Generator(device="cuda").manual_seed(8)
     q, k, v, do = [torch.randn(1, 2, 200, 64, device="cuda", generator=g) for _ in range(4)]
@@ -148,12 +148,37 @@ def test_attention_on_values_the_parts_cannot_carry(what):
     if what == "q nan": q[0, 0, 30, 1] = float("nan")
     if what == "do nan": do[0, 0, 130, 1] = float("nan")
     if what == "do tiny": do *= 1e-34
+    if what == "do 1e-30": do *= 1e-30
     for i, (a, r) in enumerate(zip(attention(q, k, v, do), causal_attention_64(q, k, v, do, 0.125))):
         if what == "v inf" and i == 0:      # infinite where 64 bits are, and nowhere else
             assert torch.equal(torch.isinf(a), torch.isinf(r.float()))
         bad = ~torch.isfinite(r)
-        if what == "k -inf" and i:          # 0 * inf in the gradients of rows that give the key no weight
+        if what == "k -inf" and i:          # 0 * inf in the gradients of rows that give the key no weight: no more than these
+            assert torch.isfinite(a[0, 0]).all()
             continue
         assert torch.equal(~torch.isfinite(a), bad)
-        # do tiny: dS around 1e-35 has subnormal terms
-        assert (a.double() - r)[~bad].norm() <= (1e-2 if what == "do tiny" else 12 * 2.0 ** -24) * r[~bad].norm()
+        # do tiny: dS around 1e-35 has subnormal terms, which y and dV know nothing of
+        assert (a.double() - r)[~bad].norm() <= (1e-2 if what == "do tiny" and i in (1, 2) else 12 * 2.0 ** -24) * r[~bad].norm()
+
+
+# the operand, its row (or feature) and size, and the size of v or do, which it is multiplied with
+@pytest.mark.parametrize("what,at,tiny,other", [("v", "column", 1e-35, 1.0), ("v", "column", 1e-36, 1e10), ("do", "column", 1e-35, 1.0),
+                                                ("do", "row", 1e-30, 1.0), ("do", "row", 1e-33, 1e3), ("v", "all", 1e-28, 1.0),
+                                                ("v", "all", 1e-36, 1e12), ("q", "row", 1e-36, 1.0), ("k", "row", 1e-36, 1.0)])
+@pytest.mark.parametrize("T", [70, 200])
+def test_attention_of_tiny_rows_and_features(T, what, at, tiny, other):
+    g = torch.Generator(device="cuda").manual_seed(9)
+    t = {n: torch.randn(1, 2, T, 64, device="cuda", generator=g) for n in ("q", "k", "v", "do")}
+    where = dict(row=(slice(None), slice(None), 60), column=(Ellipsis, 5), all=Ellipsis)[at]
+    t[what][where] *= tiny
+    if what in ("v", "do"):
+        t["do" if what == "v" else "v"] *= other
+    q, k, v, do = [x.double() for x in t.values()]
+    y, dq, dk, dv = ref = causal_attention_64(q, k, v, do, 0.125)
+    # the same sums of magnitudes: what a result is rounded against
+    p = (q @ k.mT * 0.125).masked_fill(torch.ones(T, T, device="cuda", dtype=torch.bool).triu(1), float("-inf")).softmax(-1)
+    ds = p * (do.abs() @ v.abs().mT + (do.abs() * y.abs()).sum(-1, keepdim=True)) * 0.125
+    size = p @ v.abs(), ds @ k.abs(), ds.mT @ q.abs(), p.mT @ do.abs()
+    # scores of size 8 and more rounded before they are exponentiated, sums of up to 200 terms
+    for a, r, m in zip(attention(**t), ref, size):
+        assert ((a.double() - r).abs() <= 40 * 2.0 ** -24 * m).all()
