@@ -708,13 +708,18 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant
 // tiles) is handed the next item while the other one still works, more than one phase of a shared barrier ahead of it, and
 // a wait by parity cannot tell that phase from the one before.  A tile's score products go through its four barriers in turn (at
 // most three of them are out), so that barrier and phase follow from the warpgroup's own count, and its buffer from step
-// to step: the loop is bound by its instructions, and with a bit per buffer and a division in it the launch took 1547 us where
-// it takes 1511 (9 live heads x 64, T = 16384, B = 4).
+// to step.
+// o_full, committed behind the last product of a query tile in an item, is what its warpgroup waits for before it takes O out:
+// the buffer's own buf_free would come round again when the next item has only the other warpgroup's tile, or at once where
+// there are two buffers.
+// The softmax loop is bound by its instructions and the values it carries: with a bit per buffer and a division in every step,
+// and the last buffer and its phase kept for the epilogue, the launch took 1525 us where it takes 1482 (9 live heads x 64, T =
+// 16384, B = 4).
 struct PersistBars {
   uint64_t q_full[2], q_free[2];
   uint64_t k_full[4], k_empty[4], v_full[4], v_empty[4];
   uint64_t s_full[2][4], p_full[3], buf_free[3];
-  uint64_t o_free[2];
+  uint64_t o_full[2], o_free[2];
   uint64_t w_full[2], w_empty[2];
   volatile int32_t work[2];
   uint32_t tmem_base;
@@ -810,6 +815,7 @@ flash_fwd_persistent_kernel(const __grid_constant__ CUtensorMap mapQ, const __gr
     for (int t = 0; t < 2; ++t) {
       mbar_init(&bars->q_full[t], 1);
       mbar_init(&bars->q_free[t], 1);
+      mbar_init(&bars->o_full[t], 1);
       mbar_init(&bars->o_free[t], 128);
       mbar_init(&bars->w_full[t], 1);
       mbar_init(&bars->w_empty[t], W_CONSUMERS);
@@ -1039,6 +1045,7 @@ flash_fwd_persistent_kernel(const __grid_constant__ CUtensorMap mapQ, const __gr
             for (int ks = 0; ks < FN / 16; ++ks)
               umma_ts(dO, aP + ks * 8, umma_desc_advance(dv, ks * 2048), idesc_o, (j > 0) || (ks > 0));
             umma_commit(&bars->buf_free[buf]);
+            if (j == (t ? g.nkv1 : g.nkv0) - 1) umma_commit(&bars->o_full[t]);
             if (t == 1 || !g.act1) umma_commit(&bars->v_empty[vs_]);   // last reader of V_j
           }
           __syncwarp();
@@ -1057,7 +1064,7 @@ flash_fwd_persistent_kernel(const __grid_constant__ CUtensorMap mapQ, const __gr
     const uint32_t tO = tmem + lane_base + C::O_COL + t * HD;
     const float sc = p.scale_log2;
     const bool warp_lead = (tid & 31) == 0;
-    uint32_t g_base = 0, n_s = 0;          // n_s: score tiles this warpgroup has taken
+    uint32_t g_base = 0, n_s = 0;          // n_s: score tiles this warpgroup has taken; bit 31: the parity of its items
     bool ok = true;
     for (int n = 0; ok; ++n) {
       const int it = fetch(n, warp_lead);
@@ -1069,7 +1076,6 @@ flash_fwd_persistent_kernel(const __grid_constant__ CUtensorMap mapQ, const __gr
       const int nk = t ? g.nkv1 : g.nkv0;
       if (nk > 0) {
         float m_ref = -INFINITY, l = 0.f;
-        uint32_t pbuf = 0, pph = 0;
         // buffer and phase of the running number of this tile's scores, advanced from step to step
         const uint32_t step = g.act1 ? 2 : 1, gi = g_base + (g.act1 ? t : 0);
         uint32_t buf = gi % C::NBUF, bph = (gi / C::NBUF) & 1;
@@ -1110,7 +1116,8 @@ flash_fwd_persistent_kernel(const __grid_constant__ CUtensorMap mapQ, const __gr
           } else {
             const bool need = mx > m_ref + RESCALE_THRESHOLD;
             if (__any_sync(0xffffffffu, need)) {
-              if (!mbar_wait(&bars->buf_free[pbuf], pph)) {
+              const uint32_t gp = g_base + (g.act1 ? 2 * (j - 1) + t : j - 1);     // the step before
+              if (!mbar_wait(&bars->buf_free[gp % C::NBUF], (gp / C::NBUF) & 1)) {
                 dev_set_error(p.status, SAF_DEV_TIMEOUT_SOFTMAX, 55);
                 ok = false;
                 break;
@@ -1156,8 +1163,6 @@ flash_fwd_persistent_kernel(const __grid_constant__ CUtensorMap mapQ, const __gr
           tmem_st_wait();
           tc_fence_before();
           mbar_arrive(&bars->p_full[buf]);
-          pbuf = buf;
-          pph = bph;
           buf += t && j + 2 == nk ? 1 : step;                  // (the extra diagonal step of tile 1 follows at once)
           if (buf >= (uint32_t)C::NBUF) {
             buf -= C::NBUF;
@@ -1166,11 +1171,12 @@ flash_fwd_persistent_kernel(const __grid_constant__ CUtensorMap mapQ, const __gr
         }
         if (!ok) break;
         // ---- epilogue of tile t: O / l -> bf16 -> the tile's own Q buffer -> TMA store
-        if (!mbar_wait(&bars->buf_free[pbuf], pph)) {
+        if (!mbar_wait(&bars->o_full[t], n_s >> 31)) {
           dev_set_error(p.status, SAF_DEV_TIMEOUT_SOFTMAX, 56);
           ok = false;
           break;
         }
+        n_s ^= 0x80000000u;
         tc_fence_after();
         const float inv = 1.f / l;
         const int trow = g.row0 + t * FM;

@@ -70,46 +70,91 @@ def bwd_dq(two):                           # S up to two key tiles ahead, dP one
     return issuer + [("issue", [("acc", 0)])], warp + [("wait", ("acc", 0), 0)]
 
 
-def stuck(program, two):
-    """A reachable state in which somebody waits for a phase that has gone by, or passes one that has not come."""
-    issuer, warp = program(two)
-    commits = [op[1] for op in issuer if op[0] == "issue"]
+def forward_queue(s_own, o_own, nbuf=3, items=((1, 2), (3, 0), (3, 0), (1, 2))):
+    """flash_fwd_sm100.cu, persistent: key tiles of the two query tiles of each item, longest first in a group, so that items
+    without a second tile follow those of the group before.  s_own: score barriers of each query tile's own, four in turn; o_own:
+    a barrier of its own behind the last product of a query tile."""
+    sched, scores, outs, warps = [], [], [], ([], [])
+    gs, taken, done, before = 0, [0, 0], [0, 0], [None, None]
+    for n, nk in enumerate(items):
+        sched += ([("wait", ("w_empty", n & 1), n // 2 - 1)] if n > 1 else []) + [("arrive", ("w_full", n & 1))]
+        for a in (scores, outs, *warps):
+            a += [("wait", ("w_full", n & 1), n // 2), ("arrive", ("w_empty", n & 1))]
+        order = [(t, j) for j in range(nk[0]) for t in ((0, 1) if nk[1] else (0,))] + [(1, j) for j in range(nk[0], nk[1])]
+        for t, j in order:
+            buf, k = gs % nbuf, gs // nbuf
+            s = (("s", t, taken[t] & 3), taken[t] >> 2) if s_own else (("s", buf), k)
+            scores += ([("wait", ("free", buf), k - 1)] if k else []) + [("issue", [s[0]])]
+            last = j == nk[t] - 1
+            outs += [("wait", ("o_free", t), done[t] - 1)] if j == 0 and done[t] else []
+            outs += [("wait", ("p", buf), k), ("issue", [("free", buf)] + ([("o", t)] if last else []))]
+            # (a larger row maximum rescales O, once the product of the step before is done)
+            warps[t].extend([("wait", *s)] + ([("wait", ("free", before[t][0]), before[t][1])] if j else []) + [("arrive", ("p", buf))])
+            before[t] = buf, k
+            if last:
+                warps[t].extend([("wait", ("o", t), done[t]) if o_own else ("wait", ("free", buf), k), ("arrive", ("o_free", t))])
+                done[t] += 1
+            taken[t] += 1
+            gs += 1
+    return [sched, scores, outs, *warps], {"w_empty": 4}
 
-    def phase(bar, ws, done):
-        arrived = sum(op == ("arrive", bar) for w in ws for op in warp[:w])
-        return arrived // 2 + sum(c.count(bar) for c in commits[:done])
 
-    seen, todo = set(), [(0, (0, 0), 0)]
+def stuck(agents, counts):
+    """A reachable state in which somebody waits for a phase that has gone by, or passes one that has not come.  counts: arrivals
+    that make a phase, by the barrier's name, where it is not one; the agents that meet are the ones with such an operation."""
+    commits = [[op[1] for op in a if op[0] == "issue"] for a in agents]
+    bars = {op[1] for a in agents for op in a if op[0] in ("wait", "arrive")}
+    arrived = {b: [[sum(op == ("arrive", b) for op in a[:n]) for n in range(len(a) + 1)] for a in agents] for b in bars}
+    committed = {b: [[sum(x.count(b) for x in c[:n]) for n in range(len(c) + 1)] for c in commits] for b in bars}
+    issued = [[sum(op[0] == "issue" for op in a[:n]) for n in range(len(a) + 1)] for a in agents]
+
+    def phase(b, at, done):
+        return (sum(arrived[b][i][n] for i, n in enumerate(at)) // counts.get(b[0], 1)
+                + sum(committed[b][i][n] for i, n in enumerate(done)))
+
+    seen, todo = set(), [((0,) * len(agents), (0,) * len(agents))]
     while todo:
         state = todo.pop()
         if state in seen:
             continue
         seen.add(state)
-        ip, ws, done = state
-        if done < sum(op[0] == "issue" for op in issuer[:ip]):
-            todo.append((ip, ws, done + 1))
-        for who, ops, at in [(-1, issuer, ip), (0, warp, ws[0]), (1, warp, ws[1])]:
-            if at == len(ops):
+        at, done = state
+        for i, ops in enumerate(agents):
+            if done[i] < issued[i][at[i]]:
+                todo.append((at, done[:i] + (done[i] + 1,) + done[i + 1:]))
+            if at[i] == len(ops):
                 continue
-            op = ops[at]
+            op = ops[at[i]]
             if op[0] == "wait":
-                now = phase(op[1], ws, done)
+                now = phase(op[1], at, done)
                 if not now - op[2] in (0, 1):
                     return state
                 if now == op[2]:
                     continue
-            # bar.sync of the compute warps: both have to be there, or the other one is past it
-            if op[0] == "meet" and ws[1 - who] < at:
+            # bar.sync: everybody is there, or past it
+            if op[0] == "meet" and any(at[k] < at[i] for k, a in enumerate(agents) if ("meet",) in a):
                 continue
-            todo.append((ip + 1, ws, done) if who < 0 else (ip, tuple(w + (k == who) for k, w in enumerate(ws)), done))
+            todo.append((at[:i] + (at[i] + 1,) + at[i + 1:], done))
     return None
+
+
+def two_warps(program, two):
+    issuer, warp = program(two)
+    return [issuer, warp, warp], {"p": 2, "ds": 2}
 
 
 @pytest.mark.parametrize("program", [fp32_forward, fp32_dkdv, fp32_dq, bwd_dkdv_64, bwd_dkdv_128, bwd_dq])
 def test_no_wait_is_overtaken(program):
-    assert stuck(program, True) is None
+    assert stuck(*two_warps(program, True)) is None
 
 
 @pytest.mark.parametrize("program", [fp32_forward, bwd_dkdv_64])
 def test_one_barrier_for_p_is_overtaken_where_scores_run_ahead(program):
-    assert stuck(program, False) is not None
+    assert stuck(*two_warps(program, False)) is not None
+
+
+@pytest.mark.parametrize("nbuf", [2, 3])
+def test_forward_queue(nbuf):
+    assert stuck(*forward_queue(True, True, nbuf)) is None
+    assert stuck(*forward_queue(False, True, nbuf)) is not None
+    assert stuck(*forward_queue(True, False, nbuf)) is not None
