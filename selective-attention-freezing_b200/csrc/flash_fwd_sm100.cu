@@ -135,6 +135,7 @@ struct FlashBars {
   uint64_t s_full[3];     // score buffer written by the score MMAs
   uint64_t p_full[3];     // P written by the softmax warpgroup (128 arrivals)
   uint64_t buf_free[3];   // PV product that read P from this buffer has finished
+  uint64_t o_full[2];     // the last one of a query tile: the other tile's last one may go through the same buffer
   uint32_t tmem_base;
   float dec_alpha[2][128];   // decomposed heads: alpha of the current key tile, per query tile
   float dec_rho[2][256];     // and the rho values its distances can take
@@ -275,6 +276,8 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant
       mbar_init(&bars->p_full[i], 128);
       mbar_init(&bars->buf_free[i], 1);
     }
+    mbar_init(&bars->o_full[0], 1);
+    mbar_init(&bars->o_full[1], 1);
     fence_mbar_init();
   }
   if (warp == 9) {
@@ -411,6 +414,7 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant
             for (int ks = 0; ks < FN / 16; ++ks)
               umma_ts(dO, aP + ks * 8, umma_desc_advance(dv, ks * 2048), idesc_o, (j > 0) || (ks > 0));
             umma_commit(&bars->buf_free[buf]);
+            if (j == (t ? nkv1 : nkv0) - 1) umma_commit(&bars->o_full[t]);
             if (t == 1 || !act1) umma_commit(&bars->v_empty[vs_]);   // last reader of V_j
           }
           __syncwarp();
@@ -524,8 +528,6 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant
         tmem_st_wait();
         tc_fence_before();
         mbar_arrive(&bars->p_full[buf]);
-        pbuf = buf;
-        pph = bph;
         buf += kstep;
         if (buf >= C::NBUF) {
           buf -= C::NBUF;
@@ -641,7 +643,7 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap mapQ, const __grid_constant
     }
     if (nk > 0) {
       // the last PV product of this tile
-      if (ok && !mbar_wait(&bars->buf_free[pbuf], pph)) {
+      if (ok && !mbar_wait(&bars->o_full[t], 0)) {
         dev_set_error(p.status, SAF_DEV_TIMEOUT_SOFTMAX, 29);
         ok = false;
       }
