@@ -19,6 +19,9 @@
 // before (fp32 FMAs, 64 x 64 tiles) and now: forward 119 -> 33 us, backward 397 -> 78; relative error against 64 bits 3.3e-7 ->
 // 1.6e-7 (y), 4.5e-7 -> 3.0e-7 (dq), 7.9e-7 -> 3.2e-7 (dk), 8.0e-7 -> 2.6e-7 (dv).  Two threads per row instead of four:
 // 41 and 196 us; each step's products one after the other: 164.
+// Since the issuing warp's descriptors no longer spill (below), whole launches in a row, fills and delta included: forward 35.2 ->
+// 33.6 us, backward 91 -> 81; T = 4096, B = 1, 12 heads 187 -> 178 and 700 -> 590.  88 bytes of stores and 152 of loads a thread
+// are still spilled in the backward (-Xptxas -v), none in the forward.
 //
 // The same split as the reference (kernel/fused_attn.py:228-289, 415-481, 483-540): no atomics, fixed order of sums.
 // What the parts cannot carry shows in the results: they are not finite, or smaller than what may have been lost of them, which
@@ -182,7 +185,9 @@ __device__ __forceinline__ void attn_f32_tile(const SafMixedAttnBwdArgs& g, int 
   const uint32_t tmem = sl->tmem_base;
 
   if (warp < APROD / 32) {
-    asm volatile("setmaxnreg.dec.sync.aligned.u32 56;");
+    // 256 x 64 + 512 x 80 + 128 x 56 registers = 896 x 72 (forward: 72, 80, 40): the split with the fewest spills.  The backward's
+    // issuing warp needs its 56: with 40 it spilled its descriptors
+    if constexpr (MODE != A_FWD) asm volatile("setmaxnreg.dec.sync.aligned.u32 64;");
     const int row = tid >> 4, c4 = (tid & 15) * 4;           // 16 bytes of a row, 16 rows apart
     const uint32_t off = row * 128 + ((((tid & 15) >> 1) ^ (row & 7)) << 4) + (tid & 1) * 8;
     float top = 0.f;
@@ -261,7 +266,8 @@ __device__ __forceinline__ void attn_f32_tile(const SafMixedAttnBwdArgs& g, int 
     if (lane == 0) atomicMax(&sl->top, m);
     named_bar_arrive(2, APROD + ACOMP);
   } else if (warp >= AISSUER) {
-    asm volatile("setmaxnreg.dec.sync.aligned.u32 40;");
+    if constexpr (MODE == A_FWD) asm volatile("setmaxnreg.dec.sync.aligned.u32 40;");
+    else asm volatile("setmaxnreg.dec.sync.aligned.u32 56;");
     if (warp == AISSUER) {
       const bool leader = elect_one();
       const uint32_t id_k = umma_idesc_bf16(AR, AX, 0, 0), id_mn = umma_idesc_bf16(AR, AHD, 0, 1);
@@ -356,7 +362,7 @@ __device__ __forceinline__ void attn_f32_tile(const SafMixedAttnBwdArgs& g, int 
       }
     }
   } else {
-    asm volatile("setmaxnreg.inc.sync.aligned.u32 88;");
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 80;");
     const int quad = warp & 3, part = (warp - APROD / 32) >> 2, row = quad * 32 + lane, col = part * 16;
     const int t = r0 + row;                                   // this thread's query (dK / dV: key)
     const uint32_t lanes = tmem + ((uint32_t)(quad * 32) << 16) + col;
