@@ -51,7 +51,9 @@ def test_fp32_layer(seed, monkeypatch):
     entered = len(calls)
     monkeypatch.setattr(SafCausalSelfAttention, "_layer_call", lambda *a: None)
     want = run()
-    assert len(calls) == entered and entered == (0 if train and bias else 1) or hd == 96
+    # the entry takes every head width whose projection is whole 64-column blocks, and no bias gradients
+    assert len(calls) == entered and entered == int(m._plan.shapes_ok(train) and not (train and bias))
+    assert hd == 96 or m._plan.shapes_ok(train)
     # the same fp32 sums in another order at most (dx: one product over [Q | K | V] instead of two and an addition): a few
     # roundings of 2^-24 of sums of up to 1152 terms
     for a, b in zip(got, want):

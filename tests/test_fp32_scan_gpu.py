@@ -28,7 +28,12 @@ def test_structured_heads(T, B):
     for h in (0, 2):
         for got, ref in ((y[:, h], p[h] @ v[:, h].double()), (dv[:, h], p[h].T @ dy[:, h].double())):
             assert (got.double() - ref).norm() <= tol * ref.norm()
-    s = torch.nn.functional.scaled_dot_product_attention(*(x.detach().double() for x in (q, k, v[:, [1, 3]])), is_causal=True)
+    live = [x.detach().double().requires_grad_(True) for x in (q, k, v[:, [1, 3]])]
+    s = torch.nn.functional.scaled_dot_product_attention(*live, is_causal=True)
     assert (y[:, [1, 3]].double() - s).norm() <= 2e-6 * s.norm()
-    assert all(torch.isfinite(x).all() for x in (dq, dk, dv))
+    # scores of size 8 rounded by 2^-24 of that before they are exponentiated; one row has no score gradient, only what dO.V and
+    # dO.O differ by in fp32
+    none = 2 * 2.0 ** -24 * 0.125 * dy.norm() * v.norm() * max(q.norm(), k.norm()) if T == 1 else 0.0
+    for got, ref in zip((dq, dk, dv[:, [1, 3]]), torch.autograd.grad(s, live, dy[:, [1, 3]].double())):
+        assert (got.double() - ref).norm() <= 12 * 2.0 ** -24 * ref.norm() + none
     ops.device_status()

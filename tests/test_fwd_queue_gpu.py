@@ -2,11 +2,13 @@
 import pytest
 import torch
 
+from oracle import saf_oracle as O
+
 pytestmark = pytest.mark.gpu
 
 
 # (head_dim, T, B): five row tiles with whole and ragged ends, one tile, three tiles, nine
-@pytest.mark.parametrize("hd,T,B", [(128, 640, 32), (64, 640, 32), (96, 600, 32), (128, 128, 64), (128, 384, 48), (64, 384, 29), (64, 1100, 24)])
+@pytest.mark.parametrize("hd,T,B", [(128, 640, 32), (64, 640, 32), (96, 600, 32), (128, 128, 64), (128, 384, 48), (64, 384, 29), (64, 1100, 24), (96, 1, 3), (128, 1, 3), (96, 129, 40), (128, 300, 25)])
 def test_rows_of_every_item(hd, T, B):
     from saf_b200 import ops
     g = torch.Generator(device="cuda").manual_seed(T + hd)
@@ -22,4 +24,9 @@ def test_rows_of_every_item(hd, T, B):
     err = (y[:, rows].float() - ref).norm() / ref.norm()
     # weights and results in bf16: half an ulp, 2^-9, of each, and of the sum of weights
     assert err <= 3 * 2.0 ** -9
+    # the structured heads' rows are rounded once
+    p = O.sink_decay_pattern(alpha[:1].cpu().double(), rho[:1].cpu().double(), T).cuda()
+    for h in (1, 5):
+        want = p[0] @ v[:, h].double()
+        assert (y[:, h].double() - want).norm() <= 2.0 ** -9 * want.norm()
     ops.device_status()
