@@ -19,14 +19,15 @@
 // before (fp32 FMAs, 64 x 64 tiles) and now: forward 119 -> 33 us, backward 397 -> 78; relative error against 64 bits 3.3e-7 ->
 // 1.6e-7 (y), 4.5e-7 -> 3.0e-7 (dq), 7.9e-7 -> 3.2e-7 (dk), 8.0e-7 -> 2.6e-7 (dv).  Two threads per row instead of four:
 // 41 and 196 us; each step's products one after the other: 164.
-// Since the issuing warp's descriptors no longer spill (below), whole launches in a row, fills and delta included: forward 35.2 ->
-// 33.6 us, backward 91 -> 81; T = 4096, B = 1, 12 heads 187 -> 178 and 700 -> 590.  88 bytes of stores and 152 of loads a thread
-// are still spilled in the backward (-Xptxas -v), none in the forward.
+// Since the issuing warp's descriptors no longer spill (below), whole launches in a row, fills and delta included: forward 34.5 ->
+// 33.3 us, backward 91 -> 81; T = 4096, B = 1, 12 heads 182 -> 175 and 700 -> 585.  What is still spilled (-Xptxas -v, bytes of stores and
+// loads a thread) is most of it in the repeat of what the split cannot carry: 40 / 40 forward, 268 / 300 backward, none and 84 / 124
+// without it.
 //
 // The same split as the reference (kernel/fused_attn.py:228-289, 415-481, 483-540): no atomics, fixed order of sums.
 // What the parts cannot carry shows in the results: they are not finite, or smaller than what may have been lost of them, which
-// follows from the tile's largest operand (split_bf16.cuh).  The thread that holds one computes its 16 columns again with fp32
-// FMAs.
+// follows from the tile's largest operand (split_bf16.cuh).  A tile with such results is computed again with fp32 FMAs, and the threads
+// that hold one take their 16 columns from there.
 #include <string.h>
 
 #include "head_index.cuh"
@@ -114,32 +115,169 @@ __device__ __forceinline__ void tmem_parts16(uint32_t at, const float (&v)[16]) 
   tmem_st8(at + 64, w[2]);
 }
 
-__device__ __forceinline__ float row_dot(const float* x, const float* y) {
-  float s = 0.f;
-#pragma unroll 1
-  for (int d = 0; d < AHD; d += 4) {
-    const float4 a = *reinterpret_cast<const float4*>(x + d), b = *reinterpret_cast<const float4*>(y + d);
-    s = fmaf(a.x, b.x, s);
-    s = fmaf(a.y, b.y, s);
-    s = fmaf(a.z, b.z, s);
-    s = fmaf(a.w, b.w, s);
-  }
-  return s;
-}
-__device__ __forceinline__ void axpy16(float f, const float* x, float (&acc)[16]) {
-#pragma unroll
-  for (int c = 0; c < 16; c += 4) {
-    const float4 v = *reinterpret_cast<const float4*>(x + c);
-    acc[c] = fmaf(f, v.x, acc[c]);
-    acc[c + 1] = fmaf(f, v.y, acc[c + 1]);
-    acc[c + 2] = fmaf(f, v.z, acc[c + 2]);
-    acc[c + 3] = fmaf(f, v.w, acc[c + 3]);
-  }
-}
 __device__ __forceinline__ void store16(const SafTensor& t, int b, int h, int row, int col, const float (&v)[16], float f) {
   float* p = reinterpret_cast<float*>(t.ptr) + (int64_t)b * t.stride[0] + (int64_t)h * t.stride[1] + (int64_t)row * t.stride[2] + col;
 #pragma unroll
   for (int c = 0; c < 16; c += 4) *reinterpret_cast<float4*>(p + c) = make_float4(v[c] * f, v[c + 1] * f, v[c + 2] * f, v[c + 3] * f);
+}
+
+// a thread's 16 columns of row t
+template <int MODE>
+__device__ __forceinline__ void store_results(const SafMixedAttnBwdArgs& g, const HeadIdx& hx, int t, int col, const float (&acc1)[16],
+                                              const float (&acc2)[16], float m, float l) {
+  const SafMixedAttnArgs& a = g.fwd;
+  if constexpr (MODE == A_FWD) {
+    const float ls = l == 0.f ? 1.f : l;
+    store16(a.out, hx.b, hx.h, t, col, acc1, 1.f / ls);
+    if (a.lse.ptr && col == 0)
+      reinterpret_cast<float*>(a.lse.ptr)[(int64_t)hx.b * a.lse.stride[0] + (int64_t)hx.h * a.lse.stride[1] + (int64_t)t * a.lse.stride[2]] =
+          ((m == -INFINITY) ? 0.f : m) + log2f(ls);
+  } else if constexpr (MODE == A_DKDV) {
+    store16(g.dv, hx.b, hx.hv, t, col, acc1, 1.f);
+    store16(g.dk, hx.b, hx.hk, t, col, acc2, 1.f);
+  } else {
+    store16(g.dq, hx.b, hx.hq, t, col, acc1, 1.f);
+  }
+}
+
+// The tile once more with fp32 FMAs, by all compute warps; threads with `odd` set store their results.  Resident and streamed rows, and
+// the scores or what is made of them, lie in shared memory as fp32 where the parts were (68 floats a row: 8 neighbouring rows'
+// float4 reads hit all banks once), a thread has 16 columns of a row as above.  A row adds up only what it sees, so that what later
+// keys hold does not reach it, in sums of 64.  It comes when the tile's registers are free, behind the roles: as a function of its own
+// it cost the others 4 to 8 %.  9 heads, T = 1024, B = 2, all of q NaN: forward 383 us, backward 782 (one NaN 54 and 782); the FMA
+// kernels that served these calls before 126 and 411, one thread a row through global memory 6.3 and 38 ms.
+template <int MODE>
+__device__ __forceinline__ void attn_f32_repeat(const SafMixedAttnBwdArgs& g, float* sm, int r0, int x0, int x1, bool odd) {
+  constexpr int LD = 68;
+  static_assert((AR * LD * (MODE == A_FWD ? 2 : 3) + 2 * AX * LD + 4 * AR) * 4 <= AttnShape<MODE>::NRES * RES + AttnShape<MODE>::STAGES * ASTAGE,
+                "fits where the parts were");
+  const SafMixedAttnArgs& a = g.fwd;
+  const HeadIdx hx = head_index(a, blockIdx.x);
+  const int tid = threadIdx.x - APROD, T = a.T;
+  const int part = tid >> 7, row = tid & 127, col = part * 16, t = r0 + row;
+  float *R0 = sm, *R1 = R0 + AR * LD, *X0 = MODE == A_FWD ? R1 : R1 + AR * LD, *X1 = X0 + AX * LD, *W = X1 + AX * LD, *MX = W + AR * LD;
+  auto rows = [&](float* dst, const SafTensor& from, int head, int first, int n) {
+    const float* p = f32_head(from, hx.b, head);
+    for (int i = tid; i < n * 16; i += ACOMP) {
+      const int r = i >> 4, c = (i & 15) * 4;
+      *reinterpret_cast<float4*>(dst + r * LD + c) = ld4_or_0(p + (int64_t)(first + r) * from.stride[2] + c, first + r < T);
+    }
+  };
+  // this thread's 8 columns from j on of R X^T
+  auto dot8 = [&](const float* R, const float* X, int j, float (&s)[8]) {
+#pragma unroll
+    for (int e = 0; e < 8; ++e) s[e] = 0.f;
+#pragma unroll 1
+    for (int d = 0; d < AHD; d += 4) {
+      const float4 y = *reinterpret_cast<const float4*>(R + row * LD + d);
+#pragma unroll
+      for (int e = 0; e < 8; ++e) {
+        const float4 x = *reinterpret_cast<const float4*>(X + (col + j + e) * LD + d);
+        s[e] = fmaf(y.x, x.x, s[e]);
+        s[e] = fmaf(y.y, x.y, s[e]);
+        s[e] = fmaf(y.z, x.z, s[e]);
+        s[e] = fmaf(y.w, x.w, s[e]);
+      }
+    }
+  };
+  // acc += W X over the streamed rows [from, to) of the step
+  auto apply = [&](const float* X, int from, int to, float (&acc)[16]) {
+    float s[16];
+#pragma unroll
+    for (int c = 0; c < 16; ++c) s[c] = 0.f;
+#pragma unroll 1
+    for (int x = from; x < to; ++x) {
+      const float w = W[row * LD + x];
+#pragma unroll
+      for (int c = 0; c < 16; c += 4) {
+        const float4 v = *reinterpret_cast<const float4*>(X + x * LD + col + c);
+        s[c] = fmaf(w, v.x, s[c]);
+        s[c + 1] = fmaf(w, v.y, s[c + 1]);
+        s[c + 2] = fmaf(w, v.z, s[c + 2]);
+        s[c + 3] = fmaf(w, v.w, s[c + 3]);
+      }
+    }
+#pragma unroll
+    for (int c = 0; c < 16; ++c) acc[c] += s[c];
+  };
+  const bool kv = MODE == A_DKDV;
+  rows(R0, kv ? a.k : a.q, kv ? hx.hk : hx.hq, r0, AR);
+  if constexpr (MODE != A_FWD) rows(R1, kv ? a.v : g.dout, kv ? hx.hv : hx.h, r0, AR);
+  const float scale = a.sm_scale * F_LOG2E;
+  const float* lse = MODE == A_FWD ? nullptr : f32_head(a.lse, hx.b, hx.h);
+  const float* del = MODE == A_FWD ? nullptr : f32_head(g.delta, hx.b, hx.h);
+  float acc1[16], acc2[16], m = -INFINITY, l = 0.f, s[8];
+#pragma unroll
+  for (int c = 0; c < 16; ++c) acc1[c] = acc2[c] = 0.f;
+  for (int xi = x0; xi < x1; ++xi) {
+    const int xb = xi * AX;
+    named_bar_sync(1, ACOMP);                               // the step before is read
+    rows(X0, kv ? a.q : a.k, kv ? hx.hq : hx.hk, xb, AX);
+    rows(X1, kv ? g.dout : a.v, kv ? hx.h : hx.hv, xb, AX);
+    named_bar_sync(1, ACOMP);
+    // the rows of the step that this one sees
+    const int from = kv ? min(AX, max(0, t - xb)) : 0, to = t >= T ? from : (kv ? min(AX, T - xb) : max(0, min(AX, t - xb + 1)));
+    float* w = W + row * LD + col;
+    float mx = -INFINITY;
+#pragma unroll 1
+    for (int j = 0; j < 16; j += 8) {
+      dot8(R0, X0, j, s);
+#pragma unroll
+      for (int e = 0; e < 8; ++e) {
+        const int x = col + j + e;
+        const bool seen = x >= from && x < to;
+        if constexpr (MODE == A_FWD) {
+          w[j + e] = seen ? s[e] * scale : -INFINITY;
+          mx = fmaxf(mx, w[j + e]);
+        } else {
+          w[j + e] = seen ? exp2f(s[e] * scale - lse[(int64_t)(kv ? xb + x : t) * a.lse.stride[2]]) : 0.f;
+        }
+      }
+    }
+    if constexpr (MODE == A_FWD) {
+      MX[part * AR + row] = mx;
+      named_bar_sync(1, ACOMP);
+      mx = fmaxf(fmaxf(MX[row], MX[AR + row]), fmaxf(MX[2 * AR + row], MX[3 * AR + row]));
+      const float m_new = fmaxf(m, mx), m_safe = (m_new == -INFINITY) ? 0.f : m_new;
+      const float f = (m == -INFINITY) ? 0.f : exp2f(m - m_safe);
+      float sum = 0.f;
+#pragma unroll 4
+      for (int j = 0; j < 16; ++j) {
+        w[j] = exp2f(w[j] - m_safe);
+        sum += w[j];
+      }
+      l = l * f + sum;
+      m = m_new;
+      named_bar_sync(1, ACOMP);
+#pragma unroll
+      for (int c = 0; c < 16; ++c) acc1[c] *= f;
+      apply(X1, from, to, acc1);
+    } else {
+      if constexpr (MODE == A_DKDV) {
+        named_bar_sync(1, ACOMP);
+        apply(X1, from, to, acc1);
+        named_bar_sync(1, ACOMP);                           // P is read
+      }
+#pragma unroll 1
+      for (int j = 0; j < 16; j += 8) {
+        dot8(R1, X1, j, s);
+#pragma unroll
+        for (int e = 0; e < 8; ++e) {
+          const int x = col + j + e;
+          if (x >= from && x < to) w[j + e] = w[j + e] * (s[e] - del[(int64_t)(kv ? xb + x : t) * g.delta.stride[2]]) * a.sm_scale;
+        }
+      }
+      named_bar_sync(1, ACOMP);
+      if constexpr (MODE == A_DKDV) apply(X0, from, to, acc2);
+      else apply(X0, from, to, acc1);
+    }
+  }
+  if constexpr (MODE == A_FWD) {
+    MX[part * AR + row] = l;
+    named_bar_sync(1, ACOMP);
+    l = (MX[row] + MX[AR + row]) + (MX[2 * AR + row] + MX[3 * AR + row]);
+  }
+  if (odd) store_results<MODE>(g, hx, t, col, acc1, acc2, m, l);
 }
 
 // the row tile with the `rank`-th longest walk of one (batch, head)
@@ -183,11 +321,14 @@ __device__ __forceinline__ void attn_f32_tile(const SafMixedAttnBwdArgs& g, int 
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = sl->tmem_base;
+  bool again = false;                           // this thread's results have to be computed again
 
   if (warp < APROD / 32) {
-    // 256 x 64 + 512 x 80 + 128 x 56 registers = 896 x 72 (forward: 72, 80, 40): the split with the fewest spills.  The backward's
-    // issuing warp needs its 56: with 40 it spilled its descriptors
-    if constexpr (MODE != A_FWD) asm volatile("setmaxnreg.dec.sync.aligned.u32 64;");
+    // backward: 256 x 64 + 512 x 80 + 128 x 56 registers = 896 x 72, the split with the fewest spills (with 40 the issuing warp
+    // spilled its descriptors); the forward is fastest with 72 for all, said role by role: T = 4096, B = 1, 12 heads 173 us, 183 with
+    // 80 for the compute warps, 186 without the instructions (the compiler spills more)
+    if constexpr (MODE == A_FWD) asm volatile("setmaxnreg.dec.sync.aligned.u32 72;");
+    else asm volatile("setmaxnreg.dec.sync.aligned.u32 64;");
     const int row = tid >> 4, c4 = (tid & 15) * 4;           // 16 bytes of a row, 16 rows apart
     const uint32_t off = row * 128 + ((((tid & 15) >> 1) ^ (row & 7)) << 4) + (tid & 1) * 8;
     float top = 0.f;
@@ -266,7 +407,7 @@ __device__ __forceinline__ void attn_f32_tile(const SafMixedAttnBwdArgs& g, int 
     if (lane == 0) atomicMax(&sl->top, m);
     named_bar_arrive(2, APROD + ACOMP);
   } else if (warp >= AISSUER) {
-    if constexpr (MODE == A_FWD) asm volatile("setmaxnreg.dec.sync.aligned.u32 40;");
+    if constexpr (MODE == A_FWD) asm volatile("setmaxnreg.dec.sync.aligned.u32 72;");
     else asm volatile("setmaxnreg.dec.sync.aligned.u32 56;");
     if (warp == AISSUER) {
       const bool leader = elect_one();
@@ -362,7 +503,8 @@ __device__ __forceinline__ void attn_f32_tile(const SafMixedAttnBwdArgs& g, int 
       }
     }
   } else {
-    asm volatile("setmaxnreg.inc.sync.aligned.u32 80;");
+    if constexpr (MODE == A_FWD) asm volatile("setmaxnreg.inc.sync.aligned.u32 72;");
+    else asm volatile("setmaxnreg.inc.sync.aligned.u32 80;");
     const int quad = warp & 3, part = (warp - APROD / 32) >> 2, row = quad * 32 + lane, col = part * 16;
     const int t = r0 + row;                                   // this thread's query (dK / dV: key)
     const uint32_t lanes = tmem + ((uint32_t)(quad * 32) << 16) + col;
@@ -515,58 +657,20 @@ __device__ __forceinline__ void attn_f32_tile(const SafMixedAttnBwdArgs& g, int 
     if (MODE == A_FWD) {
       l = (sl->mx[0][0][row] + sl->mx[0][1][row]) + (sl->mx[0][2][row] + sl->mx[0][3][row]);
     }
-    if (odd && t < T) {
-      const float *qb = f32_head(a.q, hx.b, hx.hq), *kb = f32_head(a.k, hx.b, hx.hk), *vb = f32_head(a.v, hx.b, hx.hv);
-      const float* dob = MODE == A_FWD ? nullptr : f32_head(g.dout, hx.b, hx.h);
-#pragma unroll
-      for (int c = 0; c < 16; ++c) acc1[c] = acc2[c] = 0.f;
-      m = -INFINITY;
-      l = 0.f;
-      const int lo = MODE == A_DKDV ? t : 0, hi = MODE == A_DKDV ? T : t + 1;
-      for (int x = lo; x < hi; ++x) {
-        const int qi = MODE == A_DKDV ? x : t, ki = MODE == A_DKDV ? t : x;
-        const float s = row_dot(qb + (int64_t)qi * a.q.stride[2], kb + (int64_t)ki * a.k.stride[2]) * scale;
-        if constexpr (MODE == A_FWD) {
-          const float m_new = fmaxf(m, s), m_safe = (m_new == -INFINITY) ? 0.f : m_new;
-          const float f = (m == -INFINITY) ? 0.f : exp2f(m - m_safe), p = exp2f(s - m_safe);
-          l = l * f + p;
-          m = m_new;
-#pragma unroll
-          for (int c = 0; c < 16; ++c) acc1[c] *= f;
-          axpy16(p, vb + (int64_t)ki * a.v.stride[2] + col, acc1);
-        } else {
-          const float* dor = dob + (int64_t)qi * g.dout.stride[2];
-          const float Lx = f32_head(a.lse, hx.b, hx.h)[(int64_t)qi * a.lse.stride[2]];
-          const float dx = f32_head(g.delta, hx.b, hx.h)[(int64_t)qi * g.delta.stride[2]];
-          const float p = exp2f(s - Lx);
-          const float ds = p * (row_dot(dor, vb + (int64_t)ki * a.v.stride[2]) - dx) * a.sm_scale;
-          if constexpr (MODE == A_DKDV) {
-            axpy16(p, dor + col, acc1);
-            axpy16(ds, qb + (int64_t)qi * a.q.stride[2] + col, acc2);
-          } else {
-            axpy16(ds, kb + (int64_t)ki * a.k.stride[2] + col, acc1);
-          }
-        }
-      }
-    }
-    if (t < T) {
-      if constexpr (MODE == A_FWD) {
-        const float ls = l == 0.f ? 1.f : l;
-        store16(a.out, hx.b, hx.h, t, col, acc1, 1.f / ls);
-        if (a.lse.ptr && part == 0)
-          reinterpret_cast<float*>(a.lse.ptr)[(int64_t)hx.b * a.lse.stride[0] + (int64_t)hx.h * a.lse.stride[1] + (int64_t)t * a.lse.stride[2]] =
-              ((m == -INFINITY) ? 0.f : m) + log2f(ls);
-      } else if constexpr (MODE == A_DKDV) {
-        store16(g.dv, hx.b, hx.hv, t, col, acc1, 1.f);
-        store16(g.dk, hx.b, hx.hk, t, col, acc2, 1.f);
-      } else {
-        store16(g.dq, hx.b, hx.hq, t, col, acc1, 1.f);
-      }
-    }
+    odd &= t < T;
+    if (t < T && !odd) store_results<MODE>(g, hx, t, col, acc1, acc2, m, l);
+    again = odd;
   }
   tc_fence_before();
-  __syncthreads();
+  const bool any = __syncthreads_or(again);
   if (warp == AISSUER) tmem_dealloc(tmem, 512);
+  if (any) {
+    const bool compute = warp >= APROD / 32 && warp < AISSUER;
+    // back to one share for all
+    if (compute) asm volatile("setmaxnreg.dec.sync.aligned.u32 72;");
+    else asm volatile("setmaxnreg.inc.sync.aligned.u32 72;");
+    if (compute) attn_f32_repeat<MODE>(g, reinterpret_cast<float*>(smem), r0, x0, x1, again);
+  }
 }
 
 // A structured head's CTA of the first row of the grid runs its scan, a sequential chain that ends long before the longest

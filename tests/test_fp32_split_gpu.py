@@ -165,7 +165,7 @@ def test_attention_on_values_the_parts_cannot_carry(what):
 @pytest.mark.parametrize("what,at,tiny,other", [("v", "column", 1e-35, 1.0), ("v", "column", 1e-36, 1e10), ("do", "column", 1e-35, 1.0),
                                                 ("do", "row", 1e-30, 1.0), ("do", "row", 1e-33, 1e3), ("v", "all", 1e-28, 1.0),
                                                 ("v", "all", 1e-36, 1e12), ("q", "row", 1e-36, 1.0), ("k", "row", 1e-36, 1.0)])
-@pytest.mark.parametrize("T", [70, 200])
+@pytest.mark.parametrize("T", [70, 200, 450])
 def test_attention_of_tiny_rows_and_features(T, what, at, tiny, other):
     g = torch.Generator(device="cuda").manual_seed(9)
     t = {n: torch.randn(1, 2, T, 64, device="cuda", generator=g) for n in ("q", "k", "v", "do")}
