@@ -21,6 +21,7 @@
 // All weight gradients of one layer, 12 x 64, 8192 tokens: 260 us (three products on at most 36 CTAs, without fills
 // and conversions) -> 44 + 9 us; 16 x 128, 16384 tokens: 510 -> 495 + 31 us, the zero fills and conversions (0.1 ms) gone.
 #include <algorithm>
+#include <type_traits>
 
 #include "saf_internal.h"
 #include "sm100_prims.cuh"
@@ -52,7 +53,7 @@ struct BlockTable {
 struct BwdGemmParams {
   int I, J, KB;              // output rows, output columns, K steps of 64
   int tiles_m, tiles_n;
-  int subs;                  // 64-column blocks of a tile: 2, 3 or 4
+  int subs;                  // DW: 64-column blocks of a tile
   int n_blocks;              // selected 64-row blocks
   const void* bias;          // DX only: bf16 over the J output columns, or null
   int* status;
@@ -65,8 +66,11 @@ struct BSmem {
   uint32_t tmem_base;
 };
 
-// F32OUT: DX writes fp32, DW writes its part of the product to the workspace (mapO: splits * split_rows rows)
-template <int MODE, bool F32OUT>
+// F32OUT: DX writes fp32, DW writes its part of the product to the workspace (mapO: splits * split_rows rows).  SUBS: 64-column
+// blocks of a tile, 2, 3 or 4, known to the compiler for DX, whose producer loops over them in every K step (as a parameter of the
+// launch it cost 5 to 8 % at 256 columns: 16384 rows, 4608 -> 1536 188 us where it takes 179); 0: the launch's own, for DW (as a
+// constant 4 it cost up to 4 % there: dx and dW of 8192 rows, 768 -> 768 76.0 us where they take 73.5)
+template <int MODE, bool F32OUT, int SUBS>
 __global__ void __launch_bounds__(BGEMM_THREADS, 1)
 indexed_gemm_bwd_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUtensorMap mapB,
                         const __grid_constant__ CUtensorMap mapW0, const __grid_constant__ CUtensorMap mapW1,
@@ -91,7 +95,7 @@ indexed_gemm_bwd_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_c
     kb1 = (int)((int64_t)p.KB * (sp + 1) / splits);
   };
   const CUtensorMap* wm[4] = {&mapW0, &mapW1, &mapW2, &mapW3};
-  const int bn = p.subs * 64;                                // columns of a tile
+  const int subs = SUBS ? SUBS : p.subs, bn = subs * 64;     // columns of a tile
 
   if (tid == 0) {
     for (int s = 0; s < NSTG; ++s) {
@@ -123,7 +127,7 @@ indexed_gemm_bwd_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_c
       for (int tile = blockIdx.x; tile < total_tiles && ok; tile += gridDim.x) {
         int tm, tn, sp, kb0, kb1;
         unit(tile, tm, tn, sp, kb0, kb1);
-        const int nsub = min(p.subs, (p.J - tn * bn + 63) / 64);                      // 64-column blocks of B
+        const int nsub = min(subs, (p.J - tn * bn + 63) / 64);                      // 64-column blocks of B
         const int nrow = (MODE == MODE_DW) ? min(2, p.n_blocks - tm * 2) : 2;    // 64-feature blocks of A
         for (int kb = kb0; kb < kb1; ++kb, ++it) {
           const int s = it % NSTG;
@@ -203,7 +207,7 @@ indexed_gemm_bwd_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_c
     for (int tile = blockIdx.x; tile < total_tiles; tile += gridDim.x, ++lt) {
       int tm, tn, sp, kb0, kb1;
       unit(tile, tm, tn, sp, kb0, kb1);
-      const int nsub = min(p.subs, (p.J - tn * bn + 63) / 64);
+      const int nsub = min(subs, (p.J - tn * bn + 63) / 64);
       const int nrow = (MODE == MODE_DW) ? min(2, p.n_blocks - tm * 2) : 2;
       const int buf = lt & 1;
       // threads that meet at named barriers leave together: one whose wait ran out takes the others with it
@@ -346,22 +350,23 @@ void fill_blocks(const SafIndexedLinearArgs& a, BlockTable* tb) {
     }
 }
 
-template <int MODE, bool F32OUT = false>
+template <int MODE, bool F32OUT = false, int SUBS = 0>
 int launch_mode(const CUtensorMap& ma, const CUtensorMap& mb, const CUtensorMap* mw, const CUtensorMap& mo,
                 const BwdGemmParams& p, const BlockTable& tb, cudaStream_t st) {
   const int sm_count = device_sm_count();
   const size_t smem = 1024 + NSTG * BSTAGE + BOUT_BYTES + sizeof(BSmem);
   static PerDeviceOnce smem_once;
-  if (int rc = ensure_dyn_smem(indexed_gemm_bwd_kernel<MODE, F32OUT>, (int)smem, smem_once)) return rc;
+  if (int rc = ensure_dyn_smem(indexed_gemm_bwd_kernel<MODE, F32OUT, SUBS>, (int)smem, smem_once)) return rc;
   const int grid = std::min(sm_count, p.tiles_m * p.tiles_n * std::max(1, p.splits));
-  return launch_pdl(MODE == MODE_DX ? "indexed_gemm_bwd_kernel<dx>" : "indexed_gemm_bwd_kernel<dw>", indexed_gemm_bwd_kernel<MODE, F32OUT>,
+  return launch_pdl(MODE == MODE_DX ? "indexed_gemm_bwd_kernel<dx>" : "indexed_gemm_bwd_kernel<dw>", indexed_gemm_bwd_kernel<MODE, F32OUT, SUBS>,
                     dim3(grid), BGEMM_THREADS, smem, st, 1, ma, mb, mw[0], mw[1], mw[2], mw[3], mo, p, tb);
 }
 
 // Columns of a dx tile, in 64-column blocks, by the time the waves should take, in cycles: a K step is bound by its
 // operands' way from L2 (16 KB of dout and 8 KB of weights per block).  A last wave that is nearly empty costs as much as a
 // full one.  Measured with 256, 192 and 128 columns: 8192 rows, 1920 -> 768 29.0, 26.2 and 32.7 us (192 tiles, 256, 384 on 148
-// SMs), 768 -> 768 14.1, 12.9, 15.7; 1024 rows, 1920 -> 768 15.6, 13.7, 12.5; 3001 rows, 3840 -> 1536 29.9, 47, 43.
+// SMs), 768 -> 768 14.1, 12.9, 15.7; 1024 rows, 1920 -> 768 15.6, 13.7, 12.5; 3001 rows, 3840 -> 1536 29.9, 47, 43.  (With the
+// width a parameter of the launch; as a constant 8192 rows, 1920 -> 768 take 24.3 at 192 columns, 1024 rows 11.4 at 128.)
 int dx_subs(int tiles_m, int C, int KB) {
   const int sms = device_sm_count();
   int best = 4;
@@ -401,12 +406,16 @@ int launch_gemm_bwd_dx_sm100(const SafIndexedLinearArgs& a, const void* dout, in
   p.halves = is_halves(a) ? 1 : 0;
   p.I = a.M; p.J = a.C; p.KB = N / 64; p.n_blocks = N / 64;
   p.tiles_m = (a.M + BM - 1) / BM;
-  p.subs = dx_subs(p.tiles_m, a.C, p.KB);
-  p.tiles_n = (a.C + p.subs * 64 - 1) / (p.subs * 64);
+  const int subs = dx_subs(p.tiles_m, a.C, p.KB);
+  p.tiles_n = (a.C + subs * 64 - 1) / (subs * 64);
   p.bias = bias;
   p.status = a.status;
-  if (f32_out) return launch_mode<MODE_DX, true>(ma, ma, mw, mo, p, tb, st);
-  return launch_mode<MODE_DX>(ma, ma, mw, mo, p, tb, st);
+  auto launch = [&](auto f32) {
+    constexpr bool F = decltype(f32)::value;
+    return subs == 4 ? launch_mode<MODE_DX, F, 4>(ma, ma, mw, mo, p, tb, st)
+                     : (subs == 3 ? launch_mode<MODE_DX, F, 3>(ma, ma, mw, mo, p, tb, st) : launch_mode<MODE_DX, F, 2>(ma, ma, mw, mo, p, tb, st));
+  };
+  return f32_out ? launch(std::true_type{}) : launch(std::false_type{});
 }
 
 int launch_gemm_bwd_dw_sm100(const SafIndexedLinearArgs& a, const void* dout, int64_t lddo, cudaStream_t st) {
@@ -430,7 +439,7 @@ int launch_gemm_bwd_dw_sm100(const SafIndexedLinearArgs& a, const void* dout, in
   p.halves = is_halves(a) ? 1 : 0;
   p.I = N; p.J = a.C; p.KB = (a.M + BK - 1) / BK; p.n_blocks = N / 64;
   p.tiles_m = (p.n_blocks + 1) / 2;
-  p.subs = 4;
+  p.subs = BN / 64;
   p.tiles_n = (a.C + BN - 1) / BN;
   p.status = a.status;
   return launch_mode<MODE_DW>(ma, mb, mw, ma, p, tb, st);
@@ -550,7 +559,7 @@ int launch_gemm_bwd_dw_full_sm100(const SafIndexedLinearArgs& a, const void* dou
   memset(&p, 0, sizeof(p));
   p.I = N; p.J = a.C; p.KB = (a.M + BK - 1) / BK; p.n_blocks = N / 64;
   p.tiles_m = (p.n_blocks + 1) / 2;
-  p.subs = 4;
+  p.subs = BN / 64;
   p.tiles_n = (a.C + BN - 1) / BN;
   p.splits = d.splits;
   p.split_rows = d.split_rows;
